@@ -103,6 +103,20 @@ int tk_tree_create_from_layout(const void* structured_points, const int32_t* per
 int tk_tree_create_device(const void* dev_points, int64_t n, int dims, int dtype, int levels, int device,
                           void* stream, tk_tree** out);
 
+/* tk_tree_create_device with the caller's device memory: `image` holds the
+ * tree (tk_tree_image_size bytes; it belongs to the caller, who keeps it
+ * until the tree is destroyed and no query of it runs any more), `workspace`
+ * the build's scratch (tk_tree_build_workspace_size bytes, free again when
+ * the call returns); both 256-byte aligned.  search_levels >= levels: depth
+ * of the leaves that queries search; the getters report the layout of depth
+ * `levels` whatever it is.  A build from a caching allocator's memory needs
+ * no cudaMalloc / cudaFree, which cost as much as a small build. */
+size_t tk_tree_image_size(int64_t n, int dims, int dtype, int search_levels);
+size_t tk_tree_build_workspace_size(int64_t n, int dims, int dtype);
+int tk_tree_build_device(const void* dev_points, int64_t n, int dims, int dtype, int levels, int search_levels,
+                         int device, void* image, size_t image_bytes, void* workspace, size_t workspace_bytes,
+                         void* stream, tk_tree** out);
+
 /* Free the tree and its device memory.  Replaces ~KDTree
  * (src/interface.cpp:88-94) + freePartitionFromGPU (src/kdtree_g.cu:140-157). */
 int tk_tree_destroy(tk_tree* tree);

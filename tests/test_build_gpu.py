@@ -148,3 +148,55 @@ def test_device_build_errors():
         tk.build_kd_tree(torch.from_numpy(bad).to(cuda), levels=3)
     with pytest.raises(Exception):
         tk.build_kd_tree(torch.from_numpy(pts).to(cuda), levels=8)
+
+
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+@pytest.mark.parametrize("n", [1023, 1025, 4095, 4096, 4097, 8191, 8192, 8193, 12289, 16385])
+def test_device_build_around_block_capacities(dtype, n):
+    """One block sorts and finishes clouds and subtrees of up to 4,096 points;
+    radix tiles hold 4,096 (float32) or 2,048 keys, partition tiles 1,024."""
+    lmax = int(np.floor(np.log2(n))) + 1
+    for d in (1, 2, 3, 5, 8):
+        for levels in (1, 3, lmax - 4, lmax):
+            for kind, pts in clouds(dtype, d, n, seed=n + d):
+                try:
+                    assert_same_layout(pts, levels)
+                except AssertionError as e:
+                    raise AssertionError(f"{kind} n={n} d={d} L={levels} {dtype.__name__}") from e
+
+
+def test_device_build_one_axis_at_a_time():
+    """Above 32M points the axes are sorted and partitioned one after the
+    other: two levels of 33.6M points with many ties, against stable sorts."""
+    import torch_kdtree_gb300 as tk
+    n = 33_600_000
+    g = torch.Generator(device=cuda)
+    g.manual_seed(5)
+    pts = torch.randint(0, 1 << 20, (n, 2), generator=g, device=cuda).float()
+    tree = tk.build_kd_tree(pts, levels=2)
+    order = torch.sort(pts[:, 0], stable=True).indices
+    want = []
+    for half in (order[: n // 2], order[n // 2:]):
+        ids = half.sort().values
+        want.append(ids[torch.sort(pts[ids, 1], stable=True).indices])
+    assert torch.equal(tree.shuffled_ind, torch.cat(want))
+
+
+def test_tree_outlives_its_stream():
+    """A tree's memory belongs to the stream it was built on: dropping the tree
+    while another stream still queries it must not hand that memory on."""
+    import torch_kdtree_gb300 as tk
+    ref = torch.randn(300_000, 3, device=cuda)
+    q = torch.randn(200_000, 3, device=cuda)
+    want_d, want_i = tk.build_kd_tree(ref).query(q, nr_nns_searches=8)
+    side = torch.cuda.Stream()
+    for _ in range(5):
+        tree = tk.build_kd_tree(ref)
+        torch.cuda.synchronize()
+        with torch.cuda.stream(side):
+            d, i = tree.query(q, nr_nns_searches=8)
+        del tree
+        junk = [torch.full((1 << 22,), -1.0, device=cuda) for _ in range(8)]
+        torch.cuda.synchronize()
+        assert torch.equal(d, want_d) and torch.equal(i, want_i)
+        del junk

@@ -47,6 +47,7 @@ class BatchedKDTrees:
         h = ctypes.c_void_p()
         check(LIB.tk_batch_create(handles, len(self.trees), qc, kk, ctypes.byref(h)))
         self._h = h
+        self._stream = None  # of the last query
         self.total_queries = sum(self.query_counts)
         self.total_out = int(LIB.tk_batch_output_size(h))
         self.ws_bytes = int(LIB.tk_batch_workspace_size(h))
@@ -70,9 +71,14 @@ class BatchedKDTrees:
             raise AssertionError(f"queries must be [{self.total_queries}, {self.dims}] {self.dtype}")
         if not q_flat.is_contiguous() or q_flat.device != self.device:
             raise AssertionError("queries must be contiguous on the batch's device")
+        stream = _stream_ptr(self.device)
+        if stream != self._stream:
+            for t in self.trees:
+                t._tree.used_on(stream)
+            self._stream = stream
         check(LIB.tk_batch_query(self._h, q_flat.data_ptr(), out_dists.data_ptr(), out_idx.data_ptr(),
                                  self.threads_per_query, self.prune_boxes, self._ws.data_ptr(), self.ws_bytes,
-                                 _stream_ptr(self.device)))
+                                 stream))
 
     def split(self, flat: torch.Tensor) -> List[torch.Tensor]:
         return [flat[o:o + n * k].view(n, k) for o, n, k in zip(self._out_offsets, self.query_counts, self.ks)]

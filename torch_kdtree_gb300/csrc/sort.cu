@@ -1,4 +1,4 @@
-// Exclusive scan and stable LSD radix sort (see sort.cuh).
+// Exclusive scan and one stable radix pass (see sort.cuh).
 //
 // Radix pass over 8-bit digits, tiles of kTile = 256 threads x kRounds items:
 //   1. k_digit_hist: per-tile digit histogram, stored digit-major
@@ -175,13 +175,6 @@ cudaError_t exclusive_scan(int* data, int64_t n, void* ws, cudaStream_t s) {
     return cudaGetLastError();
 }
 
-size_t sort_workspace_bytes(int64_t n) {
-    const int64_t ntiles = std::max<int64_t>(1, (n + kTile - 1) / kTile);
-    const int64_t hist = 256 * ntiles;
-    return align256(sizeof(int) * size_t(hist)) + scan_workspace_bytes(hist) +
-           2 * align256(sizeof(uint32_t) * size_t(std::max<int64_t>(n, 1)));
-}
-
 size_t sort_pass8_workspace_bytes(int64_t n) {
     const int64_t ntiles = std::max<int64_t>(1, (n + kTile - 1) / kTile);
     const int64_t hist = 256 * ntiles;
@@ -202,42 +195,6 @@ cudaError_t sort_pass8(const uint32_t* keys_in, const uint32_t* vals_in, uint32_
     k_digit_scatter<<<unsigned(ntiles), kSortThreads, 0, s>>>(keys_in, vals_in, n, 0, int(ntiles), hist, keys_out,
                                                              vals_out);
     return cudaGetLastError();
-}
-
-cudaError_t sort_pairs(const uint32_t* keys_in, const uint32_t* vals_in, uint32_t* keys_out, uint32_t* vals_out,
-                       int64_t n, int key_bits, void* ws, size_t ws_bytes, cudaStream_t s) {
-    if (n <= 0) return cudaSuccess;
-    if (ws_bytes < sort_workspace_bytes(n)) return cudaErrorInvalidValue;
-    const int64_t ntiles = (n + kTile - 1) / kTile;
-    const int64_t hist_n = 256 * ntiles;
-    char* p = static_cast<char*>(ws);
-    int* hist = reinterpret_cast<int*>(p);
-    p += align256(sizeof(int) * size_t(hist_n));
-    void* scan_ws = p;
-    p += scan_workspace_bytes(hist_n);
-    uint32_t* tmp_k = reinterpret_cast<uint32_t*>(p);
-    p += align256(sizeof(uint32_t) * size_t(n));
-    uint32_t* tmp_v = reinterpret_cast<uint32_t*>(p);
-
-    const int passes = std::max(1, (key_bits + 7) / 8);
-    // Ping-pong so that the last pass lands in keys_out / vals_out.
-    const uint32_t* src_k = keys_in;
-    const uint32_t* src_v = vals_in;
-    for (int pass = 0; pass < passes; ++pass) {
-        const bool to_out = ((passes - 1 - pass) % 2) == 0;
-        uint32_t* dk = to_out ? keys_out : tmp_k;
-        uint32_t* dv = to_out ? vals_out : tmp_v;
-        const int shift = 8 * pass;
-        k_digit_hist<<<unsigned(ntiles), kSortThreads, 0, s>>>(src_k, n, shift, int(ntiles), hist);
-        cudaError_t e = exclusive_scan(hist, hist_n, scan_ws, s);
-        if (e != cudaSuccess) return e;
-        k_digit_scatter<<<unsigned(ntiles), kSortThreads, 0, s>>>(src_k, src_v, n, shift, int(ntiles), hist, dk, dv);
-        e = cudaGetLastError();
-        if (e != cudaSuccess) return e;
-        src_k = dk;
-        src_v = dv;
-    }
-    return cudaSuccess;
 }
 
 }  // namespace tk

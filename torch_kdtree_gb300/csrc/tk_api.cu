@@ -430,12 +430,16 @@ int upload_tree(tk_tree* t, const HostTree<T>& h) {
 }
 
 void free_tree_device(tk_tree* t) {
-    if (t->d_pts) cudaFree(t->d_pts);
-    if (t->d_perm) cudaFree(t->d_perm);
+    if (t->one_image) {
+        if (t->own_image && t->d_pts) cudaFree(t->d_pts);
+    } else {
+        if (t->d_pts) cudaFree(t->d_pts);
+        if (t->d_perm) cudaFree(t->d_perm);
+        if (t->d_medians) cudaFree(t->d_medians);
+        if (t->d_leaf_off) cudaFree(t->d_leaf_off);
+        if (t->d_boxes) cudaFree(t->d_boxes);
+    }
     t->d_perm = nullptr;
-    if (t->d_medians) cudaFree(t->d_medians);
-    if (t->d_leaf_off) cudaFree(t->d_leaf_off);
-    if (t->d_boxes) cudaFree(t->d_boxes);
     t->d_pts = t->d_medians = t->d_boxes = nullptr;
     t->d_leaf_off = nullptr;
 }
@@ -484,6 +488,71 @@ int device_layout(const tk_tree* t, T* points, int32_t* perm) {
     return TK_OK;
 }
 
+// Argument checks of the GPU builds.
+int check_device_build(const void* dev_points, int64_t n, int dims, int dtype, int levels, int device) {
+    if (dtype != TK_F32 && dtype != TK_F64) return fail(TK_EINVAL, "dtype must be TK_F32 or TK_F64");
+    if (!dev_points) return fail(TK_EINVAL, "points pointer is null");
+    if (dims < 1 || dims > kMaxDims)
+        return fail(TK_EINVAL, "KD-tree supports dims 1 to " + std::to_string(kMaxDims) + " (got " +
+                                   std::to_string(dims) + ")");
+    if (n < 1) return fail(TK_EINVAL, "the reference point cloud is empty");
+    if (n >= (int64_t(1) << 31)) return fail(TK_EINVAL, "only 32 bit signed indexing implemented (n < 2^31)");
+    if (levels < 1 || levels > kMaxLevels)
+        return fail(TK_EINVAL, "levels must be in [1, " + std::to_string(kMaxLevels) + "]");
+    // node sizes at depth t are floor / ceil of n / 2^t: a leaf parent gets no
+    // point exactly when n < 2^(levels-1)
+    if (n < (int64_t(1) << (levels - 1)))
+        return fail(TK_EINVAL,
+                    "Ran out of points while building KD-Tree. Either you required too many levels, "
+                    "or you used a lot of coplanar points");
+    int ndev = 0;
+    if (cudaGetDeviceCount(&ndev) != cudaSuccess || device < 0 || device >= ndev) {
+        cudaGetLastError();
+        return fail(TK_EINVAL, "CUDA device " + std::to_string(device) + " is not available");
+    }
+    cudaPointerAttributes attr;
+    if (cudaPointerGetAttributes(&attr, dev_points) != cudaSuccess ||
+        (attr.type != cudaMemoryTypeDevice && attr.type != cudaMemoryTypeManaged) || attr.device != device) {
+        cudaGetLastError();
+        return fail(TK_EINVAL, "points must be device memory on CUDA device " + std::to_string(device));
+    }
+    return TK_OK;
+}
+
+// GPU build of checked arguments into `image` (not owned by the tree).
+int device_build(const void* dev_points, int64_t n, int dims, int dtype, int levels, int search_levels, int device,
+                 void* image, void* workspace, void* stream, tk_tree** out) {
+    tk_tree* t = new (std::nothrow) tk_tree();
+    if (!t) return fail(TK_ENOMEM, "host allocation failed");
+    t->dtype = dtype;
+    t->dims = dims;
+    t->levels = levels;
+    t->search_levels = search_levels;
+    t->device = device;
+    t->n = n;
+    t->host_layout = false;
+    const TreeImage im = tree_image(n, dims, dtype, search_levels);
+    char* p = static_cast<char*>(image);
+    t->d_pts = p + im.pts;
+    t->d_boxes = p + im.boxes;
+    t->d_medians = p + im.medians;
+    t->d_leaf_off = reinterpret_cast<int32_t*>(p + im.leaf_off);
+    if (dims > 3) t->d_perm = reinterpret_cast<int32_t*>(p + im.perm);
+    t->one_image = true;
+    t->own_image = false;
+    t->device_bytes = int64_t(im.total);
+    const int rc = dtype == TK_F32
+                       ? build_device_tree<float>(static_cast<const float*>(dev_points), n, dims, stream, t, workspace)
+                       : build_device_tree<double>(static_cast<const double*>(dev_points), n, dims, stream, t, workspace);
+    if (rc != TK_OK) {
+        cudaStreamSynchronize(static_cast<cudaStream_t>(stream));  // nothing of it still writes the buffers
+        delete t;
+        return rc;
+    }
+    *out = t;
+    return TK_OK;
+}
+
 }  // namespace
 }  // namespace tk
 
@@ -514,7 +583,7 @@ int tk_tree_create(const void* host_points, int64_t n, int dims, int dtype, int 
     if (!t) return fail(TK_ENOMEM, "host allocation failed");
     t->dtype = dtype;
     t->dims = dims;
-    t->levels = levels;
+    t->levels = t->search_levels = levels;
     t->device = device;
     t->n = n;
     int rc = dtype == TK_F32
@@ -560,7 +629,7 @@ int tk_tree_create_from_layout(const void* structured_points, const int32_t* per
     if (!t) return fail(TK_ENOMEM, "host allocation failed");
     t->dtype = dtype;
     t->dims = dims;
-    t->levels = levels;
+    t->levels = t->search_levels = levels;
     t->device = device;
     t->n = n;
     int rc = dtype == TK_F32
@@ -592,52 +661,53 @@ int tk_tree_create_device(const void* dev_points, int64_t n, int dims, int dtype
     clear_error();
     if (!out) return fail(TK_EINVAL, "out is null");
     *out = nullptr;
-    if (dtype != TK_F32 && dtype != TK_F64) return fail(TK_EINVAL, "dtype must be TK_F32 or TK_F64");
-    if (!dev_points) return fail(TK_EINVAL, "points pointer is null");
-    if (dims < 1 || dims > kMaxDims)
-        return fail(TK_EINVAL, "KD-tree supports dims 1 to " + std::to_string(kMaxDims) + " (got " +
-                                   std::to_string(dims) + ")");
-    if (n < 1) return fail(TK_EINVAL, "the reference point cloud is empty");
-    if (n >= (int64_t(1) << 31)) return fail(TK_EINVAL, "only 32 bit signed indexing implemented (n < 2^31)");
-    if (levels < 1 || levels > kMaxLevels)
-        return fail(TK_EINVAL, "levels must be in [1, " + std::to_string(kMaxLevels) + "]");
-    // node sizes at depth t are floor / ceil of n / 2^t: a leaf parent gets no
-    // point exactly when n < 2^(levels-1)
-    if (n < (int64_t(1) << (levels - 1)))
-        return fail(TK_EINVAL,
-                    "Ran out of points while building KD-Tree. Either you required too many levels, "
-                    "or you used a lot of coplanar points");
-    int ndev = 0;
-    if (cudaGetDeviceCount(&ndev) != cudaSuccess || device < 0 || device >= ndev) {
-        cudaGetLastError();
-        return fail(TK_EINVAL, "CUDA device " + std::to_string(device) + " is not available");
-    }
-    cudaPointerAttributes attr;
-    if (cudaPointerGetAttributes(&attr, dev_points) != cudaSuccess ||
-        (attr.type != cudaMemoryTypeDevice && attr.type != cudaMemoryTypeManaged) || attr.device != device) {
-        cudaGetLastError();
-        return fail(TK_EINVAL, "points must be device memory on CUDA device " + std::to_string(device));
-    }
-    tk_tree* t = new (std::nothrow) tk_tree();
-    if (!t) return fail(TK_ENOMEM, "host allocation failed");
-    t->dtype = dtype;
-    t->dims = dims;
-    t->levels = levels;
-    t->device = device;
-    t->n = n;
-    t->host_layout = false;
+    int rc = check_device_build(dev_points, n, dims, dtype, levels, device);
+    if (rc != TK_OK) return rc;
     DeviceGuard g(device);
-    const int rc = dtype == TK_F32
-                       ? build_device_tree<float>(static_cast<const float*>(dev_points), n, dims, levels, stream, t)
-                       : build_device_tree<double>(static_cast<const double*>(dev_points), n, dims, levels, stream, t);
-    if (rc != TK_OK) {
-        cudaStreamSynchronize(static_cast<cudaStream_t>(stream));
-        free_tree_device(t);
-        delete t;
-        return rc;
+    void* image = nullptr;
+    void* ws = nullptr;
+    const size_t image_bytes = tree_image(n, dims, dtype, levels).total, ws_bytes = build_workspace_bytes(n, dims, dtype);
+    cudaError_t e = cudaMalloc(&image, image_bytes);
+    if (e == cudaSuccess) e = cudaMalloc(&ws, ws_bytes);
+    if (e != cudaSuccess) {
+        if (image) cudaFree(image);
+        return fail(TK_ENOMEM, std::string("device allocation: ") + cudaGetErrorString(e));
     }
-    *out = t;
-    return TK_OK;
+    rc = device_build(dev_points, n, dims, dtype, levels, levels, device, image, ws, stream, out);
+    if (rc == TK_OK) (*out)->own_image = true;
+    else cudaFree(image);
+    cudaFree(ws);
+    return rc;
+}
+
+size_t tk_tree_image_size(int64_t n, int dims, int dtype, int search_levels) {
+    if (n < 1 || dims < 1 || dims > kMaxDims || search_levels < 1 || search_levels > kMaxLevels) return 0;
+    return tree_image(n, dims, dtype, search_levels).total;
+}
+
+size_t tk_tree_build_workspace_size(int64_t n, int dims, int dtype) {
+    if (n < 1 || dims < 1 || dims > kMaxDims) return 0;
+    return build_workspace_bytes(n, dims, dtype);
+}
+
+int tk_tree_build_device(const void* dev_points, int64_t n, int dims, int dtype, int levels, int search_levels,
+                         int device, void* image, size_t image_bytes, void* workspace, size_t workspace_bytes,
+                         void* stream, tk_tree** out) {
+    clear_error();
+    if (!out) return fail(TK_EINVAL, "out is null");
+    *out = nullptr;
+    int rc = check_device_build(dev_points, n, dims, dtype, levels, device);
+    if (rc != TK_OK) return rc;
+    if (search_levels < levels || search_levels > kMaxLevels || n < (int64_t(1) << (search_levels - 1)))
+        return fail(TK_EINVAL, "search_levels must be at least levels, and leave a point for every leaf parent");
+    if (!image || image_bytes < tree_image(n, dims, dtype, search_levels).total)
+        return fail(TK_EWORKSPACE, "tree image buffer too small");
+    if (!workspace || workspace_bytes < build_workspace_bytes(n, dims, dtype))
+        return fail(TK_EWORKSPACE, "workspace too small");
+    if (ws_misaligned(workspace) || ws_misaligned(image))
+        return fail(TK_EINVAL, "image and workspace must be 256-byte aligned");
+    DeviceGuard g(device);
+    return device_build(dev_points, n, dims, dtype, levels, search_levels, device, image, workspace, stream, out);
 }
 
 int tk_tree_destroy(tk_tree* t) {

@@ -67,19 +67,32 @@ namespace tk {
 // created on a tree's first host-buffer query.
 struct HostPipe;
 void free_host_pipe(HostPipe* p);
+// Byte offsets of a GPU-built tree's device image, one allocation: points,
+// node boxes, split values, leaf offsets and (4-8 dims) original indices of
+// a tree whose leaves lie at depth `levels`.
+struct TreeImage {
+    size_t pts = 0, boxes = 0, medians = 0, leaf_off = 0, perm = 0, total = 0;
+};
+TreeImage tree_image(int64_t n, int dims, int dtype, int levels);
+// Scratch bytes of a GPU build.
+size_t build_workspace_bytes(int64_t n, int dims, int dtype);
 // Builds the tree on the GPU from device points straight into t's device
-// image (tree_build_gpu.cu), same layout as build_host_tree.  The arguments
-// are validated by the caller; runs on and synchronises the CUDA stream
-// `stream` before returning.
+// image (tree_build_gpu.cu), leaves at depth t->search_levels, same layout as
+// build_host_tree.  The arguments are validated by the caller; runs on and
+// synchronises the CUDA stream `stream` before returning.
 template <typename T>
-int build_device_tree(const T* pts, int64_t n, int dims, int levels, void* stream, tk_tree* t);
+int build_device_tree(const T* pts, int64_t n, int dims, void* stream, tk_tree* t, void* workspace);
 }  // namespace tk
 
 // Opaque handle behind the C ABI.
 struct tk_tree {
     int dtype = TK_F32;
     int dims = 0;
-    int levels = 0;
+    int levels = 0;         // depth of the layout that the getters report
+    int search_levels = 0;  // depth of the device image's leaves (>= levels)
+    // The library chose search_levels: a query may stop at any shallower depth
+    // (every node of the image knows its point range), see query_levels.
+    bool auto_depth = false;
     int device = 0;
     int64_t n = 0;
     // host layout (one of the two is filled when the tree was built on the
@@ -90,10 +103,12 @@ struct tk_tree {
     tk::HostTree<double> h64;
     // device image
     void* d_pts = nullptr;       // point records: coordinates + original index (see tk_device.cuh)
-    void* d_medians = nullptr;   // T[2^L - 1]
+    void* d_medians = nullptr;   // T[2^L - 1], L = search_levels
     int32_t* d_leaf_off = nullptr;  // int32[2^L + 1]
     void* d_boxes = nullptr;     // per node {lo.xyz, 0}, {hi.xyz, 0} (see tk_device.cuh); lo / hi rows when wide
     int32_t* d_perm = nullptr;   // trees of 4-8 dims: original index of each point (records hold coordinates only)
+    bool one_image = false;      // the arrays above are parts of one allocation that starts at d_pts ...
+    bool own_image = true;       // ... which the tree frees, unless the caller provided it
     int64_t device_bytes = 0;
     mutable tk::HostPipe* pipe = nullptr;  // host-buffer query resources (see tk_tree_query_host)
 };

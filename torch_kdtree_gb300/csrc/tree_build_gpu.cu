@@ -7,316 +7,728 @@
 //
 // Presorted-axes construction instead of per-node sorting:
 //   1. for every axis a, P_a = all point ids stably radix-sorted by the
-//      coordinate's order-preserving key (ties keep ascending ids);
-//   2. level by level, every node's points occupy the same range [lo, lo+n)
-//      in every P_a, sorted along that axis.  The split axis's array gives
-//      the split value (ranks h-1, h) and each point's side; every other
-//      axis's array is stably partitioned by side within its node (one
-//      global exclusive scan of the "goes left" flags and one scatter), which
-//      keeps both children's ranges sorted;
-//   3. node sizes depend only on n (left = floor(n/2)), so the node ranges of
-//      the next level come from the current ones without looking at data;
-//   4. after the last split, the leaf parents' axis array is the final point
-//      order; point records, split values, leaf offsets and node bounding
-//      boxes are written straight into the tree's device image.
-// Work per level is a few coalesced passes over n ids, with no per-node
-// selection or sort: dims radix sorts plus about 4 (dims - 1) + 2 passes per
-// level.
+//      coordinate's order-preserving key (ties keep ascending ids), all axes
+//      in the same launches;
+//   2. every node's points occupy the same range [lo, lo + c) in every P_a,
+//      and node ranges depend only on n (left child = floor(c / 2)), so a
+//      position finds its node by arithmetic (locate).  The split axis's
+//      array gives the split value and each point's side, and the first and
+//      last entry of a node's range in each P_a give its bounding box.  The
+//      other axes' arrays are stably partitioned by side within their nodes,
+//      which keeps both children's ranges sorted.  While nodes hold more than
+//      kSub points this takes three launches a level for the whole array;
+//   3. from there on a block per node does all remaining levels in shared
+//      memory (k_subtrees) and writes split values, leaf offsets, node boxes
+//      and point records straight into the tree's device image.
+//
+// What bounds it: launches and dependent gathers for small clouds, then the
+// level passes' L2 traffic (a gather of the split coordinate per point, axis
+// and level).  One sort per axis, seven launches per axis and level, boxes
+// bottom-up and seventeen allocations took (1M / 4M points, default levels,
+// build_kd_tree with the synchronisation) 2.7 / 4.7 ms and 0.93 ms for 10,000
+// points; this takes 0.58 / 1.75 ms and 0.24 ms.
 #include <algorithm>
 #include <cstring>
 #include <limits>
 #include <string>
 #include <vector>
 
-#include "sort.cuh"
 #include "tk_device.cuh"
 #include "tk_internal.h"
 
 namespace tk {
 namespace {
 
-constexpr int kThreads = 256;
+constexpr int kSortThreads = 512;
+constexpr int kScanThreads = 256;
+constexpr int kTile = 1024;        // positions per block of the partition passes
+constexpr int kSub = 4096;         // points of a subtree that one block finishes in shared memory
+constexpr int kSubThreads = 1024;
+constexpr int kSubItems = kSub / kSubThreads;
 
-unsigned blocks_for(int64_t n) { return unsigned((n + kThreads - 1) / kThreads); }
+template <typename T>
+struct KeyBits;
+template <>
+struct KeyBits<float> {
+    using type = uint32_t;
+    static constexpr int kItems = 8;  // per thread and radix tile: 41 KiB of shared memory
+};
+template <>
+struct KeyBits<double> {
+    using type = unsigned long long;
+    static constexpr int kItems = 4;
+};
+template <typename T>
+constexpr int radix_tile() {
+    return kSortThreads * KeyBits<T>::kItems;
+}
+
+// One id array per axis (or per axis of a group), as a kernel argument: equal
+// arrays of one buffer, array a in slot `slots` byte a.  (An array of pointers
+// that a kernel indexes at run time is copied to every thread's local memory;
+// that copy was most of the memory traffic of the level passes.)
+struct Arrays {
+    uint32_t* base = nullptr;
+    int64_t stride = 0;
+    uint64_t slots = 0;
+    __host__ __device__ __forceinline__ uint32_t* operator[](int a) const {
+        return base + int64_t((slots >> (8 * a)) & 255u) * stride;
+    }
+    void set(int a, int slot) {
+        slots &= ~(uint64_t(255) << (8 * a));
+        slots |= uint64_t(slot) << (8 * a);
+    }
+    int slot(int a) const { return int((slots >> (8 * a)) & 255u); }
+};
 
 // Order-preserving unsigned keys; -0 and +0 get the same key (they compare
 // equal on the host, so their order falls to the original index).
-__device__ __forceinline__ uint32_t coord_key32(float v) {
-    uint32_t b = __float_as_uint(v == 0.0f ? 0.0f : v);
+__device__ __forceinline__ uint32_t coord_key(float v) {
+    const uint32_t b = __float_as_uint(v == 0.0f ? 0.0f : v);
     return (b & 0x80000000u) ? ~b : (b | 0x80000000u);
 }
-__device__ __forceinline__ unsigned long long coord_key64(double v) {
-    unsigned long long b = (unsigned long long)__double_as_longlong(v == 0.0 ? 0.0 : v);
+__device__ __forceinline__ unsigned long long coord_key(double v) {
+    const unsigned long long b = (unsigned long long)__double_as_longlong(v == 0.0 ? 0.0 : v);
     return (b & 0x8000000000000000ull) ? ~b : (b | 0x8000000000000000ull);
 }
 
-template <typename T>
-__global__ void k_axis_keys(const T* __restrict__ pts, int64_t n, int dims, int ax, uint32_t* __restrict__ key_lo,
-                            uint32_t* __restrict__ key_hi, int* __restrict__ nan_flag) {
-    const int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const T v = pts[i * dims + ax];
-    if (v != v) *nan_flag = 1;
-    if constexpr (sizeof(T) == 4) {
-        key_lo[i] = coord_key32(float(v));
-    } else {
-        const unsigned long long k = coord_key64(double(v));
-        key_lo[i] = uint32_t(k);
-        key_hi[i] = uint32_t(k >> 32);
+// Lanes of the warp whose 8-bit digit equals this lane's, among the valid
+// ones (an invalid lane gets the other invalid lanes).  Eight ballots: faster
+// here than __match_any_sync.
+__device__ __forceinline__ unsigned same_digit(int digit, bool valid) {
+    unsigned peers = __ballot_sync(0xFFFFFFFFu, valid);
+    if (!valid) peers = ~peers;
+#pragma unroll
+    for (int b = 0; b < 8; ++b) {
+        const bool bit = (digit >> b) & 1;
+        const unsigned m = __ballot_sync(0xFFFFFFFFu, bit);
+        peers &= bit ? m : ~m;
+    }
+    return peers;
+}
+
+// Exclusive sum over the block of one value per thread; warp_sums holds 32 ints.
+__device__ __forceinline__ int block_exclusive(int v, int* warp_sums, int* total = nullptr) {
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    int x = v;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int t = __shfl_up_sync(0xFFFFFFFFu, x, o);
+        if (lane >= o) x += t;
+    }
+    if (lane == 31) warp_sums[wid] = x;
+    __syncthreads();
+    if (wid == 0) {
+        int w = lane < nw ? warp_sums[lane] : 0;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int t = __shfl_up_sync(0xFFFFFFFFu, w, o);
+            if (lane >= o) w += t;
+        }
+        if (lane < nw) warp_sums[lane] = w;
+    }
+    __syncthreads();
+    const int excl = x - v + (wid > 0 ? warp_sums[wid - 1] : 0);
+    if (total) *total = warp_sums[nw - 1];
+    __syncthreads();
+    return excl;
+}
+
+// ----------------------------------------------------------- radix sort --
+//
+// Stable LSD radix sort by 8-bit digits, every axis of a group in the same
+// launches (blockIdx.y): per pass a histogram per tile, an exclusive scan of
+// each digit's row of tiles, and a scatter that ranks a tile's items in
+// registers (ballots within a warp, a table across warps) and
+// reorders them in shared memory so that equal digits leave as runs.
+
+template <typename T, bool FIRST>
+__global__ void __launch_bounds__(kSortThreads) k_radix_hist(const T* __restrict__ pts, int64_t n, int dims, int ax0,
+                                                             const typename KeyBits<T>::type* __restrict__ keys,
+                                                             int shift, int ntiles, int* __restrict__ hist,
+                                                             int* __restrict__ nan_flag) {
+    __shared__ int h[256];
+    const int t = threadIdx.x, a = blockIdx.y;
+    if (t < 256) h[t] = 0;
+    __syncthreads();
+    const int64_t base = int64_t(blockIdx.x) * radix_tile<T>();
+#pragma unroll
+    for (int i = 0; i < KeyBits<T>::kItems; ++i) {
+        const int64_t e = base + i * kSortThreads + t;
+        if (e < n) {
+            typename KeyBits<T>::type k;
+            if constexpr (FIRST) {
+                const T v = pts[e * dims + ax0 + a];
+                if (v != v) *nan_flag = 1;
+                k = coord_key(v);
+            } else {
+                k = keys[a * n + e];
+            }
+            atomicAdd(&h[int(k >> shift) & 255], 1);
+        }
+    }
+    __syncthreads();
+    if (t < 256) hist[(int64_t(a) * 256 + t) * ntiles + blockIdx.x] = h[t];
+}
+
+// Exclusive scan of every row (blockIdx.y * gridDim.x + blockIdx.x) of `len`
+// counts in place; the row's total goes to totals.
+__global__ void __launch_bounds__(kScanThreads) k_row_scan(int* __restrict__ rows, int len, int* __restrict__ totals) {
+    __shared__ int warp_sums[32];
+    const int64_t row = int64_t(blockIdx.y) * gridDim.x + blockIdx.x;
+    int* d = rows + row * len;
+    int carry = 0;
+    for (int base = 0; base < len; base += 4 * kScanThreads) {
+        const int e = base + 4 * int(threadIdx.x);
+        int v[4], s = 0;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            v[i] = e + i < len ? d[e + i] : 0;
+            s += v[i];
+        }
+        int total = 0;
+        int run = carry + block_exclusive(s, warp_sums, &total);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            if (e + i < len) d[e + i] = run;
+            run += v[i];
+        }
+        carry += total;
+    }
+    if (threadIdx.x == 0) totals[row] = carry;
+}
+
+template <typename T, bool FIRST, bool LAST>
+__global__ void __launch_bounds__(kSortThreads, 2) k_radix_scatter(
+    const T* __restrict__ pts, int64_t n, int dims, int ax0, const typename KeyBits<T>::type* __restrict__ kin,
+    const Arrays vin, int shift, int ntiles, const int* __restrict__ hist, const int* __restrict__ totals,
+    typename KeyBits<T>::type* __restrict__ kout, const Arrays vout) {
+    using K = typename KeyBits<T>::type;
+    constexpr int ITEMS = KeyBits<T>::kItems, TILE = radix_tile<T>(), WARPS = kSortThreads / 32;
+    __shared__ K skey[TILE];
+    __shared__ uint32_t sval[TILE];
+    __shared__ uint16_t cnt[WARPS][256];
+    __shared__ int gbase[256];
+    __shared__ int warp_sums[32];
+    const int t = threadIdx.x, lane = t & 31, w = t >> 5, a = blockIdx.y;
+    const int64_t base = int64_t(blockIdx.x) * TILE;
+    const int64_t e0 = base + w * (32 * ITEMS) + lane;
+    for (int i = t; i < WARPS * 128; i += kSortThreads) reinterpret_cast<uint32_t*>(&cnt[0][0])[i] = 0;
+    __syncthreads();
+    K key[ITEMS];
+    uint32_t val[ITEMS];
+    int rank[ITEMS];
+#pragma unroll
+    for (int i = 0; i < ITEMS; ++i) {
+        const int64_t e = e0 + i * 32;
+        key[i] = 0;
+        val[i] = 0;
+        if (e < n) {
+            key[i] = FIRST ? coord_key(pts[e * dims + ax0 + a]) : kin[a * n + e];
+            val[i] = FIRST ? uint32_t(e) : vin[a][e];
+        }
+    }
+    const unsigned below = (1u << lane) - 1u;
+#pragma unroll
+    for (int i = 0; i < ITEMS; ++i) {
+        const bool valid = e0 + i * 32 < n;
+        const int digit = int(key[i] >> shift) & 255;
+        const unsigned peers = same_digit(digit, valid);
+        const int before = cnt[w][digit];
+        __syncwarp();
+        if (valid && (peers & below) == 0) cnt[w][digit] = uint16_t(before + __popc(peers));
+        __syncwarp();
+        rank[i] = before + __popc(peers & below);
+    }
+    __syncthreads();
+    // thread t < 256 owns digit t: place of every warp's run within the tile
+    int run = 0;
+    if (t < 256)
+        for (int i = 0; i < WARPS; ++i) {
+            const int c = cnt[i][t];
+            cnt[i][t] = uint16_t(run);
+            run += c;
+        }
+    const int lstart = block_exclusive(run, warp_sums);
+    const int gstart = block_exclusive(t < 256 ? totals[a * 256 + t] : 0, warp_sums);
+    if (t < 256) {
+        gbase[t] = gstart + hist[(int64_t(a) * 256 + t) * ntiles + blockIdx.x] - lstart;
+        for (int i = 0; i < WARPS; ++i) cnt[i][t] = uint16_t(cnt[i][t] + lstart);
+    }
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < ITEMS; ++i) {
+        if (e0 + i * 32 < n) {
+            const int pos = cnt[w][int(key[i] >> shift) & 255] + rank[i];
+            skey[pos] = key[i];
+            sval[pos] = val[i];
+        }
+    }
+    __syncthreads();
+    const int m = int(min(int64_t(TILE), n - base));
+    for (int j = t; j < m; j += kSortThreads) {
+        const K k = skey[j];
+        const int64_t dst = int64_t(gbase[int(k >> shift) & 255]) + j;
+        if (!LAST) kout[a * n + dst] = k;
+        vout[a][dst] = sval[j];
     }
 }
 
-__global__ void k_gather_u32(const uint32_t* __restrict__ src, const uint32_t* __restrict__ idx, int64_t n,
-                             uint32_t* __restrict__ dst) {
-    const int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (i < n) dst[i] = src[idx[i]];
+// Clouds of up to kSub points: one block per axis sorts in shared memory, all
+// digits in one launch.
+template <typename T>
+__global__ void __launch_bounds__(kSubThreads) k_small_sort(const T* __restrict__ pts, int n, int dims,
+                                                            const Arrays out, int* __restrict__ nan_flag) {
+    using K = typename KeyBits<T>::type;
+    constexpr int WARPS = kSubThreads / 32;
+    extern __shared__ __align__(16) unsigned char smem[];
+    K* skey = reinterpret_cast<K*>(smem);                                      // [kSub]
+    uint16_t* sval = reinterpret_cast<uint16_t*>(skey + kSub);                 // [kSub]
+    uint16_t* cnt = sval + kSub;                                               // [WARPS][256]
+    __shared__ int warp_sums[32];
+    const int t = threadIdx.x, lane = t & 31, w = t >> 5, a = blockIdx.x;
+    for (int i = t; i < n; i += kSubThreads) {
+        const T v = pts[int64_t(i) * dims + a];
+        if (v != v) *nan_flag = 1;
+        skey[i] = coord_key(v);
+        sval[i] = uint16_t(i);
+    }
+    __syncthreads();
+    const int e0 = w * (32 * kSubItems) + lane;
+    const unsigned below = (1u << lane) - 1u;
+    for (int shift = 0; shift < int(sizeof(K)) * 8; shift += 8) {
+        for (int i = t; i < WARPS * 256; i += kSubThreads) cnt[i] = 0;
+        K key[kSubItems];
+        uint16_t val[kSubItems];
+        int rank[kSubItems];
+#pragma unroll
+        for (int i = 0; i < kSubItems; ++i) {
+            const int e = e0 + i * 32;
+            key[i] = e < n ? skey[e] : K(0);
+            val[i] = e < n ? sval[e] : uint16_t(0);
+        }
+        __syncthreads();
+#pragma unroll
+        for (int i = 0; i < kSubItems; ++i) {
+            const bool valid = e0 + i * 32 < n;
+            const int digit = int(key[i] >> shift) & 255;
+            const unsigned peers = same_digit(digit, valid);
+            const int before = cnt[w * 256 + digit];
+            __syncwarp();
+            if (valid && (peers & below) == 0) cnt[w * 256 + digit] = uint16_t(before + __popc(peers));
+            __syncwarp();
+            rank[i] = before + __popc(peers & below);
+        }
+        __syncthreads();
+        int run = 0;
+        if (t < 256) {
+            for (int i = 0; i < WARPS; ++i) {
+                const int c = cnt[i * 256 + t];
+                cnt[i * 256 + t] = uint16_t(run);
+                run += c;
+            }
+        }
+        const int start = block_exclusive(t < 256 ? run : 0, warp_sums);
+        if (t < 256)
+            for (int i = 0; i < WARPS; ++i) cnt[i * 256 + t] = uint16_t(cnt[i * 256 + t] + start);
+        __syncthreads();
+#pragma unroll
+        for (int i = 0; i < kSubItems; ++i) {
+            if (e0 + i * 32 < n) {
+                const int pos = cnt[w * 256 + (int(key[i] >> shift) & 255)] + rank[i];
+                skey[pos] = key[i];
+                sval[pos] = val[i];
+            }
+        }
+        __syncthreads();
+    }
+    for (int i = t; i < n; i += kSubThreads) out[a][i] = sval[i];
 }
 
-__device__ __forceinline__ float add_t(float a, float b) { return __fadd_rn(a, b); }
-__device__ __forceinline__ double add_t(double a, double b) { return __dadd_rn(a, b); }
-__device__ __forceinline__ float half_t(float s) { return __double2float_rn(__dmul_rn(0.5, double(s))); }
-__device__ __forceinline__ double half_t(double s) { return __dmul_rn(0.5, s); }
-
-// Split values of the 2^t nodes of level t (and, at the leaf parents, the
-// leaf offsets).  compMedian (src/kdtree.hpp:392-401): odd n -> element h,
-// even n -> 0.5 * (element h-1 + element h), the sum rounded in T and the
-// product taken in double.
 template <typename T>
-__global__ void k_level_split(const T* __restrict__ pts, int dims, int ax, const uint32_t* __restrict__ pa,
-                              const int32_t* __restrict__ off, int nodes, T* __restrict__ medians,
-                              int32_t* __restrict__ leaf_off, bool last) {
-    const int j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= nodes) return;
-    const int32_t lo = off[j], cnt = off[j + 1] - lo, h = cnt / 2;
-    const T upper = pts[int64_t(pa[lo + h]) * dims + ax];
-    const T lower = h > 0 ? pts[int64_t(pa[lo + h - 1]) * dims + ax] : upper;
-    medians[nodes - 1 + j] = (cnt & 1) ? upper : half_t(add_t(lower, upper));
-    if (last) {
-        leaf_off[2 * j] = lo;
-        leaf_off[2 * j + 1] = lo + h;
+size_t small_sort_smem() {
+    return kSub * sizeof(typename KeyBits<T>::type) + kSub * sizeof(uint16_t) + (kSubThreads / 32) * 256 * sizeof(uint16_t);
+}
+
+// --------------------------------------------------------- node arithmetic --
+
+// Node of depth t that position p of the n points falls into: index j in its
+// level, first position lo, point count c, and the number of points that go
+// left at depth t in all nodes before it (`lefts`).  A node of c points gives
+// floor(c / 2) to its left child, so the 2^r nodes r levels below a node of c
+// points hold floor(c / 2^r) points each, the last c mod 2^r in bit-reversed
+// order one more: the number of odd ones among them follows.
+struct NodeAt {
+    int j, lo, c, lefts;
+};
+__device__ __forceinline__ int lefts_below(int c, int r) {
+    const int f = c >> r, m = c & ((1 << r) - 1);
+    const int odd = (f & 1) ? (1 << r) - m : m;
+    return (c - odd) >> 1;
+}
+__device__ __forceinline__ NodeAt locate(int n, int t, int p) {
+    NodeAt a{0, 0, n, 0};
+    for (int s = 0; s < t; ++s) {
+        const int h = a.c >> 1;
+        a.j <<= 1;
+        if (p - a.lo >= h) {
+            a.lefts += lefts_below(h, t - 1 - s);
+            a.lo += h;
+            a.c -= h;
+            a.j |= 1;
+        } else {
+            a.c = h;
+        }
+    }
+    return a;
+}
+// First position and point count of node j of depth t.
+__device__ __forceinline__ void node_range(int n, int t, int j, int& lo, int& c) {
+    lo = 0;
+    c = n;
+    for (int s = t - 1; s >= 0; --s) {
+        const int h = c >> 1;
+        if ((j >> s) & 1) {
+            lo += h;
+            c -= h;
+        } else {
+            c = h;
+        }
     }
 }
 
-// side[id] = 1 if point id goes to the right child of its node.
-__global__ void k_mark_side(const uint32_t* __restrict__ pa, int64_t n, const int32_t* __restrict__ node_of,
-                            const int32_t* __restrict__ off, uint8_t* __restrict__ side) {
-    const int64_t p = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (p >= n) return;
-    const int j = node_of[p];
-    const int32_t lo = off[j], h = (off[j + 1] - lo) / 2;
-    side[pa[p]] = uint8_t(int32_t(p) - lo >= h);
+__device__ __forceinline__ float half_sum(float a, float b) {
+    return __double2float_rn(__dmul_rn(0.5, double(__fadd_rn(a, b))));
 }
+__device__ __forceinline__ double half_sum(double a, double b) { return __dmul_rn(0.5, __dadd_rn(a, b)); }
+__device__ __forceinline__ float index_bits(uint32_t v, float) { return __uint_as_float(v); }
+__device__ __forceinline__ double index_bits(uint32_t v, double) { return __longlong_as_double((long long)v); }
 
-__global__ void k_left_flags(const uint32_t* __restrict__ pb, int64_t n, const uint8_t* __restrict__ side,
-                             int* __restrict__ flags) {
-    const int64_t p = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (p < n) flags[p] = side[pb[p]] ^ 1;
-}
+// The tree's device image (see tk_internal.h).
+template <typename T>
+struct Image {
+    T* pts;             // point records, or rows of W coordinates (trees of 4-8 dims)
+    int32_t* perm;      // trees of 4-8 dims
+    T* medians;
+    int32_t* leaf_off;
+    T* boxes;
+    int levels;         // depth of the leaves
+    int W;              // record_width(dims)
+};
 
-// Stable partition of every node's range of pb by side: lefts first.  pre is
-// the exclusive prefix sum of the left flags over the whole array.
-__global__ void k_partition(const uint32_t* __restrict__ pb, int64_t n, const uint8_t* __restrict__ side,
-                            const int32_t* __restrict__ node_of, const int32_t* __restrict__ off,
-                            const int* __restrict__ pre, uint32_t* __restrict__ out) {
-    const int64_t p = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (p >= n) return;
-    const int j = node_of[p];
-    const int32_t lo = off[j], h = (off[j + 1] - lo) / 2;
-    const uint32_t id = pb[p];
-    const int32_t left_before = pre[p] - pre[lo];
-    const int32_t dst = side[id] == 0 ? lo + left_before : lo + h + (int32_t(p) - lo - left_before);
-    out[dst] = id;
-}
-
-// Node of every position at the next level, and the next level's ranges.
-__global__ void k_next_nodes(int64_t n, const int32_t* __restrict__ off, int32_t* __restrict__ node_of) {
-    const int64_t p = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (p >= n) return;
-    const int j = node_of[p];
-    const int32_t lo = off[j], h = (off[j + 1] - lo) / 2;
-    node_of[p] = 2 * j + (int32_t(p) - lo >= h ? 1 : 0);
-}
-
-__global__ void k_child_offsets(const int32_t* __restrict__ off, int nodes, int32_t* __restrict__ next) {
-    const int j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j > nodes) return;
-    if (j == nodes) {
-        next[2 * nodes] = off[nodes];
+// One of the node_parts(dims) entries of node j of depth s, whose c points
+// stand in positions lo .. lo + c of every axis's order: the lower and upper
+// bound of each axis (its order starts at the minimum and ends at the
+// maximum), then the rest (point range, split value or leaf offset).  A
+// thread per entry: a thread per node waited for one gather after the other.
+// id_at(axis, i): id of the i-th point of the node along the axis.
+// compMedian (src/kdtree.hpp:392-401): odd n -> element h, even n -> 0.5 *
+// (element h-1 + element h), the sum rounded in T and the product in double.
+__device__ __forceinline__ int node_parts(int dims) { return 2 * dims + 1; }
+template <typename T, typename IdAt>
+__device__ __forceinline__ void write_node_part(const T* __restrict__ pts, int dims, const Image<T>& im, int s, int j,
+                                                int lo, int c, int part, IdAt id_at) {
+    const int64_t node = (int64_t(1) << s) - 1 + j;
+    const T inf = std::numeric_limits<T>::infinity();
+    const bool wide = dims > 3;
+    const int bs = wide ? im.W : 4;  // coordinates per box row
+    T* lo_row = im.boxes + (2 * node) * bs;
+    T* hi_row = lo_row + bs;
+    if (part < 2 * dims) {
+        const int a = part >> 1, upper = part & 1;
+        const T v = c > 0 ? pts[int64_t(id_at(a, upper ? c - 1 : 0)) * dims + a] : (upper ? -inf : inf);
+        (upper ? hi_row : lo_row)[a] = v;
         return;
     }
-    const int32_t lo = off[j];
-    next[2 * j] = lo;
-    next[2 * j + 1] = lo + (off[j + 1] - lo) / 2;
-}
-
-template <typename T>
-__global__ void k_make_records(const T* __restrict__ pts, int dims, const uint32_t* __restrict__ order, int64_t n,
-                               PointRec<T>* __restrict__ recs) {
-    const int64_t p = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (p >= n) return;
-    const uint32_t id = order[p];
-    T c[3] = {T(0), T(0), T(0)};
-    for (int d = 0; d < dims; ++d) c[d] = pts[int64_t(id) * dims + d];
-    PointRec<T> r;
-    r.x = c[0];
-    r.y = c[1];
-    r.z = c[2];
-    if constexpr (sizeof(T) == 4) {
-        r.w = __uint_as_float(id);
+    for (int a = dims; a < im.W; ++a) {
+        lo_row[a] = c > 0 ? T(0) : inf;
+        hi_row[a] = c > 0 ? T(0) : -inf;
+    }
+    if (!wide) {  // the box records also carry the node's point range [begin, end)
+        lo_row[3] = index_bits(uint32_t(lo), T(0));
+        hi_row[3] = index_bits(uint32_t(lo + c), T(0));
+    }
+    if (s < im.levels) {
+        const int ax = s % dims, h = c / 2;
+        if (c > 0) {
+            const T upper = pts[int64_t(id_at(ax, h)) * dims + ax];
+            const T lower = pts[int64_t(id_at(ax, h > 0 ? h - 1 : 0)) * dims + ax];
+            im.medians[node] = (c & 1) ? upper : half_sum(lower, upper);
+        }
     } else {
-        r.w = __longlong_as_double((long long)id);
+        im.leaf_off[j] = lo;
+        if (j == (1 << s) - 1) im.leaf_off[j + 1] = lo + c;
     }
-    recs[p] = r;
 }
 
-// Box of every leaf (one warp per leaf), stored at node 2^L - 1 + leaf, with
-// the leaf's point range in the records' 4th slots.
 template <typename T>
-__global__ void k_leaf_boxes(const PointRec<T>* __restrict__ recs, const int32_t* __restrict__ leaf_off,
-                             int64_t nleaves, PointRec<T>* __restrict__ boxes) {
-    const int64_t leaf = (int64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
-    const int lane = threadIdx.x & 31;
-    if (leaf >= nleaves) return;
-    const T inf = std::numeric_limits<T>::infinity();
-    T lo[3] = {inf, inf, inf}, hi[3] = {-inf, -inf, -inf};
-    for (int32_t i = leaf_off[leaf] + lane; i < leaf_off[leaf + 1]; i += 32) {
-        const PointRec<T> r = recs[i];
-        const T c[3] = {r.x, r.y, r.z};
-#pragma unroll
-        for (int d = 0; d < 3; ++d) {
-            lo[d] = c[d] < lo[d] ? c[d] : lo[d];
-            hi[d] = hi[d] < c[d] ? c[d] : hi[d];
+__device__ __forceinline__ void write_point(const T* __restrict__ pts, int dims, const Image<T>& im, int64_t p,
+                                            uint32_t id) {
+    const T* src = pts + int64_t(id) * dims;
+    if (dims > 3) {
+        for (int d = 0; d < im.W; ++d) im.pts[p * im.W + d] = d < dims ? src[d] : T(0);
+        im.perm[p] = int32_t(id);
+    } else {
+        PointRec<T> r;
+        r.x = src[0];
+        r.y = dims > 1 ? src[1] : T(0);
+        r.z = dims > 2 ? src[2] : T(0);
+        r.w = index_bits(id, T(0));
+        reinterpret_cast<PointRec<T>*>(im.pts)[p] = r;
+    }
+}
+
+// ------------------------------------------------------------ top levels --
+
+// Level s over the whole array.  Slice blockIdx.y < naxes: which points of a
+// group of axes' orders go left -- those before the middle element of their
+// node's order along the split axis, by (coordinate, id) -- as bits, with
+// their count per tile.  The slice after them writes the nodes' entries of
+// the image.  (Marking each point's side in an array by id first, to be
+// gathered here instead of the coordinate, cost another pass of scattered
+// byte writes: 22 us a level at 1M points.)
+template <typename T>
+__global__ void __launch_bounds__(256) k_level_count(const T* __restrict__ pts, int n, int dims, int s, const Arrays P,
+                                                     const Image<T> im, const Arrays in, int naxes,
+                                                     uint32_t* __restrict__ bits, int words, int ntiles,
+                                                     int* __restrict__ counts) {
+    __shared__ int warp_cnt[8];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, b = blockIdx.y;
+    if (b == naxes) {
+        const int64_t v = int64_t(blockIdx.x) * 256 + threadIdx.x;
+        if (v < (int64_t(1) << s) * node_parts(dims)) {
+            const int j = int(v / node_parts(dims)), part = int(v % node_parts(dims));
+            int lo, c;
+            node_range(n, s, j, lo, c);
+            write_node_part<T>(pts, dims, im, s, j, lo, c, part, [&](int ax, int i) { return P[ax][lo + i]; });
         }
+        return;
     }
+    const int ax = s % dims;
+    const uint32_t* pa = P[ax];
+    const uint32_t* pb = in[b];
+    int c = 0;
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-#pragma unroll
-        for (int d = 0; d < 3; ++d) {
-            const T l = __shfl_xor_sync(0xFFFFFFFFu, lo[d], o);
-            const T h = __shfl_xor_sync(0xFFFFFFFFu, hi[d], o);
-            lo[d] = l < lo[d] ? l : lo[d];
-            hi[d] = hi[d] < h ? h : hi[d];
+    for (int i = 0; i < kTile / 256; ++i) {
+        const int word = blockIdx.x * (kTile / 32) + w * (kTile / 256) + i;
+        const int64_t p = int64_t(word) * 32 + lane;
+        bool left = false;
+        if (p < n) {
+            const NodeAt a = locate(n, s, int(p));
+            const uint32_t id = pb[p], mid = pa[a.lo + (a.c >> 1)];
+            const T v = pts[int64_t(id) * dims + ax], m = pts[int64_t(mid) * dims + ax];
+            left = v < m || (v == m && id < mid);
         }
+        const unsigned m = __ballot_sync(0xFFFFFFFFu, left);
+        if (lane == 0 && word < words) bits[int64_t(b) * words + word] = m;
+        c += __popc(m);
     }
-    if (lane == 0) {  // the box records also carry the leaf's point range [begin, end)
-        const int64_t node = nleaves - 1 + leaf;
-        PointRec<T> a{lo[0], lo[1], lo[2], T(0)}, b{hi[0], hi[1], hi[2], T(0)};
-        if constexpr (sizeof(T) == 4) {
-            a.w = __uint_as_float(uint32_t(leaf_off[leaf]));
-            b.w = __uint_as_float(uint32_t(leaf_off[leaf + 1]));
-        } else {
-            a.w = __longlong_as_double((long long)uint32_t(leaf_off[leaf]));
-            b.w = __longlong_as_double((long long)uint32_t(leaf_off[leaf + 1]));
+    if (lane == 0) warp_cnt[w] = c;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        int sum = 0;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) sum += warp_cnt[i];
+        counts[int64_t(b) * ntiles + blockIdx.x] = sum;
+    }
+}
+
+// Stable partition of every node's range by side (lefts first); counts holds
+// the exclusive scan of the tiles' left counts.
+__global__ void __launch_bounds__(256) k_level_partition(int n, int s, const Arrays in, const Arrays out,
+                                                         const uint32_t* __restrict__ bits, int words, int ntiles,
+                                                         const int* __restrict__ counts) {
+    __shared__ int warp_cnt[8];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, b = blockIdx.y;
+    const uint32_t* pb = in[b];
+    uint32_t* po = out[b];
+    constexpr int WORDS = kTile / 256;
+    const int word0 = blockIdx.x * (kTile / 32) + w * WORDS;
+    const uint32_t mine = lane < WORDS && word0 + lane < words ? bits[int64_t(b) * words + word0 + lane] : 0u;
+    int c = __popc(mine);
+    c = __reduce_add_sync(0xFFFFFFFFu, c);
+    if (lane == 0) warp_cnt[w] = c;
+    __syncthreads();
+    int run = counts[int64_t(b) * ntiles + blockIdx.x];
+    for (int i = 0; i < w; ++i) run += warp_cnt[i];
+    const unsigned below = (1u << lane) - 1u;
+#pragma unroll
+    for (int i = 0; i < WORDS; ++i) {
+        const unsigned m = __shfl_sync(0xFFFFFFFFu, mine, i);
+        const int64_t p64 = int64_t(word0 + i) * 32 + lane;
+        if (p64 < n) {
+            const int p = int(p64);
+            const NodeAt a = locate(n, s, p);
+            const int before = run + __popc(m & below) - a.lefts;  // lefts before p in its node
+            const int dst = (m >> lane) & 1 ? a.lo + before : a.lo + (a.c >> 1) + (p - a.lo - before);
+            po[dst] = pb[p];
         }
-        boxes[2 * node] = a;
-        boxes[2 * node + 1] = b;
+        run += __popc(m);
     }
 }
 
-// Boxes of the 2^t inner nodes of level t from their children.
 template <typename T>
-__global__ void k_inner_boxes(int nodes, PointRec<T>* __restrict__ boxes) {
-    const int j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= nodes) return;
-    const int64_t id = int64_t(nodes) - 1 + j;
-    const PointRec<T> al = boxes[2 * (2 * id + 1)], ah = boxes[2 * (2 * id + 1) + 1];
-    const PointRec<T> bl = boxes[2 * (2 * id + 2)], bh = boxes[2 * (2 * id + 2) + 1];
-    PointRec<T> lo, hi;
-    lo.x = bl.x < al.x ? bl.x : al.x;
-    lo.y = bl.y < al.y ? bl.y : al.y;
-    lo.z = bl.z < al.z ? bl.z : al.z;
-    lo.w = T(0);
-    hi.x = ah.x < bh.x ? bh.x : ah.x;
-    hi.y = ah.y < bh.y ? bh.y : ah.y;
-    hi.z = ah.z < bh.z ? bh.z : ah.z;
-    hi.w = T(0);
-    boxes[2 * id] = lo;
-    boxes[2 * id + 1] = hi;
+__global__ void __launch_bounds__(256) k_write_points(const T* __restrict__ pts, int n, int dims,
+                                                      const uint32_t* __restrict__ order, const Image<T> im) {
+    const int64_t p = int64_t(blockIdx.x) * 256 + threadIdx.x;
+    if (p < n) write_point<T>(pts, dims, im, p, order[p]);
 }
 
-// Trees of 4-8 dimensions: coordinate rows of W (zero padded) and the
-// original indices, in leaf order.
-template <typename T>
-__global__ void k_make_rows(const T* __restrict__ pts, int dims, int W, const uint32_t* __restrict__ order,
-                            int64_t n, T* __restrict__ rows, int32_t* __restrict__ perm) {
-    const int64_t p = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (p >= n) return;
-    const uint32_t id = order[p];
-    for (int d = 0; d < W; ++d) rows[p * W + d] = d < dims ? pts[int64_t(id) * dims + d] : T(0);
-    perm[p] = int32_t(id);
-}
+// -------------------------------------------------------------- subtrees --
 
-// Leaf boxes of such a tree (one warp per leaf): lo row at node 2i, hi at 2i+1.
+// One block per node of depth t0 (at most kSub points): all levels below it.
+// The node's ids and, per axis, its order as 16-bit places live in shared
+// memory; a thread keeps the node range of its kSubItems consecutive places
+// in registers.  Two axes' left counts share one block scan (16 bits each).
 template <typename T>
-__global__ void k_leaf_boxes_wide(const T* __restrict__ rows, int W, const int32_t* __restrict__ leaf_off,
-                                  int64_t nleaves, T* __restrict__ boxes) {
-    const int64_t leaf = (int64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
-    const int lane = threadIdx.x & 31;
-    if (leaf >= nleaves) return;
-    const T inf = std::numeric_limits<T>::infinity();
-    T lo[kMaxDims], hi[kMaxDims];
-#pragma unroll
-    for (int d = 0; d < kMaxDims; ++d) {
-        lo[d] = inf;
-        hi[d] = -inf;
+__global__ void __launch_bounds__(kSubThreads) k_subtrees(const T* __restrict__ pts, int n, int dims, int t0,
+                                                          const Arrays P, const Image<T> im,
+                                                          uint16_t* __restrict__ place) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    uint32_t* ids = reinterpret_cast<uint32_t*>(smem);                    // [kSub]
+    uint32_t* start = ids + kSub;                                         // [kSub] scan at each node's start
+    uint16_t* arr = reinterpret_cast<uint16_t*>(start + kSub);            // [dims][kSub]
+    uint8_t* side = reinterpret_cast<uint8_t*>(arr + dims * kSub);        // [kSub]
+    __shared__ int warp_sums[32];
+    int glo, cnt;
+    node_range(n, t0, blockIdx.x, glo, cnt);
+    const int t = threadIdx.x;
+    for (int i = t; i < cnt; i += kSubThreads) {
+        const uint32_t id = P[0][glo + i];
+        ids[i] = id;
+        arr[i] = uint16_t(i);
+        if (dims > 1) place[id] = uint16_t(i);
     }
-    for (int32_t i = leaf_off[leaf] + lane; i < leaf_off[leaf + 1]; i += 32) {
+    __syncthreads();  // the block's own writes to `place` are visible to all its threads
+    for (int a = 1; a < dims; ++a)
+        for (int i = t; i < cnt; i += kSubThreads) arr[a * kSub + i] = place[P[a][glo + i]];
+
+    int lo[kSubItems], c[kSubItems], j[kSubItems];
 #pragma unroll
-        for (int d = 0; d < kMaxDims; ++d) {
-            if (d < W) {
-                const T c = rows[int64_t(i) * W + d];
-                lo[d] = c < lo[d] ? c : lo[d];
-                hi[d] = hi[d] < c ? c : hi[d];
+    for (int e = 0; e < kSubItems; ++e) {
+        lo[e] = 0;
+        c[e] = cnt;
+        j[e] = 0;
+    }
+    __syncthreads();
+    for (int s = t0;; ++s) {
+        const int entries = node_parts(dims) << (s - t0);
+        for (int v = t; v < entries; v += kSubThreads) {
+            const int nj = v / node_parts(dims), part = v % node_parts(dims);
+            int nlo, nc;
+            node_range(cnt, s - t0, nj, nlo, nc);
+            write_node_part<T>(pts, dims, im, s, (int(blockIdx.x) << (s - t0)) + nj, glo + nlo, nc, part,
+                               [&](int ax, int i) { return ids[arr[ax * kSub + nlo + i]]; });
+        }
+        if (s == im.levels) break;
+        const int ax = s % dims;
+#pragma unroll
+        for (int e = 0; e < kSubItems; ++e) {
+            const int p = t * kSubItems + e;
+            if (p < cnt) side[arr[ax * kSub + p]] = uint8_t(p - lo[e] >= (c[e] >> 1));
+        }
+        __syncthreads();
+        for (int o = 1; o < dims; o += 2) {
+            // the next two axes after the split axis (cyclically); the second may not exist
+            const int b0 = (ax + o) % dims, b1 = (ax + o + 1) % dims;
+            const bool two = o + 1 < dims;
+            uint16_t v0[kSubItems], v1[kSubItems];
+            uint32_t f[kSubItems], sum = 0;
+#pragma unroll
+            for (int e = 0; e < kSubItems; ++e) {
+                const int p = t * kSubItems + e;
+                v0[e] = v1[e] = 0;
+                f[e] = 0;
+                if (p < cnt) {
+                    v0[e] = arr[b0 * kSub + p];
+                    f[e] = side[v0[e]] ^ 1u;
+                    if (two) {
+                        v1[e] = arr[b1 * kSub + p];
+                        f[e] |= uint32_t(side[v1[e]] ^ 1u) << 16;
+                    }
+                }
+                sum += f[e];
+            }
+            uint32_t run = uint32_t(block_exclusive(int(sum), warp_sums));
+            uint32_t ex[kSubItems];
+#pragma unroll
+            for (int e = 0; e < kSubItems; ++e) {
+                const int p = t * kSubItems + e;
+                ex[e] = run;
+                if (p < cnt && p == lo[e]) start[j[e]] = run;
+                run += f[e];
+            }
+            __syncthreads();
+#pragma unroll
+            for (int e = 0; e < kSubItems; ++e) {
+                const int p = t * kSubItems + e;
+                if (p < cnt) {
+                    const uint32_t d = ex[e] - start[j[e]];  // both halves: lefts before p in its node
+                    const int h = c[e] >> 1, d0 = int(d & 0xFFFFu), d1 = int(d >> 16);
+                    arr[b0 * kSub + ((f[e] & 1u) ? lo[e] + d0 : lo[e] + h + (p - lo[e] - d0))] = v0[e];
+                    if (two) arr[b1 * kSub + ((f[e] >> 16) ? lo[e] + d1 : lo[e] + h + (p - lo[e] - d1))] = v1[e];
+                }
+            }
+            __syncthreads();
+        }
+#pragma unroll
+        for (int e = 0; e < kSubItems; ++e) {
+            const int p = t * kSubItems + e, h = c[e] >> 1;
+            j[e] *= 2;
+            if (p - lo[e] >= h) {
+                lo[e] += h;
+                c[e] -= h;
+                j[e] += 1;
+            } else {
+                c[e] = h;
             }
         }
     }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-#pragma unroll
-        for (int d = 0; d < kMaxDims; ++d) {
-            const T l = __shfl_xor_sync(0xFFFFFFFFu, lo[d], o);
-            const T h = __shfl_xor_sync(0xFFFFFFFFu, hi[d], o);
-            lo[d] = l < lo[d] ? l : lo[d];
-            hi[d] = hi[d] < h ? h : hi[d];
-        }
-    }
-    if (lane == 0) {
-        const int64_t node = nleaves - 1 + leaf;
-        for (int d = 0; d < W; ++d) {
-            boxes[(2 * node) * W + d] = lo[d];
-            boxes[(2 * node + 1) * W + d] = hi[d];
-        }
-    }
+    // points in leaf order: the leaf parent's axis (left as it was by the last partition)
+    const int fa = (im.levels - 1) % dims;
+    for (int i = t; i < cnt; i += kSubThreads) write_point<T>(pts, dims, im, glo + i, ids[arr[fa * kSub + i]]);
 }
 
-template <typename T>
-__global__ void k_inner_boxes_wide(int nodes, int W, T* __restrict__ boxes) {
-    const int j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= nodes) return;
-    const int64_t id = int64_t(nodes) - 1 + j, a = 2 * id + 1, b = 2 * id + 2;
-    for (int d = 0; d < W; ++d) {
-        const T al = boxes[(2 * a) * W + d], ah = boxes[(2 * a + 1) * W + d];
-        const T bl = boxes[(2 * b) * W + d], bh = boxes[(2 * b + 1) * W + d];
-        boxes[(2 * id) * W + d] = bl < al ? bl : al;
-        boxes[(2 * id + 1) * W + d] = ah < bh ? bh : ah;
-    }
-}
+size_t subtree_smem(int dims) { return size_t(kSub) * (4 + 4 + 2 * dims + 1); }
 
-// Device scratch of one build, freed on every exit path.
-struct Scratch {
-    std::vector<void*> ptrs;
-    cudaError_t err = cudaSuccess;
-    template <typename X>
-    X* get(size_t count) {
-        void* p = nullptr;
-        if (err == cudaSuccess) err = cudaMalloc(&p, std::max<size_t>(count * sizeof(X), 16));
-        if (err == cudaSuccess) ptrs.push_back(p);
-        return static_cast<X*>(p);
-    }
-    ~Scratch() {
-        for (void* p : ptrs) cudaFree(p);
-    }
+size_t align256(size_t v) { return (v + 255) / 256 * 256; }
+
+// Axes sorted (and partitioned) in one launch: all of them up to 32M points,
+// above that one after the other, with the scratch of one.
+int axes_at_once(int64_t n, int dims) { return n <= (int64_t(32) << 20) ? dims : 1; }
+
+// Scratch of a build: id orders (one per axis), then spare orders, two key
+// arrays (whose space the level passes use afterwards), digit histograms.
+struct BuildWs {
+    size_t orders = 0, key_a = 0, key_b = 0, hist = 0, totals = 0, nan_flag = 0, total = 0;
+    size_t order_bytes = 0;
+    int at_once = 1;
 };
+BuildWs build_ws(int64_t n, int dims, size_t key_bytes) {
+    BuildWs w;
+    const bool small = n <= kSub;
+    const int A = w.at_once = axes_at_once(n, dims);
+    w.order_bytes = align256(4 * size_t(n));
+    size_t o = 0;
+    w.nan_flag = o;
+    o += 256;
+    w.orders = o;
+    o += w.order_bytes * (small ? dims : dims + A);
+    w.key_b = o;  // small clouds: the places of k_subtrees only
+    o += small ? align256(2 * size_t(n)) : align256(key_bytes * size_t(n) * A);
+    if (!small) {
+        w.key_a = o;
+        o += align256(key_bytes * size_t(n) * A);
+        const size_t tile = key_bytes == 4 ? radix_tile<float>() : radix_tile<double>();
+        const size_t ntiles = (size_t(n) + tile - 1) / tile;
+        w.hist = o;  // the level passes' tile counts use it too
+        o += align256(sizeof(int) * 256 * ntiles * A);
+        w.totals = o;
+        o += align256(sizeof(int) * 256 * A);
+    }
+    w.total = o;
+    return w;
+}
 
 #define TK_TRY(expr)                                                                          \
     do {                                                                                      \
@@ -326,121 +738,138 @@ struct Scratch {
 
 }  // namespace
 
-template <typename T>
-int build_device_tree(const T* pts, int64_t n, int dims, int levels, void* stream, tk_tree* t) {
-    const cudaStream_t s = static_cast<cudaStream_t>(stream);
-    const int L = levels;
-    const int64_t nleaves = int64_t(1) << L;
-    const int64_t nparts = nleaves - 1;
-    const int64_t nnodes = 2 * nleaves - 1;
+size_t build_workspace_bytes(int64_t n, int dims, int dtype) {
+    return build_ws(n, dims, dtype == TK_F32 ? 4 : 8).total;
+}
 
-    Scratch sc;
-    uint32_t* P[kMaxDims] = {};
-    for (int a = 0; a < dims; ++a) P[a] = sc.get<uint32_t>(n);
-    uint32_t* spare = sc.get<uint32_t>(n);
-    uint32_t* key_lo = sc.get<uint32_t>(n);
-    uint32_t* key_hi = sizeof(T) == 8 ? sc.get<uint32_t>(n) : nullptr;
-    uint32_t* tmp_k = sc.get<uint32_t>(n);
-    uint32_t* tmp_v = sizeof(T) == 8 ? sc.get<uint32_t>(n) : nullptr;
-    uint8_t* side = sc.get<uint8_t>(n);
-    int32_t* node_of = sc.get<int32_t>(n);
-    int* flags = sc.get<int>(n);
-    int32_t* off_a = sc.get<int32_t>(nleaves + 1);
-    int32_t* off_b = sc.get<int32_t>(nleaves + 1);
-    int* nan_flag = sc.get<int>(1);
-    const size_t sort_ws_bytes = sort_workspace_bytes(n);
-    void* sort_ws = sc.get<unsigned char>(sort_ws_bytes);
-    void* scan_ws = sc.get<unsigned char>(scan_workspace_bytes(n));
-    if (sc.err != cudaSuccess) return fail(TK_ENOMEM, std::string("device build scratch: ") + cudaGetErrorString(sc.err));
-
-    // the tree's device image (wide trees: coordinate rows, indices, box rows)
+TreeImage tree_image(int64_t n, int dims, int dtype, int levels) {
+    TreeImage im;
+    const size_t es = dtype == TK_F32 ? 4 : 8;
+    const size_t nleaves = size_t(1) << levels;
     const bool wide = dims > 3;
-    const int W = record_width(dims);
-    const size_t b_pts = wide ? sizeof(T) * W * size_t(n) : sizeof(PointRec<T>) * size_t(n);
-    const size_t b_perm = wide ? sizeof(int32_t) * size_t(n) : 0;
-    const size_t b_med = sizeof(T) * size_t(nparts);
-    const size_t b_off = sizeof(int32_t) * size_t(nleaves + 1);
-    const size_t b_box = wide ? sizeof(T) * W * 2 * size_t(nnodes) : sizeof(PointRec<T>) * 2 * size_t(nnodes);
-    TK_TRY(cudaMalloc(&t->d_pts, b_pts));
-    if (wide) TK_TRY(cudaMalloc(reinterpret_cast<void**>(&t->d_perm), b_perm));
-    TK_TRY(cudaMalloc(&t->d_medians, std::max<size_t>(b_med, 16)));
-    TK_TRY(cudaMalloc(reinterpret_cast<void**>(&t->d_leaf_off), b_off));
-    TK_TRY(cudaMalloc(&t->d_boxes, b_box));
-    t->device_bytes = int64_t(b_pts + b_perm + b_med + b_off + b_box);
-    T* medians = static_cast<T*>(t->d_medians);
-    PointRec<T>* recs = static_cast<PointRec<T>*>(t->d_pts);
-    PointRec<T>* boxes = static_cast<PointRec<T>*>(t->d_boxes);
+    const size_t row = es * (wide ? record_width(dims) : 4);
+    size_t o = 0;
+    im.pts = o;
+    o += align256(row * size_t(n));
+    im.boxes = o;
+    o += align256(row * 2 * (2 * nleaves - 1));
+    im.medians = o;
+    o += align256(es * nleaves);
+    im.leaf_off = o;
+    o += align256(sizeof(int32_t) * (nleaves + 1));
+    im.perm = o;
+    if (wide) o += align256(sizeof(int32_t) * size_t(n));
+    im.total = o;
+    return im;
+}
+
+template <typename T>
+int build_device_tree(const T* pts, int64_t n, int dims, void* stream, tk_tree* t, void* workspace) {
+    using K = typename KeyBits<T>::type;
+    const cudaStream_t s = static_cast<cudaStream_t>(stream);
+    const int L = t->search_levels;
+    const BuildWs w = build_ws(n, dims, sizeof(K));
+    char* ws = static_cast<char*>(workspace);
+    int* nan_flag = reinterpret_cast<int*>(ws + w.nan_flag);
+    Arrays P, spare;  // P's arrays, then the spares
+    P.base = spare.base = reinterpret_cast<uint32_t*>(ws + w.orders);
+    P.stride = spare.stride = int64_t(w.order_bytes / 4);
+    const int A = w.at_once;
+    for (int a = 0; a < dims; ++a) P.set(a, a);
+    for (int a = 0; a < A; ++a) spare.set(a, dims + a);
+    const int n32 = int(n);
+
+    Image<T> im;
+    im.pts = static_cast<T*>(t->d_pts);
+    im.perm = t->d_perm;
+    im.medians = static_cast<T*>(t->d_medians);
+    im.leaf_off = t->d_leaf_off;
+    im.boxes = static_cast<T*>(t->d_boxes);
+    im.levels = L;
+    im.W = record_width(dims);
 
     // 1. presorted axes
     TK_TRY(cudaMemsetAsync(nan_flag, 0, sizeof(int), s));
-    for (int a = 0; a < dims; ++a) {
-        k_axis_keys<T><<<blocks_for(n), kThreads, 0, s>>>(pts, n, dims, a, key_lo, key_hi, nan_flag);
+    int t0 = 0;  // depth from which a block finishes a node
+    if (n <= kSub) {
+        const size_t smem = small_sort_smem<T>();
+        TK_TRY(cudaFuncSetAttribute(k_small_sort<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+        k_small_sort<T><<<dims, kSubThreads, smem, s>>>(pts, n32, dims, P, nan_flag);
         TK_TRY(cudaGetLastError());
-        if constexpr (sizeof(T) == 4) {
-            TK_TRY(sort_pairs(key_lo, nullptr, tmp_k, P[a], n, 32, sort_ws, sort_ws_bytes, s));
-        } else {
-            TK_TRY(sort_pairs(key_lo, nullptr, tmp_k, tmp_v, n, 32, sort_ws, sort_ws_bytes, s));
-            k_gather_u32<<<blocks_for(n), kThreads, 0, s>>>(key_hi, tmp_v, n, key_lo);
-            TK_TRY(cudaGetLastError());
-            TK_TRY(sort_pairs(key_lo, tmp_v, tmp_k, P[a], n, 32, sort_ws, sort_ws_bytes, s));
-        }
-    }
-
-    // 2./3. level by level
-    const int32_t init_off[2] = {0, int32_t(n)};
-    TK_TRY(cudaMemcpyAsync(off_a, init_off, sizeof(init_off), cudaMemcpyHostToDevice, s));
-    TK_TRY(cudaMemsetAsync(node_of, 0, sizeof(int32_t) * size_t(n), s));
-    int32_t* off = off_a;
-    int32_t* off_next = off_b;
-    for (int lev = 0; lev < L; ++lev) {
-        const int ax = lev % dims;
-        const int nodes = 1 << lev;
-        const bool last = lev == L - 1;
-        k_level_split<T><<<blocks_for(nodes), kThreads, 0, s>>>(pts, dims, ax, P[ax], off, nodes, medians,
-                                                                t->d_leaf_off, last);
-        TK_TRY(cudaGetLastError());
-        if (last) break;
-        k_mark_side<<<blocks_for(n), kThreads, 0, s>>>(P[ax], n, node_of, off, side);
-        TK_TRY(cudaGetLastError());
-        for (int b = 0; b < dims; ++b) {
-            if (b == ax) continue;
-            k_left_flags<<<blocks_for(n), kThreads, 0, s>>>(P[b], n, side, flags);
-            TK_TRY(cudaGetLastError());
-            TK_TRY(exclusive_scan(flags, n, scan_ws, s));
-            k_partition<<<blocks_for(n), kThreads, 0, s>>>(P[b], n, side, node_of, off, flags, spare);
-            TK_TRY(cudaGetLastError());
-            std::swap(P[b], spare);
-        }
-        k_next_nodes<<<blocks_for(n), kThreads, 0, s>>>(n, off, node_of);
-        k_child_offsets<<<blocks_for(nodes + 1), kThreads, 0, s>>>(off, nodes, off_next);
-        TK_TRY(cudaGetLastError());
-        std::swap(off, off_next);
-    }
-    const int32_t n32 = int32_t(n);
-    TK_TRY(cudaMemcpyAsync(t->d_leaf_off + nleaves, &n32, sizeof(int32_t), cudaMemcpyHostToDevice, s));
-
-    // 4. records in leaf order, node boxes bottom-up
-    if (wide) {
-        T* rows = static_cast<T*>(t->d_pts);
-        T* wboxes = static_cast<T*>(t->d_boxes);
-        k_make_rows<T><<<blocks_for(n), kThreads, 0, s>>>(pts, dims, W, P[(L - 1) % dims], n, rows, t->d_perm);
-        k_leaf_boxes_wide<T><<<unsigned((nleaves * 32 + kThreads - 1) / kThreads), kThreads, 0, s>>>(
-            rows, W, t->d_leaf_off, nleaves, wboxes);
-        TK_TRY(cudaGetLastError());
-        for (int lev = L - 1; lev >= 0; --lev) {
-            k_inner_boxes_wide<T><<<blocks_for(int64_t(1) << lev), kThreads, 0, s>>>(1 << lev, W, wboxes);
-            TK_TRY(cudaGetLastError());
-        }
     } else {
-        k_make_records<T><<<blocks_for(n), kThreads, 0, s>>>(pts, dims, P[(L - 1) % dims], n, recs);
-        k_leaf_boxes<T><<<unsigned((nleaves * 32 + kThreads - 1) / kThreads), kThreads, 0, s>>>(recs, t->d_leaf_off,
-                                                                                                nleaves, boxes);
-        TK_TRY(cudaGetLastError());
-        for (int lev = L - 1; lev >= 0; --lev) {
-            k_inner_boxes<T><<<blocks_for(int64_t(1) << lev), kThreads, 0, s>>>(1 << lev, boxes);
+        while (t0 < L && ((n - 1) >> t0) + 1 > kSub) ++t0;
+        K* key_a = reinterpret_cast<K*>(ws + w.key_a);
+        K* key_b = reinterpret_cast<K*>(ws + w.key_b);
+        int* hist = reinterpret_cast<int*>(ws + w.hist);
+        int* totals = reinterpret_cast<int*>(ws + w.totals);
+        const int rtiles = int((n + radix_tile<T>() - 1) / radix_tile<T>());
+        const int passes = int(sizeof(K));
+        for (int a0 = 0; a0 < dims; a0 += A) {
+            const int na = std::min(A, dims - a0);
+            const dim3 grid(rtiles, na);
+            Arrays dst = P;
+            for (int a = 0; a < na; ++a) dst.set(a, P.slot(a0 + a));
+            for (int pass = 0; pass < passes; ++pass) {
+                const K* kin = pass & 1 ? key_a : key_b;  // pass 0 reads the points
+                K* kout = pass & 1 ? key_b : key_a;
+                const Arrays& vin = pass & 1 ? spare : dst;
+                const Arrays& vout = pass & 1 ? dst : spare;  // an even number of passes ends in dst
+                const int shift = 8 * pass;
+                if (pass == 0) k_radix_hist<T, true><<<grid, kSortThreads, 0, s>>>(pts, n, dims, a0, kin, shift, rtiles, hist, nan_flag);
+                else k_radix_hist<T, false><<<grid, kSortThreads, 0, s>>>(pts, n, dims, a0, kin, shift, rtiles, hist, nan_flag);
+                k_row_scan<<<dim3(256, na), kScanThreads, 0, s>>>(hist, rtiles, totals);
+                if (pass == 0) k_radix_scatter<T, true, false><<<grid, kSortThreads, 0, s>>>(pts, n, dims, a0, kin, vin, shift, rtiles, hist, totals, kout, vout);
+                else if (pass + 1 < passes) k_radix_scatter<T, false, false><<<grid, kSortThreads, 0, s>>>(pts, n, dims, a0, kin, vin, shift, rtiles, hist, totals, kout, vout);
+                else k_radix_scatter<T, false, true><<<grid, kSortThreads, 0, s>>>(pts, n, dims, a0, kin, vin, shift, rtiles, hist, totals, kout, vout);
+                TK_TRY(cudaGetLastError());
+            }
+        }
+    }
+
+    // 2. levels whose nodes exceed a block's capacity
+    const int ntiles = int((n + kTile - 1) / kTile);
+    if (t0 > 0) {
+        uint32_t* bits = reinterpret_cast<uint32_t*>(ws + w.key_a);  // the keys' space
+        int* counts = reinterpret_cast<int*>(ws + w.hist);
+        int* totals = reinterpret_cast<int*>(ws + w.totals);
+        const int words = int((n + 31) / 32);
+        for (int lev = 0; lev < t0; ++lev) {
+            int axes[kMaxDims], na = 0;
+            for (int b = 0; b < dims; ++b)
+                if (b != lev % dims) axes[na++] = b;
+            int g = 0;
+            do {
+                const int m = std::min(A, na - g);
+                Arrays in = P;
+                const Arrays out = spare;
+                for (int i = 0; i < m; ++i) in.set(i, P.slot(axes[g + i]));
+                // the nodes' entries need every axis's order as it was before this level: with the first group
+                k_level_count<T><<<dim3(ntiles, m + (g == 0)), 256, 0, s>>>(pts, n32, dims, lev, P, im, in, m, bits, words, ntiles, counts);
+                if (m > 0) {
+                    k_row_scan<<<dim3(1, m), kScanThreads, 0, s>>>(counts, ntiles, totals);
+                    k_level_partition<<<dim3(ntiles, m), 256, 0, s>>>(n32, lev, in, out, bits, words, ntiles, counts);
+                }
+                for (int i = 0; i < m; ++i) {
+                    P.set(axes[g + i], out.slot(i));
+                    spare.set(i, in.slot(i));
+                }
+                g += A;
+            } while (g < na);
             TK_TRY(cudaGetLastError());
         }
     }
+
+    // 3. the rest, a block per node
+    if (n > kSub && ((n - 1) >> t0) + 1 > kSub) {  // leaves larger than a block's capacity
+        k_level_count<T><<<dim3(ntiles, 1), 256, 0, s>>>(pts, n32, dims, L, P, im, P, 0, nullptr, 0, ntiles, nullptr);
+        k_write_points<T><<<unsigned((n + 255) / 256), 256, 0, s>>>(pts, n32, dims, P[(L - 1) % dims], im);
+    } else {
+        const size_t smem = subtree_smem(dims);
+        TK_TRY(cudaFuncSetAttribute(k_subtrees<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+        k_subtrees<T><<<1u << t0, kSubThreads, smem, s>>>(pts, n32, dims, t0, P, im,
+                                                        reinterpret_cast<uint16_t*>(ws + w.key_b));
+    }
+    TK_TRY(cudaGetLastError());
     int nan_host = 0;
     TK_TRY(cudaMemcpyAsync(&nan_host, nan_flag, sizeof(int), cudaMemcpyDeviceToHost, s));
     TK_TRY(cudaStreamSynchronize(s));
@@ -448,7 +877,7 @@ int build_device_tree(const T* pts, int64_t n, int dims, int levels, void* strea
     return TK_OK;
 }
 
-template int build_device_tree<float>(const float*, int64_t, int, int, void*, tk_tree*);
-template int build_device_tree<double>(const double*, int64_t, int, int, void*, tk_tree*);
+template int build_device_tree<float>(const float*, int64_t, int, void*, tk_tree*, void*);
+template int build_device_tree<double>(const double*, int64_t, int, void*, tk_tree*, void*);
 
 }  // namespace tk

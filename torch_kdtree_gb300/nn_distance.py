@@ -56,10 +56,15 @@ def _workspace(nbytes: int, device: torch.device) -> torch.Tensor:
 
 class _Tree:
     """Owner of a tk_tree handle: built on the host from a numpy array, or
-    (``from_device``) on the GPU from a CUDA tensor."""
+    (``from_device``) on the GPU from a CUDA tensor.  A tree built on the GPU
+    lives in a tensor (``image``) of the stream it was built on; ``used_on``
+    has to be told every stream that queries it."""
 
     def __init__(self, points: Optional[np.ndarray], levels: int, device_index: int):
         self.handle = None
+        self.image = None
+        self.stream = None
+        self.other_streams = False
         if points is None:
             return
         n, d = points.shape
@@ -72,11 +77,21 @@ class _Tree:
     def from_device(cls, points: torch.Tensor, levels: int) -> "_Tree":
         t = cls(None, levels, points.device.index)
         n, d = points.shape
+        dt = _DTYPES[points.dtype]
         h = ctypes.c_void_p()
-        check(LIB.tk_tree_create_device(points.data_ptr(), n, d, _DTYPES[points.dtype], levels, points.device.index,
-                                        _stream_ptr(points.device), ctypes.byref(h)))
-        t.handle = h
+        # sizes are 0 for arguments that the build refuses; it then says why
+        image = _workspace(LIB.tk_tree_image_size(n, d, dt, levels), points.device)
+        ws = _workspace(LIB.tk_tree_build_workspace_size(n, d, dt), points.device)
+        stream = _stream_ptr(points.device)
+        check(LIB.tk_tree_build_device(points.data_ptr(), n, d, dt, levels, levels, points.device.index,
+                                       image.data_ptr(), image.numel(), ws.data_ptr(), ws.numel(), stream,
+                                       ctypes.byref(h)))
+        t.handle, t.image, t.stream = h, image, stream
         return t
+
+    def used_on(self, stream: int) -> None:
+        if stream != self.stream:
+            self.other_streams = True
 
     def info(self) -> TreeInfo:
         info = TreeInfo()
@@ -86,6 +101,10 @@ class _Tree:
     def __del__(self):
         h = getattr(self, "handle", None)
         if h is not None and h.value:
+            if self.image is not None and self.other_streams:
+                # the image's memory goes back to its own stream's pool: let the
+                # other streams' queries end first (what cudaFree would wait for)
+                torch.cuda.synchronize(self.image.device)
             LIB.tk_tree_destroy(h)
             self.handle = None
 
@@ -96,9 +115,10 @@ def knn_query_raw(tree: _Tree, q: torch.Tensor, k: int, dists: torch.Tensor, idx
     nq = q.shape[0]
     ws_bytes = LIB.tk_tree_query_workspace_size(tree.handle, nq)
     ws = _workspace(ws_bytes, q.device)
+    stream = _stream_ptr(q.device)
+    tree.used_on(stream)
     check(LIB.tk_tree_query(tree.handle, q.data_ptr(), nq, k, dists.data_ptr(), idx.data_ptr(),
-                            ctypes.byref(opts) if opts is not None else None, ws.data_ptr(), ws_bytes,
-                            _stream_ptr(q.device)))
+                            ctypes.byref(opts) if opts is not None else None, ws.data_ptr(), ws_bytes, stream))
 
 
 def knn_query_host(tree: _Tree, q: torch.Tensor, k: int, dists: torch.Tensor, idx: torch.Tensor, device: torch.device,
