@@ -2,7 +2,7 @@
 // the plan and launch of batch.cu with the wide trees' records and search
 // (kd_wide.cuh).  Every cloud of a batch has the same dims, so one record
 // width W serves the whole launch; each group looks up its query's cloud and
-// runs kd_search_wide with that cloud's tree and k.
+// runs the search of kd_wide.cuh with that cloud's tree and k.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -68,7 +68,7 @@ __global__ void k_batch_bin_count_wide(const WideBatchArgs<T> a, int* counts, in
 
 template <typename T, int W, int G, int R>
 __device__ __forceinline__ void batch_search_wide(const WideCloudDesc<T>& cd, int dims, const T (&q)[W],
-                                                  T* out_d, int32_t* out_i, unsigned gmask, int gl, int gbase) {
+                                                  T* out_d, int32_t* out_i, Key<T>* buf, int lane) {
     KdWideArgs<T> wa{};
     wa.pts = cd.pts;
     wa.perm = cd.perm;
@@ -79,16 +79,19 @@ __device__ __forceinline__ void batch_search_wide(const WideCloudDesc<T>& cd, in
     wa.smem_levels = 0;  // split values come from L1 / L2: one launch serves many trees
     wa.dims = dims;
     wa.k = cd.k;
-    kd_search_wide<T, W, G, R>(wa, nullptr, q, out_d, out_i, gmask, gl, gbase);
+    if constexpr (G == 32) kd_search_wide_warp<T, W, R>(wa, q, out_d, out_i, buf, lane);
+    else kd_search_wide<T, W, R>(wa, nullptr, q, out_d, out_i);
 }
 
 // G = 1: k <= 16 (R in {1, 4, 16}); G = 32: k <= 128 (R in {1, 2, 4}).
 template <typename T, int W, int G>
 __device__ __forceinline__ void batch_query_wide(const WideBatchArgs<T>& a) {
     const int lane = threadIdx.x & 31;
-    const int gl = lane & (G - 1);
-    const int gbase = lane & ~(G - 1);
-    const unsigned gmask = group_mask<G>(lane);
+    Key<T>* buf = nullptr;
+    if constexpr (G == 32) {
+        __shared__ Key<T> bufs[8][64];
+        buf = bufs[threadIdx.x >> 5];
+    }
     constexpr int kGroupsPerWarp = 32 / G;
     const int gid = lane / G;
     for (;;) {
@@ -108,13 +111,13 @@ __device__ __forceinline__ void batch_query_wide(const WideBatchArgs<T>& a) {
             T* od = a.out_d + o;
             int32_t* oi = a.out_i + o;
             if (G == 1) {
-                if (cd.k <= 1) batch_search_wide<T, W, G, 1>(cd, a.dims, q, od, oi, gmask, gl, gbase);
-                else if (cd.k <= 4) batch_search_wide<T, W, G, 4>(cd, a.dims, q, od, oi, gmask, gl, gbase);
-                else batch_search_wide<T, W, G, 16>(cd, a.dims, q, od, oi, gmask, gl, gbase);
+                if (cd.k <= 1) batch_search_wide<T, W, G, 1>(cd, a.dims, q, od, oi, buf, lane);
+                else if (cd.k <= 4) batch_search_wide<T, W, G, 4>(cd, a.dims, q, od, oi, buf, lane);
+                else batch_search_wide<T, W, G, 16>(cd, a.dims, q, od, oi, buf, lane);
             } else {
-                if (cd.k <= 32) batch_search_wide<T, W, G, 1>(cd, a.dims, q, od, oi, gmask, gl, gbase);
-                else if (cd.k <= 64) batch_search_wide<T, W, G, 2>(cd, a.dims, q, od, oi, gmask, gl, gbase);
-                else batch_search_wide<T, W, G, 4>(cd, a.dims, q, od, oi, gmask, gl, gbase);
+                if (cd.k <= 32) batch_search_wide<T, W, G, 1>(cd, a.dims, q, od, oi, buf, lane);
+                else if (cd.k <= 64) batch_search_wide<T, W, G, 2>(cd, a.dims, q, od, oi, buf, lane);
+                else batch_search_wide<T, W, G, 4>(cd, a.dims, q, od, oi, buf, lane);
             }
         }
         __syncwarp();

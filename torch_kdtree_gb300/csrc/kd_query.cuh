@@ -36,6 +36,7 @@
 
 #include <cuda_runtime.h>
 
+#include "kd_warp.cuh"
 #include "tk_device.cuh"
 #include "tk_internal.h"
 
@@ -312,15 +313,71 @@ __device__ __forceinline__ void kd_search(const TreeView<T>& tv, const T (&q)[D]
     list.store(k, gl, out_d, out_i, 0);
 }
 
+// The same search with a whole warp per query (kd_warp.cuh).
+template <typename T, int D, int R>
+__device__ __forceinline__ void kd_search_warp(const TreeView<T>& tv, const T (&q)[D], int k, T* out_d,
+                                               int32_t* out_i, Key<T>* buf, int lane) {
+    WarpList<T, R> wl;
+    wl.init(k, buf, lane);
+    const int L = tv.levels;
+    bool nan_q = false;  // all distances are NaN and enter no list: the home leaf is enough
+#pragma unroll
+    for (int c = 0; c < D; ++c) nan_q |= q[c] != q[c];
+    auto qa = [&](int ax) { return pick<T, D>(q, ax); };
+
+    int leaf = warp_descend(tv.medians, 0, 0, L, D, lane, qa);
+    T bound = T(0);       // of this lane's sibling (lane 31: of the leaf)
+    bool pending = false;
+    int range = 0, range_end = 0;
+    for (int fresh = 0;;) {  // lanes fresh .. L - 1 have new siblings
+        const bool mine = lane >= fresh && lane < L;
+        if (mine || lane == 31) {
+            const int node = lane == 31 ? leaf : path_sibling(leaf, L, lane);
+            const PointRec<T> lo = load_rec(tv.boxes + 2 * node);
+            const PointRec<T> hi = load_rec(tv.boxes + 2 * node + 1);
+            bound = box_bound_of<T, D>(lo, hi, q);
+            range = int(rec_index(lo));
+            range_end = int(rec_index(hi));
+            pending = lane != 31 && !nan_q;
+        }
+        const int beg = __shfl_sync(0xFFFFFFFFu, range, 31);
+        const int end = __shfl_sync(0xFFFFFFFFu, range_end, 31);
+        if (__shfl_sync(0xFFFFFFFFu, bound, 31) <= wl.worst.dist()) {
+            for (int j = beg + lane; j - lane < end; j += 64) {
+                // two records in flight
+                Key<T> k0 = Key<T>::sentinel(), k1 = Key<T>::sentinel();
+                PointRec<T> p0, p1;
+                const bool h0 = j < end, h1 = j + 32 < end;
+                if (h0) p0 = load_rec(tv.pts + j);
+                if (h1) p1 = load_rec(tv.pts + j + 32);
+                if (h0) k0 = Key<T>::make(sqdist<T, D>(q, p0), rec_index(p0));
+                if (h1) k1 = Key<T>::make(sqdist<T, D>(q, p1), rec_index(p1));
+                wl.offer(k0, lane);
+                if (j - lane + 32 < end) wl.offer(k1, lane);
+            }
+            wl.flush(lane);
+        }
+        const unsigned m = __ballot_sync(0xFFFFFFFFu, pending && bound <= wl.worst.dist());
+        if (!m) break;
+        const int t = 31 - __clz(m);
+        pending = pending && lane < t;
+        leaf = warp_descend(tv.medians, path_sibling(leaf, L, t), t + 1, L, D, lane, qa);
+        fresh = t + 1;
+    }
+    wl.list.store(k, lane, out_d, out_i, 0);
+}
+
 template <typename T, int D, int G, int R>
-__device__ __forceinline__ void kd_query_one(const KdArgs<T>& a, const T* s_med, int qi, unsigned gmask, int gl,
-                                             int gbase) {
+__device__ __forceinline__ void kd_query_one(const KdArgs<T>& a, const T* s_med, Key<T>* buf, int qi, unsigned gmask,
+                                             int gl, int gbase) {
     T q[D];
 #pragma unroll
     for (int c = 0; c < D; ++c) q[c] = a.q[(long long)qi * D + c];
     const TreeView<T> tv{a.pts, a.medians, a.leaf_off, a.levels, a.smem_levels, s_med, a.boxes};
-    kd_search<T, D, G, R>(tv, q, a.k, a.out_d + (long long)qi * a.k, a.out_i + (long long)qi * a.k, gmask, gl,
-                          gbase);
+    T* out_d = a.out_d + (long long)qi * a.k;
+    int32_t* out_i = a.out_i + (long long)qi * a.k;
+    if constexpr (G == 32) kd_search_warp<T, D, R>(tv, q, a.k, out_d, out_i, buf, gl);
+    else kd_search<T, D, G, R>(tv, q, a.k, out_d, out_i, gmask, gl, gbase);
 }
 
 constexpr int kKdBlock = 256;  // threads per block of the KD query kernels
@@ -335,9 +392,15 @@ template <typename T, int D, int G, int R>
 __global__ void __launch_bounds__(kKdBlock) k_kd_query(const KdArgs<T> a) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     T* s_med = reinterpret_cast<T*>(smem_raw);
-    const int n_smem = (1 << a.smem_levels) - 1;
-    for (int i = threadIdx.x; i < n_smem; i += blockDim.x) s_med[i] = a.medians[i];
-    __syncthreads();
+    Key<T>* buf = nullptr;
+    if constexpr (G == 32) {
+        __shared__ Key<T> bufs[kKdBlock / 32][64];
+        buf = bufs[threadIdx.x >> 5];
+    } else {
+        const int n_smem = (1 << a.smem_levels) - 1;
+        for (int i = threadIdx.x; i < n_smem; i += blockDim.x) s_med[i] = a.medians[i];
+        __syncthreads();
+    }
 
     const int lane = threadIdx.x & 31;
     const int gl = lane & (G - 1);
@@ -354,7 +417,7 @@ __global__ void __launch_bounds__(kKdBlock) k_kd_query(const KdArgs<T> a) {
         const int t = base + gid;
         if (t < a.nq) {
             const int qi = a.order ? __ldg(a.order + t) : t;
-            kd_query_one<T, D, G, R>(a, s_med, qi, gmask, gl, gbase);
+            kd_query_one<T, D, G, R>(a, s_med, buf, qi, gmask, gl, gbase);
         }
         __syncwarp();
     }

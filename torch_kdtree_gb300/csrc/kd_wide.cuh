@@ -11,9 +11,9 @@
 // the reference's ((0 + d0^2) + d1^2) + ... bit for bit.  The split axis
 // cycles with the real `dims`.
 //
-// The search is kd_search's (exact per-axis plane bounds on a stack of far
-// cells, node-box pruning, queries binned by cell, persistent warps), with
-// one lane per query (k <= 16) or a 32-lane group per query (k <= 128).  A
+// Queries are binned by cell, warps persistent.  One lane per query (k <= 16)
+// searches with exact per-axis plane bounds on a stack of far cells and
+// node-box pruning; a warp per query (k <= 128) walks as kd_warp.cuh says.  A
 // leaf point is first tested as a float against the list's worst distance;
 // only candidates that pass load their original index and build the
 // (distance, index) key.
@@ -21,6 +21,7 @@
 
 #include <cuda_runtime.h>
 
+#include "kd_warp.cuh"
 #include "tk_device.cuh"
 #include "tk_internal.h"
 
@@ -124,24 +125,15 @@ __device__ __forceinline__ T box_bound_w(const T* boxes, int node, const T (&q)[
     return sum_w<T, W>(e);
 }
 
-template <typename T, int W, int G, int R>
+// One lane per query.
+template <typename T, int W, int R>
 __device__ __forceinline__ void kd_search_wide(const KdWideArgs<T>& a, const T* s_med, const T (&q)[W], T* out_d,
-                                               int32_t* out_i, unsigned gmask, int gl, int gbase) {
-    TopK<T, G, R> list;
-    list.init(a.k, gl);
+                                               int32_t* out_i) {
+    TopK<T, 1, R> list;
+    list.init(a.k, 0);
     Key<T> worst = Key<T>::sentinel();
     T worst_d = worst.dist();
-    // Stack of far cells.  A 32-lane group's control flow is uniform, so its
-    // stack lives in the group's registers, entry j in lane j (levels <= 24 <
-    // 32): a push is a register move in one lane, a pop W + 1 shuffles.  Each
-    // lane holding its own copy of the 36-byte entries in local memory missed
-    // L1 on 98% of the pops (1M-point 8-D tree), and this form measured 2-6%
-    // faster at d = 6-8.  (For 3-D trees the private copies mostly hit L1 and
-    // measured faster.)  One lane per query keeps a private local array.
-    constexpr bool RS = G == 32;
-    WideEntry<T, W> stk[RS ? 1 : kMaxLevels];
-    int rs_node = 0;
-    T rs_e[W];
+    WideEntry<T, W> stk[kMaxLevels];  // far cells
     int sp = 0;
     int node = 0, depth = 0;
     T e[W];
@@ -163,15 +155,7 @@ __device__ __forceinline__ void kd_search_wide(const KdWideArgs<T>& a, const T* 
 #pragma unroll
             for (int c = 0; c < W; ++c) far.e[c] = (c == ax) ? plane : e[c];
             if (sum_w<T, W>(far.e) <= worst_d) {
-                if constexpr (RS) {
-                    if (gl == sp) {
-                        rs_node = far.node;
-#pragma unroll
-                        for (int c = 0; c < W; ++c) rs_e[c] = far.e[c];
-                    }
-                } else {
-                    stk[sp] = far;
-                }
+                stk[sp] = far;
                 ++sp;
             }
             node = 2 * node + (go_left ? 1 : 2);
@@ -182,41 +166,19 @@ __device__ __forceinline__ void kd_search_wide(const KdWideArgs<T>& a, const T* 
             const int leaf = node - first_leaf;
             const int beg = __ldg(a.leaf_off + leaf);
             const int end = __ldg(a.leaf_off + leaf + 1);
-            if constexpr (G == 1) {
-                for (int j = beg; j < end; ++j) {
-                    T p[W];
-                    load_row<T, W>(a.pts + size_t(j) * W, p);
-                    const T d = sqdist_w<T, W>(q, p);
-                    if (d <= worst.dist())
-                        worst = offer<T, G, R>(list, Key<T>::make(d, uint32_t(__ldg(a.perm + j))), worst, gmask,
-                                               gl, gbase);
-                }
-            } else {
-                for (int j0 = beg; j0 < end; j0 += G) {
-                    const int j = j0 + gl;
-                    Key<T> mine = Key<T>::sentinel();
-                    if (j < end) {
-                        T p[W];
-                        load_row<T, W>(a.pts + size_t(j) * W, p);
-                        const T d = sqdist_w<T, W>(q, p);
-                        if (d <= worst.dist()) mine = Key<T>::make(d, uint32_t(__ldg(a.perm + j)));
-                    }
-                    worst = offer<T, G, R>(list, mine, worst, gmask, gl, gbase);
-                }
+            for (int j = beg; j < end; ++j) {
+                T p[W];
+                load_row<T, W>(a.pts + size_t(j) * W, p);
+                const T d = sqdist_w<T, W>(q, p);
+                if (d <= worst.dist())
+                    worst = offer<T, 1, R>(list, Key<T>::make(d, uint32_t(__ldg(a.perm + j))), worst, 0u, 0, 0);
             }
             worst_d = worst.dist();
         }
         bool resumed = false;
         while (sp > 0) {
             --sp;
-            WideEntry<T, W> s;
-            if constexpr (RS) {
-                s.node = __shfl_sync(gmask, rs_node, sp);
-#pragma unroll
-                for (int c = 0; c < W; ++c) s.e[c] = __shfl_sync(gmask, rs_e[c], sp);
-            } else {
-                s = stk[sp];
-            }
+            const WideEntry<T, W> s = stk[sp];
             if (sum_w<T, W>(s.e) <= worst_d && (!a.boxes || box_bound_w<T, W>(a.boxes, s.node, q) <= worst_d)) {
                 node = s.node;
 #pragma unroll
@@ -228,21 +190,77 @@ __device__ __forceinline__ void kd_search_wide(const KdWideArgs<T>& a, const T* 
         }
         if (!resumed) break;
     }
-    list.store(a.k, gl, out_d, out_i, 0);
+    list.store(a.k, 0, out_d, out_i, 0);
 }
 
+// The same search with a whole warp per query (kd_warp.cuh); always prunes
+// with node boxes.
+template <typename T, int W, int R>
+__device__ __forceinline__ void kd_search_wide_warp(const KdWideArgs<T>& a, const T (&q)[W], T* out_d, int32_t* out_i,
+                                                    Key<T>* buf, int lane) {
+    WarpList<T, R> wl;
+    wl.init(a.k, buf, lane);
+    const int L = a.levels, dims = a.dims;
+    const int first_leaf = (1 << L) - 1;
+    bool nan_q = false;  // all distances are NaN and enter no list: the home leaf is enough
+#pragma unroll
+    for (int c = 0; c < W; ++c) nan_q |= q[c] != q[c];
+    auto qa = [&](int ax) { return pick_w<T, W>(q, ax); };
+
+    int leaf = warp_descend(a.medians, 0, 0, L, dims, lane, qa);
+    T bound = T(0);  // of this lane's sibling (lane 31: of the leaf)
+    bool pending = false;
+    int range = 0;  // lanes 29, 30: the leaf's point range
+    for (int fresh = 0;;) {  // lanes fresh .. L - 1 have new siblings
+        if ((lane >= fresh && lane < L) || lane == 31) {
+            bound = box_bound_w<T, W>(a.boxes, lane == 31 ? leaf : path_sibling(leaf, L, lane), q);
+            pending = lane != 31 && !nan_q;
+        } else if (lane >= 29) {
+            range = __ldg(a.leaf_off + (leaf - first_leaf) + (lane - 29));
+        }
+        const int beg = __shfl_sync(0xFFFFFFFFu, range, 29);
+        const int end = __shfl_sync(0xFFFFFFFFu, range, 30);
+        if (__shfl_sync(0xFFFFFFFFu, bound, 31) <= wl.worst.dist()) {
+            T p[W];
+            if (beg + lane < end) load_row<T, W>(a.pts + size_t(beg + lane) * W, p);
+            for (int j = beg + lane; j - lane < end; j += 32) {
+                T d = T(0);
+                if (j < end) d = sqdist_w<T, W>(q, p);
+                if (j + 32 < end) load_row<T, W>(a.pts + size_t(j + 32) * W, p);
+                Key<T> mine = Key<T>::sentinel();
+                if (j < end && d <= wl.worst.dist()) mine = Key<T>::make(d, uint32_t(__ldg(a.perm + j)));
+                wl.offer(mine, lane);
+            }
+            wl.flush(lane);
+        }
+        const unsigned m = __ballot_sync(0xFFFFFFFFu, pending && bound <= wl.worst.dist());
+        if (!m) break;
+        const int t = 31 - __clz(m);
+        pending = pending && lane < t;
+        leaf = warp_descend(a.medians, path_sibling(leaf, L, t), t + 1, L, dims, lane, qa);
+        fresh = t + 1;
+    }
+    wl.list.store(a.k, lane, out_d, out_i, 0);
+}
+
+// A warp per query at 5 blocks of 256 per SM (48 registers): 7% faster at 6
+// and 8 dims than the 62 registers it takes freely; the next rows loaded
+// while the last are offered: 4%.
 template <typename T, int W, int G, int R>
-__global__ void __launch_bounds__(256) k_kd_wide(const KdWideArgs<T> a) {
+__global__ void __launch_bounds__(256, G == 32 && sizeof(T) == 4 ? (R < 4 ? 5 : 4) : 1) k_kd_wide(const KdWideArgs<T> a) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     T* s_med = reinterpret_cast<T*>(smem_raw);
-    const int n_smem = (1 << a.smem_levels) - 1;
-    for (int i = threadIdx.x; i < n_smem; i += blockDim.x) s_med[i] = a.medians[i];
-    __syncthreads();
+    Key<T>* buf = nullptr;
+    if constexpr (G == 32) {
+        __shared__ Key<T> bufs[8][64];
+        buf = bufs[threadIdx.x >> 5];
+    } else {
+        const int n_smem = (1 << a.smem_levels) - 1;
+        for (int i = threadIdx.x; i < n_smem; i += blockDim.x) s_med[i] = a.medians[i];
+        __syncthreads();
+    }
 
     const int lane = threadIdx.x & 31;
-    const int gl = lane & (G - 1);
-    const int gbase = lane & ~(G - 1);
-    const unsigned gmask = group_mask<G>(lane);
     constexpr int kGroupsPerWarp = 32 / G;
     const int gid = lane / G;
     for (;;) {
@@ -256,8 +274,10 @@ __global__ void __launch_bounds__(256) k_kd_wide(const KdWideArgs<T> a) {
             T q[W];
 #pragma unroll
             for (int c = 0; c < W; ++c) q[c] = c < a.dims ? a.q[(long long)qi * a.dims + c] : T(0);
-            kd_search_wide<T, W, G, R>(a, s_med, q, a.out_d + (long long)qi * a.k, a.out_i + (long long)qi * a.k,
-                                       gmask, gl, gbase);
+            T* out_d = a.out_d + (long long)qi * a.k;
+            int32_t* out_i = a.out_i + (long long)qi * a.k;
+            if constexpr (G == 32) kd_search_wide_warp<T, W, R>(a, q, out_d, out_i, buf, lane);
+            else kd_search_wide<T, W, R>(a, s_med, q, out_d, out_i);
         }
         __syncwarp();
     }

@@ -1,6 +1,7 @@
 // C ABI of the engine (include/tk_knn.h): error reporting, tree life cycle,
 // and the KD query pipeline (query binning + KD kernel launch).
 #include <algorithm>
+#include <cmath>
 #include <cstring>
 #include <mutex>
 #include <string>
@@ -116,29 +117,28 @@ bool gr_available(int dtype, int dims, int G, int R) {
     return true;
 }
 
-// Lanes per query when the caller leaves it to the library (measured on the
-// large workloads): one lane per query up to ~192 points per leaf and k <= 16
-// (its list fits one lane's registers); 32 lanes for larger leaves or k > 16,
-// which spread both the leaf scan and the list (k = 100: 21 ms on 32 lanes,
-// 35 ms on 8).  Calls with fewer queries than half a wave (SMs x 512) spread
-// each query over 4, 8, 16 or 32 lanes until queries x lanes fill a wave of
-// SMs x 1024 threads: 10,000 queries on one lane each fill 40 of 152 SMs and
-// ran 1.6x slower than on 16 lanes; at 32,768 (65,536) queries 8 (4) lanes
-// beat one by 25% (6%), while at 131,072 one lane beat two by 20%.  Two-lane
-// groups were the slowest shape in every measurement and are skipped.  Trees
+// Lanes per query when the caller leaves it to the library: one lane or a
+// whole warp (2 to 16 lanes were never the fastest shape; a warp's walk tests
+// a path's siblings side by side, see kd_warp.cuh).  One lane's list holds
+// k <= 16.  A lane takes far fewer instructions per query but its search is
+// one long chain of dependent steps, longer in larger clouds, so calls need
+// enough queries to hide it: the crossing was measured, at depths of 22 and
+// ~100 points per leaf, near 50,000 queries for 10,000 points, 110,000 for
+// 100,000, 220,000 for 1M and 260,000 for 4M (k = 5 and 8; ms on one lane
+// against a warp: 1M points, 65,536 queries, k=8 0.32 / 0.19; 1,048,576
+// queries 0.97 / 2.1), lower for k = 1 and higher for k = 16.  Leaves of more
+// than 192 points always take a warp.  Trees
 // of 4-8 dimensions (1M refs x 262k queries N(0,1), depth 12-13): one lane
-// only for k = 1 up to 6 dimensions (d=4: 0.40 vs 0.70 ms), 32 otherwise
-// (d=8, k=16: 21.4 vs 38.3 ms; d=8, k=1: 8.5 vs 9.1 ms).
+// only for k = 1 up to 6 dimensions from a wave of queries on (d=4: 0.40 vs
+// 0.70 ms), a warp otherwise (d=8, k=16: 21.4 vs 38.3 ms).
 int auto_lanes(const tk_tree* t, int64_t nq, int k) {
+    if (k > 16) return 32;
+    const double sms = sm_count(t->device);
+    if (t->dims > 3) return k == 1 && t->dims <= 6 && double(nq) >= sms * 512 ? 1 : 32;
     const double avg_leaf = double(t->n) / double(int64_t(1) << t->levels);
-    int g = (k > 16 || avg_leaf > 192) ? 32 : 1;
-    if (t->dims > 3) g = (k == 1 && t->dims <= 6) ? 1 : 32;
-    const int64_t wave = int64_t(sm_count(t->device)) * 1024;  // resident threads
-    if (g == 1 && 2 * nq < wave) {
-        g = 4;
-        while (g < 32 && nq * g < wave) g <<= 1;
-    }
-    return g;
+    if (avg_leaf > 192) return 32;
+    const double crossing = sms * 120.0 * std::max(1.0, std::log2(double(t->n)) - 10.3);
+    return double(nq) >= crossing * (k == 1 ? 0.6 : (k > 8 ? 1.4 : 1.0)) ? 1 : 32;
 }
 
 int pow2_ceil(int v) {
@@ -156,7 +156,7 @@ int pow2_ceil(int v) {
 // do not end up in the last chunks (the launch's tail), and a warp's 32
 // queries have similar costs (a warp runs as long as its slowest lane).
 template <typename CountFn>
-int prepare_order(const tk_tree* t, int nq, const tk_query_opts& o, char* ws, cudaStream_t s, int** counter,
+int prepare_order(const tk_tree* t, int G, int nq, int k, const tk_query_opts& o, char* ws, cudaStream_t s, int** counter,
                   const int32_t** order, bool classes, CountFn count) {
     const int L = t->levels;
     const WsLayout w = ws_layout(L, nq);
@@ -168,8 +168,14 @@ int prepare_order(const tk_tree* t, int nq, const tk_query_opts& o, char* ws, cu
     // lengthens the slowest warp, which then sets the launch time (131,072
     // queries: 1.33 ms binned vs 1.17 ms in input order; 1,048,576: 3.53 vs
     // 5.84 ms on the cube-and-sphere workload).
-    const bool bin = o.bin_queries == 1 ||
-                     (o.bin_queries < 0 && L >= 2 && int64_t(nq) >= int64_t(sm_count(t->device)) * 1024);
+    // A warp per query gains by the cost order already where a search is long
+    // (4-8 dims, or long lists), from ten queries per resident warp on:
+    // 65,536 queries of 1M points, ms in input order / binned: 6 dims k=16
+    // 1.93 / 1.78, 8 dims 8.0 / 7.0, 3 dims k=100 0.66 / 0.60; but 3 dims k=16
+    // 0.24 / 0.25, and 10,000 queries lose wherever they are.
+    const int64_t sms = sm_count(t->device);
+    const bool long_search = G == 32 && (t->dims > 3 ? k > 4 : k > 48) && int64_t(nq) >= sms * 320;
+    const bool bin = o.bin_queries == 1 || (o.bin_queries < 0 && L >= 2 && (int64_t(nq) >= sms * 1024 || long_search));
     cudaError_t e;
     if (bin) {
         const int B = bin_levels(L, nq);
@@ -230,6 +236,7 @@ int run_query(const tk_tree* t, const T* q, int nq, int k, T* dists, int32_t* id
     // resident per SM on the one-lane shape.
     int S = o.smem_levels >= 0 ? o.smem_levels : 10;
     S = std::max(0, std::min({S, L, sizeof(T) == 4 ? 15 : 14}));  // <= 128 KiB of shared memory
+    if (!packet && G == 32) S = 0;  // a warp per query reads split values five levels at a time instead
     const int block = kKdBlock;
     const size_t smem = kd_smem_bytes<T>(S);
     const void* kfn = packet ? kd_packet_kernel<T, D>(R) : kd_query_kernel<T, D>(G, R);
@@ -249,7 +256,7 @@ int run_query(const tk_tree* t, const T* q, int nq, int k, T* dists, int32_t* id
     int* counter = nullptr;
     const int32_t* order = nullptr;
     const PointRec<T>* boxes = static_cast<const PointRec<T>*>(t->d_boxes);
-    int rc0 = prepare_order(t, nq, o, ws, s, &counter, &order, true, [&](int B, int* counts, int* bin_of, int* pos_of) {
+    int rc0 = prepare_order(t, G, nq, k, o, ws, s, &counter, &order, true, [&](int B, int* counts, int* bin_of, int* pos_of) {
         bin_count_launch<T, D>(q, nq, static_cast<const T*>(t->d_medians), B, L, boxes, counts, bin_of, pos_of, s);
     });
     if (rc0 != TK_OK) return rc0;
@@ -292,6 +299,7 @@ int run_query_wide(const tk_tree* t, const T* q, int nq, int k, T* dists, int32_
     const int L = t->levels;
     int S = o.smem_levels >= 0 ? o.smem_levels : 10;
     S = std::max(0, std::min({S, L, sizeof(T) == 4 ? 15 : 14}));
+    if (G == 32) S = 0;  // a warp per query reads split values five levels at a time instead
     const int block = kKdBlock;
     const size_t smem = kd_smem_bytes<T>(S);
     const void* kfn = kd_wide_kernel<T>(W, G, R);
@@ -310,7 +318,7 @@ int run_query_wide(const tk_tree* t, const T* q, int nq, int k, T* dists, int32_
 
     int* counter = nullptr;
     const int32_t* order = nullptr;
-    const int rc0 = prepare_order(t, nq, o, ws, s, &counter, &order, true, [&](int B, int* counts, int* bin_of, int* pos_of) {
+    const int rc0 = prepare_order(t, G, nq, k, o, ws, s, &counter, &order, true, [&](int B, int* counts, int* bin_of, int* pos_of) {
         bin_count_wide_launch<T>(q, nq, t->dims, static_cast<const T*>(t->d_medians), B, L,
                                  static_cast<const T*>(t->d_boxes), W, counts, bin_of, pos_of, s);
     });
@@ -321,7 +329,8 @@ int run_query_wide(const tk_tree* t, const T* q, int nq, int k, T* dists, int32_
     a.perm = t->d_perm;
     a.medians = static_cast<const T*>(t->d_medians);
     a.leaf_off = t->d_leaf_off;
-    a.boxes = o.prune_boxes == 0 ? nullptr : static_cast<const T*>(t->d_boxes);
+    // a warp per query prunes with node boxes always: one round trip tests all of a path's siblings
+    a.boxes = o.prune_boxes == 0 && G == 1 ? nullptr : static_cast<const T*>(t->d_boxes);
     a.levels = L;
     a.smem_levels = S;
     a.dims = t->dims;
