@@ -108,9 +108,12 @@ int tk_tree_create_device(const void* dev_points, int64_t n, int dims, int dtype
  * until the tree is destroyed and no query of it runs any more), `workspace`
  * the build's scratch (tk_tree_build_workspace_size bytes, free again when
  * the call returns); both 256-byte aligned.  search_levels >= levels: depth
- * of the leaves that queries search; the getters report the layout of depth
- * `levels` whatever it is.  A build from a caching allocator's memory needs
+ * of the leaves that queries search; 0 lets the library choose
+ * (tk_tree_search_levels, the depth to size the image for) and each query
+ * stop at the depth that suits its shape.  The getters report the layout of
+ * depth `levels` whatever it is.  A build from a caching allocator's memory needs
  * no cudaMalloc / cudaFree, which cost as much as a small build. */
+int tk_tree_search_levels(int64_t n, int dims, int dtype, int levels);
 size_t tk_tree_image_size(int64_t n, int dims, int dtype, int search_levels);
 size_t tk_tree_build_workspace_size(int64_t n, int dims, int dtype);
 int tk_tree_build_device(const void* dev_points, int64_t n, int dims, int dtype, int levels, int search_levels,

@@ -200,3 +200,39 @@ def test_tree_outlives_its_stream():
         torch.cuda.synchronize()
         assert torch.equal(d, want_d) and torch.equal(i, want_i)
         del junk
+
+
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+@pytest.mark.parametrize("d", [1, 2, 3, 6])
+def test_default_depth_tree(dtype, d, oracle, tmp_path):
+    """With the default depth the library searches deeper or shallower leaves
+    than the layout it reports: the layout stays the host build's, and every
+    launch shape, a saved and re-loaded tree and a batch give the exhaustive
+    answer."""
+    import torch_kdtree_gb300 as tk
+    from torch_kdtree_gb300._lib import QueryOpts
+    from torch_kdtree_gb300.batched import BatchedKDTrees
+    for n in (1, 2, 40, 700, 9000, 300_000):
+        for kind, ref in list(clouds(dtype, d, n, seed=n + 3 * d))[:3]:
+            q = np.concatenate([ref[:50], np.random.default_rng(n).standard_normal((150, d)).astype(dtype)])
+            rt, qt = torch.from_numpy(ref).to(cuda), torch.from_numpy(q).to(cuda)
+            tree = tk.build_kd_tree(rt)
+            host = tk.build_kd_tree(rt, build="host")
+            assert tree.levels == host.levels and tree.built_on == "device"
+            assert torch.equal(tree.shuffled_ind, host.shuffled_ind)
+            assert torch.equal(tree.structured_points, host.structured_points)
+            tree.save(tmp_path / "t.npz")
+            loaded = tk.load_kd_tree(tmp_path / "t.npz")
+            for k in sorted({1, min(n, 16), min(n, 70)}):
+                bd, bi = oracle.brute(ref, q, k)
+                for lanes in (0, 1, 4, 32):
+                    for traversal in (0, 2):
+                        tree.query_opts = QueryOpts.make(threads_per_query=lanes, traversal=traversal)
+                        dd, ii = tree.query(qt, nr_nns_searches=k)
+                        np.testing.assert_array_equal(dd.cpu().numpy(), bd, err_msg=f"{kind} {n} {k} {lanes}")
+                        np.testing.assert_array_equal(ii.cpu().numpy(), bi)
+                dd, ii = loaded.query(qt, nr_nns_searches=k)
+                np.testing.assert_array_equal(ii.cpu().numpy(), bi)
+                bdd, bii = BatchedKDTrees([rt, rt], [k, 1], [len(q), 0]).query([qt, qt[:0]])
+                np.testing.assert_array_equal(bii[0].cpu().numpy(), bi)
+                np.testing.assert_array_equal(bdd[0].cpu().numpy(), bd)

@@ -73,6 +73,7 @@ SIGNATURES = {
     "tk_cuda_available": (_int, []),
     "tk_tree_create": (_int, [_vp, _i64, _int, _int, _int, _int, _int, ctypes.POINTER(_vp)]),
     "tk_tree_create_device": (_int, [_vp, _i64, _int, _int, _int, _int, _vp, ctypes.POINTER(_vp)]),
+    "tk_tree_search_levels": (_int, [_i64, _int, _int, _int]),
     "tk_tree_image_size": (_sz, [_i64, _int, _int, _int]),
     "tk_tree_build_workspace_size": (_sz, [_i64, _int, _int]),
     "tk_tree_build_device": (_int, [_vp, _i64, _int, _int, _int, _int, _int, _vp, _sz, _vp, _sz, _vp,

@@ -35,6 +35,7 @@ struct CloudDesc {
     const PointRec<T>* boxes;  // null: prune with split planes only
     long long out_off;  // element offset of the cloud's [nq_c, k_c] block in the outputs
     int levels;
+    int leaf_shift;  // image leaves below the searched depth (unused: boxes carry their ranges)
     int k;
     int bins;       // 2^B_c cells used for binning
     int bin_base;   // first cell of this cloud in the global cell array
@@ -210,9 +211,11 @@ int upload_descs(tk_batch* b, const tk_tree* const* trees, const int64_t* q_coun
         Desc& d = h[c];
         fill_desc<T>(d, t);
         d.out_off = b->out_off[c];
-        d.levels = t->levels;
+        // the batch runs one lane per query up to k = 16, else 8 lanes (32 with 4-8 dims)
+        d.levels = query_levels(t, b->max_k <= 16 ? 1 : (t->dims > 3 ? 32 : 8), ks[c]);
+        d.leaf_shift = t->search_levels - d.levels;
         d.k = ks[c];
-        const int B = batch_bin_levels(t->levels, std::max<int64_t>(q_counts[c], 1));
+        const int B = batch_bin_levels(d.levels, std::max<int64_t>(q_counts[c], 1));
         d.bins = 1 << B;
         d.bin_base = bin_base;
         bin_base += d.bins;

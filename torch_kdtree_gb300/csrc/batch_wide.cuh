@@ -30,6 +30,7 @@ struct WideCloudDesc {
     const T* boxes;           // lo / hi rows of W per node
     long long out_off;        // element offset of the cloud's [nq_c, k_c] block in the outputs
     int levels, k;
+    int leaf_shift;           // see KdWideArgs
     int bins;                 // 2^B_c cells used for binning
     int bin_base;             // first cell of this cloud in the global cell array
 };
@@ -76,6 +77,7 @@ __device__ __forceinline__ void batch_search_wide(const WideCloudDesc<T>& cd, in
     wa.leaf_off = cd.leaf_off;
     wa.boxes = cd.boxes;
     wa.levels = cd.levels;
+    wa.leaf_shift = cd.leaf_shift;
     wa.smem_levels = 0;  // split values come from L1 / L2: one launch serves many trees
     wa.dims = dims;
     wa.k = cd.k;

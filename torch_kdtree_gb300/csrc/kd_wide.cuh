@@ -32,9 +32,10 @@ struct KdWideArgs {
     const T* pts;             // [n][W] coordinates in leaf order, zero padded
     const int32_t* perm;      // [n] original index of each point
     const T* medians;         // [2^L - 1] heap order
-    const int32_t* leaf_off;  // [2^L + 1]
+    const int32_t* leaf_off;  // [2^(L + leaf_shift) + 1]
     const T* boxes;           // [2 (2^(L+1) - 1)][W]: node i's lo row at 2i, hi row at 2i+1; or null
     int levels, smem_levels, dims;
+    int leaf_shift;           // the image's leaves lie this many levels below the searched ones
     const T* q;               // [nq, dims]
     int nq, k;
     const int32_t* order;     // [nq] processing order (binned), or null
@@ -164,8 +165,8 @@ __device__ __forceinline__ void kd_search_wide(const KdWideArgs<T>& a, const T* 
         }
         if (!a.boxes || box_bound_w<T, W>(a.boxes, node, q) <= worst_d) {
             const int leaf = node - first_leaf;
-            const int beg = __ldg(a.leaf_off + leaf);
-            const int end = __ldg(a.leaf_off + leaf + 1);
+            const int beg = __ldg(a.leaf_off + (leaf << a.leaf_shift));
+            const int end = __ldg(a.leaf_off + ((leaf + 1) << a.leaf_shift));
             for (int j = beg; j < end; ++j) {
                 T p[W];
                 load_row<T, W>(a.pts + size_t(j) * W, p);
@@ -216,7 +217,7 @@ __device__ __forceinline__ void kd_search_wide_warp(const KdWideArgs<T>& a, cons
             bound = box_bound_w<T, W>(a.boxes, lane == 31 ? leaf : path_sibling(leaf, L, lane), q);
             pending = lane != 31 && !nan_q;
         } else if (lane >= 29) {
-            range = __ldg(a.leaf_off + (leaf - first_leaf) + (lane - 29));
+            range = __ldg(a.leaf_off + ((leaf - first_leaf + lane - 29) << a.leaf_shift));
         }
         const int beg = __shfl_sync(0xFFFFFFFFu, range, 29);
         const int end = __shfl_sync(0xFFFFFFFFu, range, 30);

@@ -117,6 +117,11 @@ bool gr_available(int dtype, int dims, int G, int R) {
     return true;
 }
 
+constexpr double kOneLaneLeaf = 22;  // points per leaf, see query_levels
+
+// round(log2(v)), at least 0
+int log2_round(double v) { return v <= 1.0 ? 0 : int(std::lround(std::log2(v))); }
+
 // Lanes per query when the caller leaves it to the library: one lane or a
 // whole warp (2 to 16 lanes were never the fastest shape; a warp's walk tests
 // a path's siblings side by side, see kd_warp.cuh).  One lane's list holds
@@ -127,7 +132,7 @@ bool gr_available(int dtype, int dims, int G, int R) {
 // 100,000, 220,000 for 1M and 260,000 for 4M (k = 5 and 8; ms on one lane
 // against a warp: 1M points, 65,536 queries, k=8 0.32 / 0.19; 1,048,576
 // queries 0.97 / 2.1), lower for k = 1 and higher for k = 16.  Leaves of more
-// than 192 points always take a warp.  Trees
+// than 192 points (a depth the caller asked for) always take a warp.  Trees
 // of 4-8 dimensions (1M refs x 262k queries N(0,1), depth 12-13): one lane
 // only for k = 1 up to 6 dimensions from a wave of queries on (d=4: 0.40 vs
 // 0.70 ms), a warp otherwise (d=8, k=16: 21.4 vs 38.3 ms).
@@ -135,8 +140,8 @@ int auto_lanes(const tk_tree* t, int64_t nq, int k) {
     if (k > 16) return 32;
     const double sms = sm_count(t->device);
     if (t->dims > 3) return k == 1 && t->dims <= 6 && double(nq) >= sms * 512 ? 1 : 32;
-    const double avg_leaf = double(t->n) / double(int64_t(1) << t->levels);
-    if (avg_leaf > 192) return 32;
+    const double avg_leaf = double(t->n) / double(int64_t(1) << t->search_levels);
+    if (!t->auto_depth && avg_leaf > 192) return 32;
     const double crossing = sms * 120.0 * std::max(1.0, std::log2(double(t->n)) - 10.3);
     return double(nq) >= crossing * (k == 1 ? 0.6 : (k > 8 ? 1.4 : 1.0)) ? 1 : 32;
 }
@@ -156,10 +161,9 @@ int pow2_ceil(int v) {
 // do not end up in the last chunks (the launch's tail), and a warp's 32
 // queries have similar costs (a warp runs as long as its slowest lane).
 template <typename CountFn>
-int prepare_order(const tk_tree* t, int G, int nq, int k, const tk_query_opts& o, char* ws, cudaStream_t s, int** counter,
+int prepare_order(const tk_tree* t, int L, int G, int nq, int k, const tk_query_opts& o, char* ws, cudaStream_t s, int** counter,
                   const int32_t** order, bool classes, CountFn count) {
-    const int L = t->levels;
-    const WsLayout w = ws_layout(L, nq);
+    const WsLayout w = ws_layout(t->search_levels, nq);
     *counter = reinterpret_cast<int*>(ws + w.counter);
     *order = nullptr;
     // Automatic binning from one wave of queries (SMs x 1024) on: below that
@@ -209,6 +213,26 @@ int prepare_order(const tk_tree* t, int G, int nq, int k, const tk_query_opts& o
     return TK_OK;
 }
 
+}  // namespace
+
+// Points per leaf a search works best with: one lane follows its own path and
+// wants small leaves; a warp scans 32 points at a time and, with a longer
+// list, has more to gain from scanning on than from another descent.  Best
+// depths measured (k; points per leaf at 10,000 / 100,000 / 1M / 4M points):
+// one lane 20 / 24 / 30 / 16; a warp k=1 39 / 49 / 61 / 64, k=8 156 / 98 / 61 /
+// 128, k=16 156 / 98 / 122 / 128, k=100 156 / 195 / 244 / 128; 4-8 dims 61 to
+// 122.  float64 pays more for a point than for a descent.
+int query_levels(const tk_tree* t, int lanes, int k) {
+    if (!t->auto_depth) return t->search_levels;
+    double leaf = kOneLaneLeaf;
+    if (t->dims > 3) leaf = lanes == 1 ? kOneLaneLeaf : 90;
+    else if (lanes == 32) leaf = t->dtype == TK_F64 ? 50 : (k <= 2 ? 50 : (k <= 48 ? 110 : 180));
+    else if (lanes > 1) leaf = 40;
+    return std::max(1, std::min(t->search_levels, log2_round(double(t->n) / leaf)));
+}
+
+namespace {
+
 template <typename T, int D>
 int run_query(const tk_tree* t, const T* q, int nq, int k, T* dists, int32_t* idx, const tk_query_opts& o,
               char* ws, cudaStream_t s) {
@@ -230,7 +254,7 @@ int run_query(const tk_tree* t, const T* q, int nq, int k, T* dists, int32_t* id
         if (!gr_available(t->dtype, D, G, R)) return fail(TK_EUNSUPPORTED, "no kernel shape for this k");
     }
 
-    const int L = t->levels;
+    const int L = packet ? t->search_levels : query_levels(t, G, k);
     // 10 levels (4 KiB for float): deeper staging measured no faster, and at
     // 12 levels (16 KiB) only 3 of the 4 blocks the registers allow stayed
     // resident per SM on the one-lane shape.
@@ -256,7 +280,7 @@ int run_query(const tk_tree* t, const T* q, int nq, int k, T* dists, int32_t* id
     int* counter = nullptr;
     const int32_t* order = nullptr;
     const PointRec<T>* boxes = static_cast<const PointRec<T>*>(t->d_boxes);
-    int rc0 = prepare_order(t, G, nq, k, o, ws, s, &counter, &order, true, [&](int B, int* counts, int* bin_of, int* pos_of) {
+    int rc0 = prepare_order(t, L, G, nq, k, o, ws, s, &counter, &order, true, [&](int B, int* counts, int* bin_of, int* pos_of) {
         bin_count_launch<T, D>(q, nq, static_cast<const T*>(t->d_medians), B, L, boxes, counts, bin_of, pos_of, s);
     });
     if (rc0 != TK_OK) return rc0;
@@ -296,7 +320,7 @@ int run_query_wide(const tk_tree* t, const T* q, int nq, int k, T* dists, int32_
     if (G != 1 || k > 16) G = 32;  // kernels of wide trees: 1 (k <= 16) or 32 lanes per query
     const int R = pow2_ceil((k + G - 1) / G);
     const int W = record_width(t->dims);
-    const int L = t->levels;
+    const int L = query_levels(t, G, k);
     int S = o.smem_levels >= 0 ? o.smem_levels : 10;
     S = std::max(0, std::min({S, L, sizeof(T) == 4 ? 15 : 14}));
     if (G == 32) S = 0;  // a warp per query reads split values five levels at a time instead
@@ -318,7 +342,7 @@ int run_query_wide(const tk_tree* t, const T* q, int nq, int k, T* dists, int32_
 
     int* counter = nullptr;
     const int32_t* order = nullptr;
-    const int rc0 = prepare_order(t, G, nq, k, o, ws, s, &counter, &order, true, [&](int B, int* counts, int* bin_of, int* pos_of) {
+    const int rc0 = prepare_order(t, L, G, nq, k, o, ws, s, &counter, &order, true, [&](int B, int* counts, int* bin_of, int* pos_of) {
         bin_count_wide_launch<T>(q, nq, t->dims, static_cast<const T*>(t->d_medians), B, L,
                                  static_cast<const T*>(t->d_boxes), W, counts, bin_of, pos_of, s);
     });
@@ -332,6 +356,7 @@ int run_query_wide(const tk_tree* t, const T* q, int nq, int k, T* dists, int32_
     // a warp per query prunes with node boxes always: one round trip tests all of a path's siblings
     a.boxes = o.prune_boxes == 0 && G == 1 ? nullptr : static_cast<const T*>(t->d_boxes);
     a.levels = L;
+    a.leaf_shift = t->search_levels - L;
     a.smem_levels = S;
     a.dims = t->dims;
     a.q = q;
@@ -453,10 +478,10 @@ void free_tree_device(tk_tree* t) {
     t->d_leaf_off = nullptr;
 }
 
-// Layout of a tree built on the GPU: points (T[n*dims]) and / or the
-// permutation (int32[n]) copied out of its device point records.
+// Points (T[n*dims]) and / or permutation (int32[n]) of a GPU-built tree in
+// the order of its device image.
 template <typename T>
-int device_layout(const tk_tree* t, T* points, int32_t* perm) {
+int image_layout(const tk_tree* t, T* points, int32_t* perm) {
     DeviceGuard g(t->device);
     if (t->dims > 3) {  // coordinate rows + separate indices
         const int W = record_width(t->dims);
@@ -493,6 +518,38 @@ int device_layout(const tk_tree* t, T* points, int32_t* perm) {
                 perm[i] = int32_t(bits);
             }
         }
+    }
+    return TK_OK;
+}
+
+// The same in the layout's order (depth `levels`).  A deeper image holds the
+// same points in each range of a leaf of that depth, ordered along the axes
+// of its own leaf parents: order each range along the layout's.
+template <typename T>
+int device_layout(const tk_tree* t, T* points, int32_t* perm) {
+    if (t->search_levels == t->levels) return image_layout<T>(t, points, perm);
+    const size_t n = size_t(t->n);
+    const int dims = t->dims, ax = (t->levels - 1) % dims;
+    std::vector<T> pts(n * dims);
+    std::vector<int32_t> ids(n), offs(size_t(1) << t->search_levels | 1), at(n);
+    int rc = image_layout<T>(t, pts.data(), ids.data());
+    if (rc != TK_OK) return rc;
+    {
+        DeviceGuard g(t->device);
+        const cudaError_t e = cudaMemcpy(offs.data(), t->d_leaf_off, sizeof(int32_t) * offs.size(), cudaMemcpyDeviceToHost);
+        if (e != cudaSuccess) return fail(TK_ECUDA, std::string("layout copy: ") + cudaGetErrorString(e));
+    }
+    for (size_t i = 0; i < n; ++i) at[i] = int32_t(i);
+    const int shift = t->search_levels - t->levels;
+    for (size_t l = 0; l < size_t(1) << t->levels; ++l)
+        std::sort(at.begin() + offs[l << shift], at.begin() + offs[(l + 1) << shift], [&](int32_t a, int32_t b) {
+            const T x = pts[size_t(a) * dims + ax], y = pts[size_t(b) * dims + ax];
+            return x < y || (!(y < x) && ids[a] < ids[b]);
+        });
+    for (size_t i = 0; i < n; ++i) {
+        if (points)
+            for (int d = 0; d < dims; ++d) points[i * dims + d] = pts[size_t(at[i]) * dims + d];
+        if (perm) perm[i] = ids[at[i]];
     }
     return TK_OK;
 }
@@ -694,6 +751,13 @@ size_t tk_tree_image_size(int64_t n, int dims, int dtype, int search_levels) {
     return tree_image(n, dims, dtype, search_levels).total;
 }
 
+int tk_tree_search_levels(int64_t n, int dims, int dtype, int levels) {
+    (void)dtype;
+    // the deepest that query_levels asks for
+    const int deep = log2_round(double(std::max<int64_t>(n, 1)) / (dims > 3 ? 90.0 : kOneLaneLeaf));
+    return std::min(kMaxLevels, std::max(levels, deep));
+}
+
 size_t tk_tree_build_workspace_size(int64_t n, int dims, int dtype) {
     if (n < 1 || dims < 1 || dims > kMaxDims) return 0;
     return build_workspace_bytes(n, dims, dtype);
@@ -707,6 +771,8 @@ int tk_tree_build_device(const void* dev_points, int64_t n, int dims, int dtype,
     *out = nullptr;
     int rc = check_device_build(dev_points, n, dims, dtype, levels, device);
     if (rc != TK_OK) return rc;
+    const bool auto_depth = search_levels == 0;
+    if (auto_depth) search_levels = tk_tree_search_levels(n, dims, dtype, levels);
     if (search_levels < levels || search_levels > kMaxLevels || n < (int64_t(1) << (search_levels - 1)))
         return fail(TK_EINVAL, "search_levels must be at least levels, and leave a point for every leaf parent");
     if (!image || image_bytes < tree_image(n, dims, dtype, search_levels).total)
@@ -716,7 +782,9 @@ int tk_tree_build_device(const void* dev_points, int64_t n, int dims, int dtype,
     if (ws_misaligned(workspace) || ws_misaligned(image))
         return fail(TK_EINVAL, "image and workspace must be 256-byte aligned");
     DeviceGuard g(device);
-    return device_build(dev_points, n, dims, dtype, levels, search_levels, device, image, workspace, stream, out);
+    rc = device_build(dev_points, n, dims, dtype, levels, search_levels, device, image, workspace, stream, out);
+    if (rc == TK_OK) (*out)->auto_depth = auto_depth;
+    return rc;
 }
 
 int tk_tree_destroy(tk_tree* t) {
@@ -773,8 +841,10 @@ int tk_tree_get_splits(const tk_tree* t, void* medians, int32_t* leaf_offsets) {
         cudaError_t e = cudaSuccess;
         if (medians)
             e = cudaMemcpy(medians, t->d_medians, (t->dtype == TK_F32 ? 4 : 8) * nparts, cudaMemcpyDeviceToHost);
-        if (e == cudaSuccess && leaf_offsets)
-            e = cudaMemcpy(leaf_offsets, t->d_leaf_off, sizeof(int32_t) * (nparts + 2), cudaMemcpyDeviceToHost);
+        if (e == cudaSuccess && leaf_offsets)  // every 2^(search_levels - levels)-th offset of the image
+            e = cudaMemcpy2D(leaf_offsets, sizeof(int32_t), t->d_leaf_off,
+                             sizeof(int32_t) << (t->search_levels - t->levels), sizeof(int32_t), nparts + 2,
+                             cudaMemcpyDeviceToHost);
         if (e != cudaSuccess) return fail(TK_ECUDA, std::string("split copy: ") + cudaGetErrorString(e));
         return TK_OK;
     }
@@ -793,7 +863,7 @@ int tk_tree_get_splits(const tk_tree* t, void* medians, int32_t* leaf_offsets) {
 
 size_t tk_tree_query_workspace_size(const tk_tree* t, int64_t nq) {
     if (!t || nq < 0) return 0;
-    return ws_layout(t->levels, std::max<int64_t>(nq, 1)).total;
+    return ws_layout(t->search_levels, std::max<int64_t>(nq, 1)).total;
 }
 
 int tk_tree_query(const tk_tree* t, const void* q, int64_t nq, int k, void* dists, int32_t* idx,
@@ -807,7 +877,7 @@ int tk_tree_query(const tk_tree* t, const void* q, int64_t nq, int k, void* dist
     if (t->device < 0 || !t->d_pts) return fail(TK_EINVAL, "tree was built host-only (device < 0); it has no device image");
     if (nq == 0) return TK_OK;
     if (!q || !dists || !idx) return fail(TK_EINVAL, "null query or output pointer");
-    const size_t need = ws_layout(t->levels, nq).total;
+    const size_t need = ws_layout(t->search_levels, nq).total;
     if (!workspace || workspace_bytes < need)
         return fail(TK_EWORKSPACE, "workspace too small: need " + std::to_string(need) + " bytes");
     if (ws_misaligned(workspace)) return fail(TK_EINVAL, "workspace must be 256-byte aligned");
@@ -899,7 +969,7 @@ extern "C" int tk_tree_query_noalloc(const tk_tree* t, const void* q, int64_t nq
     void* scratch = nullptr;
     int rc = noalloc_scratch(t->device, &scratch);
     if (rc != TK_OK) return rc;
-    if (ws_layout(t->levels, nq).total > kNoAllocScratchBytes)
+    if (ws_layout(t->search_levels, nq).total > kNoAllocScratchBytes)
         return fail(TK_EINVAL, "query needs more scratch than the static array holds");
     tk_query_opts o{0, -1, -1, 0, 0, nullptr, nullptr, -1, 0};
     if (opts) o = *opts;
@@ -1022,7 +1092,7 @@ extern "C" int tk_tree_query_host(const tk_tree* t, const void* q, int64_t nq, i
     const size_t es = t->dtype == TK_F32 ? 4 : 8;
     const size_t qb = es * size_t(t->dims) * size_t(nq), db = es * size_t(k) * size_t(nq),
                  ib = 4 * size_t(k) * size_t(nq);
-    const size_t wsb = align_up(ws_layout(t->levels, nq).total, 256);
+    const size_t wsb = align_up(ws_layout(t->search_levels, nq).total, 256);
     const size_t need = wsb + align_up(qb, 256) + (direct ? 0 : align_up(db, 256) + align_up(ib, 256));
     char* buf = nullptr;
     int rc = pipe_buffer(p, need, &buf);

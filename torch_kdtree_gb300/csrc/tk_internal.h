@@ -84,6 +84,12 @@ template <typename T>
 int build_device_tree(const T* pts, int64_t n, int dims, void* stream, tk_tree* t, void* workspace);
 }  // namespace tk
 
+namespace tk {
+// Depth at which a query of tree t with `lanes` lanes per query stops
+// (tk_api.cu): search_levels, or a shallower one where the library chooses.
+int query_levels(const tk_tree* t, int lanes, int k);
+}  // namespace tk
+
 // Opaque handle behind the C ABI.
 struct tk_tree {
     int dtype = TK_F32;

@@ -74,17 +74,18 @@ class _Tree:
         self.handle = h
 
     @classmethod
-    def from_device(cls, points: torch.Tensor, levels: int) -> "_Tree":
+    def from_device(cls, points: torch.Tensor, levels: int, auto_depth: bool) -> "_Tree":
         t = cls(None, levels, points.device.index)
         n, d = points.shape
         dt = _DTYPES[points.dtype]
         h = ctypes.c_void_p()
         # sizes are 0 for arguments that the build refuses; it then says why
-        image = _workspace(LIB.tk_tree_image_size(n, d, dt, levels), points.device)
+        depth = LIB.tk_tree_search_levels(n, d, dt, levels) if auto_depth else levels
+        image = _workspace(LIB.tk_tree_image_size(n, d, dt, depth), points.device)
         ws = _workspace(LIB.tk_tree_build_workspace_size(n, d, dt), points.device)
         stream = _stream_ptr(points.device)
-        check(LIB.tk_tree_build_device(points.data_ptr(), n, d, dt, levels, levels, points.device.index,
-                                       image.data_ptr(), image.numel(), ws.data_ptr(), ws.numel(), stream,
+        check(LIB.tk_tree_build_device(points.data_ptr(), n, d, dt, levels, 0 if auto_depth else levels,
+                                       points.device.index, image.data_ptr(), image.numel(), ws.data_ptr(), ws.numel(), stream,
                                        ctypes.byref(h)))
         t.handle, t.image, t.stream = h, image, stream
         return t
@@ -133,8 +134,10 @@ def knn_query_host(tree: _Tree, q: torch.Tensor, k: int, dists: torch.Tensor, id
 
 class TorchKDTree:
     def __init__(self, points_ref: torch.Tensor, device: torch.device, levels: int, squared_distances: bool,
-                 query_opts: Optional[QueryOpts] = None, build: str = "auto"):
-        """Builds the KD-tree.  See :func:`build_kd_tree`."""
+                 query_opts: Optional[QueryOpts] = None, build: str = "auto", auto_depth: bool = False):
+        """Builds the KD-tree.  See :func:`build_kd_tree`.  ``auto_depth``: the
+        layout has ``levels`` levels, but searches of a tree built on the GPU
+        may go as deep as suits them."""
         if device.type not in ("cuda", "cpu"):
             raise RuntimeError(f"Could not find the KD-Tree for your specified options (device {device}).")
         if points_ref.shape[0] >= 2 ** 31:
@@ -163,7 +166,7 @@ class TorchKDTree:
             build = "device" if points_ref.is_cuda else "host"
         if build == "device":
             pts = points_ref.detach().to(device).contiguous()
-            self._tree = _Tree.from_device(pts, self.levels)
+            self._tree = _Tree.from_device(pts, self.levels, auto_depth)
         else:
             host = np.ascontiguousarray(points_ref.detach().cpu().numpy())
             self._tree = _Tree(host, self.levels, device.index)
@@ -357,11 +360,14 @@ def build_kd_tree(points_ref: Union[torch.Tensor, np.ndarray], device: Optional[
     input, else "host".  With ``device='cpu'`` (the reference's KDTreeCPU
     trees) it is built and queried on the host.  ``device`` defaults to
     ``points_ref.device``; ``levels`` defaults to the reference's heuristic
-    and may range 1..24."""
+    and may range 1..24.  A depth that is asked for is the depth searched;
+    with the default, a tree built on the GPU reports the layout of the
+    heuristic's depth and is searched at the depth that suits each query."""
     if issubclass(type(points_ref), np.ndarray):
         points_ref = torch.from_numpy(points_ref)
     if device is None:
         device = points_ref.device
+    auto_depth = levels is None
     if levels is None:
         levels = default_levels(points_ref.shape[0])
     if issubclass(type(device), str):
@@ -370,7 +376,7 @@ def build_kd_tree(points_ref: Union[torch.Tensor, np.ndarray], device: Optional[
     assert issubclass(type(points_ref), torch.Tensor)
     assert device.type != "cuda" or gpu_available, "You requested the KD-Tree on the GPU, but no CUDA device is visible"
     assert device.type in ["cuda", "cpu"]
-    return TorchKDTree(points_ref, device, levels, squared_distances, query_opts, build)
+    return TorchKDTree(points_ref, device, levels, squared_distances, query_opts, build, auto_depth)
 
 
 TREE_FORMAT = "torch_kdtree_gb300.kdtree/1"
