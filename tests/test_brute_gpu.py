@@ -298,3 +298,49 @@ def test_random_configurations(oracle):
         msg = f"case {case}: d={d} n={n} nq={nq} k={k} {mode} {np.dtype(dtype).name}"
         np.testing.assert_array_equal(dd.cpu().numpy(), bd, err_msg=msg)
         np.testing.assert_array_equal(ii.cpu().numpy(), bi, err_msg=msg)
+
+
+@pytest.mark.parametrize("mode", ["tf32", "bf16_split"])
+@pytest.mark.parametrize("order", ["clustered", "sorted", "one_column"])
+@pytest.mark.parametrize("k", [1, 16, 32])
+def test_tensor_core_lists_that_fill_up(mode, order, k, oracle):
+    """Clouds whose near neighbours are neighbours in memory, or all sit where
+    one thread keeps its list: the sampled thresholds let too much through and
+    lists are pruned on the way."""
+    rng = np.random.default_rng(k)
+    n, d, nq = 40_000, 12, 300
+    if order == "clustered":
+        ref = np.repeat(rng.standard_normal((40, d)) * 8, n // 40, axis=0) + rng.standard_normal((n, d)) * 0.1
+    else:
+        ref = rng.standard_normal((n, d))
+        if order == "sorted":
+            ref = ref[np.argsort(ref[:, 0])]
+            ref[:, 0] *= 30
+        else:  # 157 tiles: every 157th reference shares a tile
+            ref[::157] *= 0.01
+    ref = ref.astype(np.float32)
+    q = (ref[rng.integers(0, n, nq)] + 0.05 * rng.standard_normal((nq, d))).astype(np.float32)
+    if order == "one_column":
+        q = (0.01 * rng.standard_normal((nq, d))).astype(np.float32)
+    bd, bi = oracle.brute(ref, q, k)
+    dd, ii = tk().nn_distance(torch.from_numpy(ref).to(cuda), torch.from_numpy(q).to(cuda), k, mode=mode)
+    np.testing.assert_array_equal(dd.cpu().numpy(), bd)
+    np.testing.assert_array_equal(ii.cpu().numpy(), bi)
+
+
+@pytest.mark.parametrize("n_listed", [3, 300, 2500])
+@pytest.mark.parametrize("k", [1, 32, 64])
+def test_recomputed_queries(n_listed, k, oracle):
+    """Queries without a certificate (their nearest references are all equally
+    far) among ordinary ones: few of them take a warp per slice, many the
+    tiled kernel."""
+    rng = np.random.default_rng(n_listed + k)
+    ref = np.concatenate([rng.standard_normal((6000, 8)), np.tile(rng.standard_normal((1, 8)) + 20, (700, 1))])
+    ref = ref[rng.permutation(len(ref))].astype(np.float32)
+    q = rng.standard_normal((3000, 8)).astype(np.float32)
+    hard = rng.permutation(len(q))[:n_listed]
+    q[hard] = (20 + 0.1 * rng.standard_normal((n_listed, 8))).astype(np.float32)
+    bd, bi = oracle.brute(ref, q, k)
+    dd, ii = tk().nn_distance(torch.from_numpy(ref).to(cuda), torch.from_numpy(q).to(cuda), k, mode="tf32")
+    np.testing.assert_array_equal(dd.cpu().numpy(), bd)
+    np.testing.assert_array_equal(ii.cpu().numpy(), bi)

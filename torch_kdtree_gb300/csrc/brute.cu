@@ -7,6 +7,7 @@
 
 #include "brute.cuh"
 #include "brute_tc.cuh"
+#include "kd_warp.cuh"
 
 namespace tk {
 namespace {
@@ -47,6 +48,9 @@ int padded_dims(int d) {
 BrutePlan plan_brute(int64_t n, int64_t nq, int d, int k, bool f32) {
     BrutePlan p;
     p.DP = padded_dims(d);
+    // long lists of narrow points: padded to 4 they fit the path below
+    // (262,144 x 65,536, d=3, k=32: 131 ms on two lanes per query, 24 ms)
+    if (f32 && d < 4 && k > 16 && k <= 32) p.DP = 4;
     if (f32 && p.DP % 4 == 0 && p.DP <= 32 && k <= 32) {
         // one lane per query with broadcast 16-byte row loads (brute.cuh)
         p.G = 1;
@@ -125,45 +129,163 @@ int check_common(const void* ref, int64_t n, const void* q, int64_t nq, int d, i
 
 }  // namespace
 
-// The fallback expects few listed queries: it slices the references finely
-// (as planned for 1,024 queries) and launches for the worst case of all nq;
-// blocks past the device-side count exit at once.
+// ------------------------------------------------- listed queries --
+//
+// The exact answers of the queries on a device-side list, whose length only
+// the device knows.  Usually it is empty or short: up to kFew queries, a warp
+// takes (query, slice) pairs, a lane per reference row read from global
+// memory (0.8 us per query of 262,144 references, d=32).  Longer lists go
+// through the tiled kernel above, its blocks looping over (query tile, slice)
+// pairs.  A last kernel merges a query's slices, a warp per query; whichever
+// kernel is not meant exits at once.  (The tiled kernel for any list, with a
+// lane merging a query's 128 slices, took 1.0 ms for a few dozen queries.)
+namespace {
+
+constexpr int kFew = 256;
+constexpr int kFewSlices = 64;
+constexpr int kMaxSlices = 128;
+constexpr int kSlots = 65536;  // (query, slice) pairs with a list in the shared buffer
+
+struct ListArgs {
+    const float* ref;
+    const float* q;
+    int n, d, k;
+    const int* qlist;
+    const int* qcount;
+    Key<float>* part;  // [listed query][slice][k]
+    int max_slices;    // of the tiled kernel
+    float* out_d;
+    int32_t* out_i;
+};
+
+// Rows of d floats, 16 bytes at a time when `vec`; the reference's order.
+__device__ __forceinline__ float row_dist(const float* __restrict__ q, const float* __restrict__ r, int d, bool vec) {
+    float acc = 0.f;
+    if (vec) {
+        for (int c = 0; c < d; c += 4) {
+            const float4 a = __ldg(reinterpret_cast<const float4*>(q + c)), b = __ldg(reinterpret_cast<const float4*>(r + c));
+            const float d0 = sub_rn(a.x, b.x), d1 = sub_rn(a.y, b.y), d2 = sub_rn(a.z, b.z), d3 = sub_rn(a.w, b.w);
+            acc = add_rn(add_rn(add_rn(add_rn(acc, mul_rn(d0, d0)), mul_rn(d1, d1)), mul_rn(d2, d2)), mul_rn(d3, d3));
+        }
+    } else {
+        for (int c = 0; c < d; ++c) {
+            const float t = sub_rn(q[c], r[c]);
+            acc = add_rn(acc, mul_rn(t, t));
+        }
+    }
+    return acc;
+}
+
+template <int R>
+__global__ void __launch_bounds__(256) k_few_search(const ListArgs a) {
+    __shared__ Key<float> bufs[8][64];
+    const int count = *a.qcount;
+    if (count > kFew) return;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const bool vec = (a.d & 3) == 0 && ((reinterpret_cast<uintptr_t>(a.ref) | reinterpret_cast<uintptr_t>(a.q)) & 15) == 0;
+    const int per = (a.n + kFewSlices - 1) / kFewSlices;
+    for (int item = blockIdx.x * 8 + w; item < count * kFewSlices; item += gridDim.x * 8) {
+        const int slot = item / kFewSlices, slice = item % kFewSlices;
+        const float* q = a.q + (long long)a.qlist[slot] * a.d;
+        const int r0 = int(min((long long)a.n, (long long)per * slice)), r1 = int(min((long long)a.n, (long long)r0 + per));
+        WarpList<float, R> wl;
+        wl.init(a.k, bufs[w], lane);
+        for (int r = r0; r < r1; r += 32) {
+            Key<float> mine = Key<float>::sentinel();
+            if (r + lane < r1) mine = Key<float>::make(row_dist(q, a.ref + (long long)(r + lane) * a.d, a.d, vec), uint32_t(r + lane));
+            wl.offer(mine, lane);
+        }
+        wl.flush(lane);
+        Key<float>* out = a.part + (long long)item * a.k;
+#pragma unroll
+        for (int i = 0; i < R; ++i) {
+            const int o = i * 32 + lane - (32 * R - a.k);
+            if (o >= 0) out[o] = wl.list.slot[i];
+        }
+    }
+}
+
+template <int R>
+__global__ void __launch_bounds__(256) k_list_merge(const ListArgs a) {
+    __shared__ Key<float> bufs[8][64];
+    const int count = *a.qcount;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int slices = count <= kFew ? kFewSlices : list_slices(count, kSlots, a.max_slices);
+    if (slices == 1) return;  // already in the outputs
+    for (int slot = blockIdx.x * 8 + w; slot < count; slot += gridDim.x * 8) {
+        WarpList<float, R> wl;
+        wl.init(a.k, bufs[w], lane);
+        const Key<float>* src = a.part + (long long)slot * slices * a.k;
+        const int total = slices * a.k;
+        for (int e = lane; e - lane < total; e += 32) wl.offer(e < total ? src[e] : Key<float>::sentinel(), lane);
+        wl.flush(lane);
+        wl.list.store(a.k, lane, a.out_d, a.out_i, a.qlist[slot]);
+    }
+}
+
+}  // namespace
+
+// Both kernels share one buffer of per-slice lists: 16.8 MB for k = 32,
+// whatever the list's length.
 size_t brute_fallback_workspace_bytes(int64_t n, int64_t nq, int d, int k) {
-    BrutePlan p = plan_brute(n, std::min<int64_t>(std::max<int64_t>(nq, 1), 1024), d, k, true);
-    if (p.nsplit <= 1) return 256;
-    return align256(sizeof(Key<float>) * size_t(std::max<int64_t>(nq, 1)) * p.nsplit * k);
+    (void)n;
+    (void)d;
+    const int64_t slots = std::min<int64_t>(kSlots, std::max<int64_t>(nq, 1) * kMaxSlices);
+    return align256(sizeof(Key<float>) * size_t(slots) * k);
 }
 
 int brute_fallback(const float* ref, int64_t n, const float* q, int64_t nq, int d, int k, float* dists,
                    int32_t* idx, const int* qlist, const int* qcount, void* ws, size_t ws_bytes, cudaStream_t s) {
-    BrutePlan p = plan_brute(n, std::min<int64_t>(std::max<int64_t>(nq, 1), 1024), d, k, true);
-    const int per_block = 256 / p.G;
-    p.qtiles = int((nq + per_block - 1) / per_block);
     if (ws_bytes < brute_fallback_workspace_bytes(n, nq, d, k)) return fail(TK_EWORKSPACE, "fallback workspace");
-    BruteArgs<float> a;
-    a.ref = ref;
-    a.q = q;
-    a.n = int(n);
-    a.nq = int(nq);
-    a.d = d;
-    a.k = k;
-    a.nsplit = p.nsplit;
-    a.out_d = dists;
-    a.out_i = idx;
-    a.part = static_cast<Key<float>*>(ws);
-    a.qlist = qlist;
-    a.qcount = qcount;
-    switch (p.DP) {
-        case 1: return launch_dp<float, 1>(a, p, s);
-        case 2: return launch_dp<float, 2>(a, p, s);
-        case 3: return launch_dp<float, 3>(a, p, s);
-        case 4: return launch_dp<float, 4>(a, p, s);
-        case 8: return launch_dp<float, 8>(a, p, s);
-        case 16: return launch_dp<float, 16>(a, p, s);
-        case 32: return launch_dp<float, 32>(a, p, s);
-        case 64: return launch_dp<float, 64>(a, p, s);
-        default: return launch_dp<float, 128>(a, p, s);
+    const int sms = sm_count_dev(), few = int(std::min<int64_t>(nq, kFew));
+    const int max_slices = int(std::max<int64_t>(1, std::min<int64_t>(kMaxSlices, n / 2048)));
+    ListArgs l{ref, q, int(n), d, k, qlist, qcount, static_cast<Key<float>*>(ws), max_slices, dists, idx};
+    const unsigned gs = unsigned(std::min(4 * sms, (few * kFewSlices + 7) / 8));
+    const unsigned gm = unsigned(std::min<int64_t>(4 * sms, (nq + 7) / 8));
+    if (k <= 32) k_few_search<1><<<gs, 256, 0, s>>>(l);
+    else if (k <= 64) k_few_search<2><<<gs, 256, 0, s>>>(l);
+    else k_few_search<4><<<gs, 256, 0, s>>>(l);
+    cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) return fail(TK_ECUDA, std::string("listed queries: ") + cudaGetErrorString(e));
+    int rc = TK_OK;
+    if (nq > kFew) {
+        BrutePlan p = plan_brute(n, nq, d, k, true);
+        p.nsplit = max_slices;
+        p.list_blocks = int(std::min<int64_t>(int64_t(p.qtiles) * max_slices, 8 * sms));
+        BruteArgs<float> a;
+        a.ref = ref;
+        a.q = q;
+        a.n = int(n);
+        a.nq = int(nq);
+        a.d = d;
+        a.k = k;
+        a.nsplit = p.nsplit;
+        a.out_d = dists;
+        a.out_i = idx;
+        a.part = static_cast<Key<float>*>(ws);
+        a.qlist = qlist;
+        a.qcount = qcount;
+        a.qmore = kFew;
+        a.slots = kSlots;
+        switch (p.DP) {
+            case 1: rc = launch_dp<float, 1>(a, p, s); break;
+            case 2: rc = launch_dp<float, 2>(a, p, s); break;
+            case 3: rc = launch_dp<float, 3>(a, p, s); break;
+            case 4: rc = launch_dp<float, 4>(a, p, s); break;
+            case 8: rc = launch_dp<float, 8>(a, p, s); break;
+            case 16: rc = launch_dp<float, 16>(a, p, s); break;
+            case 32: rc = launch_dp<float, 32>(a, p, s); break;
+            case 64: rc = launch_dp<float, 64>(a, p, s); break;
+            default: rc = launch_dp<float, 128>(a, p, s); break;
+        }
+        if (rc != TK_OK) return rc;
     }
+    if (k <= 32) k_list_merge<1><<<gm, 256, 0, s>>>(l);
+    else if (k <= 64) k_list_merge<2><<<gm, 256, 0, s>>>(l);
+    else k_list_merge<4><<<gm, 256, 0, s>>>(l);
+    e = cudaGetLastError();
+    if (e != cudaSuccess) return fail(TK_ECUDA, std::string("listed queries: ") + cudaGetErrorString(e));
+    return TK_OK;
 }
 
 }  // namespace tk

@@ -33,11 +33,20 @@ struct BruteArgs {
     T* out_d;       // [nq, k]   (nsplit == 1)
     int32_t* out_i; // [nq, k]
     Key<T>* part;   // [nq, nsplit, k] per-slice lists (nsplit > 1)
-    // Optional gather: when qlist is set, block slots index qlist[0..*qcount)
-    // and results go to rows qlist[slot]; slots past *qcount do nothing.
+    // Optional gather: when qlist is set, the queries are qlist[0..*qcount)
+    // and results go to their rows (the caller merges the slices).
     const int* qlist = nullptr;
     const int* qcount = nullptr;
+    int qmore = 0;  // a list of at most this many queries is not served here
+    int slots = 0;  // (query, slice) pairs that `part` has room for (qlist only)
 };
+
+// Slices of a listed search: as many as there is room for (with one, its
+// lists go straight to the outputs).
+__host__ __device__ __forceinline__ int list_slices(int count, int slots, int most) {
+    const int s = slots / (count > 0 ? count : 1);
+    return s < 1 ? 1 : (s > most ? most : s);
+}
 
 // Reference rows per shared-memory tile: 32 KiB of coordinates, 32 to 256 rows.
 template <typename T, int DP>
@@ -58,22 +67,17 @@ __device__ __forceinline__ T sqdist_padded(const T (&q)[DP], const T* r) {
     return acc;
 }
 
-template <typename T, int DP, int G, int R>
-__global__ void __launch_bounds__(256) k_brute(const BruteArgs<T> a) {
+// One query tile against one slice (LIST: of the listed queries).
+template <typename T, int DP, int G, int R, bool LIST>
+__device__ __forceinline__ void brute_block(const BruteArgs<T>& a, T* tile, int live, int nsplit, int qtile, int slice) {
     constexpr int TR = BruteTile<T, DP>::kRefs;
-    __shared__ __align__(16) T tile[TR * DP];
     const int lane = threadIdx.x & 31;
     const int gl = lane & (G - 1);
     const int gbase = lane & ~(G - 1);
     const unsigned gmask = group_mask<G>(lane);
-    const int slot = blockIdx.x * (blockDim.x / G) + threadIdx.x / G;
-    int live = a.nq;
-    if (a.qlist) {
-        live = *a.qcount;
-        if (int(blockIdx.x * (blockDim.x / G)) >= live) return;  // whole block idle (uniform)
-    }
+    const int slot = qtile * (blockDim.x / G) + threadIdx.x / G;
     const bool active = slot < live;
-    const int qi = active ? (a.qlist ? a.qlist[slot] : slot) : 0;
+    const int qi = active ? (LIST ? a.qlist[slot] : slot) : 0;
 
     T q[DP];
 #pragma unroll
@@ -83,9 +87,9 @@ __global__ void __launch_bounds__(256) k_brute(const BruteArgs<T> a) {
     list.init(a.k, gl);
     Key<T> worst = Key<T>::sentinel();
 
-    const long long per = ((long long)a.n + a.nsplit - 1) / a.nsplit;
-    const int r0 = int(min((long long)a.n, per * blockIdx.y));
-    const int r1 = int(min((long long)a.n, per * (blockIdx.y + 1)));
+    const long long per = ((long long)a.n + nsplit - 1) / nsplit;
+    const int r0 = int(min((long long)a.n, per * slice));
+    const int r1 = int(min((long long)a.n, per * (slice + 1)));
     for (int t0 = r0; t0 < r1; t0 += TR) {
         const int len = min(TR, r1 - t0);
         __syncthreads();
@@ -174,10 +178,10 @@ __global__ void __launch_bounds__(256) k_brute(const BruteArgs<T> a) {
         }
     }
     if (!active) return;
-    if (a.nsplit == 1) {
+    if (nsplit == 1) {
         list.store(a.k, gl, a.out_d, a.out_i, qi);
     } else {
-        Key<T>* dst = a.part + ((long long)slot * a.nsplit + blockIdx.y) * a.k;
+        Key<T>* dst = a.part + ((long long)slot * nsplit + slice) * a.k;
 #pragma unroll
         for (int r = 0; r < R; ++r) {
             const int s = r * G + gl;
@@ -185,6 +189,24 @@ __global__ void __launch_bounds__(256) k_brute(const BruteArgs<T> a) {
             if (o >= 0) dst[o] = list.slot[r];
         }
     }
+}
+
+template <typename T, int DP, int G, int R>
+__global__ void __launch_bounds__(256) k_brute(const BruteArgs<T> a) {
+    __shared__ __align__(16) T tile[BruteTile<T, DP>::kRefs * DP];
+    brute_block<T, DP, G, R, false>(a, tile, a.nq, a.nsplit, blockIdx.x, blockIdx.y);
+}
+
+// The queries of a list: blocks loop over its (query tile, slice) pairs.
+template <typename T, int DP, int G, int R>
+__global__ void __launch_bounds__(256) k_brute_list(const BruteArgs<T> a) {
+    __shared__ __align__(16) T tile[BruteTile<T, DP>::kRefs * DP];
+    const int live = *a.qcount;
+    if (live <= a.qmore) return;
+    const int nsplit = list_slices(live, a.slots, a.nsplit);
+    const int per_tile = blockDim.x / G, qtiles = (live + per_tile - 1) / per_tile;
+    for (int item = blockIdx.x; item < qtiles * nsplit; item += gridDim.x)
+        brute_block<T, DP, G, R, true>(a, tile, live, nsplit, item % qtiles, item / qtiles);
 }
 
 // Combine the per-slice lists of every query (group of G lanes per query).
@@ -195,9 +217,7 @@ __global__ void __launch_bounds__(256) k_brute_merge(const BruteArgs<T> a) {
     const int gbase = lane & ~(G - 1);
     const unsigned gmask = group_mask<G>(lane);
     const int slot = blockIdx.x * (blockDim.x / G) + threadIdx.x / G;
-    const int live = a.qlist ? *a.qcount : a.nq;
-    if (slot >= live) return;  // whole groups leave together
-    const int qi = a.qlist ? a.qlist[slot] : slot;
+    if (slot >= a.nq) return;  // whole groups leave together
     TopK<T, G, R> list;
     list.init(a.k, gl);
     Key<T> worst = Key<T>::sentinel();
@@ -208,7 +228,7 @@ __global__ void __launch_bounds__(256) k_brute_merge(const BruteArgs<T> a) {
         const Key<T> mine = e < total ? src[e] : Key<T>::sentinel();
         worst = offer<T, G, R>(list, mine, worst, gmask, gl, gbase);
     }
-    list.store(a.k, gl, a.out_d, a.out_i, qi);
+    list.store(a.k, gl, a.out_d, a.out_i, slot);
 }
 
 // Exact search for the queries listed on the device (qlist[0..*qcount)),
@@ -220,6 +240,7 @@ int brute_fallback(const float* ref, int64_t n, const float* q, int64_t nq, int 
 // Launch shape of an exhaustive search (brute.cu: plan_brute).
 struct BrutePlan {
     int DP, G, R, nsplit, qtiles;
+    int list_blocks = 0;  // blocks of a search of listed queries
 };
 
 template <typename T, int DP>
@@ -228,8 +249,12 @@ int launch_dp(const BruteArgs<T>& a, const BrutePlan& p, cudaStream_t s) {
     bool done = false;
 #define TK_BR(g, r)                                                          \
     if (!done && p.G == g && p.R == r) {                                     \
-        k_brute<T, DP, g, r><<<grid, 256, 0, s>>>(a);                        \
-        if (p.nsplit > 1) k_brute_merge<T, g, r><<<p.qtiles, 256, 0, s>>>(a); \
+        if (p.list_blocks) {                                                 \
+            if constexpr (sizeof(T) == 4) k_brute_list<T, DP, g, r><<<p.list_blocks, 256, 0, s>>>(a); \
+        } else {                                                             \
+            k_brute<T, DP, g, r><<<grid, 256, 0, s>>>(a);                    \
+            if (p.nsplit > 1) k_brute_merge<T, g, r><<<p.qtiles, 256, 0, s>>>(a); \
+        }                                                                    \
         done = true;                                                         \
     }
     TK_BR(1, 1) TK_BR(1, 4) TK_BR(1, 16) TK_BR(2, 16) TK_BR(4, 16) TK_BR(8, 16)

@@ -6,13 +6,16 @@
 //
 // 1. k_tc_pack: operands for the tensor cores (TF32 rounded to nearest, or a
 //    BF16 hi/lo split x = hi + lo) and |x|^2 in FP32.
-// 2. k_tc_select: a block owns 128 queries and one slice of the references;
+// 2. k_tc5_select (brute_tc_kernels.cuh): tcgen05 products of 128 queries and
+//    256 references at a time; every row collects the references that score
+//    below a sampled threshold tau.  Depths and k that it does not take go to
+//    k_tc_select: a block owns 128 queries and one slice of the references;
 //    tiles of 128 references are multiplied with mma.sync (TF32 m16n8k8 or
 //    BF16 m16n8k16 with three products hi*hi + hi*lo + lo*hi, FP32 accumulate),
 //    the score tile goes through shared memory, and one thread per query keeps
 //    the C = over-fetch best scores of its row (C >= 2k) plus the row
 //    threshold tau (the C-th score; +inf while fewer than C were seen).
-// 3. k_tc_rerank: one warp per query recomputes the exact distance of every
+// 3. k_tc5_rerank / k_tc_rerank: one warp per query recomputes the exact distance of every
 //    candidate with the reference arithmetic (sqdist order, no fused
 //    multiply-add), keeps the k best (distance, index) keys, and certifies:
 //    with D = k-th exact distance, E = bound on |score_tc - score_exact| for
@@ -27,6 +30,7 @@
 // parallel.
 #include <algorithm>
 #include <atomic>
+#include <cmath>
 #include <string>
 
 #include "brute_tc.cuh"
@@ -37,8 +41,10 @@ using namespace tcx;
 namespace {
 
 struct TcWs {
-    size_t a_pack, b_pack, a_lo, b_lo, rnorm, qnorm, cand_s, cand_i, tau, fail_count, fail_list, brute, err, total;
-    int KP, C, nsplit;
+    size_t a_pack, b_pack, a_lo, b_lo, rnorm, qnorm, fail_count, fail_list, brute, err, total;
+    size_t cand_s, cand_i, tau;  // mma.sync search
+    size_t hits, counts, thr;    // tcgen05 search
+    int KP, C, nsplit, pstride, rank, wanted;
     bool tc5;  // tcgen05 path
 };
 
@@ -68,7 +74,7 @@ int tc_over(int k) {
 }
 
 TcWs tc_layout(int64_t n, int64_t nq, int d, int k, int mode, int sms) {
-    TcWs w;
+    TcWs w{};
     w.tc5 = tc5_eligible(d, k, mode);
     w.KP = w.tc5 ? tc5_kp(d, mode) : tc_kp(d, mode);
     w.C = tc_over(k);
@@ -76,9 +82,39 @@ TcWs tc_layout(int64_t n, int64_t nq, int d, int k, int mode, int sms) {
     size_t o = 0;
     if (w.tc5) {
         const int qblocks = int((nq + kT5Rows - 1) / kT5Rows);
-        int ns = std::max(1, (8 * sms + qblocks / 2) / std::max(1, qblocks));
-        ns = int(std::min<int64_t>({int64_t(ns), int64_t(8), std::max<int64_t>(1, n / (8 * kT5Cols))}));
-        w.nsplit = ns;
+        // Slices of the references per row block, and the sample that gives a
+        // slice's threshold: max(150, 5k) references of a row are to score
+        // below the thresholds of its slices together (the certificate wants
+        // about 2k with room), by the rank-th smallest minimum of every
+        // pstride-th tile, rank about 25 (the threshold scatters by 1 / sqrt(rank)) --
+        // so the more slices, the larger the sampled share.  One block per
+        // SM: the slice count with the least (1 + share) / SMs used, of at
+        // least 8 tiles a slice.
+        const int64_t tiles = (n + kT5Cols - 1) / kT5Cols;
+        const int most = int(std::min<int64_t>(24, std::max<int64_t>(1, tiles / 8)));
+        // small calls, where it costs little, want more: their many short
+        // slices scatter more, and TF32's error is large against the spacing
+        // of near neighbours in few dimensions
+        double wanted = std::max(150.0, 5.0 * k);
+        if (qblocks <= (mode == TK_BRUTE_TF32 && d <= 8 ? sms : sms / 8)) wanted = std::max(wanted, 16.0 * k);
+        w.wanted = int(wanted);
+        double best = 1e30;
+        for (int ns = 1; ns <= most; ++ns) {
+            const int64_t per = (tiles + ns - 1) / ns;
+            const double below = wanted / ns;
+            const int stride = per >= 64 ? std::max(1, std::min(8, int(below / 25.0))) : 1;
+            const double blocks = double(qblocks) * ns;
+            const double cost = (1.0 + 1.0 / stride) * std::ceil(blocks / sms) * sms / blocks;
+            if (cost < 0.98 * best) {
+                best = cost;
+                w.nsplit = ns;
+                w.pstride = stride;
+                // of at most 0.8 of the minima there are (see k_tc5_select)
+                const int64_t pre = (per + stride - 1) / stride;
+                const int minima = int(pre <= 8 ? 16 * pre : std::min<int64_t>(kT5Minima, 4 * std::min<int64_t>(pre, 32)));
+                w.rank = std::max(8, std::min({64, minima * 4 / 5, int(below / stride + 0.5)}));
+            }
+        }
         const size_t nq_pad = size_t(qblocks) * kT5Rows;
         const size_t n_pad = size_t((n + kT5Cols - 1) / kT5Cols) * kT5Cols;
         w.a_pack = o; o += align256(es * nq_pad * w.KP);
@@ -99,9 +135,16 @@ TcWs tc_layout(int64_t n, int64_t nq, int d, int k, int mode, int sms) {
         w.qnorm = o; o += align256(4 * size_t(nq));
     }
     w.err = o; o += 256;
-    w.cand_s = o; o += align256(4 * size_t(nq) * w.nsplit * w.C);
-    w.cand_i = o; o += align256(4 * size_t(nq) * w.nsplit * w.C);
-    w.tau = o; o += align256(4 * size_t(nq) * w.nsplit);
+    if (w.tc5) {
+        const size_t lists = (size_t(nq) + kT5Rows - 1) / kT5Rows * kT5Rows * w.nsplit * kT5Parts;
+        w.hits = o; o += align256(8 * lists * kT5Cap);
+        w.counts = o; o += align256(4 * lists);
+        w.thr = o; o += align256(4 * lists);
+    } else {
+        w.cand_s = o; o += align256(4 * size_t(nq) * w.nsplit * w.C);
+        w.cand_i = o; o += align256(4 * size_t(nq) * w.nsplit * w.C);
+        w.tau = o; o += align256(4 * size_t(nq) * w.nsplit);
+    }
     w.fail_count = o; o += 256;
     w.fail_list = o; o += align256(4 * size_t(nq));
     w.brute = o; o += brute_fallback_workspace_bytes(n, nq, d, k);
@@ -167,40 +210,39 @@ int run_brute_tc(const float* ref, int64_t n, const float* q, int64_t nq, int d,
     int crc = TK_OK;
     if (w.tc5) {
         // 1-2. pack into the core-matrix layout and run the tcgen05 candidate kernel
-        const int qblocks = (nq32 + kT5Rows - 1) / kT5Rows;
-        const int n_pad = int((n + kT5Cols - 1) / kT5Cols) * kT5Cols;
+        const int qblocks = (nq32 + kT5Rows - 1) / kT5Rows, tiles = int((n + kT5Cols - 1) / kT5Cols);
         unsigned char* ahi = reinterpret_cast<unsigned char*>(p + w.a_pack);
         unsigned char* alo = reinterpret_cast<unsigned char*>(p + w.a_lo);
         unsigned char* bhi = reinterpret_cast<unsigned char*>(p + w.b_pack);
         unsigned char* blo = reinterpret_cast<unsigned char*>(p + w.b_lo);
-        const int nq_pad = qblocks * kT5Rows;
+        const int chunks = w.KP * (mode == TK_BRUTE_TF32 ? 4 : 2) / 16;  // 16-byte pieces of a packed row
+        auto grid = [&](int64_t rows) { return unsigned((rows * chunks + 255) / 256); };
+        const unsigned ga = grid(int64_t(qblocks) * kT5Rows), gb = grid(int64_t(tiles) * kT5Cols);
         if (mode == TK_BRUTE_TF32) {
-            k_tc5_pack<TK_BRUTE_TF32><<<(nq_pad + 255) / 256, 256, 0, s>>>(q, nq32, nq_pad, d, w.KP, kT5Rows, 1, ahi, alo,
-                                                                         err);
-            k_tc5_pack<TK_BRUTE_TF32><<<(n_pad + 255) / 256, 256, 0, s>>>(ref, n32, n_pad, d, w.KP, kT5Cols, 0, bhi, blo,
-                                                                        err);
+            k_tc5_pack<TK_BRUTE_TF32><<<ga, 256, 0, s>>>(q, nq32, qblocks, d, w.KP, 1, ahi, alo, err);
+            k_tc5_pack<TK_BRUTE_TF32><<<gb, 256, 0, s>>>(ref, n32, tiles, d, w.KP, 0, bhi, blo, err);
         } else {
-            k_tc5_pack<TK_BRUTE_BF16_SPLIT><<<(nq_pad + 255) / 256, 256, 0, s>>>(q, nq32, nq_pad, d, w.KP, kT5Rows, 1,
-                                                                               ahi, alo, err);
-            k_tc5_pack<TK_BRUTE_BF16_SPLIT><<<(n_pad + 255) / 256, 256, 0, s>>>(ref, n32, n_pad, d, w.KP, kT5Cols, 0,
-                                                                              bhi, blo, err);
+            k_tc5_pack<TK_BRUTE_BF16_SPLIT><<<ga, 256, 0, s>>>(q, nq32, qblocks, d, w.KP, 1, ahi, alo, err);
+            k_tc5_pack<TK_BRUTE_BF16_SPLIT><<<gb, 256, 0, s>>>(ref, n32, tiles, d, w.KP, 0, bhi, blo, err);
         }
         Tc5Args t5{};
         t5.a_hi = ahi;
         t5.a_lo = alo;
         t5.b_hi = bhi;
         t5.b_lo = blo;
-        t5.n = n32;
         t5.nq = nq32;
+        t5.tiles = tiles;
         t5.nsplit = w.nsplit;
-        t5.cand_s = reinterpret_cast<float*>(p + w.cand_s);
-        t5.cand_i = reinterpret_cast<int32_t*>(p + w.cand_i);
-        t5.tau = reinterpret_cast<float*>(p + w.tau);
+        t5.pstride = w.pstride;
+        t5.rank = w.rank;
+        t5.hits = reinterpret_cast<uint2*>(p + w.hits);
+        t5.counts = reinterpret_cast<int*>(p + w.counts);
+        t5.thr = reinterpret_cast<float*>(p + w.thr);
         t5.err = reinterpret_cast<int*>(p + w.err);
         const uint32_t polls = g_wait_polls.load();
         t5.max_tries = polls ? polls : kT5MaxTries;
-        crc = mode == TK_BRUTE_TF32 ? tc5_dispatch_tf32(t5, w.KP, w.C / 2, qblocks, s)
-                                    : tc5_dispatch_bf16(t5, w.KP, w.C / 2, qblocks, s);
+        crc = mode == TK_BRUTE_TF32 ? tc5_dispatch_tf32(t5, w.KP, qblocks, s)
+                                    : tc5_dispatch_bf16(t5, w.KP, qblocks, s);
         if (crc != TK_OK) return crc;
     } else if (mode == TK_BRUTE_TF32) {
         k_tc_pack<TK_BRUTE_TF32><<<(nq32 + 255) / 256, 256, 0, s>>>(q, nq32, d, w.KP, reinterpret_cast<uint32_t*>(p + w.a_pack),
@@ -254,16 +296,22 @@ int run_brute_tc(const float* ref, int64_t n, const float* q, int64_t nq, int d,
     ra.cand_s = a.cand_s;
     ra.cand_i = a.cand_i;
     ra.tau = a.tau;
+    ra.keep = w.wanted;
+    ra.hits = reinterpret_cast<const uint2*>(p + w.hits);
+    ra.counts = reinterpret_cast<const int*>(p + w.counts);
+    ra.thr = reinterpret_cast<const float*>(p + w.thr);
     const double u = 1.0 / 16777216.0;
-    ra.eps_dot = mode == TK_BRUTE_TF32 ? (1.0 / 1024.0 + 1.0 / 4194304.0 + (d + 2) * 2.0 * u)
-                                       : (3.1 / 65536.0 + 3.0 * (d + 2) * 2.0 * u);
+    ra.eps_dot = float(mode == TK_BRUTE_TF32 ? (1.0 / 1024.0 + 1.0 / 4194304.0 + (d + 2) * 2.0 * u)
+                                             : (3.1 / 65536.0 + 3.0 * (d + 2) * 2.0 * u));
     ra.out_d = dists;
     ra.out_i = idx;
     ra.fail_count = reinterpret_cast<int*>(p + w.fail_count);
     ra.fail_list = reinterpret_cast<int*>(p + w.fail_list);
     ra.err = reinterpret_cast<const int*>(p + w.err);
     const int rb = (nq32 + 7) / 8;
-    if (k <= 32) k_tc_rerank<1><<<rb, 256, 0, s>>>(ra);
+    if (w.tc5) {
+        k_tc5_rerank<<<rb, 256, 0, s>>>(ra);
+    } else if (k <= 32) k_tc_rerank<1><<<rb, 256, 0, s>>>(ra);
     else k_tc_rerank<2><<<rb, 256, 0, s>>>(ra);
     e = cudaGetLastError();
     if (e != cudaSuccess) return fail(TK_ECUDA, std::string("tc launch: ") + cudaGetErrorString(e));

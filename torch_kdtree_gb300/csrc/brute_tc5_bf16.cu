@@ -4,11 +4,11 @@
 namespace tk {
 namespace tcx {
 
-int tc5_dispatch_bf16(const Tc5Args& a, int KP, int CH, int qblocks, cudaStream_t s) {
+int tc5_dispatch_bf16(const Tc5Args& a, int KP, int qblocks, cudaStream_t s) {
     switch (KP) {
-        case 16: return tc5_dispatch_ch<TK_BRUTE_BF16_SPLIT, 16>(a, CH, qblocks, s);
-        case 32: return tc5_dispatch_ch<TK_BRUTE_BF16_SPLIT, 32>(a, CH, qblocks, s);
-        case 48: return tc5_dispatch_ch<TK_BRUTE_BF16_SPLIT, 48>(a, CH, qblocks, s);
+        case 16: return launch_tc5<TK_BRUTE_BF16_SPLIT, 16>(a, qblocks, s);
+        case 32: return launch_tc5<TK_BRUTE_BF16_SPLIT, 32>(a, qblocks, s);
+        case 48: return launch_tc5<TK_BRUTE_BF16_SPLIT, 48>(a, qblocks, s);
         default: return fail(TK_EUNSUPPORTED, "tcgen05 path: unsupported depth");
     }
 }

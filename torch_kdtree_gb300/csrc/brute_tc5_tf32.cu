@@ -4,12 +4,12 @@
 namespace tk {
 namespace tcx {
 
-int tc5_dispatch_tf32(const Tc5Args& a, int KP, int CH, int qblocks, cudaStream_t s) {
+int tc5_dispatch_tf32(const Tc5Args& a, int KP, int qblocks, cudaStream_t s) {
     switch (KP) {
-        case 8: return tc5_dispatch_ch<TK_BRUTE_TF32, 8>(a, CH, qblocks, s);
-        case 16: return tc5_dispatch_ch<TK_BRUTE_TF32, 16>(a, CH, qblocks, s);
-        case 24: return tc5_dispatch_ch<TK_BRUTE_TF32, 24>(a, CH, qblocks, s);
-        default: return tc5_dispatch_tf32_deep(a, KP, CH, qblocks, s);  // 32, 40
+        case 8: return launch_tc5<TK_BRUTE_TF32, 8>(a, qblocks, s);
+        case 16: return launch_tc5<TK_BRUTE_TF32, 16>(a, qblocks, s);
+        case 24: return launch_tc5<TK_BRUTE_TF32, 24>(a, qblocks, s);
+        default: return tc5_dispatch_tf32_deep(a, KP, qblocks, s);  // 32, 40
     }
 }
 

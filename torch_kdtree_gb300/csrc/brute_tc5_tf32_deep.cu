@@ -4,10 +4,10 @@
 namespace tk {
 namespace tcx {
 
-int tc5_dispatch_tf32_deep(const Tc5Args& a, int KP, int CH, int qblocks, cudaStream_t s) {
+int tc5_dispatch_tf32_deep(const Tc5Args& a, int KP, int qblocks, cudaStream_t s) {
     switch (KP) {
-        case 32: return tc5_dispatch_ch<TK_BRUTE_TF32, 32>(a, CH, qblocks, s);
-        case 40: return tc5_dispatch_ch<TK_BRUTE_TF32, 40>(a, CH, qblocks, s);
+        case 32: return launch_tc5<TK_BRUTE_TF32, 32>(a, qblocks, s);
+        case 40: return launch_tc5<TK_BRUTE_TF32, 40>(a, qblocks, s);
         default: return fail(TK_EUNSUPPORTED, "tcgen05 path: unsupported depth");
     }
 }

@@ -11,6 +11,7 @@
 #include <string>
 
 #include "brute.cuh"
+#include "kd_warp.cuh"
 #include "tc_sm100.cuh"
 #include "tk_internal.h"
 
@@ -253,18 +254,17 @@ __global__ void __launch_bounds__(kThreads, 1) k_tc_select(const TcArgs a) {
 // no-swizzle K-major layout (8-row x 16-byte core matrices; core matrices
 // adjacent along K 128 bytes apart, 8-row groups 8*KB bytes apart), one
 // contiguous block per 128 query rows / 256 reference rows, so each tile is
-// a single bulk copy.  Reference padding rows carry a huge |r|^2 and never
-// become candidates.
+// a single bulk copy.  Reference r sits in tile r % tiles, at column r / tiles
+// turned by a step per tile (packed_ref): references that are neighbours in
+// memory, often neighbours in space, fall into different tiles (see the sample
+// below) and different column groups (see the lists).  Padding rows carry a
+// huge |r|^2.
 constexpr int kT5Rows = 128;   // M (queries per block)
 constexpr int kT5Cols = 256;   // N (references per tile)
 constexpr int kT5EpiWarps = 16; // 4 per 32-lane quarter of the accumulator when reading tensor memory
-constexpr int kT5Chunk = 64;    // accumulator columns per phase (16 per column-group warp)
-constexpr int kT5Buf = 48;      // hit buffer per row and tile parity (a redo phase: 32 columns)
-constexpr int kT5BufStride = kT5Buf + 1;  // row stride of the hit buffer (keys), spreads rows over banks
-// Row stride (words) of the sample's group minima (2C <= 128 per row); 132 = 4
-// mod 32 puts the 32 lanes of a bisection read (8 rows x 4 interleaved lanes)
-// on 32 different banks.
-constexpr int kT5MinStride = 132;
+constexpr int kT5Parts = kT5EpiWarps / 4;           // column groups of 64: lists per row and slice
+constexpr int kT5Minima = 128;                      // sample minima per row
+constexpr int kT5MinStride = kT5Minima + 2;         // their row stride (16-bit words): lanes of a read on other banks
 constexpr int kT5Threads = 32 * (kT5EpiWarps + 1);
 constexpr float kT5PadNorm = 1e30f;
 constexpr uint32_t kT5MaxTries = 1u << 22;  // bounded mbarrier polls (default; Tc5Args::max_tries)
@@ -273,40 +273,60 @@ __device__ __forceinline__ uint32_t core_offset(int row, int kb, int KB) {
     return uint32_t((row >> 3) * (8 * KB) + (kb >> 4) * 128 + (row & 7) * 16 + (kb & 15));
 }
 
-// rows: logical rows; padded to a multiple of tile_rows.  is_query selects
-// [-2q, 1] (queries) or [r, |r|^2] (references).
+// Reference at column `col` of tile `tile`; padding when >= n.
+__device__ __forceinline__ uint32_t packed_ref(uint32_t tile, uint32_t col, uint32_t tiles) {
+    return ((col - 67u * tile) & uint32_t(kT5Cols - 1)) * tiles + tile;
+}
+
+// A thread per 16 bytes of a packed row.  is_query selects [-2q, 1]
+// (tiles of kT5Rows rows) or [r, |r|^2] (tiles of kT5Cols rows).
 template <int MODE>
-__global__ void k_tc5_pack(const float* __restrict__ x, int rows, int rows_pad, int d, int KP, int tile_rows,
-                           int is_query, unsigned char* __restrict__ hi, unsigned char* __restrict__ lo,
-                           int* __restrict__ err) {
-    const int r = blockIdx.x * blockDim.x + threadIdx.x;
-    if (r >= rows_pad) return;
+__global__ void __launch_bounds__(256) k_tc5_pack(const float* __restrict__ x, int rows, int tiles, int d, int KP,
+                                                  int is_query, unsigned char* __restrict__ hi,
+                                                  unsigned char* __restrict__ lo, int* __restrict__ err) {
     constexpr int ESZ = MODE == TK_BRUTE_TF32 ? 4 : 2;
-    const int KB = KP * ESZ;
+    constexpr int E = 16 / ESZ;  // elements of 16 bytes
+    const int KB = KP * ESZ, chunks = KB / 16;
+    const int tile_rows = is_query ? kT5Rows : kT5Cols;
+    const long long i = (long long)blockIdx.x * 256 + threadIdx.x;
+    const long long p = i / chunks;
+    const int cb = int(i - p * chunks);
+    if (p >= (long long)tiles * tile_rows) return;
+    const int tile = int(p / tile_rows), c = int(p - (long long)tile * tile_rows);
+    const long long r = is_query ? p : (long long)packed_ref(uint32_t(tile), uint32_t(c), uint32_t(tiles));
     const bool real = r < rows;
-    float nrm = 0.f;
-    if (real && !is_query) {
-        for (int c = 0; c < d; ++c) nrm = fmaf(x[(long long)r * d + c], x[(long long)r * d + c], nrm);
-        if (!(nrm < kTcNormLimit)) atomicOr(err, kTcErrRange);  // see kTcNormLimit
+    const float* row = x + r * d;
+    float v[E];
+#pragma unroll
+    for (int e = 0; e < E; ++e) {
+        const int k = cb * E + e;
+        v[e] = 0.f;
+        if (k < d) {
+            v[e] = real ? row[k] : 0.f;
+            if (is_query) v[e] = -2.f * v[e];
+        } else if (k == d) {
+            if (is_query) {
+                v[e] = real ? 1.f : 0.f;
+            } else {
+                float nrm = 0.f;
+                for (int j = 0; real && j < d; ++j) nrm = fmaf(row[j], row[j], nrm);
+                if (!(nrm < kTcNormLimit)) atomicOr(err, kTcErrRange);  // see kTcNormLimit
+                v[e] = real ? nrm : kT5PadNorm;
+            }
+        }
     }
-    const long long tile_base = (long long)(r / tile_rows) * tile_rows * KB;
-    const int rr = r % tile_rows;
-    for (int c = 0; c < KP; ++c) {
-        float v = 0.f;
-        if (c < d) {
-            v = real ? x[(long long)r * d + c] : 0.f;
-            if (is_query) v = -2.f * v;
-        } else if (c == d) {
-            v = is_query ? (real ? 1.f : 0.f) : (real ? nrm : kT5PadNorm);
+    const long long off = (long long)tile * tile_rows * KB + core_offset(c, cb * 16, KB);
+    if constexpr (MODE == TK_BRUTE_TF32) {
+        *reinterpret_cast<uint4*>(hi + off) = make_uint4(to_tf32(v[0]), to_tf32(v[1]), to_tf32(v[2]), to_tf32(v[3]));
+    } else {
+        __align__(16) __nv_bfloat16 h[E], l[E];
+#pragma unroll
+        for (int e = 0; e < E; ++e) {
+            h[e] = __float2bfloat16_rn(v[e]);
+            l[e] = __float2bfloat16_rn(v[e] - __bfloat162float(h[e]));
         }
-        const long long off = tile_base + core_offset(rr, c * ESZ, KB);
-        if (MODE == TK_BRUTE_TF32) {
-            *reinterpret_cast<uint32_t*>(hi + off) = to_tf32(v);
-        } else {
-            const __nv_bfloat16 h = __float2bfloat16_rn(v);
-            *reinterpret_cast<__nv_bfloat16*>(hi + off) = h;
-            *reinterpret_cast<__nv_bfloat16*>(lo + off) = __float2bfloat16_rn(v - __bfloat162float(h));
-        }
+        *reinterpret_cast<uint4*>(hi + off) = *reinterpret_cast<const uint4*>(h);
+        *reinterpret_cast<uint4*>(lo + off) = *reinterpret_cast<const uint4*>(l);
     }
 }
 
@@ -315,26 +335,17 @@ struct Tc5Args {
     const unsigned char* a_lo;
     const unsigned char* b_hi;  // packed references, tiles of 256 rows
     const unsigned char* b_lo;
-    int n, nq, nsplit;
-    float* cand_s;              // [nq, nsplit, 2 * CH]
-    int32_t* cand_i;
-    float* tau;                 // [nq, nsplit]
+    int nq, tiles, nsplit;
+    int pstride;                // every pstride-th tile of a slice is sampled
+    int rank;                   // the threshold is the rank-th smallest of the sample's minima
+    uint2* hits;                // [padded nq][nsplit][kT5Parts][CAP]: score bits, reference
+    int* counts;                // [padded nq][nsplit][kT5Parts]
+    float* thr;                 // same shape: every reference of the part scoring below it is in its list
     int* err;                   // kTcErrTimeout set when a bounded wait ran out
     uint32_t max_tries;         // polls of each mbarrier wait before giving up
 };
 
-// Score keys: order-preserving uint32 image of the float score (negative
-// scores included) in the high word, reference index in the low word.
-__device__ __forceinline__ unsigned long long score_key(float sc, uint32_t idx) {
-    uint32_t u = __float_as_uint(sc);
-    u = (u & 0x80000000u) ? ~u : (u | 0x80000000u);
-    return (static_cast<unsigned long long>(u) << 32) | idx;
-}
-__device__ __forceinline__ float key_score(unsigned long long key) {
-    const uint32_t u = uint32_t(key >> 32);
-    return __uint_as_float((u & 0x80000000u) ? (u & 0x7FFFFFFFu) : ~u);
-}
-constexpr unsigned long long kScoreSentinel = (0xFF800000ull << 32) | 0xFFFFFFFFull;  // score +inf
+// Order-preserving uint32 image of a score (negative scores included).
 __device__ __forceinline__ uint32_t score_bits(float sc) {
     const uint32_t u = __float_as_uint(sc);
     return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
@@ -343,40 +354,12 @@ __device__ __forceinline__ float bits_score(uint32_t u) {
     return __uint_as_float((u & 0x80000000u) ? (u & 0x7FFFFFFFu) : ~u);
 }
 
-// A row's over-fetch list of up to 32 * R keys spread over a warp (slot s on
-// lane s % 32, register s / 32; the first 32 R - C slots are padding below
-// every key), as TopK in tk_device.cuh.
-// The over-fetch list of one query row held by a group of 4 lanes: ascending
-// score keys, lane g of the group holding ranks [RS g, RS g + RS) in its
-// registers (RS = C / 4).  An insertion shifts every lane's run in registers
-// and moves one key across each lane boundary with a single shuffle, so the 8
-// groups of a warp insert into their 8 rows side by side.
-template <int RS>
-struct GroupList {
-    unsigned long long slot[RS];
-    __device__ __forceinline__ void init() {
-#pragma unroll
-        for (int i = 0; i < RS; ++i) slot[i] = kScoreSentinel;
-    }
-    // Insert c (the sentinel leaves the list as it is); every lane of the
-    // warp calls it.  gl: this lane's place in its group.
-    __device__ __forceinline__ void insert(unsigned long long c, int gl) {
-        const unsigned long long before = __shfl_up_sync(0xFFFFFFFFu, slot[RS - 1], 1, 4);
-#pragma unroll
-        for (int i = RS - 1; i >= 0; --i) {  // top down: slot[i - 1] is still the old value
-            const unsigned long long old = slot[i];
-            const bool has_prev = i > 0 || gl > 0;
-            const unsigned long long prev = i > 0 ? slot[i - 1] : before;
-            slot[i] = old <= c ? old : ((!has_prev || prev <= c) ? c : prev);
-        }
-    }
-    __device__ __forceinline__ unsigned long long worst() const {
-        return __shfl_sync(0xFFFFFFFFu, slot[RS - 1], 3, 4);
-    }
-};
+// Entries of one part's list, and how many of them survive when it fills up
+// (before it may lack room for 16 more).  Enough for every k the path takes.
+constexpr int kT5Kept = 64;
+constexpr int kT5Cap = 2 * kT5Kept + 16;
 
-
-template <int MODE, int KP, int CH>
+template <int MODE, int KP>
 struct Tc5Shape {
     static constexpr int ESZ = MODE == TK_BRUTE_TF32 ? 4 : 2;
     static constexpr int KB = KP * ESZ;
@@ -384,37 +367,85 @@ struct Tc5Shape {
     static constexpr uint32_t A_BYTES = uint32_t(kT5Rows) * KB;
     static constexpr uint32_t B_BYTES = uint32_t(kT5Cols) * KB;
     static constexpr int KSTEPS = KB / 32;
-    static constexpr size_t SMEM = size_t(PL) * A_BYTES + 2 * size_t(PL) * B_BYTES +
-                                   2 * size_t(kT5Rows) * kT5BufStride * 8 +  // hit buffers by tile parity
-                                   size_t(kT5Rows) * sizeof(float) +         // row thresholds
-                                   2 * size_t(kT5Rows) * sizeof(int) +       // hit counts by tile parity
-                                   40 * sizeof(int);                         // overflow / abort flags: block, per quarter
-    static_assert(SMEM <= 232448, "shared memory of the select kernel");
-    static_assert(size_t(kT5Rows) * kT5MinStride * 4 <= 2 * size_t(kT5Rows) * kT5BufStride * 8 && 4 * CH <= 128,
-                  "the sample's minima fit the hit buffers");
+    static constexpr size_t FIXED = size_t(PL) * A_BYTES + size_t(kT5Rows) * kT5MinStride * 2 + kT5Rows * sizeof(float);
+    // reference tiles in flight: as many as fit, at most 4
+    static constexpr int STAGES = (232448 - FIXED) / (PL * B_BYTES) < 4 ? int((232448 - FIXED) / (PL * B_BYTES)) : 4;
+    static_assert(STAGES >= 3, "reference stages of the select kernel");
+    static constexpr size_t SMEM = FIXED + size_t(STAGES) * PL * B_BYTES;
 };
 
+// A part's list of n >= kT5Kept entries (n <= kT5Cap), by the whole warp:
+// lower its threshold to its kT5Kept-th smallest score and keep what scores
+// below.  Returns (entries kept, threshold's bits).  By the list's own lane
+// alone this took 0.5 ms.
+static __device__ __noinline__ uint2 prune_hits(uint2* list, int n, int lane) {
+    constexpr int E = (kT5Cap + 31) / 32;
+    uint2 k[E];
+    uint32_t u[E], lo = 0xFFFFFFFFu, hi = 0u;
+    __syncwarp();
+#pragma unroll
+    for (int e = 0; e < E; ++e) {
+        const bool in = 32 * e + lane < n;
+        k[e] = in ? list[32 * e + lane] : make_uint2(0u, 0u);
+        u[e] = in ? score_bits(__uint_as_float(k[e].x)) : 0xFFFFFFFFu;
+        lo = min(lo, u[e]);
+        if (in) hi = max(hi, u[e]);
+    }
+    lo = __reduce_min_sync(0xFFFFFFFFu, lo);
+    hi = __reduce_max_sync(0xFFFFFFFFu, hi);
+    while (lo < hi) {
+        const uint32_t mid = lo + ((hi - lo) >> 1);
+        int c = 0;
+#pragma unroll
+        for (int e = 0; e < E; ++e) c += u[e] <= mid ? 1 : 0;
+        c = __reduce_add_sync(0xFFFFFFFFu, c);
+        if (c >= kT5Kept) hi = mid;
+        else lo = mid + 1u;
+    }
+    int kept = 0;
+#pragma unroll
+    for (int e = 0; e < E; ++e) {
+        const unsigned m = __ballot_sync(0xFFFFFFFFu, u[e] < lo);
+        if (u[e] < lo) list[kept + __popc(m & ((1u << lane) - 1u))] = k[e];
+        kept += __popc(m);
+    }
+    __syncwarp();
+    return make_uint2(uint32_t(kept), __float_as_uint(bits_score(lo)));
+}
+
+__device__ __forceinline__ float min3(float a, float b, float c) {
+    float r;
+    asm("min.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+    return r;
+}
+
 // Candidate search of one block: 128 query rows against one slice of the
-// references, C = 2 CH candidates per row.
+// references.
 //
-// Sampled first threshold.  Before its slice a block runs PS = C / 2 full
-// tiles spread over the slice (a sample); each epilogue thread takes the
-// minimum of its 64 scores of a sample tile (a group of 64 references of its
-// row), and the row's four list lanes find T0 = the C-th smallest of the
-// row's 2C group minima (bisection on their order-preserving images).  At
-// least C distinct references of the slice score <= T0 (the minima of C
-// groups), so the slice's C-th best score is <= T0 and T0 is a valid
-// threshold from the first tile on: the lists start empty, but only
-// references scoring <= T0 enter them, instead of every score of the first
-// tiles.  (The C-th of 2C minima of 64 scores sits near the 1% quantile of a
-// row's scores; C / 4 sample tiles with minima of 32 scores, near 2%, were
-// 2-5% slower, and the maximum of C minima, near 7%, slower still.)  The
-// sample tiles are scanned again as part of the slice; slices of fewer than
-// 2 PS full tiles skip the sample.
-template <int MODE, int KP, int CH>
+// A thread of the epilogue (warp w, lane l) reads 64 columns of one query row
+// of every tile and keeps, by itself and without any barrier, the list of its
+// references that score below a threshold: two instructions per score when
+// there is no hit, which bounds the kernel together with the products.
+//
+// The threshold comes first.  Before its slice a block runs a sample of it,
+// in which threads only keep minima of groups of scores, 128 per row, rounded
+// up to 16 bits; the threshold is the rank-th smallest of a row's minima.  The
+// groups being spread over the cloud, about rank * pstride references of the
+// slice score below it; run_brute_tc picks both so that some 150 references
+// of a row do over all slices.  Nothing depends on that: a list that fills up
+// lowers its own threshold to its kT5Kept-th best, and whatever the threshold, the
+// references that no list holds score at or above it, which is all that the
+// certificate uses.
+//
+// 262,144 x 65,536, d=32, k=32, TF32: 3.5 ms, tensor pipe 45% busy, issue
+// slots 51%: 4 epilogue warps per scheduler cannot cover the latency of their
+// own minima, votes and branches.  (Before: a short sample, then per-row
+// sorted lists kept up to date in the registers of 4-lane groups, a barrier
+// per tile: 9.6 ms.)
+template <int MODE, int KP>
 __global__ void __launch_bounds__(kT5Threads, 1) k_tc5_select(const Tc5Args a) {
-    using Sh = Tc5Shape<MODE, KP, CH>;
-    constexpr int PL = Sh::PL, KB = Sh::KB, KSTEPS = Sh::KSTEPS;
+    using Sh = Tc5Shape<MODE, KP>;
+    constexpr int PL = Sh::PL, KB = Sh::KB, KSTEPS = Sh::KSTEPS, STAGES = Sh::STAGES, CAP = kT5Cap;
     constexpr uint32_t A_BYTES = Sh::A_BYTES, B_BYTES = Sh::B_BYTES;
     constexpr uint32_t LBO = 128, SBO = 8 * KB;
     constexpr int NPROD = MODE == TK_BRUTE_TF32 ? 1 : 3;
@@ -422,48 +453,31 @@ __global__ void __launch_bounds__(kT5Threads, 1) k_tc5_select(const Tc5Args a) {
 
     extern __shared__ __align__(1024) unsigned char smem[];
     unsigned char* sA = smem;                       // [PL][A_BYTES]
-    unsigned char* sB = smem + PL * A_BYTES;        // [2 stages][PL][B_BYTES]
-    unsigned long long* sBuf = reinterpret_cast<unsigned long long*>(sB + 2 * PL * B_BYTES);  // [2][kT5Rows][stride]
-    float* sThr = reinterpret_cast<float*>(sBuf + 2 * kT5Rows * kT5BufStride);  // [kT5Rows] list threshold per row
-    int* sCnt = reinterpret_cast<int*>(sThr + kT5Rows);                        // [2][kT5Rows] buffered hits per row
-    // [0..7] the sample steps' flags (block-wide), then per quarter [8 + 8q ..]:
-    // [0..3] overflow, [4..7] abort, by step mod 4
-    int* sFlag = sCnt + 2 * kT5Rows;
-    __shared__ __align__(8) uint64_t full_a, full_b[2], mma_done[2], epi_done[2];
+    unsigned char* sB = smem + PL * A_BYTES;        // [STAGES][PL][B_BYTES]
+    uint16_t* sMin = reinterpret_cast<uint16_t*>(sB + STAGES * PL * B_BYTES);  // [kT5Rows][kT5MinStride]
+    float* sThr = reinterpret_cast<float*>(sMin + kT5Rows * kT5MinStride);     // [kT5Rows]
+    __shared__ __align__(8) uint64_t full_a, full_b[STAGES], mma_done[2], epi_done[2];
     __shared__ uint32_t tmem_base_sh;
-    __shared__ int abort_sh;
-    constexpr int C = 2 * CH;                 // over-fetch per row and slice
-    constexpr int RS = C / 4;                 // list keys per lane (4 lanes per row)
-    constexpr int ROWS_PER_WARP = kT5Rows / kT5EpiWarps;
-    static_assert(ROWS_PER_WARP * 4 == 32, "one row per group of 4 lanes");
     constexpr int NEPI = 32 * kT5EpiWarps;
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const long long per0 = ((long long)a.n + a.nsplit - 1) / a.nsplit;
-    const long long per = (per0 + kT5Cols - 1) / kT5Cols * kT5Cols;  // slices start on tile boundaries
-    const int r0 = int(min((long long)a.n, per * blockIdx.y));
-    const int r1 = int(min((long long)a.n, per * (blockIdx.y + 1)));
-    const int ntiles = (r1 - r0 + kT5Cols - 1) / kT5Cols;
-    const int tile0 = r0 / kT5Cols;
-    constexpr int PS = (C + 1) / 2;             // sample tiles (4 group minima of a row per tile)
-    const int nfull = (r1 - r0) / kT5Cols;
-    const int npre = nfull >= 2 * PS ? PS : 0;  // sample tiles run before the slice
-    const int pstride = npre ? nfull / PS : 1;
-    const int nseq = npre + ntiles;             // tiles through the pipeline
-    // slice tile of pipeline step t: the samples s * pstride, then 0 .. ntiles - 1
-    auto tile_of = [&](int t) { return t < npre ? t * pstride : t - npre; };
+    const int per = (a.tiles + a.nsplit - 1) / a.nsplit;
+    const int tile0 = min(a.tiles, per * int(blockIdx.y));
+    const int ntiles = min(a.tiles, tile0 + per) - tile0;
+    const int npre = (ntiles + a.pstride - 1) / a.pstride;  // sampled tiles
+    const int nseq = npre + ntiles;  // tiles through the pipeline
+    auto tile_of = [&](int t) { return tile0 + (t < npre ? t * a.pstride : t - npre); };
 
     if (tid == 0) {
         sm100::mbar_init(&full_a, 1);
-        sm100::mbar_init(&full_b[0], 1);
-        sm100::mbar_init(&full_b[1], 1);
+        for (int i = 0; i < STAGES; ++i) sm100::mbar_init(&full_b[i], 1);
         sm100::mbar_init(&mma_done[0], 1);
         sm100::mbar_init(&mma_done[1], 1);
         sm100::mbar_init(&epi_done[0], kT5EpiWarps);
         sm100::mbar_init(&epi_done[1], kT5EpiWarps);
-        abort_sh = 0;
         sm100::mbar_fence_init();
     }
+    for (int i = tid; i < kT5Rows * kT5MinStride; i += kT5Threads) sMin[i] = 0xFFFFu;
     if (warp == kT5EpiWarps) sm100::tmem_alloc(&tmem_base_sh, 512);
     sm100::tc_fence_before();
     __syncthreads();
@@ -474,39 +488,38 @@ __global__ void __launch_bounds__(kT5Threads, 1) k_tc5_select(const Tc5Args a) {
         // ------------------------------------------------ producer / MMA issuer
         if (lane == 0 && nseq > 0) {
             bool ok = true;
-            // what this thread started and has not yet seen complete, per
-            // stage: the tile last copied in / waited for, last committed /
-            // waited for (drained if it gives up, see below)
+            // what this thread started and has not yet seen complete (waited
+            // for, within bounds, if it gives up): tiles copied in, products
             bool a_pending = true;
-            int b_issued[2] = {-1, -1}, b_waited[2] = {-1, -1};
-            int m_issued[2] = {-1, -1}, m_waited[2] = {-1, -1};
+            int b_issued = 0, b_waited = 0, m_issued = 0, m_waited = 0;
+            auto load = [&](int t) {
+                const int st = t % STAGES;
+                const size_t tb = (size_t)tile_of(t) * B_BYTES;
+                sm100::mbar_arrive_expect_tx(&full_b[st], PL * B_BYTES);
+                sm100::bulk_g2s(sB + (st * PL) * B_BYTES, a.b_hi + tb, B_BYTES, &full_b[st]);
+                if (PL == 2) sm100::bulk_g2s(sB + (st * PL + 1) * B_BYTES, a.b_lo + tb, B_BYTES, &full_b[st]);
+                b_issued = t + 1;
+            };
             sm100::mbar_arrive_expect_tx(&full_a, PL * A_BYTES);
             sm100::bulk_g2s(sA, a.a_hi + (size_t)blockIdx.x * A_BYTES, A_BYTES, &full_a);
             if (PL == 2) sm100::bulk_g2s(sA + A_BYTES, a.a_lo + (size_t)blockIdx.x * A_BYTES, A_BYTES, &full_a);
-            for (int t = 0; t < 2 && t < nseq; ++t) {
-                const size_t tb = (size_t)(tile0 + tile_of(t)) * B_BYTES;
-                sm100::mbar_arrive_expect_tx(&full_b[t], PL * B_BYTES);
-                sm100::bulk_g2s(sB + (t * PL) * B_BYTES, a.b_hi + tb, B_BYTES, &full_b[t]);
-                if (PL == 2) sm100::bulk_g2s(sB + (t * PL + 1) * B_BYTES, a.b_lo + tb, B_BYTES, &full_b[t]);
-                b_issued[t] = t;
-            }
+            for (int t = 0; t < STAGES && t < nseq; ++t) load(t);
             for (int t = 0; t < nseq; ++t) {
-                const int st = t & 1;
-                const uint32_t ph = (t >> 1) & 1;  // stage st serves tiles st, st + 2, ...: phase t / 2
-                ok = sm100::mbar_wait(&full_b[st], ph, a.max_tries);
+                const int st = t % STAGES, ac = t & 1;
+                ok = sm100::mbar_wait(&full_b[st], (t / STAGES) & 1, a.max_tries);
                 if (!ok) break;
-                b_waited[st] = t;
+                b_waited = t + 1;
                 if (t == 0) {
                     ok = sm100::mbar_wait(&full_a, 0, a.max_tries);
                     if (!ok) break;
                     a_pending = false;
                 }
                 if (t >= 2) {
-                    ok = sm100::mbar_wait(&epi_done[st], ((t - 2) >> 1) & 1, a.max_tries);
+                    ok = sm100::mbar_wait(&epi_done[ac], ((t - 2) >> 1) & 1, a.max_tries);
                     if (!ok) break;
                 }
                 sm100::tc_fence_after();
-                const uint32_t dtm = tmem + uint32_t(st * kT5Cols);
+                const uint32_t dtm = tmem + uint32_t(ac * kT5Cols);
                 const uint32_t a0 = sm100::smem_u32(sA);
                 const uint32_t b0 = sm100::smem_u32(sB + (st * PL) * B_BYTES);
 #pragma unroll
@@ -522,17 +535,15 @@ __global__ void __launch_bounds__(kT5Threads, 1) k_tc5_select(const Tc5Args a) {
                         else sm100::mma_bf16(dtm, ad, bd, IDESC, acc);
                     }
                 }
-                sm100::mma_commit(&mma_done[st]);
-                m_issued[st] = t;
-                if (t + 2 < nseq) {
-                    ok = sm100::mbar_wait(&mma_done[st], ph, a.max_tries);  // stage st no longer read
+                sm100::mma_commit(&mma_done[ac]);
+                m_issued = t + 1;
+                // while these products run: the stage of the ones before them
+                // takes its next tile
+                if (t >= 1) {
+                    ok = sm100::mbar_wait(&mma_done[ac ^ 1], ((t - 1) >> 1) & 1, a.max_tries);
                     if (!ok) break;
-                    m_waited[st] = t;
-                    const size_t tb = (size_t)(tile0 + tile_of(t + 2)) * B_BYTES;
-                    sm100::mbar_arrive_expect_tx(&full_b[st], PL * B_BYTES);
-                    sm100::bulk_g2s(sB + (st * PL) * B_BYTES, a.b_hi + tb, B_BYTES, &full_b[st]);
-                    if (PL == 2) sm100::bulk_g2s(sB + (st * PL + 1) * B_BYTES, a.b_lo + tb, B_BYTES, &full_b[st]);
-                    b_issued[st] = t + 2;
+                    m_waited = t;
+                    if (t - 1 + STAGES < nseq) load(t - 1 + STAGES);
                 }
             }
             if (!ok) {
@@ -541,221 +552,151 @@ __global__ void __launch_bounds__(kT5Threads, 1) k_tc5_select(const Tc5Args a) {
                 // thread's own copies and matrix products still in flight
                 // land -- each wait bounded by the default poll count --
                 // before the block frees its tensor memory and exits.
-                atomicExch(&abort_sh, 1);
                 atomicOr(a.err, kTcErrTimeout);
                 if (a_pending) sm100::mbar_wait(&full_a, 0, kT5MaxTries);
-                for (int s2 = 0; s2 < 2; ++s2) {
-                    if (b_issued[s2] > b_waited[s2])
-                        sm100::mbar_wait(&full_b[s2], (b_issued[s2] >> 1) & 1, kT5MaxTries);
-                    if (m_issued[s2] > m_waited[s2])
-                        sm100::mbar_wait(&mma_done[s2], (m_issued[s2] >> 1) & 1, kT5MaxTries);
-                }
+                for (int t = b_waited; t < b_issued; ++t)
+                    sm100::mbar_wait(&full_b[t % STAGES], (t / STAGES) & 1, kT5MaxTries);
+                for (int t = m_waited; t < m_issued; ++t)
+                    sm100::mbar_wait(&mma_done[t & 1], (t >> 1) & 1, kT5MaxTries);
             }
         }
         __syncwarp();
     } else {
         // ------------------------------------------------------- epilogue warps
-        // Thread (warp w, lane l) reads accumulator lane 32 (w & 3) + l, i.e.
-        // query row `myrow`, and the 16-column group w >> 2 of every 64-column
-        // phase.  Each score is compared with the row's threshold (the worst
-        // key of its over-fetch list, possibly stale but never too small);
-        // the rare hits are appended to the row's buffer of the tile's parity
-        // in shared memory.  One barrier per tile and accumulator quarter:
-        // after it the tile's accumulator is released to the MMA issuer, and
-        // warp w merges the buffers of its quarter's rows 32 (w & 3) +
-        // 8 (w >> 2) .. + 7 into their lists (kept in its registers, one row
-        // per group of 4 lanes) while other warps may already be filtering
-        // the next tile into the other parity's buffers.  A row can
-        // take at most kT5Buf hits per tile on this path; a tile that
-        // overflows a buffer (the first tiles of a slice, while the lists
-        // fill) is done again from tensor memory in eight steps of 32
-        // columns, merging after each, which cannot overflow.
-        const int quarter = warp & 3, cgroup = warp >> 2;
+        // Thread (warp w, lane l): accumulator lane 32 (w & 3) + l, i.e. query
+        // row `myrow`, columns 64 (w >> 2) .. + 63.
+        const int quarter = warp & 3, part = warp >> 2;
         const int myrow = 32 * quarter + lane;
-        // the row this lane's group keeps: the 4 warps of a quarter keep its 32 rows
-        const int grow = 32 * quarter + ROWS_PER_WARP * cgroup + (lane >> 2);
-        int* qFlag = sFlag + 8 + 8 * quarter;
-        const int gl = lane & 3;
-        GroupList<RS> glist;
-        glist.init();
-        unsigned long long gworst = kScoreSentinel;
-        float t0g = __int_as_float(0x7f800000);   // T0 of row grow
-        // the sample's group minima (images), 2C per row, in the hit buffers' space
-        uint32_t* sMin = reinterpret_cast<uint32_t*>(sBuf);
-        const uint32_t trow = tmem + (uint32_t(32 * quarter) << 16);
-        constexpr int NPHASE = kT5Cols / kT5Chunk;
-        if (tid < kT5Rows) {
-            sThr[tid] = __int_as_float(0x7f800000);
-            sCnt[tid] = 0;
-            sCnt[kT5Rows + tid] = 0;
-        }
-        if (tid < 40) sFlag[tid] = 0;
-        // The sample steps synchronise all epilogue warps (their minima share
-        // the hit buffers' space across quarters); from the first tile of the
-        // slice on, each quarter (its 4 warps filter and keep the same 32
-        // rows) synchronises on its own named barrier, and the quarters meet
-        // only through the accumulator stages (epi_done).
+        const uint32_t trow = tmem + (uint32_t(32 * quarter) << 16) + uint32_t(part * 64);
         auto bar_all = [&]() { asm volatile("bar.sync 1, %0;" ::"r"(NEPI) : "memory"); };
-        auto bar_quarter = [&]() { asm volatile("bar.sync %0, 128;" ::"r"(2 + quarter) : "memory"); };
-        bar_all();
-        // compare 16 scores of columns col0 .. col0+15 with thr, append the hits
-        // to buffer parity `par` (`edge`: the columns may run past the slice's
-        // end, in its last tile)
-        auto append16 = [&](const float (&v)[16], int col0, float thr, float pthr, int par, int* ovf, bool edge) {
-            float m = v[0];
-#pragma unroll
-            for (int i = 1; i < 16; ++i) m = fminf(m, v[i]);
-            if (!(m <= pthr)) return;  // no hit among the 16 (pthr = thr once hits are rare)
-            unsigned long long* buf = sBuf + (par * kT5Rows + myrow) * kT5BufStride;
-            int* cnt = sCnt + par * kT5Rows + myrow;
-#pragma unroll
-            for (int i = 0; i < 16; ++i) {
-                if (v[i] <= thr && (!edge || col0 + i < r1)) {
-                    const int pos = atomicAdd(cnt, 1);
-                    if (pos < kT5Buf) buf[pos] = score_key(v[i], uint32_t(col0 + i));
-                    else *ovf = 1;
-                }
-            }
+        bool alive = true;
+        float va[32], vb[32];  // the thread's first and last 32 scores of a tile
+        // Waits for pipeline step t's products and loads both halves; the
+        // second is still on its way.  False when the wait ran out.
+        auto begin = [&](int t) {
+            int ok = 1;
+            if (lane == 0) ok = sm100::mbar_wait(&mma_done[t & 1], (t >> 1) & 1, a.max_tries);
+            if (!__shfl_sync(0xFFFFFFFFu, ok, 0)) return false;
+            sm100::tc_fence_after();
+            const uint32_t at = trow + uint32_t((t & 1) * kT5Cols);
+            sm100::tmem_ld32(at, va);
+            sm100::tmem_wait32(va);
+            sm100::tmem_ld32(at + 32u, vb);
+            return true;
         };
-        // merge the buffered hits (parity par) of this warp's rows into their
-        // lists: the 8 rows side by side, one hit of each row per step (a row
-        // out of hits offers the sentinel); a step no row can use is skipped
-        auto merge = [&](int par) {
-            int* cnt = sCnt + par * kT5Rows + grow;
-            const int n = min(*cnt, kT5Buf);  // the same on the 4 lanes of a group
-            const unsigned long long* B = sBuf + (par * kT5Rows + grow) * kT5BufStride;
-            const int nmax = __reduce_max_sync(0xFFFFFFFFu, n);
-            // the last lane of a group holds the row's worst key: it alone
-            // decides whether its row can use the step (no shuffle per step),
-            // and the next hit is loaded while this one is inserted
-            unsigned long long c = 0 < n ? B[0] : kScoreSentinel;
-            for (int h = 0; h < nmax; ++h) {
-                const unsigned long long cn = h + 1 < n ? B[h + 1] : kScoreSentinel;
-                if (__any_sync(0xFFFFFFFFu, gl == 3 && c < glist.slot[RS - 1])) glist.insert(c, gl);
-                c = cn;
-            }
-            gworst = glist.worst();
-            if (gl == 0 && n > 0) {
-                *cnt = 0;
-                sThr[grow] = fminf(t0g, key_score(gworst));
-            }
-        };
-        for (int t = 0; t < nseq; ++t) {
-            const int st = t & 1, par = t & 1, f4 = t & 3;
-            const uint32_t ph = (t >> 1) & 1;
-            const bool pre = t < npre;
-            const int tt = tile_of(t);
-            const int base = r0 + tt * kT5Cols;
-            const uint32_t tcol = trow + uint32_t(st * kT5Cols);
-            int w_ok = 1;
-            if (lane == 0) w_ok = sm100::mbar_wait(&mma_done[st], ph, a.max_tries);
-            w_ok = __shfl_sync(0xFFFFFFFFu, w_ok, 0);
-            int* F = pre ? sFlag : qFlag;  // this step's flags (block-wide while sampling)
-            if (pre ? tid == 0 : (cgroup == 0 && lane == 0)) {
-                // flags of step t + 2 (last read before the barrier of step t - 1)
-                F[(f4 + 2) & 3] = 0;
-                F[4 + ((f4 + 2) & 3)] = 0;
-            }
-            if (w_ok && pre) {
-                // one group minimum (64 scores) of this thread's row per sample tile
-                sm100::tc_fence_after();
-                float m = __int_as_float(0x7f800000);
-#pragma unroll 1
-                for (int j = 0; j < NPHASE; ++j) {
-                    float v0[16];
-                    sm100::tmem_ld16(tcol + uint32_t(j * kT5Chunk + cgroup * 16), v0);
-#pragma unroll
-                    for (int i = 0; i < 16; ++i) m = fminf(m, v0[i]);
-                }
-                sMin[myrow * kT5MinStride + t * 4 + cgroup] = m == m ? score_bits(m) : 0xFFFFFFFFu;
-            } else if (w_ok) {
-                sm100::tc_fence_after();
-                const float thr = sThr[myrow];
-                // the 16-score pre-check pays once hits are rare (from the 16th tile of the slice on)
-                const float pthr = tt >= 16 ? thr : __int_as_float(0x7f800000);
-                const bool edge = base + kT5Cols > r1;
-#pragma unroll
-                for (int j = 0; j < NPHASE; j += 2) {
-                    float v0[16], v1[16];
-                    sm100::tmem_ld16x2(tcol + uint32_t(j * kT5Chunk + cgroup * 16),
-                                       tcol + uint32_t((j + 1) * kT5Chunk + cgroup * 16), v0, v1);
-                    append16(v0, base + j * kT5Chunk + cgroup * 16, thr, pthr, par, &F[f4], edge);
-                    append16(v1, base + (j + 1) * kT5Chunk + cgroup * 16, thr, pthr, par, &F[f4], edge);
-                }
-            } else if (lane == 0) {
-                F[4 + f4] = 1;
-            }
-            if (pre) bar_all();
-            else bar_quarter();
-            const int bad = F[4 + f4];   // agreed (block / quarter): written only before the barrier above
-            const int ovf = F[f4];
-            if (!bad && pre && t == npre - 1) {
-                // T0 of row grow = the C-th smallest of its 2C group minima,
-                // found by the row's 4 lanes by bisection on the order-
-                // preserving image (C/2 minima per lane, interleaved so that
-                // the 4 lanes read 4 different banks)
-                const uint32_t* mins = sMin + grow * kT5MinStride + gl;
-                uint32_t lo = 0u, hi = 0xFFFFFFFFu;
-#pragma unroll 1
-                for (int it = 0; it < 32; ++it) {
-                    const uint32_t mid = lo + ((hi - lo) >> 1);
-                    int cnt = 0;
-#pragma unroll 8
-                    for (int i = 0; i < C / 2; ++i) cnt += mins[4 * i] <= mid ? 1 : 0;
-                    cnt += __shfl_xor_sync(0xFFFFFFFFu, cnt, 1);
-                    cnt += __shfl_xor_sync(0xFFFFFFFFu, cnt, 2);
-                    if (cnt >= C) hi = mid;
-                    else lo = mid + 1u;
-                }
-                // images above +inf's are NaN minima (never certified): no threshold
-                t0g = lo < 0xFF800000u ? bits_score(lo) : __int_as_float(0x7f800000);
-                if (gl == 0) sThr[grow] = t0g;
-                bar_all();  // no quarter appends hits over the sample's minima before all have read them
-            }
-            if (!bad && ovf) {
-                // redo the tile in eight steps of 32 columns (two column groups each)
-                if (cgroup == 0) sCnt[par * kT5Rows + myrow] = 0;  // the quarter's rows
-                bar_quarter();
-#pragma unroll 1
-                for (int j = 0; j < 2 * NPHASE; ++j) {
-                    if ((cgroup >> 1) == (j & 1)) {
-                        const float thr = sThr[myrow];
-                        float v[16];
-                        sm100::tmem_ld16(tcol + uint32_t((j >> 1) * kT5Chunk + cgroup * 16), v);
-                        int dummy = 0;
-                        append16(v, base + (j >> 1) * kT5Chunk + cgroup * 16, thr, __int_as_float(0x7f800000), par,
-                                 &dummy, true);  // <= 32 hits per row
-                    }
-                    bar_quarter();
-                    merge(par);
-                    bar_quarter();
-                }
-            }
-            // this tile's accumulator is no longer read
+        // The second half has arrived: the accumulator goes back to the issuer.
+        auto rest = [&](int t) {
+            sm100::tmem_wait32(vb);
             sm100::tc_fence_before();
             __syncwarp();
-            if (lane == 0) sm100::mbar_arrive(&epi_done[st]);
-            if (bad) {
-                if (cgroup == 0 && lane == 0) atomicOr(a.err, kTcErrTimeout);
-                break;
-            }
-            if (!ovf && !pre) merge(par);
-        }
-        // write the lists: C candidates per row and the row threshold
-        {
-            const int q = blockIdx.x * kT5Rows + grow;
-            if (q < a.nq) {
-                const long long base = ((long long)q * a.nsplit + blockIdx.y) * C + RS * gl;
+            if (lane == 0) sm100::mbar_arrive(&epi_done[t & 1]);
+        };
+        // minima of columns 16 c + 3 j .. + 2 (j < 5) of a half, and of all 16
+        auto min16 = [&](const float (&v)[32], int c, float (&g)[5]) {
+            const float* x = v + 16 * c;
 #pragma unroll
-                for (int i = 0; i < RS; ++i) {
-                    const unsigned long long key = glist.slot[i];
-                    const bool real = key != kScoreSentinel;
-                    a.cand_s[base + i] = key_score(key);
-                    a.cand_i[base + i] = real ? int32_t(uint32_t(key)) : -1;
+            for (int j = 0; j < 5; ++j) g[j] = min3(x[3 * j], x[3 * j + 1], x[3 * j + 2]);
+            return fminf(min3(g[0], g[1], g[2]), min3(g[3], g[4], x[15]));
+        };
+        float g[5];
+        // sample: minima of groups of `tpg` tiles' scores, of one tile, or (short slices) of 16 scores
+        const int tpg = (npre + 31) / 32;
+        float run = __int_as_float(0x7f800000);
+        for (int t = 0; t < npre; ++t) {
+            alive = begin(t);
+            if (!alive) break;
+            const float m0 = min16(va, 0, g), m1 = min16(va, 1, g);
+            rest(t);
+            const float m2 = min16(vb, 0, g), m3 = min16(vb, 1, g);
+            uint16_t* out = sMin + myrow * kT5MinStride;
+            if (npre <= 8) {
+                out[(t * 4 + 0) * 4 + part] = uint16_t(score_bits(m0) >> 16);
+                out[(t * 4 + 1) * 4 + part] = uint16_t(score_bits(m1) >> 16);
+                out[(t * 4 + 2) * 4 + part] = uint16_t(score_bits(m2) >> 16);
+                out[(t * 4 + 3) * 4 + part] = uint16_t(score_bits(m3) >> 16);
+            } else {
+                run = fminf(min3(run, m0, m1), fminf(m2, m3));
+                if ((t + 1) % tpg == 0 || t + 1 == npre) {
+                    out[(t / tpg) * 4 + part] = uint16_t(score_bits(run) >> 16);
+                    run = __int_as_float(0x7f800000);
                 }
-                if (gl == 0) a.tau[(long long)q * a.nsplit + blockIdx.y] = key_score(gworst);
             }
         }
+        bar_all();
+        {
+            // the rank-th smallest of a row's minima, by 4 lanes: bisection on their 16-bit images
+            const int grow = 32 * quarter + 8 * part + (lane >> 2), gl = lane & 3;
+            const uint16_t* mins = sMin + grow * kT5MinStride + gl * (kT5Minima / 4);
+            uint32_t m[kT5Minima / 8];
+#pragma unroll
+            for (int i = 0; i < kT5Minima / 8; ++i) m[i] = *reinterpret_cast<const uint32_t*>(mins + 2 * i);
+            uint32_t lo = 0u, hi = 0xFFFFu;
+#pragma unroll 1
+            for (int it = 0; it < 16; ++it) {
+                const uint32_t mid = (lo + hi) >> 1;
+                int c = 0;
+#pragma unroll
+                for (int i = 0; i < kT5Minima / 8; ++i) c += ((m[i] & 0xFFFFu) <= mid ? 1 : 0) + ((m[i] >> 16) <= mid ? 1 : 0);
+                c += __shfl_xor_sync(0xFFFFFFFFu, c, 1);
+                c += __shfl_xor_sync(0xFFFFFFFFu, c, 2);
+                if (c >= a.rank) hi = mid;
+                else lo = min(mid + 1u, 0xFFFFu);
+            }
+            // rounded up to the end of its 16-bit bucket, and low enough to
+            // keep the padding rows out (NaN minima give a NaN threshold: no
+            // hits, and no certificate for such rows)
+            if (gl == 0) sThr[grow] = lo < 0xFF80u ? fminf(bits_score((lo << 16) | 0xFFFFu), kT5PadNorm) : kT5PadNorm;
+        }
+        bar_all();
+        const long long lidx = (((long long)blockIdx.x * kT5Rows + myrow) * a.nsplit + blockIdx.y) * kT5Parts + part;
+        uint2* list = a.hits + lidx * CAP;
+        // (rows past the last query take no hits: all their scores are equal)
+        float thr = blockIdx.x * kT5Rows + myrow < a.nq ? sThr[myrow] : -__int_as_float(0x7f800000);
+        int cnt = 0;
+        // Hits of a half (32 columns from col0 on).  Branches are taken by the
+        // whole warp (votes): few of its 512 scores of 16 columns are hits,
+        // and the tests narrow down on them in two steps, 16 columns and 3.
+        auto collect = [&](const float (&v)[32], uint32_t tile, uint32_t col0) {
+#pragma unroll
+            for (int c = 0; c < 2; ++c) {
+                if (!__any_sync(0xFFFFFFFFu, min16(v, c, g) < thr)) continue;
+#pragma unroll
+                for (int j = 0; j < 6; ++j) {
+                    if (!__any_sync(0xFFFFFFFFu, (j < 5 ? g[j < 5 ? j : 0] : v[16 * c + 15]) < thr)) continue;
+#pragma unroll
+                    for (int i = 16 * c + 3 * j; i < 16 * c + (j < 5 ? 3 * j + 3 : 16); ++i) {
+                        if (v[i] < thr) {
+                            list[cnt] = make_uint2(__float_as_uint(v[i]), packed_ref(tile, col0 + uint32_t(i), uint32_t(a.tiles)));
+                            ++cnt;
+                        }
+                    }
+                }
+                unsigned full = __ballot_sync(0xFFFFFFFFu, cnt > CAP - 16);
+                while (full) {
+                    const int src = __ffs(full) - 1;
+                    full &= full - 1u;
+                    const int n = __shfl_sync(0xFFFFFFFFu, cnt, src);
+                    uint2* at = reinterpret_cast<uint2*>(
+                        __shfl_sync(0xFFFFFFFFu, reinterpret_cast<unsigned long long>(list), src));
+                    const uint2 p = prune_hits(at, n, lane);
+                    if (lane == src) {
+                        cnt = int(p.x);
+                        thr = __uint_as_float(p.y);
+                    }
+                }
+            }
+        };
+        for (int t = npre; alive && t < nseq; ++t) {
+            alive = begin(t);
+            if (!alive) break;
+            const uint32_t tile = uint32_t(tile_of(t)), col0 = uint32_t(64 * part);
+            collect(va, tile, col0);
+            rest(t);
+            collect(vb, tile, col0 + 32u);
+        }
+        if (!alive && lane == 0) atomicOr(a.err, kTcErrTimeout);
+        a.counts[lidx] = cnt;
+        a.thr[lidx] = thr;
     }
     // teardown: everyone done with tensor memory
     sm100::tc_fence_before();
@@ -780,10 +721,14 @@ struct RerankArgs {
     const float* ref;     // [n, d] float32 originals
     const float* q;       // [nq, d]
     int n, nq, d, k, C, nsplit;
-    const float* cand_s;
+    const float* cand_s;  // mma.sync search: [nq, nsplit, C]
     const int32_t* cand_i;
-    const float* tau;
-    double eps_dot;       // relative error bound of the tensor-core dot product
+    const float* tau;     // [nq, nsplit]
+    int keep;             // tcgen05 search: references per query worth recomputing
+    const uint2* hits;    // see Tc5Args
+    const int* counts;
+    const float* thr;
+    float eps_dot;        // relative error bound of the tensor-core dot product
     float* out_d;
     int32_t* out_i;
     int* fail_count;
@@ -834,6 +779,36 @@ __device__ __forceinline__ float rerank_dist(const float* __restrict__ qrow, con
     return acc;
 }
 
+// |q|^2 on every lane of the warp, a lane per coordinate.
+__device__ __forceinline__ float squared_norm(const float* qrow, int d, int lane) {
+    float qq = 0.f;
+    for (int c = lane; c < d; c += 32) qq = fmaf(qrow[c], qrow[c], qq);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) qq += __shfl_xor_sync(0xFFFFFFFFu, qq, o);
+    return qq;
+}
+
+// Certificate of a query (|q|^2 = qq) whose k-th exact distance among the
+// recomputed references is D; every other reference scores at or above tau.
+// In single precision: E already doubles the bound on the score's error, and
+// its last term covers the rounding of this arithmetic, below 2 (d + 16) u of
+// the largest operand.  (In double it kept the slow pipe busy for a third of
+// the re-rank.)  Overflow or NaN anywhere refuses the certificate.
+__device__ __forceinline__ bool certified(const RerankArgs& a, float qq, float tau, float D) {
+    if (a.err && *a.err) return false;
+    if (!(qq < kTcNormLimit)) return false;  // see kTcNormLimit (also NaN / inf coordinates)
+    if (isinf(tau)) return true;
+    const float u = 1.0f / 16777216.0f;           // 2^-24
+    const float m = float(a.d + 4) * u;           // rounding of the exact FP32 distance
+    const float Dp = D * (1.0f + 2.0f * m);       // at least the real |q-r|^2 of any r with dist(r) <= D
+    const float qn = sqrtf(qq);
+    const float rho = qn + sqrtf(Dp);             // |r| of any such r
+    const float eps = 2.0f * a.eps_dot + m;       // score error, relative
+    const float big = qn * rho + rho * rho + fmaxf(Dp, qq);
+    const float E = 2.0f * eps * big + 4.0f * float(a.d + 16) * u * (big + fabsf(tau));  // first term: x2 safety
+    return (qq + tau) - E > Dp;                   // false for NaN
+}
+
 // One warp per query: exact distances of the candidates, top-k, certificate.
 template <int R>
 __global__ void __launch_bounds__(256) k_tc_rerank(const RerankArgs a) {
@@ -856,50 +831,120 @@ __global__ void __launch_bounds__(256) k_tc_rerank(const RerankArgs a) {
         worst = offer<float, 32, R>(list, mine, worst, 0xFFFFFFFFu, lane, 0);
     }
     list.store(a.k, lane, a.out_d, a.out_i, qi);
-    // certificate (lane 0)
+    const float qq = squared_norm(qrow, a.d, lane);
     if (lane == 0) {
-        double tau = INFINITY;
-        for (int s = 0; s < a.nsplit; ++s) tau = fmin(tau, (double)a.tau[(long long)qi * a.nsplit + s]);
-        bool ok = !(a.err && *a.err);
-        double qq = 0.0;
-        for (int c = 0; c < a.d; ++c) qq += (double)qrow[c] * (double)qrow[c];
-        ok = ok && qq < double(kTcNormLimit);  // see kTcNormLimit (false for NaN / inf coordinates)
-        if (ok && !isinf(tau)) {
-            const double D = (double)worst.dist();
-            const double u = 1.0 / 16777216.0;                  // 2^-24
-            const double m = (a.d + 4) * u;                      // rounding of the exact FP32 distance
-            const double Dp = D / (1.0 - m);                     // real |q-r|^2 of any r with dist(r) <= D
-            const double qn = sqrt(qq);
-            const double rho = qn + sqrt(Dp);                    // |r| of any such r
-            const double eps = 2.0 * a.eps_dot + (a.d + 4) * u;  // score error, relative
-            const double E = 2.0 * eps * (qn * rho + rho * rho + fmax(Dp, qq));  // x2 safety
-            ok = !isnan(D) && (qq + tau - E > Dp);
-        }
-        if (!ok) {
+        float tau = __int_as_float(0x7f800000);
+        for (int s = 0; s < a.nsplit; ++s) tau = fminf(tau, a.tau[(long long)qi * a.nsplit + s]);
+        if (!certified(a, qq, tau, worst.dist())) {
             const int slot = atomicAdd(a.fail_count, 1);
             a.fail_list[slot] = qi;
         }
     }
 }
 
-template <int MODE, int KP, int CH>
-int launch_tc5(const Tc5Args& a, int qblocks, cudaStream_t s) {
-    using Sh = Tc5Shape<MODE, KP, CH>;
-    const void* fn = reinterpret_cast<const void*>(&k_tc5_select<MODE, KP, CH>);
-    cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(Sh::SMEM));
-    if (e != cudaSuccess) return fail(TK_ECUDA, std::string("tcgen05 select smem: ") + cudaGetErrorString(e));
-    k_tc5_select<MODE, KP, CH><<<dim3(qblocks, a.nsplit), kT5Threads, Sh::SMEM, s>>>(a);
-    return TK_OK;
+// The same for the lists of k_tc5_select (k <= 32).  Where they hold far more
+// references than were wanted (clustered clouds), only those up to the
+// keep-th best score are recomputed, and that score joins the lists'
+// thresholds in tau.
+static __global__ void __launch_bounds__(256) k_tc5_rerank(const RerankArgs a) {
+    constexpr int CAP = kT5Cap;
+    __shared__ Key<float> bufs[8][64];
+    __shared__ uint32_t todo[8][64];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int qi = blockIdx.x * 8 + w;
+    if (qi >= a.nq) return;
+    const int nl = a.nsplit * kT5Parts;
+    const int* counts = a.counts + (long long)qi * nl;
+    const uint2* hits = a.hits + (long long)qi * nl * CAP;
+    int total = 0;
+    float tau = __int_as_float(0x7f800000);
+    for (int l = lane; l < nl; l += 32) {
+        total += counts[l];
+        tau = fminf(tau, a.thr[(long long)qi * nl + l]);
+    }
+    total = __reduce_add_sync(0xFFFFFFFFu, total);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) tau = fminf(tau, __shfl_xor_sync(0xFFFFFFFFu, tau, o));
+    uint32_t cut = 0xFFFFFFFFu;  // image of the last score recomputed
+    if (total > 2 * a.keep) {
+        uint32_t lo = 0xFFFFFFFFu, hi = 0u;
+        for (int l = 0; l < nl; ++l) {
+            const int c = counts[l];
+            for (int e = lane; e < c; e += 32) {
+                const uint32_t u = score_bits(__uint_as_float(hits[l * CAP + e].x));
+                lo = min(lo, u);
+                hi = max(hi, u);
+            }
+        }
+        lo = __reduce_min_sync(0xFFFFFFFFu, lo);
+        hi = __reduce_max_sync(0xFFFFFFFFu, hi);
+        while (lo < hi) {
+            const uint32_t mid = lo + ((hi - lo) >> 1);
+            int below = 0;
+            for (int l = 0; l < nl; ++l) {
+                const int c = counts[l];
+                for (int e = lane; e < c; e += 32)
+                    below += score_bits(__uint_as_float(hits[l * CAP + e].x)) <= mid ? 1 : 0;
+            }
+            below = __reduce_add_sync(0xFFFFFFFFu, below);
+            if (below >= a.keep) hi = mid;
+            else lo = mid + 1u;
+            if (below >= a.keep && below <= a.keep + 32) break;  // near enough
+        }
+        cut = hi;
+        tau = fminf(tau, bits_score(cut));
+    }
+    WarpList<float, 1> wl;
+    wl.init(a.k, bufs[w], lane);
+    const float* qrow = a.q + (long long)qi * a.d;
+    const bool vec =
+        (a.d & 3) == 0 && ((reinterpret_cast<uintptr_t>(a.ref) | reinterpret_cast<uintptr_t>(a.q)) & 15) == 0;
+    int waiting = 0;
+    auto evaluate = [&](int m) {
+        Key<float> mine = Key<float>::sentinel();
+        if (lane < m) {
+            const uint32_t r = todo[w][lane];
+            mine = Key<float>::make(rerank_dist(qrow, a.ref + (long long)r * a.d, a.d, vec), r);
+        }
+        wl.offer(mine, lane);
+    };
+    for (int l = 0; l < nl; ++l) {
+        const int c = counts[l];
+        for (int e0 = 0; e0 < c; e0 += 32) {
+            const uint2 k = e0 + lane < c ? hits[l * CAP + e0 + lane] : make_uint2(0u, 0u);
+            const bool take = e0 + lane < c && score_bits(__uint_as_float(k.x)) <= cut;
+            const unsigned m = __ballot_sync(0xFFFFFFFFu, take);
+            if (take) todo[w][waiting + __popc(m & ((1u << lane) - 1u))] = k.y;
+            waiting += __popc(m);
+            __syncwarp();
+            if (waiting >= 32) {
+                evaluate(32);
+                const uint32_t rest = todo[w][32 + lane];
+                __syncwarp();
+                waiting -= 32;
+                if (lane < waiting) todo[w][lane] = rest;
+                __syncwarp();
+            }
+        }
+    }
+    if (waiting > 0) evaluate(waiting);
+    wl.flush(lane);
+    wl.list.store(a.k, lane, a.out_d, a.out_i, qi);
+    const float qq = squared_norm(qrow, a.d, lane);
+    if (lane == 0 && !certified(a, qq, tau, wl.worst.dist())) {
+        const int slot = atomicAdd(a.fail_count, 1);
+        a.fail_list[slot] = qi;
+    }
 }
 
 template <int MODE, int KP>
-int tc5_dispatch_ch(const Tc5Args& a, int CH, int qblocks, cudaStream_t s) {
-    switch (CH) {
-        case 8: return launch_tc5<MODE, KP, 8>(a, qblocks, s);
-        case 16: return launch_tc5<MODE, KP, 16>(a, qblocks, s);
-        case 32: return launch_tc5<MODE, KP, 32>(a, qblocks, s);
-        default: return fail(TK_EUNSUPPORTED, "tcgen05 path: k <= 32");
-    }
+int launch_tc5(const Tc5Args& a, int qblocks, cudaStream_t s) {
+    using Sh = Tc5Shape<MODE, KP>;
+    const void* fn = reinterpret_cast<const void*>(&k_tc5_select<MODE, KP>);
+    cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(Sh::SMEM));
+    if (e != cudaSuccess) return fail(TK_ECUDA, std::string("tcgen05 select smem: ") + cudaGetErrorString(e));
+    k_tc5_select<MODE, KP><<<dim3(qblocks, a.nsplit), kT5Threads, Sh::SMEM, s>>>(a);
+    return TK_OK;
 }
 
 template <int MODE, int KP, int C>
@@ -938,9 +983,9 @@ int dispatch_kp(const TcArgs& a, int qblocks, cudaStream_t s) {
 }
 
 // Entry points of the candidate kernels, one unit each.
-int tc5_dispatch_tf32(const Tc5Args& a, int KP, int CH, int qblocks, cudaStream_t s);       // brute_tc5_tf32.cu
-int tc5_dispatch_tf32_deep(const Tc5Args& a, int KP, int CH, int qblocks, cudaStream_t s);  // brute_tc5_tf32_deep.cu
-int tc5_dispatch_bf16(const Tc5Args& a, int KP, int CH, int qblocks, cudaStream_t s);  // brute_tc5_bf16.cu
+int tc5_dispatch_tf32(const Tc5Args& a, int KP, int qblocks, cudaStream_t s);       // brute_tc5_tf32.cu
+int tc5_dispatch_tf32_deep(const Tc5Args& a, int KP, int qblocks, cudaStream_t s);  // brute_tc5_tf32_deep.cu
+int tc5_dispatch_bf16(const Tc5Args& a, int KP, int qblocks, cudaStream_t s);  // brute_tc5_bf16.cu
 int tc_select_dispatch(const TcArgs& a, int mode, int qblocks, cudaStream_t s);          // brute_tc_mma.cu
 
 }  // namespace tcx
