@@ -236,3 +236,23 @@ def test_default_depth_tree(dtype, d, oracle, tmp_path):
                 bdd, bii = BatchedKDTrees([rt, rt], [k, 1], [len(q), 0]).query([qt, qt[:0]])
                 np.testing.assert_array_equal(bii[0].cpu().numpy(), bi)
                 np.testing.assert_array_equal(bdd[0].cpu().numpy(), bd)
+
+
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+@pytest.mark.parametrize("n", [4000, 5000, 100_000])
+def test_device_build_refuses_nan_at_every_size(dtype, n):
+    """NaN coordinates have a place in the sort order, so the passes stay inside
+    their arrays and the build ends with the error."""
+    import torch_kdtree_gb300 as tk
+    from torch_kdtree_gb300._lib import TK_EINVAL
+    rng = np.random.default_rng(n)
+    for share in (1, n // 3):
+        pts = rng.standard_normal((n, 3)).astype(dtype)
+        pts[rng.permutation(n)[:share], rng.integers(0, 3, share)] = np.nan
+        st, h = device_tree(pts, 9)
+        assert st == TK_EINVAL and not h.value
+        with pytest.raises(Exception, match="NaN"):
+            tk.build_kd_tree(torch.from_numpy(pts).to(cuda))
+    good = torch.randn(n, 3, device=cuda)
+    d, _ = tk.build_kd_tree(good).query(good[:100])
+    assert float(d.max()) == 0.0

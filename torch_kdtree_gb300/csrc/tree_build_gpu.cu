@@ -516,7 +516,10 @@ __global__ void __launch_bounds__(256) k_level_count(const T* __restrict__ pts, 
         if (p < n) {
             const NodeAt a = locate(n, s, int(p));
             const uint32_t id = pb[p], mid = pa[a.lo + (a.c >> 1)];
-            const T v = pts[int64_t(id) * dims + ax], m = pts[int64_t(mid) * dims + ax];
+            // by the sort's keys: exactly h of a node's points go left whatever
+            // the values (NaN compares false with everything; with it the
+            // places below would run past the node's range)
+            const auto v = coord_key(pts[int64_t(id) * dims + ax]), m = coord_key(pts[int64_t(mid) * dims + ax]);
             left = v < m || (v == m && id < mid);
         }
         const unsigned m = __ballot_sync(0xFFFFFFFFu, left);
