@@ -255,7 +255,9 @@ int tk_batch_query(const tk_batch* batch, const void* q, void* dists, int32_t* i
 typedef enum tk_brute_mode {
     TK_BRUTE_EXACT = 0,      /* CUDA cores, the reference's distance arithmetic (float or double) */
     TK_BRUTE_TF32 = 1,       /* q.r on tensor cores in TF32, over-fetch, exact FP32 re-rank */
-    TK_BRUTE_BF16_SPLIT = 2  /* q.r as BF16 hi/lo split products with FP32 accumulation, then exact re-rank */
+    TK_BRUTE_BF16_SPLIT = 2, /* q.r as BF16 hi/lo split products with FP32 accumulation, then exact re-rank */
+    TK_BRUTE_ROUTED = 3      /* whichever search is fastest for the sizes, any dtype, dims and k of TK_BRUTE_EXACT:
+                                CUDA cores, BF16 hi/lo, or (1-3 dims) a KD-tree that lives for the call */
 } tk_brute_mode;
 
 /* Bytes of device scratch tk_nn_distance needs. */
@@ -281,8 +283,8 @@ int tk_nn_distance(const void* ref, int64_t n, const void* q, int64_t nq, int di
  * shared memory would not fit a block).
  * The answer is exact in every case: an unfinished or uncertifiable
  * candidate search only sends its queries to the exact kernel.  Returns
- * TK_ETIMEOUT when bit 0 is set, else TK_OK; TK_BRUTE_EXACT calls report
- * zeros.  Replaces the reference's exit() on a device error
+ * TK_ETIMEOUT when bit 0 is set, else TK_OK; TK_BRUTE_EXACT and
+ * TK_BRUTE_ROUTED calls report zeros.  Replaces the reference's exit() on a device error
  * (src/cutils.cuh:34-43), which left the caller nothing to inspect. */
 int tk_nn_distance_report(const void* workspace, int64_t n, int64_t nq, int dims, int k, int dtype, int mode,
                           int* flags, int* recomputed);

@@ -344,3 +344,49 @@ def test_recomputed_queries(n_listed, k, oracle):
     dd, ii = tk().nn_distance(torch.from_numpy(ref).to(cuda), torch.from_numpy(q).to(cuda), k, mode="tf32")
     np.testing.assert_array_equal(dd.cpu().numpy(), bd)
     np.testing.assert_array_equal(ii.cpu().numpy(), bi)
+
+
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+@pytest.mark.parametrize("d", [1, 2, 3])
+@pytest.mark.parametrize("data", ["normal", "repeated", "grid", "nan", "inf"])
+def test_exact_mode_through_a_tree(dtype, d, data, oracle):
+    """Large calls in 1-3 dimensions build a tree for the call; clouds with NaN
+    or infinite coordinates are searched exhaustively after all."""
+    rng = np.random.default_rng(d)
+    n, nq = 20_011, 5_003
+    ref = rng.standard_normal((n, d)).astype(dtype)
+    q = rng.standard_normal((nq, d)).astype(dtype)
+    if data == "repeated":
+        ref = ref[rng.integers(0, 50, n)]
+    elif data == "grid":
+        ref, q = np.round(ref * 2), np.round(q * 2)
+    elif data == "nan":
+        ref[rng.integers(0, n, 3), rng.integers(0, d, 3)] = np.nan
+        q[7, 0] = np.nan
+    elif data == "inf":
+        ref[rng.integers(0, n, n // 2), 0] = np.inf
+        q[:3, 0] = (np.inf, -np.inf, np.nan)
+    rt, qt = torch.from_numpy(ref).to(cuda), torch.from_numpy(q).to(cuda)
+    for k in (1, 5, 17, 100):
+        bd, bi = oracle.brute(ref, q, k)
+        bi = np.where(bi == 2 ** 31 - 1, -1, bi)  # the oracle's mark of a NaN query's empty slots
+        dd, ii = tk().nn_distance(rt, qt, k)
+        np.testing.assert_array_equal(dd.cpu().numpy(), bd)
+        np.testing.assert_array_equal(ii.cpu().numpy(), bi)
+
+
+def test_exact_mode_captured_in_a_graph():
+    """Every route of the exact mode is device work only."""
+    for n, nq, d, k in ((30_000, 30_000, 3, 1), (4_000, 2_000, 16, 8), (300, 50, 3, 2)):
+        ref, q = torch.randn(n, d, device=cuda), torch.randn(nq, d, device=cuda)
+        want = tk().nn_distance(ref, q, k)
+        static_q = torch.zeros_like(q)
+        tk().nn_distance(ref, static_q, k)
+        torch.cuda.synchronize()
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g):
+            dd, ii = tk().nn_distance(ref, static_q, k)
+        static_q.copy_(q)
+        g.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(dd, want[0]) and torch.equal(ii, want[1])

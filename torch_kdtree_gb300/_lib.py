@@ -24,6 +24,7 @@ TK_F64 = 1
 TK_BRUTE_EXACT = 0
 TK_BRUTE_TF32 = 1
 TK_BRUTE_BF16_SPLIT = 2
+TK_BRUTE_ROUTED = 3
 TK_NOALLOC_MAX_QUERIES = 262144
 
 _STATUS_NAMES = {

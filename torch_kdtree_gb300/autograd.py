@@ -67,7 +67,7 @@ class BruteDistances(torch.autograd.Function):
         from .nn_distance import nn_distance_raw
         d = torch.empty((q.shape[0], k), dtype=q.dtype, device=q.device)
         i = torch.empty((q.shape[0], k), dtype=torch.int32, device=q.device)
-        nn_distance_raw(ref.detach(), q.detach(), k, d, i, mode)
+        nn_distance_raw(ref.detach(), q.detach(), k, d, i, mode, routed=True)
         ctx.save_for_backward(q, ref, i)
         ctx.mark_non_differentiable(i)
         return d, i

@@ -154,13 +154,13 @@ def autotune_brute(points_ref: torch.Tensor, points_query: torch.Tensor, k: int,
     ii = torch.empty(q.shape[0], k, dtype=torch.int32, device=ref.device)
     best, table = None, []
     for m in modes:
-        nn_distance_raw(ref, q, k, dd, ii, m)  # warm-up
+        nn_distance_raw(ref, q, k, dd, ii, m, routed=True)  # warm-up
         times = []
         for _ in range(reps):
             s = torch.cuda.Event(enable_timing=True)
             e = torch.cuda.Event(enable_timing=True)
             s.record()
-            nn_distance_raw(ref, q, k, dd, ii, m)
+            nn_distance_raw(ref, q, k, dd, ii, m, routed=True)
             e.record()
             e.synchronize()
             times.append(s.elapsed_time(e))

@@ -77,7 +77,7 @@ size_t brute_ws_bytes(const BrutePlan& p, int64_t nq, int k) {
 
 template <typename T>
 int run_brute(const T* ref, int64_t n, const T* q, int64_t nq, int d, int k, T* dists, int32_t* idx, void* ws,
-              size_t ws_bytes, cudaStream_t s) {
+              size_t ws_bytes, cudaStream_t s, const int* gate = nullptr) {
     const BrutePlan p = plan_brute(n, nq, d, k, sizeof(T) == 4);
     if (ws_bytes < brute_ws_bytes<T>(p, nq, k) || (p.nsplit > 1 && !ws))
         return fail(TK_EWORKSPACE, "workspace too small");
@@ -92,6 +92,7 @@ int run_brute(const T* ref, int64_t n, const T* q, int64_t nq, int d, int k, T* 
     a.out_d = dists;
     a.out_i = idx;
     a.part = static_cast<Key<T>*>(ws);
+    a.gate = gate;
     switch (p.DP) {
         case 1: return launch_dp<T, 1>(a, p, s);
         case 2: return launch_dp<T, 2>(a, p, s);
@@ -112,6 +113,60 @@ int run_brute(const T* ref, int64_t n, const T* q, int64_t nq, int d, int k, T* 
         return launch_brute_f64_wide(a, p, s);  // brute_f64.cu: d = 5 .. 128
     }
     return fail(TK_EUNSUPPORTED, "no brute-force kernel for this dimension");
+}
+
+// Route of a call that only wants the exact answer (TK_BRUTE_ROUTED).
+enum class Route { kCudaCores, kTensorCores, kTree };
+
+// Queries per pass over the tensor cores: bounds the workspace (4.6 KB of hit
+// lists per query and slice).
+constexpr int64_t kRoutePass = 262144;
+constexpr size_t kRouteBytes = size_t(4) << 30;
+
+// Up to three dimensions a tree that is built for the call pays from the
+// pairs on at which the comparisons cost more than its build (ms, exhaustive /
+// tree: 65,536 x 65,536, d=3, k=1 1.87 / 0.29; 20,000 x 20,000 k=1 0.22 / 0.21,
+// k=4 0.33 / 0.23, k=16 1.24 / 0.26; 65,536 x 2,000 k=4 0.18 / 0.23; float64
+// 10,000 x 10,000 3.4 / 0.28).  Otherwise the tensor-core search (BF16 hi/lo:
+// an error bound 60 times smaller than TF32's leaves hardly any query without
+// a certificate) beats the CUDA cores wherever it applies but for the smallest
+// calls, whose launches cost more than the work (ms, CUDA cores / tensor
+// cores: 262,144 x 65,536, k=32, d=32 69 / 4.7, d=8 30 / 3.8; 20,000 x 20,000,
+// d=8, k=1 0.44 / 0.45, k=8 1.02 / 0.45; 1,000 x 128, d=8, k=1 0.06 / 0.07,
+// k=8 0.11 / 0.07, d=32, k=8 0.17 / 0.07; d=3, k=4 1,000 x 1,000 0.08 / 0.07,
+// 10,000 x 10,000 0.19 / 0.18; k=1 0.13 / 0.18).
+Route route_of(int64_t n, int64_t nq, int d, int k, int dtype) {
+    const double pairs = double(n) * double(nq);
+    const bool narrow = d <= 3;
+    if (narrow && n >= 512) {
+        const double worth = dtype == TK_F64 ? 3e5 : (k == 1 ? 4e8 : (k < 8 ? 2.5e8 : 1e8));
+        if (pairs >= worth) return Route::kTree;
+    }
+    if (dtype != TK_F32 || d > 47 || k > 32 || n < 512 || pairs < 6e4) return Route::kCudaCores;
+    if (narrow && (k < 4 || (k < 8 && pairs > 5e7))) return Route::kCudaCores;
+    if (k < 4 && pairs < (d <= 8 ? 5e8 : 1e6)) return Route::kCudaCores;
+    if (brute_tc_workspace_bytes(n, std::min(nq, kRoutePass), d, k, TK_BRUTE_BF16_SPLIT) > kRouteBytes)
+        return Route::kCudaCores;
+    return Route::kTensorCores;
+}
+
+// Workspace of the tree route: the exhaustive search's (for clouds with NaN
+// or infinite coordinates), then the tree's.
+size_t exact_ws_bytes(int64_t n, int64_t nq, int d, int k, int dtype) {
+    const BrutePlan p = plan_brute(n, nq, d, k, dtype != TK_F64);
+    return dtype == TK_F64 ? brute_ws_bytes<double>(p, nq, k) : brute_ws_bytes<float>(p, nq, k);
+}
+
+template <typename T>
+int run_tree_route(const T* ref, int64_t n, const T* q, int64_t nq, int d, int k, int dtype, T* dists, int32_t* idx,
+                   char* ws, size_t ws_bytes, cudaStream_t s) {
+    const size_t eb = exact_ws_bytes(n, nq, d, k, dtype);
+    if (!ws || ws_bytes < eb + transient_tree_workspace_bytes(n, nq, d, k, dtype))
+        return fail(TK_EWORKSPACE, "workspace too small");
+    const int* odd = nullptr;
+    const int rc = transient_tree_query(ref, n, q, nq, d, k, dtype, dists, idx, ws + eb, s, &odd);
+    if (rc != TK_OK) return rc;
+    return run_brute<T>(ref, n, q, nq, d, k, dists, idx, ws, eb, s, odd + 1);
 }
 
 int check_common(const void* ref, int64_t n, const void* q, int64_t nq, int d, int k, int dtype, const void* dists,
@@ -297,9 +352,12 @@ extern "C" {
 size_t tk_nn_distance_workspace_size(int64_t n, int64_t nq, int dims, int k, int dtype, int mode) {
     if (n < 1 || nq < 0 || k < 1 || dims < 1) return 0;
     if (mode == TK_BRUTE_TF32 || mode == TK_BRUTE_BF16_SPLIT) return brute_tc_workspace_bytes(n, nq, dims, k, mode);
-    const BrutePlan p = plan_brute(n, std::max<int64_t>(nq, 1), dims, k, dtype != TK_F64);
-    return dtype == TK_F64 ? brute_ws_bytes<double>(p, std::max<int64_t>(nq, 1), k)
-                           : brute_ws_bytes<float>(p, std::max<int64_t>(nq, 1), k);
+    nq = std::max<int64_t>(nq, 1);
+    const Route route = mode == TK_BRUTE_ROUTED ? route_of(n, nq, dims, k, dtype) : Route::kCudaCores;
+    if (route == Route::kTensorCores)
+        return brute_tc_workspace_bytes(n, std::min(nq, kRoutePass), dims, k, TK_BRUTE_BF16_SPLIT);
+    return exact_ws_bytes(n, nq, dims, k, dtype) +
+           (route == Route::kTree ? transient_tree_workspace_bytes(n, nq, dims, k, dtype) : 0);
 }
 
 int tk_nn_distance(const void* ref, int64_t n, const void* q, int64_t nq, int dims, int k, int dtype, int mode,
@@ -310,7 +368,23 @@ int tk_nn_distance(const void* ref, int64_t n, const void* q, int64_t nq, int di
     if (nq == 0) return TK_OK;
     if (ws_misaligned(workspace)) return fail(TK_EINVAL, "workspace must be 256-byte aligned");
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    if (mode == TK_BRUTE_EXACT) {
+    const Route route = mode == TK_BRUTE_ROUTED ? route_of(n, nq, dims, k, dtype) : Route::kCudaCores;
+    if (route == Route::kTree) {
+        char* ws = static_cast<char*>(workspace);
+        if (dtype == TK_F32)
+            return run_tree_route<float>(static_cast<const float*>(ref), n, static_cast<const float*>(q), nq, dims, k,
+                                         dtype, static_cast<float*>(dists), idx, ws, workspace_bytes, s);
+        return run_tree_route<double>(static_cast<const double*>(ref), n, static_cast<const double*>(q), nq, dims, k,
+                                      dtype, static_cast<double*>(dists), idx, ws, workspace_bytes, s);
+    }
+    if (route == Route::kTensorCores) {
+        for (int64_t q0 = 0; q0 < nq && rc == TK_OK; q0 += kRoutePass)
+            rc = run_brute_tc(static_cast<const float*>(ref), n, static_cast<const float*>(q) + q0 * dims,
+                              std::min(kRoutePass, nq - q0), dims, k, TK_BRUTE_BF16_SPLIT,
+                              static_cast<float*>(dists) + q0 * k, idx + q0 * k, workspace, workspace_bytes, s);
+        return rc;
+    }
+    if (mode == TK_BRUTE_EXACT || mode == TK_BRUTE_ROUTED) {
         if (dtype == TK_F32)
             return run_brute<float>(static_cast<const float*>(ref), n, static_cast<const float*>(q), nq, dims, k,
                                     static_cast<float*>(dists), idx, workspace, workspace_bytes, s);

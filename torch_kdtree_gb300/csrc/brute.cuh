@@ -37,6 +37,7 @@ struct BruteArgs {
     // and results go to their rows (the caller merges the slices).
     const int* qlist = nullptr;
     const int* qcount = nullptr;
+    const int* gate = nullptr;  // do nothing while *gate is 0
     int qmore = 0;  // a list of at most this many queries is not served here
     int slots = 0;  // (query, slice) pairs that `part` has room for (qlist only)
 };
@@ -194,6 +195,7 @@ __device__ __forceinline__ void brute_block(const BruteArgs<T>& a, T* tile, int 
 template <typename T, int DP, int G, int R>
 __global__ void __launch_bounds__(256) k_brute(const BruteArgs<T> a) {
     __shared__ __align__(16) T tile[BruteTile<T, DP>::kRefs * DP];
+    if (a.gate && *a.gate == 0) return;
     brute_block<T, DP, G, R, false>(a, tile, a.nq, a.nsplit, blockIdx.x, blockIdx.y);
 }
 
@@ -217,7 +219,7 @@ __global__ void __launch_bounds__(256) k_brute_merge(const BruteArgs<T> a) {
     const int gbase = lane & ~(G - 1);
     const unsigned gmask = group_mask<G>(lane);
     const int slot = blockIdx.x * (blockDim.x / G) + threadIdx.x / G;
-    if (slot >= a.nq) return;  // whole groups leave together
+    if (slot >= a.nq || (a.gate && *a.gate == 0)) return;  // whole groups leave together
     TopK<T, G, R> list;
     list.init(a.k, gl);
     Key<T> worst = Key<T>::sentinel();

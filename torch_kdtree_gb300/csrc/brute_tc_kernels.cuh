@@ -30,7 +30,8 @@ inline size_t align256(size_t v) { return (v + 255) / 256 * 256; }
 // non-finite coordinates) enter no list, and overflowing ones break the error
 // bound, so a query is certified only when |q|^2 < 2^125 and every reference
 // has |r|^2 < 2^125 (the pack kernel flags any other reference in `err`,
-// which certifies nothing).  Then every partial sum of a score is below
+// which certifies nothing; the tcgen05 path takes references with infinite or
+// NaN coordinates for padding).  Then every partial sum of a score is below
 // |r|^2 + 2|q||r| <= 2 (|q|^2 + |r|^2) < 2^127: finite.  Uncertified queries
 // are answered by the exact kernel.
 constexpr float kTcNormLimit = 0x1p125f;
@@ -308,10 +309,18 @@ __global__ void __launch_bounds__(256) k_tc5_pack(const float* __restrict__ x, i
             if (is_query) {
                 v[e] = real ? 1.f : 0.f;
             } else {
-                float nrm = 0.f;
-                for (int j = 0; real && j < d; ++j) nrm = fmaf(row[j], row[j], nrm);
-                if (!(nrm < kTcNormLimit)) atomicOr(err, kTcErrRange);  // see kTcNormLimit
-                v[e] = real ? nrm : kT5PadNorm;
+                float nrm = 0.f, odd = 0.f;  // odd: NaN if a coordinate is not finite
+                for (int j = 0; real && j < d; ++j) {
+                    nrm = fmaf(row[j], row[j], nrm);
+                    odd += row[j] - row[j];
+                }
+                // An infinite or NaN coordinate puts the reference at distance
+                // inf or NaN: it is in no certified answer (those have k
+                // finite distances) and counts as padding.  For the rest see
+                // kTcNormLimit.
+                const bool finite = odd == 0.f;
+                if (finite && !(nrm < kTcNormLimit)) atomicOr(err, kTcErrRange);
+                v[e] = real && finite ? nrm : kT5PadNorm;
             }
         }
     }

@@ -372,6 +372,29 @@ int run_query_wide(const tk_tree* t, const T* q, int nq, int k, T* dists, int32_
     return rc;
 }
 
+int run_query_any(const tk_tree* t, const void* q, int n32, int k, void* dists, int32_t* idx, const tk_query_opts& o,
+                  char* ws, cudaStream_t s) {
+    if (t->dtype == TK_F32) {
+        auto* qq = static_cast<const float*>(q);
+        auto* dd = static_cast<float*>(dists);
+        switch (t->dims) {
+            case 1: return run_query<float, 1>(t, qq, n32, k, dd, idx, o, ws, s);
+            case 2: return run_query<float, 2>(t, qq, n32, k, dd, idx, o, ws, s);
+            case 3: return run_query<float, 3>(t, qq, n32, k, dd, idx, o, ws, s);
+            default: return run_query_wide<float>(t, qq, n32, k, dd, idx, o, ws, s);
+        }
+    } else {
+        auto* qq = static_cast<const double*>(q);
+        auto* dd = static_cast<double*>(dists);
+        switch (t->dims) {
+            case 1: return run_query<double, 1>(t, qq, n32, k, dd, idx, o, ws, s);
+            case 2: return run_query<double, 2>(t, qq, n32, k, dd, idx, o, ws, s);
+            case 3: return run_query<double, 3>(t, qq, n32, k, dd, idx, o, ws, s);
+            default: return run_query_wide<double>(t, qq, n32, k, dd, idx, o, ws, s);
+        }
+    }
+}
+
 // The 4th slot of a point record holds an index as raw bits: the original
 // index of a point, or the begin / end offset of a leaf in its box records.
 template <typename T>
@@ -585,6 +608,18 @@ int check_device_build(const void* dev_points, int64_t n, int dims, int dtype, i
     return TK_OK;
 }
 
+// The parts of a tree's image (tree_image) at `image`.
+void set_image(tk_tree* t, void* image) {
+    const TreeImage im = tree_image(t->n, t->dims, t->dtype, t->search_levels);
+    char* p = static_cast<char*>(image);
+    t->d_pts = p + im.pts;
+    t->d_boxes = p + im.boxes;
+    t->d_medians = p + im.medians;
+    t->d_leaf_off = reinterpret_cast<int32_t*>(p + im.leaf_off);
+    if (t->dims > 3) t->d_perm = reinterpret_cast<int32_t*>(p + im.perm);
+    t->device_bytes = int64_t(im.total);
+}
+
 // GPU build of checked arguments into `image` (not owned by the tree).
 int device_build(const void* dev_points, int64_t n, int dims, int dtype, int levels, int search_levels, int device,
                  void* image, void* workspace, void* stream, tk_tree** out) {
@@ -597,16 +632,9 @@ int device_build(const void* dev_points, int64_t n, int dims, int dtype, int lev
     t->device = device;
     t->n = n;
     t->host_layout = false;
-    const TreeImage im = tree_image(n, dims, dtype, search_levels);
-    char* p = static_cast<char*>(image);
-    t->d_pts = p + im.pts;
-    t->d_boxes = p + im.boxes;
-    t->d_medians = p + im.medians;
-    t->d_leaf_off = reinterpret_cast<int32_t*>(p + im.leaf_off);
-    if (dims > 3) t->d_perm = reinterpret_cast<int32_t*>(p + im.perm);
     t->one_image = true;
     t->own_image = false;
-    t->device_bytes = int64_t(im.total);
+    set_image(t, image);
     const int rc = dtype == TK_F32
                        ? build_device_tree<float>(static_cast<const float*>(dev_points), n, dims, stream, t, workspace)
                        : build_device_tree<double>(static_cast<const double*>(dev_points), n, dims, stream, t, workspace);
@@ -886,29 +914,68 @@ int tk_tree_query(const tk_tree* t, const void* q, int64_t nq, int k, void* dist
     DeviceGuard g(t->device);
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     char* ws = static_cast<char*>(workspace);
-    const int n32 = int(nq);
-    if (t->dtype == TK_F32) {
-        auto* qq = static_cast<const float*>(q);
-        auto* dd = static_cast<float*>(dists);
-        switch (t->dims) {
-            case 1: return run_query<float, 1>(t, qq, n32, k, dd, idx, o, ws, s);
-            case 2: return run_query<float, 2>(t, qq, n32, k, dd, idx, o, ws, s);
-            case 3: return run_query<float, 3>(t, qq, n32, k, dd, idx, o, ws, s);
-            default: return run_query_wide<float>(t, qq, n32, k, dd, idx, o, ws, s);
-        }
-    } else {
-        auto* qq = static_cast<const double*>(q);
-        auto* dd = static_cast<double*>(dists);
-        switch (t->dims) {
-            case 1: return run_query<double, 1>(t, qq, n32, k, dd, idx, o, ws, s);
-            case 2: return run_query<double, 2>(t, qq, n32, k, dd, idx, o, ws, s);
-            case 3: return run_query<double, 3>(t, qq, n32, k, dd, idx, o, ws, s);
-            default: return run_query_wide<double>(t, qq, n32, k, dd, idx, o, ws, s);
-        }
-    }
+    return run_query_any(t, q, int(nq), k, dists, idx, o, ws, s);
 }
 
 }  // extern "C"
+
+// ------------------------------------------------------ transient trees --
+
+namespace tk {
+namespace {
+
+// The tree of one call, its depth the one that the call's query wants.
+tk_tree transient_tree(int64_t n, int64_t nq, int dims, int k, int dtype) {
+    tk_tree t;
+    t.dtype = dtype;
+    t.dims = dims;
+    t.n = n;
+    if (cudaGetDevice(&t.device) != cudaSuccess) t.device = 0;
+    t.host_layout = false;
+    t.one_image = true;
+    t.own_image = false;
+    t.auto_depth = true;
+    t.search_levels = kMaxLevels;
+    t.search_levels = query_levels(&t, auto_lanes(&t, nq, k), k);
+    t.levels = t.search_levels;
+    return t;
+}
+
+struct TransientWs {
+    size_t image = 0, build = 0, query = 0, total = 0;
+};
+TransientWs transient_ws(const tk_tree& t, int64_t nq) {
+    TransientWs w;
+    size_t o = align_up(tree_image(t.n, t.dims, t.dtype, t.search_levels).total, 256);
+    w.build = o;
+    o += align_up(build_workspace_bytes(t.n, t.dims, t.dtype), 256);
+    w.query = o;
+    o += align_up(ws_layout(t.search_levels, nq).total, 256);
+    w.total = o;
+    return w;
+}
+
+}  // namespace
+
+size_t transient_tree_workspace_bytes(int64_t n, int64_t nq, int dims, int k, int dtype) {
+    return transient_ws(transient_tree(n, nq, dims, k, dtype), nq).total;
+}
+
+int transient_tree_query(const void* ref, int64_t n, const void* q, int64_t nq, int dims, int k, int dtype,
+                         void* dists, int32_t* idx, void* workspace, void* stream, const int** odd) {
+    tk_tree t = transient_tree(n, nq, dims, k, dtype);
+    const TransientWs w = transient_ws(t, nq);
+    char* ws = static_cast<char*>(workspace);
+    set_image(&t, ws + w.image);
+    const int rc = dtype == TK_F32
+                       ? enqueue_device_tree<float>(static_cast<const float*>(ref), n, dims, stream, &t, ws + w.build, odd)
+                       : enqueue_device_tree<double>(static_cast<const double*>(ref), n, dims, stream, &t, ws + w.build, odd);
+    if (rc != TK_OK) return rc;
+    const tk_query_opts o{0, -1, -1, 0, 0, nullptr, nullptr, -1, 0};
+    return run_query_any(&t, q, int(nq), k, dists, idx, o, ws + w.query, static_cast<cudaStream_t>(stream));
+}
+
+}  // namespace tk
 
 // ------------------------------------------------ allocation-free query --
 //
@@ -975,25 +1042,7 @@ extern "C" int tk_tree_query_noalloc(const tk_tree* t, const void* q, int64_t nq
     if (opts) o = *opts;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     char* ws = static_cast<char*>(scratch);
-    const int n32 = int(nq);
-    if (t->dtype == TK_F32) {
-        auto* qq = static_cast<const float*>(q);
-        auto* dd = static_cast<float*>(dists);
-        switch (t->dims) {
-            case 1: return run_query<float, 1>(t, qq, n32, k, dd, idx, o, ws, s);
-            case 2: return run_query<float, 2>(t, qq, n32, k, dd, idx, o, ws, s);
-            case 3: return run_query<float, 3>(t, qq, n32, k, dd, idx, o, ws, s);
-            default: return run_query_wide<float>(t, qq, n32, k, dd, idx, o, ws, s);
-        }
-    }
-    auto* qq = static_cast<const double*>(q);
-    auto* dd = static_cast<double*>(dists);
-    switch (t->dims) {
-        case 1: return run_query<double, 1>(t, qq, n32, k, dd, idx, o, ws, s);
-        case 2: return run_query<double, 2>(t, qq, n32, k, dd, idx, o, ws, s);
-        case 3: return run_query<double, 3>(t, qq, n32, k, dd, idx, o, ws, s);
-        default: return run_query_wide<double>(t, qq, n32, k, dd, idx, o, ws, s);
-    }
+    return run_query_any(t, q, int(nq), k, dists, idx, o, ws, s);
 }
 
 // ------------------------------------------------- host-buffer query --

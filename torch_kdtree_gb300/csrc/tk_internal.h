@@ -82,6 +82,17 @@ size_t build_workspace_bytes(int64_t n, int dims, int dtype);
 // synchronises the CUDA stream `stream` before returning.
 template <typename T>
 int build_device_tree(const T* pts, int64_t n, int dims, void* stream, tk_tree* t, void* workspace);
+// The same without waiting: *odd points to two device ints, whether some
+// coordinate is NaN, and whether some is NaN or infinite.
+template <typename T>
+int enqueue_device_tree(const T* pts, int64_t n, int dims, void* stream, const tk_tree* t, void* workspace,
+                        const int** odd);
+// k nearest neighbours (1-3 dims) through a tree that is built and dropped in
+// the workspace (tk_api.cu): device work only.  *odd as above: where it says
+// so, the caller has to search exhaustively.
+size_t transient_tree_workspace_bytes(int64_t n, int64_t nq, int dims, int k, int dtype);
+int transient_tree_query(const void* ref, int64_t n, const void* q, int64_t nq, int dims, int k, int dtype,
+                         void* dists, int32_t* idx, void* workspace, void* stream, const int** odd);
 }  // namespace tk
 
 namespace tk {

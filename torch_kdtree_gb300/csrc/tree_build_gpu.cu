@@ -92,6 +92,15 @@ __device__ __forceinline__ unsigned long long coord_key(double v) {
     return (b & 0x8000000000000000ull) ? ~b : (b | 0x8000000000000000ull);
 }
 
+// odd[0]: some coordinate is NaN; odd[1]: some coordinate is NaN or infinite.
+template <typename T>
+__device__ __forceinline__ void mark_odd(T v, int* odd) {
+    if (v - v != T(0)) {
+        odd[1] = 1;
+        if (v != v) odd[0] = 1;
+    }
+}
+
 // Lanes of the warp whose 8-bit digit equals this lane's, among the valid
 // ones (an invalid lane gets the other invalid lanes).  Eight ballots: faster
 // here than __match_any_sync.
@@ -146,7 +155,7 @@ template <typename T, bool FIRST>
 __global__ void __launch_bounds__(kSortThreads) k_radix_hist(const T* __restrict__ pts, int64_t n, int dims, int ax0,
                                                              const typename KeyBits<T>::type* __restrict__ keys,
                                                              int shift, int ntiles, int* __restrict__ hist,
-                                                             int* __restrict__ nan_flag) {
+                                                             int* __restrict__ odd) {
     __shared__ int h[256];
     const int t = threadIdx.x, a = blockIdx.y;
     if (t < 256) h[t] = 0;
@@ -159,7 +168,7 @@ __global__ void __launch_bounds__(kSortThreads) k_radix_hist(const T* __restrict
             typename KeyBits<T>::type k;
             if constexpr (FIRST) {
                 const T v = pts[e * dims + ax0 + a];
-                if (v != v) *nan_flag = 1;
+                mark_odd(v, odd);
                 k = coord_key(v);
             } else {
                 k = keys[a * n + e];
@@ -278,7 +287,7 @@ __global__ void __launch_bounds__(kSortThreads, 2) k_radix_scatter(
 // digits in one launch.
 template <typename T>
 __global__ void __launch_bounds__(kSubThreads) k_small_sort(const T* __restrict__ pts, int n, int dims,
-                                                            const Arrays out, int* __restrict__ nan_flag) {
+                                                            const Arrays out, int* __restrict__ odd) {
     using K = typename KeyBits<T>::type;
     constexpr int WARPS = kSubThreads / 32;
     extern __shared__ __align__(16) unsigned char smem[];
@@ -289,7 +298,7 @@ __global__ void __launch_bounds__(kSubThreads) k_small_sort(const T* __restrict_
     const int t = threadIdx.x, lane = t & 31, w = t >> 5, a = blockIdx.x;
     for (int i = t; i < n; i += kSubThreads) {
         const T v = pts[int64_t(i) * dims + a];
-        if (v != v) *nan_flag = 1;
+        mark_odd(v, odd);
         skey[i] = coord_key(v);
         sval[i] = uint16_t(i);
     }
@@ -703,7 +712,7 @@ int axes_at_once(int64_t n, int dims) { return n <= (int64_t(32) << 20) ? dims :
 // Scratch of a build: id orders (one per axis), then spare orders, two key
 // arrays (whose space the level passes use afterwards), digit histograms.
 struct BuildWs {
-    size_t orders = 0, key_a = 0, key_b = 0, hist = 0, totals = 0, nan_flag = 0, total = 0;
+    size_t orders = 0, key_a = 0, key_b = 0, hist = 0, totals = 0, odd = 0, total = 0;
     size_t order_bytes = 0;
     int at_once = 1;
 };
@@ -713,7 +722,7 @@ BuildWs build_ws(int64_t n, int dims, size_t key_bytes) {
     const int A = w.at_once = axes_at_once(n, dims);
     w.order_bytes = align256(4 * size_t(n));
     size_t o = 0;
-    w.nan_flag = o;
+    w.odd = o;
     o += 256;
     w.orders = o;
     o += w.order_bytes * (small ? dims : dims + A);
@@ -767,13 +776,15 @@ TreeImage tree_image(int64_t n, int dims, int dtype, int levels) {
 }
 
 template <typename T>
-int build_device_tree(const T* pts, int64_t n, int dims, void* stream, tk_tree* t, void* workspace) {
+int enqueue_device_tree(const T* pts, int64_t n, int dims, void* stream, const tk_tree* t, void* workspace,
+                        const int** odd_out) {
     using K = typename KeyBits<T>::type;
     const cudaStream_t s = static_cast<cudaStream_t>(stream);
     const int L = t->search_levels;
     const BuildWs w = build_ws(n, dims, sizeof(K));
     char* ws = static_cast<char*>(workspace);
-    int* nan_flag = reinterpret_cast<int*>(ws + w.nan_flag);
+    int* odd = reinterpret_cast<int*>(ws + w.odd);
+    *odd_out = odd;
     Arrays P, spare;  // P's arrays, then the spares
     P.base = spare.base = reinterpret_cast<uint32_t*>(ws + w.orders);
     P.stride = spare.stride = int64_t(w.order_bytes / 4);
@@ -792,12 +803,12 @@ int build_device_tree(const T* pts, int64_t n, int dims, void* stream, tk_tree* 
     im.W = record_width(dims);
 
     // 1. presorted axes
-    TK_TRY(cudaMemsetAsync(nan_flag, 0, sizeof(int), s));
+    TK_TRY(cudaMemsetAsync(odd, 0, 2 * sizeof(int), s));
     int t0 = 0;  // depth from which a block finishes a node
     if (n <= kSub) {
         const size_t smem = small_sort_smem<T>();
         TK_TRY(cudaFuncSetAttribute(k_small_sort<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
-        k_small_sort<T><<<dims, kSubThreads, smem, s>>>(pts, n32, dims, P, nan_flag);
+        k_small_sort<T><<<dims, kSubThreads, smem, s>>>(pts, n32, dims, P, odd);
         TK_TRY(cudaGetLastError());
     } else {
         while (t0 < L && ((n - 1) >> t0) + 1 > kSub) ++t0;
@@ -818,8 +829,8 @@ int build_device_tree(const T* pts, int64_t n, int dims, void* stream, tk_tree* 
                 const Arrays& vin = pass & 1 ? spare : dst;
                 const Arrays& vout = pass & 1 ? dst : spare;  // an even number of passes ends in dst
                 const int shift = 8 * pass;
-                if (pass == 0) k_radix_hist<T, true><<<grid, kSortThreads, 0, s>>>(pts, n, dims, a0, kin, shift, rtiles, hist, nan_flag);
-                else k_radix_hist<T, false><<<grid, kSortThreads, 0, s>>>(pts, n, dims, a0, kin, shift, rtiles, hist, nan_flag);
+                if (pass == 0) k_radix_hist<T, true><<<grid, kSortThreads, 0, s>>>(pts, n, dims, a0, kin, shift, rtiles, hist, odd);
+                else k_radix_hist<T, false><<<grid, kSortThreads, 0, s>>>(pts, n, dims, a0, kin, shift, rtiles, hist, odd);
                 k_row_scan<<<dim3(256, na), kScanThreads, 0, s>>>(hist, rtiles, totals);
                 if (pass == 0) k_radix_scatter<T, true, false><<<grid, kSortThreads, 0, s>>>(pts, n, dims, a0, kin, vin, shift, rtiles, hist, totals, kout, vout);
                 else if (pass + 1 < passes) k_radix_scatter<T, false, false><<<grid, kSortThreads, 0, s>>>(pts, n, dims, a0, kin, vin, shift, rtiles, hist, totals, kout, vout);
@@ -873,13 +884,24 @@ int build_device_tree(const T* pts, int64_t n, int dims, void* stream, tk_tree* 
                                                         reinterpret_cast<uint16_t*>(ws + w.key_b));
     }
     TK_TRY(cudaGetLastError());
+    return TK_OK;
+}
+
+template <typename T>
+int build_device_tree(const T* pts, int64_t n, int dims, void* stream, tk_tree* t, void* workspace) {
+    const cudaStream_t s = static_cast<cudaStream_t>(stream);
+    const int* odd = nullptr;
+    const int rc = enqueue_device_tree<T>(pts, n, dims, stream, t, workspace, &odd);
+    if (rc != TK_OK) return rc;
     int nan_host = 0;
-    TK_TRY(cudaMemcpyAsync(&nan_host, nan_flag, sizeof(int), cudaMemcpyDeviceToHost, s));
+    TK_TRY(cudaMemcpyAsync(&nan_host, odd, sizeof(int), cudaMemcpyDeviceToHost, s));
     TK_TRY(cudaStreamSynchronize(s));
     if (nan_host) return fail(TK_EINVAL, "reference points contain NaN");
     return TK_OK;
 }
 
+template int enqueue_device_tree<float>(const float*, int64_t, int, void*, const tk_tree*, void*, const int**);
+template int enqueue_device_tree<double>(const double*, int64_t, int, void*, const tk_tree*, void*, const int**);
 template int build_device_tree<float>(const float*, int64_t, int, void*, tk_tree*, void*);
 template int build_device_tree<double>(const double*, int64_t, int, void*, tk_tree*, void*);
 

@@ -427,9 +427,12 @@ _BRUTE_MODES = {"exact": _lib.TK_BRUTE_EXACT, "fp32": _lib.TK_BRUTE_EXACT, "fp64
 
 
 def nn_distance_raw(points_ref: torch.Tensor, points_query: torch.Tensor, k: int, dists: torch.Tensor,
-                    idx: torch.Tensor, mode: str = "exact") -> None:
-    """Enqueue one tk_nn_distance on the current stream (inputs on the device)."""
+                    idx: torch.Tensor, mode: str = "exact", routed: bool = False) -> None:
+    """Enqueue one tk_nn_distance on the current stream (inputs on the device).
+    ``routed``: "exact" may take any search that gives the exact answer."""
     m = _BRUTE_MODES[mode]
+    if routed and m == _lib.TK_BRUTE_EXACT:
+        m = _lib.TK_BRUTE_ROUTED
     n, d = points_ref.shape
     nq = points_query.shape[0]
     dt = _DTYPES[points_ref.dtype]
@@ -445,9 +448,10 @@ def nn_distance(points_ref: torch.Tensor, points_query: torch.Tensor, nr_nns_sea
     """Exhaustive exact KNN: ``(dists, inds)`` of every query among all
     reference points, squared distances ``[Q, k]`` and int32 indices.
 
-    ``mode``: "exact" (CUDA cores, float32 or float64), "tf32" or
-    "bf16_split" (tensor-core candidate search with an exact float32 re-rank;
-    same answer), or "auto" (the fastest of these for the shapes, timed once
+    ``mode``: "exact" (float32 or float64; the fastest search for the sizes:
+    CUDA cores, tensor cores with an exact re-rank, or in 1-3 dimensions a
+    KD-tree that lives for the call), "tf32" or "bf16_split" (tensor-core
+    candidate search with an exact float32 re-rank; same answer), or "auto" (the fastest of these for the shapes, timed once
     by :func:`torch_kdtree_gb300.autotune.autotune_brute` and cached).
     Differentiable in both point sets.  The reference shipped this search as
     an unbound CUDA launcher (src/nndistance_g.cu:191-220) for d = 3 only;
@@ -476,7 +480,7 @@ def nn_distance(points_ref: torch.Tensor, points_query: torch.Tensor, nr_nns_sea
     nq = q_c.shape[0]
     dists = torch.empty((nq, k), dtype=ref_c.dtype, device=ref_c.device)
     idx = torch.empty((nq, k), dtype=torch.int32, device=ref_c.device)
-    nn_distance_raw(ref_c.detach(), q_c.detach(), k, dists, idx, mode)
+    nn_distance_raw(ref_c.detach(), q_c.detach(), k, dists, idx, mode, routed=True)
     return dists, idx
 
 
