@@ -157,6 +157,9 @@ typedef struct tk_query_opts {
 
 /* Bytes of device scratch tk_tree_query needs for nq queries. */
 size_t tk_tree_query_workspace_size(const tk_tree* tree, int64_t nq);
+/* Calls of at most this many queries may pass a null workspace (unless the
+ * options ask for binning or limit the blocks per SM). */
+int64_t tk_tree_query_scratch_free(const tk_tree* tree);
 
 /* Exact k nearest neighbours of nq device-resident query points.
  * q: device [nq, dims] (tree dtype); dists: device [nq, k] squared

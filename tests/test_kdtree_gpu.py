@@ -401,3 +401,39 @@ def test_random_configurations(oracle):
         msg = f"case {case}: dims={dims} {np.dtype(dtype).name} n={n} nq={nq} k={k} L={levels} {opts}"
         np.testing.assert_array_equal(d, bd, err_msg=msg)
         np.testing.assert_array_equal(i, bi, err_msg=msg)
+
+
+@pytest.mark.parametrize("d,dtype", [(3, np.float32), (3, np.float64), (8, np.float64)])
+def test_calls_without_a_workspace(d, dtype, oracle):
+    """Up to tk_tree_query_scratch_free queries one round of the grid holds the
+    call in every launch shape; above, or with binning, a workspace is due."""
+    import ctypes
+    from torch_kdtree_gb300._lib import LIB, TK_EWORKSPACE, QueryOpts
+    rng = np.random.default_rng(d)
+    ref = rng.standard_normal((5000, d)).astype(dtype)
+    tree = tk().build_kd_tree(torch.from_numpy(ref).to(cuda))
+    h = tree._tree.handle
+    most = LIB.tk_tree_query_scratch_free(h)
+    assert most >= 8
+    q = rng.standard_normal((most + 1, d)).astype(dtype)
+    qt = torch.from_numpy(q).to(cuda)
+    stream = torch.cuda.current_stream().cuda_stream
+
+    def call(nq, k, **opts):
+        dd = torch.empty(nq, k, dtype=qt.dtype, device=cuda)
+        ii = torch.empty(nq, k, dtype=torch.int32, device=cuda)
+        o = QueryOpts.make(**opts)
+        st = LIB.tk_tree_query(h, qt.data_ptr(), nq, k, dd.data_ptr(), ii.data_ptr(), ctypes.byref(o), None, 0, stream)
+        return st, dd, ii
+
+    for k in (1, 16, 128):
+        bd, bi = oracle.brute(ref, q[:most], k)
+        for lanes in (0, 1, 32):
+            for traversal in (0, 2):
+                st, dd, ii = call(most, k, threads_per_query=lanes, traversal=traversal)
+                assert st == 0
+                np.testing.assert_array_equal(dd.cpu().numpy(), bd)
+                np.testing.assert_array_equal(ii.cpu().numpy(), bi)
+    assert call(most + 1, 4)[0] == TK_EWORKSPACE
+    assert call(most, 4, bin_queries=1)[0] == TK_EWORKSPACE
+    assert call(most, 4, blocks_per_sm=1)[0] == TK_EWORKSPACE

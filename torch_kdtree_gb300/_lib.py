@@ -85,6 +85,7 @@ SIGNATURES = {
     "tk_tree_get_perm": (_int, [_vp, _vp]),
     "tk_tree_get_points": (_int, [_vp, _vp]),
     "tk_tree_get_splits": (_int, [_vp, _vp, _vp]),
+    "tk_tree_query_scratch_free": (_i64, [_vp]),
     "tk_tree_query_workspace_size": (_sz, [_vp, _i64]),
     "tk_tree_query": (_int, [_vp, _vp, _i64, _int, _vp, _vp, ctypes.POINTER(QueryOpts), _vp, _sz, _vp]),
     "tk_batch_create": (_int, [ctypes.POINTER(_vp), _int, ctypes.POINTER(_i64), ctypes.POINTER(_i32),

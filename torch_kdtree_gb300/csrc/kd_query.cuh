@@ -56,7 +56,7 @@ struct KdArgs {
     const int32_t* order;    // [nq] processing order (binned), or null for identity
     T* out_d;                // [nq, k]
     int32_t* out_i;          // [nq, k]
-    int* work;               // global work counter, zero at launch
+    int* work;               // global work counter, zero at launch; null: the grid covers all queries once
 };
 
 template <typename T, int D>
@@ -409,10 +409,8 @@ __global__ void __launch_bounds__(kKdBlock) k_kd_query(const KdArgs<T> a) {
     constexpr int kGroupsPerWarp = 32 / G;
     const int gid = lane / G;
 
-    for (;;) {
-        int base = 0;
-        if (lane == 0) base = atomicAdd(a.work, kGroupsPerWarp);
-        base = __shfl_sync(0xFFFFFFFFu, base, 0);
+    for (int round = 0;;) {
+        const int base = next_queries(a.work, kGroupsPerWarp, a.nq, round);
         if (base >= a.nq) break;
         const int t = base + gid;
         if (t < a.nq) {
@@ -550,10 +548,8 @@ __global__ void __launch_bounds__(256) k_kd_packet(const KdArgs<T> a) {
 
     const int lane = threadIdx.x & 31;
     const TreeView<T> tv{a.pts, a.medians, a.leaf_off, a.levels, a.smem_levels, s_med, a.boxes};
-    for (;;) {
-        int base = 0;
-        if (lane == 0) base = atomicAdd(a.work, 32);
-        base = __shfl_sync(0xFFFFFFFFu, base, 0);
+    for (int round = 0;;) {
+        const int base = next_queries(a.work, 32, a.nq, round);
         if (base >= a.nq) break;
         const int t = base + lane;
         const bool active = t < a.nq;

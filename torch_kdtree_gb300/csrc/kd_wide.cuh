@@ -41,7 +41,7 @@ struct KdWideArgs {
     const int32_t* order;     // [nq] processing order (binned), or null
     T* out_d;                 // [nq, k]
     int32_t* out_i;           // [nq, k]
-    int* work;                // global work counter, zero at launch
+    int* work;                // global work counter, zero at launch; null: see next_queries
 };
 
 template <typename T, int W>
@@ -264,10 +264,8 @@ __global__ void __launch_bounds__(256, G == 32 && sizeof(T) == 4 ? (R < 4 ? 5 : 
     const int lane = threadIdx.x & 31;
     constexpr int kGroupsPerWarp = 32 / G;
     const int gid = lane / G;
-    for (;;) {
-        int base = 0;
-        if (lane == 0) base = atomicAdd(a.work, kGroupsPerWarp);
-        base = __shfl_sync(0xFFFFFFFFu, base, 0);
+    for (int round = 0;;) {
+        const int base = next_queries(a.work, kGroupsPerWarp, a.nq, round);
         if (base >= a.nq) break;
         const int t = base + gid;
         if (t < a.nq) {

@@ -3,8 +3,10 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <map>
 #include <mutex>
 #include <string>
+#include <tuple>
 #include <vector>
 
 #include "kd_query.cuh"
@@ -152,6 +154,41 @@ int pow2_ceil(int v) {
     return p;
 }
 
+// Blocks of `kfn` that fit an SM.  A property of the code and the launch, asked
+// of the driver once per kernel (0.8 us a call).
+int blocks_per_sm(const void* kfn, int block, size_t smem) {
+    static std::mutex mu;
+    static std::map<std::tuple<int, const void*, int, size_t>, int> known;
+    int dev = 0;
+    cudaGetDevice(&dev);
+    std::lock_guard<std::mutex> lock(mu);
+    int& v = known[std::make_tuple(dev, kfn, block, smem)];
+    if (v == 0 && (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&v, kfn, block, smem) != cudaSuccess || v <= 0)) v = 1;
+    return v;
+}
+
+// Whether a call's queries are ordered by cell and cost class.
+// Automatic binning from one wave of queries (SMs x 1024) on: below that each
+// thread takes about one query, the cell order gains little leaf sharing, and
+// grouping a region's expensive queries into the same warps lengthens the
+// slowest warp, which then sets the launch time (131,072 queries: 1.33 ms
+// binned vs 1.17 ms in input order; 1,048,576: 3.53 vs 5.84 ms on the
+// cube-and-sphere workload).  A warp per query gains by the cost order already
+// where a search is long (4-8 dims, or long lists), from ten queries per
+// resident warp on: 65,536 queries of 1M points, ms in input order / binned:
+// 6 dims k=16 1.93 / 1.78, 8 dims 8.0 / 7.0, 3 dims k=100 0.66 / 0.60; but 3
+// dims k=16 0.24 / 0.25, and 10,000 queries lose wherever they are.
+bool binned(const tk_tree* t, int L, int G, int64_t nq, int k, const tk_query_opts& o) {
+    if (o.bin_queries >= 0) return o.bin_queries == 1;
+    const int64_t sms = sm_count(t->device);
+    const bool long_search = G == 32 && (t->dims > 3 ? k > 4 : k > 48) && nq >= sms * 320;
+    return L >= 2 && (nq >= sms * 1024 || long_search);
+}
+
+// Queries that one round of any kernel's grid holds (a warp each, one block
+// per SM): no counter, and too few to be binned, so no workspace.
+int64_t scratch_free(const tk_tree* t) { return int64_t(sm_count(t->device)) * (kKdBlock / 32); }
+
 // Zero the work counter and, when binning is on, order the queries by the
 // tree cell at depth B they fall into (count, exclusive scan, scatter).
 // `count(B, counts, bin_of, pos_of)` launches the counting kernel.  With
@@ -164,22 +201,8 @@ template <typename CountFn>
 int prepare_order(const tk_tree* t, int L, int G, int nq, int k, const tk_query_opts& o, char* ws, cudaStream_t s, int** counter,
                   const int32_t** order, bool classes, CountFn count) {
     const WsLayout w = ws_layout(t->search_levels, nq);
-    *counter = reinterpret_cast<int*>(ws + w.counter);
     *order = nullptr;
-    // Automatic binning from one wave of queries (SMs x 1024) on: below that
-    // each thread takes about one query, the cell order gains little leaf
-    // sharing, and grouping a region's expensive queries into the same warps
-    // lengthens the slowest warp, which then sets the launch time (131,072
-    // queries: 1.33 ms binned vs 1.17 ms in input order; 1,048,576: 3.53 vs
-    // 5.84 ms on the cube-and-sphere workload).
-    // A warp per query gains by the cost order already where a search is long
-    // (4-8 dims, or long lists), from ten queries per resident warp on:
-    // 65,536 queries of 1M points, ms in input order / binned: 6 dims k=16
-    // 1.93 / 1.78, 8 dims 8.0 / 7.0, 3 dims k=100 0.66 / 0.60; but 3 dims k=16
-    // 0.24 / 0.25, and 10,000 queries lose wherever they are.
-    const int64_t sms = sm_count(t->device);
-    const bool long_search = G == 32 && (t->dims > 3 ? k > 4 : k > 48) && int64_t(nq) >= sms * 320;
-    const bool bin = o.bin_queries == 1 || (o.bin_queries < 0 && L >= 2 && (int64_t(nq) >= sms * 1024 || long_search));
+    const bool bin = binned(t, L, G, nq, k, o);
     cudaError_t e;
     if (bin) {
         const int B = bin_levels(L, nq);
@@ -206,7 +229,7 @@ int prepare_order(const tk_tree* t, int L, int G, int nq, int k, const tk_query_
             if (e != cudaSuccess) return fail(TK_ECUDA, std::string("cost-class pass: ") + cudaGetErrorString(e));
             *order = reinterpret_cast<const int32_t*>(final_order);
         }
-    } else {
+    } else if (*counter) {
         e = cudaMemsetAsync(*counter, 0, sizeof(int), s);
         if (e != cudaSuccess) return fail(TK_ECUDA, std::string("memset: ") + cudaGetErrorString(e));
     }
@@ -269,15 +292,14 @@ int run_query(const tk_tree* t, const T* q, int nq, int k, T* dists, int32_t* id
         cudaError_t e = cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
         if (e != cudaSuccess) return fail(TK_ECUDA, std::string("smem attribute: ") + cudaGetErrorString(e));
     }
-    int per_sm = 0;
-    cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kfn, block, smem);
-    if (e != cudaSuccess || per_sm <= 0) per_sm = 1;
+    int per_sm = blocks_per_sm(kfn, block, smem);
     if (o.blocks_per_sm > 0) per_sm = std::min(per_sm, int(o.blocks_per_sm));
     const int groups_per_block = block / G;
     const int need = (nq + groups_per_block - 1) / groups_per_block;
     const int grid = std::max(1, std::min(need, per_sm * sm_count(t->device)));
 
-    int* counter = nullptr;
+    // a grid that holds all queries at once needs no counter
+    int* counter = grid < need || binned(t, L, G, nq, k, o) ? reinterpret_cast<int*>(ws + ws_layout(t->search_levels, nq).counter) : nullptr;
     const int32_t* order = nullptr;
     const PointRec<T>* boxes = static_cast<const PointRec<T>*>(t->d_boxes);
     int rc0 = prepare_order(t, L, G, nq, k, o, ws, s, &counter, &order, true, [&](int B, int* counts, int* bin_of, int* pos_of) {
@@ -332,15 +354,13 @@ int run_query_wide(const tk_tree* t, const T* q, int nq, int k, T* dists, int32_
         cudaError_t e = cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
         if (e != cudaSuccess) return fail(TK_ECUDA, std::string("smem attribute: ") + cudaGetErrorString(e));
     }
-    int per_sm = 0;
-    cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kfn, block, smem);
-    if (e != cudaSuccess || per_sm <= 0) per_sm = 1;
+    int per_sm = blocks_per_sm(kfn, block, smem);
     if (o.blocks_per_sm > 0) per_sm = std::min(per_sm, int(o.blocks_per_sm));
     const int groups_per_block = block / G;
     const int need = (nq + groups_per_block - 1) / groups_per_block;
     const int grid = std::max(1, std::min(need, per_sm * sm_count(t->device)));
 
-    int* counter = nullptr;
+    int* counter = grid < need || binned(t, L, G, nq, k, o) ? reinterpret_cast<int*>(ws + ws_layout(t->search_levels, nq).counter) : nullptr;
     const int32_t* order = nullptr;
     const int rc0 = prepare_order(t, L, G, nq, k, o, ws, s, &counter, &order, true, [&](int B, int* counts, int* bin_of, int* pos_of) {
         bin_count_wide_launch<T>(q, nq, t->dims, static_cast<const T*>(t->d_medians), B, L,
@@ -889,6 +909,8 @@ int tk_tree_get_splits(const tk_tree* t, void* medians, int32_t* leaf_offsets) {
     return TK_OK;
 }
 
+int64_t tk_tree_query_scratch_free(const tk_tree* t) { return t && t->device >= 0 ? scratch_free(t) : 0; }
+
 size_t tk_tree_query_workspace_size(const tk_tree* t, int64_t nq) {
     if (!t || nq < 0) return 0;
     return ws_layout(t->search_levels, std::max<int64_t>(nq, 1)).total;
@@ -905,12 +927,13 @@ int tk_tree_query(const tk_tree* t, const void* q, int64_t nq, int k, void* dist
     if (t->device < 0 || !t->d_pts) return fail(TK_EINVAL, "tree was built host-only (device < 0); it has no device image");
     if (nq == 0) return TK_OK;
     if (!q || !dists || !idx) return fail(TK_EINVAL, "null query or output pointer");
-    const size_t need = ws_layout(t->search_levels, nq).total;
-    if (!workspace || workspace_bytes < need)
-        return fail(TK_EWORKSPACE, "workspace too small: need " + std::to_string(need) + " bytes");
-    if (ws_misaligned(workspace)) return fail(TK_EINVAL, "workspace must be 256-byte aligned");
     tk_query_opts o{0, -1, -1, 0, 0, nullptr, nullptr, -1, 0};
     if (opts) o = *opts;
+    const bool free_of_scratch = !workspace && o.bin_queries <= 0 && o.blocks_per_sm <= 0 && nq <= scratch_free(t);
+    const size_t need = free_of_scratch ? 0 : ws_layout(t->search_levels, nq).total;
+    if (!free_of_scratch && (!workspace || workspace_bytes < need))
+        return fail(TK_EWORKSPACE, "workspace too small: need " + std::to_string(need) + " bytes");
+    if (ws_misaligned(workspace)) return fail(TK_EINVAL, "workspace must be 256-byte aligned");
     DeviceGuard g(t->device);
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     char* ws = static_cast<char*>(workspace);

@@ -327,6 +327,19 @@ __device__ __forceinline__ unsigned group_mask(int lane) {
     }
 }
 
+// First of the next `count` queries for this warp, past nq when there are
+// none.  Without a counter every warp takes its share of one round (`round`
+// counts the calls).
+__device__ __forceinline__ int next_queries(int* work, int count, int nq, int& round) {
+    int base = nq;
+    if (work) {
+        if ((threadIdx.x & 31) == 0) base = atomicAdd(work, count);
+        return __shfl_sync(0xFFFFFFFFu, base, 0);
+    }
+    if (round++ == 0) base = int(blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * count;
+    return base;
+}
+
 // Cost class of a query for the launch order (smaller = costlier).  The
 // squared distance from the query to the farthest corner of its home leaf's
 // bounding box bounds its distance to every point of that leaf, so it tracks

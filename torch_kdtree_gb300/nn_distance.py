@@ -47,7 +47,9 @@ def default_levels(n: int) -> int:
 
 
 def _stream_ptr(device: torch.device) -> int:
-    return torch.cuda.current_stream(device).cuda_stream
+    if device.index is None:
+        return torch.cuda.current_stream(device).cuda_stream
+    return torch._C._cuda_getCurrentRawStream(device.index)  # the same, without a Stream object
 
 
 def _workspace(nbytes: int, device: torch.device) -> torch.Tensor:
@@ -65,6 +67,7 @@ class _Tree:
         self.image = None
         self.stream = None
         self.other_streams = False
+        self._scratch_free = None
         if points is None:
             return
         n, d = points.shape
@@ -90,6 +93,13 @@ class _Tree:
         t.handle, t.image, t.stream = h, image, stream
         return t
 
+    @property
+    def scratch_free(self) -> int:
+        """Queries per call that need no workspace."""
+        if self._scratch_free is None:
+            self._scratch_free = int(LIB.tk_tree_query_scratch_free(self.handle))
+        return self._scratch_free
+
     def used_on(self, stream: int) -> None:
         if stream != self.stream:
             self.other_streams = True
@@ -114,12 +124,19 @@ def knn_query_raw(tree: _Tree, q: torch.Tensor, k: int, dists: torch.Tensor, idx
                   opts: Optional[QueryOpts] = None) -> None:
     """Enqueue one tk_tree_query on the current stream (inputs already on the device)."""
     nq = q.shape[0]
-    ws_bytes = LIB.tk_tree_query_workspace_size(tree.handle, nq)
-    ws = _workspace(ws_bytes, q.device)
     stream = _stream_ptr(q.device)
-    tree.used_on(stream)
-    check(LIB.tk_tree_query(tree.handle, q.data_ptr(), nq, k, dists.data_ptr(), idx.data_ptr(),
-                            ctypes.byref(opts) if opts is not None else None, ws.data_ptr(), ws_bytes, stream))
+    if stream != tree.stream:
+        tree.used_on(stream)
+    if nq <= tree.scratch_free and (opts is None or (opts.bin_queries <= 0 and opts.blocks_per_sm <= 0)):
+        ws_ptr, ws_bytes = None, 0
+    else:
+        ws_bytes = LIB.tk_tree_query_workspace_size(tree.handle, nq)
+        ws = _workspace(ws_bytes, q.device)
+        ws_ptr = ws.data_ptr()
+    status = LIB.tk_tree_query(tree.handle, q.data_ptr(), nq, k, dists.data_ptr(), idx.data_ptr(),
+                               ctypes.byref(opts) if opts is not None else None, ws_ptr, ws_bytes, stream)
+    if status:
+        check(status)
 
 
 def knn_query_host(tree: _Tree, q: torch.Tensor, k: int, dists: torch.Tensor, idx: torch.Tensor, device: torch.device,
@@ -246,6 +263,16 @@ class TorchKDTree:
             return self._query_cpu(points_query, k, result_dists, result_idx)
         if k > MAX_K:
             raise RuntimeError(f"nr_nns_searches is limited to {MAX_K} on the GPU")
+        if (result_dists is None and result_idx is None and points_query.dtype == self.dtype
+                and points_query.device == self.device and points_query.dim() == 2
+                and points_query.shape[1] == self.dims and points_query.is_contiguous()
+                and not (torch.is_grad_enabled() and (points_query.requires_grad or self.ref_requires_grad))):
+            # nothing to check, move or differentiate: the common call
+            shape = (points_query.shape[0], k)
+            dists = torch.empty(shape, dtype=self.dtype, device=self.device)
+            inds = torch.empty(shape, dtype=self.dtype_idx, device=self.device)
+            knn_query_raw(self._tree, points_query, k, dists, inds, self.query_opts)
+            return (dists if self.squared_distances else torch.sqrt(dists)), inds
         host_out = (result_dists is not None and result_idx is not None and result_dists.device.type == "cpu"
                     and result_idx.device.type == "cpu")
         need_grad = torch.is_grad_enabled() and (points_query.requires_grad or self.ref_requires_grad)
