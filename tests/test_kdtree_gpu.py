@@ -437,3 +437,44 @@ def test_calls_without_a_workspace(d, dtype, oracle):
     assert call(most + 1, 4)[0] == TK_EWORKSPACE
     assert call(most, 4, bin_queries=1)[0] == TK_EWORKSPACE
     assert call(most, 4, blocks_per_sm=1)[0] == TK_EWORKSPACE
+
+
+@pytest.mark.parametrize("d", [1, 2, 3])
+@pytest.mark.parametrize("data", ["normal", "far_away", "tiny", "huge", "underflow", "overflow", "clusters", "inf", "grid"])
+def test_float64_filter(d, data, oracle):
+    """float64 trees search float images first: clouds far from the origin, at
+    the ends of the double range, with distances that under- or overflow, in
+    clusters far below float resolution, with infinite coordinates."""
+    rng = np.random.default_rng(d)
+    n, nq = 20_000, 400
+    ref, q = rng.standard_normal((n, d)), rng.standard_normal((nq, d))
+    if data == "far_away":
+        ref, q = 4.5e6 + 1e-2 * ref, 4.5e6 + 1e-2 * q
+    elif data == "tiny":
+        ref, q = 1e-140 * ref, 1e-140 * q
+    elif data == "huge":
+        ref, q = 1e150 * ref, 1e150 * q
+    elif data == "underflow":
+        ref, q = 1e-170 * ref, 1e-170 * q
+    elif data == "overflow":
+        ref, q = 1e160 * ref, 1e160 * q
+    elif data == "clusters":
+        c = rng.standard_normal((20, d)) * 1e3
+        ref = c[rng.integers(0, 20, n)] + 1e-9 * ref
+        q = c[rng.integers(0, 20, nq)] + 1e-9 * q
+    elif data == "inf":
+        ref[rng.random(n) < 0.02, 0] = np.inf
+        ref[rng.random(n) < 0.02, d - 1] = -np.inf
+        q[:4, 0] = (np.inf, -np.inf, 1e300, 0.0)
+    elif data == "grid":
+        ref, q = np.round(ref * 2), np.round(q * 2)
+    q[-50:] = ref[rng.integers(0, n, 50)]
+    with np.errstate(all="ignore"):
+        for k in (1, 8, 40):
+            bd, bi = oracle.brute(ref, q, k)
+            bi = np.where(bi == 2 ** 31 - 1, -1, bi)
+            for levels in (None, 5, 12):
+                tree = tk().build_kd_tree(torch.from_numpy(ref).to(cuda), levels=levels)
+                dd, ii = tree.query(torch.from_numpy(q).to(cuda), nr_nns_searches=k)
+                np.testing.assert_array_equal(dd.cpu().numpy(), bd, err_msg=f"{k} {levels}")
+                np.testing.assert_array_equal(ii.cpu().numpy(), bi, err_msg=f"{k} {levels}")

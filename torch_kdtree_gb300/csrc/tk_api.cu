@@ -9,6 +9,7 @@
 #include <tuple>
 #include <vector>
 
+#include "kd_filter.cuh"
 #include "kd_query.cuh"
 #include "kd_wide.cuh"
 #include "sort.cuh"
@@ -119,7 +120,8 @@ bool gr_available(int dtype, int dims, int G, int R) {
     return true;
 }
 
-constexpr double kOneLaneLeaf = 22;  // points per leaf, see query_levels
+// Points per leaf for one lane per query, see query_levels.
+double one_lane_leaf(int64_t n) { return n <= 65536 ? 11 : 22; }
 
 // round(log2(v)), at least 0
 int log2_round(double v) { return v <= 1.0 ? 0 : int(std::lround(std::log2(v))); }
@@ -131,21 +133,36 @@ int log2_round(double v) { return v <= 1.0 ? 0 : int(std::lround(std::log2(v)));
 // one long chain of dependent steps, longer in larger clouds, so calls need
 // enough queries to hide it: the crossing was measured, at depths of 22 and
 // ~100 points per leaf, near 50,000 queries for 10,000 points, 110,000 for
-// 100,000, 220,000 for 1M and 260,000 for 4M (k = 5 and 8; ms on one lane
-// against a warp: 1M points, 65,536 queries, k=8 0.32 / 0.19; 1,048,576
-// queries 0.97 / 2.1), lower for k = 1 and higher for k = 16.  Leaves of more
-// than 192 points (a depth the caller asked for) always take a warp.  Trees
-// of 4-8 dimensions (1M refs x 262k queries N(0,1), depth 12-13): one lane
-// only for k = 1 up to 6 dimensions from a wave of queries on (d=4: 0.40 vs
-// 0.70 ms), a warp otherwise (d=8, k=16: 21.4 vs 38.3 ms).
+// 100,000, 200,000 for 1M and 260,000 for 4M (d = 3, k = 5 and 8; ms on one
+// lane against a warp: 1M points, 65,536 queries, k=8 0.32 / 0.19; 1,048,576
+// queries 0.97 / 2.1; 200,000 points, 131,072 queries, k=4 0.19 / 0.24), lower
+// for k = 1, higher for k = 16, and lower in fewer dimensions, where a search
+// is shorter (131,072 queries in 200,000 points, k=4: d=2 0.10 / 0.16, d=1
+// 0.05 / 0.13).  Leaves of more than 192 points (a depth the caller asked for)
+// always take a warp.  Trees of 4-8 dimensions (1M refs x 262k queries N(0,1),
+// depth 12-13): one lane only for k = 1 up to 6 dimensions from half a wave of
+// queries on (d=4: 0.40 vs 0.70 ms), a warp otherwise (d=8, k=16: 21.4 vs 38.3).
 int auto_lanes(const tk_tree* t, int64_t nq, int k) {
     if (k > 16) return 32;
     const double sms = sm_count(t->device);
     if (t->dims > 3) return k == 1 && t->dims <= 6 && double(nq) >= sms * 512 ? 1 : 32;
+    if (t->d_filter[0]) {
+        // float64: the filtered search takes a warp per query; one lane without
+        // the filter wins where a search is short and there are many (ms, one
+        // lane / filtered, k=8: d=1 20,000 points, 65,536 queries 0.104 /
+        // 0.109, 1M queries 0.42 / 1.63; d=2 200,000 points 65,536 0.39 / 0.19,
+        // 1M 1.99 / 2.48, 1M points 4.3 / 2.6; d=3 2,000 points 4.5 / 4.0, k=1
+        // 2.7 / 2.9, 200,000 points 7.2 / 4.4; d=2, k=1, 262,144 queries, 1,000
+        // points 0.35 / 0.57, 20,000 0.41 / 0.54)
+        const double from = t->dims == 1 ? 256 : (t->dims == 2 && t->n <= 50000 ? (t->n <= 5000 ? 700 : 1300) : 2048);
+        const bool short_search = t->dims == 1 || (t->dims == 2 ? t->n <= 500000 : t->n <= 5000 && k <= 4);
+        return short_search && double(nq) >= sms * from ? 1 : 32;
+    }
     const double avg_leaf = double(t->n) / double(int64_t(1) << t->search_levels);
     if (!t->auto_depth && avg_leaf > 192) return 32;
     const double crossing = sms * 120.0 * std::max(1.0, std::log2(double(t->n)) - 10.3);
-    return double(nq) >= crossing * (k == 1 ? 0.6 : (k > 8 ? 1.4 : 1.0)) ? 1 : 32;
+    const double by_k = k == 1 ? 0.6 : (k > 8 ? 1.4 : 0.9), by_dims = t->dims == 1 ? 0.4 : (t->dims == 2 ? 0.65 : 1.0);
+    return double(nq) >= crossing * by_k * by_dims ? 1 : 32;
 }
 
 int pow2_ceil(int v) {
@@ -242,14 +259,15 @@ int prepare_order(const tk_tree* t, int L, int G, int nq, int k, const tk_query_
 // wants small leaves; a warp scans 32 points at a time and, with a longer
 // list, has more to gain from scanning on than from another descent.  Best
 // depths measured (k; points per leaf at 10,000 / 100,000 / 1M / 4M points):
-// one lane 20 / 24 / 30 / 16; a warp k=1 39 / 49 / 61 / 64, k=8 156 / 98 / 61 /
+// one lane 10 / 24 / 30 / 16 (5,000 points: 10); a warp k=1 39 / 49 / 61 / 64, k=8 156 / 98 / 61 /
 // 128, k=16 156 / 98 / 122 / 128, k=100 156 / 195 / 244 / 128; 4-8 dims 61 to
-// 122.  float64 pays more for a point than for a descent.
+// 122.  float64 without the float filter pays more for a point than for a
+// descent.
 int query_levels(const tk_tree* t, int lanes, int k) {
     if (!t->auto_depth) return t->search_levels;
-    double leaf = kOneLaneLeaf;
-    if (t->dims > 3) leaf = lanes == 1 ? kOneLaneLeaf : 90;
-    else if (lanes == 32) leaf = t->dtype == TK_F64 ? 50 : (k <= 2 ? 50 : (k <= 48 ? 110 : 180));
+    double leaf = one_lane_leaf(t->n);
+    if (t->dims > 3) leaf = lanes == 1 ? leaf : 90;
+    else if (lanes == 32) leaf = t->dtype == TK_F64 && !t->d_filter[0] ? 50 : (k <= 2 ? 50 : (k <= 48 ? 110 : 180));
     else if (lanes > 1) leaf = 40;
     return std::max(1, std::min(t->search_levels, log2_round(double(t->n) / leaf)));
 }
@@ -286,7 +304,8 @@ int run_query(const tk_tree* t, const T* q, int nq, int k, T* dists, int32_t* id
     if (!packet && G == 32) S = 0;  // a warp per query reads split values five levels at a time instead
     const int block = kKdBlock;
     const size_t smem = kd_smem_bytes<T>(S);
-    const void* kfn = packet ? kd_packet_kernel<T, D>(R) : kd_query_kernel<T, D>(G, R);
+    const bool filtered = sizeof(T) == 8 && !packet && G == 32 && t->d_filter[0];
+    const void* kfn = packet ? kd_packet_kernel<T, D>(R) : (filtered ? kd_filtered_kernel(D, R) : kd_query_kernel<T, D>(G, R));
     if (!kfn) return fail(TK_EUNSUPPORTED, "KD query kernel shape not compiled");
     if (smem > 48 * 1024) {
         cudaError_t e = cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
@@ -323,7 +342,30 @@ int run_query(const tk_tree* t, const T* q, int nq, int k, T* dists, int32_t* id
     a.work = counter;
     KdLaunch l{G, R, block, grid, smem};
     if (o.kernel_start_event) cudaEventRecord(static_cast<cudaEvent_t>(o.kernel_start_event), s);
-    const int rc = packet ? kd_packet_launch<T, D>(a, l, s) : kd_query_launch<T, D>(a, l, s);
+    int rc;
+    if constexpr (sizeof(T) == 8) {
+        if (filtered) {
+            FilterArgs f;
+            f.f.pts = static_cast<const PointRec<float>*>(t->d_filter[0]);
+            f.f.boxes = static_cast<const PointRec<float>*>(t->d_filter[1]);
+            f.f.medians = static_cast<const float*>(t->d_filter[2]);
+            f.f.frame = static_cast<const Frame*>(t->d_filter[3]);
+            f.pts = a.pts;
+            f.levels = L;
+            f.q = q;
+            f.nq = nq;
+            f.k = k;
+            f.order = order;
+            f.out_d = dists;
+            f.out_i = idx;
+            f.work = counter;
+            rc = kd_filtered_launch(f, D, R, grid, s);
+        } else {
+            rc = packet ? kd_packet_launch<T, D>(a, l, s) : kd_query_launch<T, D>(a, l, s);
+        }
+    } else {
+        rc = packet ? kd_packet_launch<T, D>(a, l, s) : kd_query_launch<T, D>(a, l, s);
+    }
     if (rc == TK_OK && o.kernel_stop_event) cudaEventRecord(static_cast<cudaEvent_t>(o.kernel_stop_event), s);
     return rc;
 }
@@ -637,6 +679,12 @@ void set_image(tk_tree* t, void* image) {
     t->d_medians = p + im.medians;
     t->d_leaf_off = reinterpret_cast<int32_t*>(p + im.leaf_off);
     if (t->dims > 3) t->d_perm = reinterpret_cast<int32_t*>(p + im.perm);
+    if (im.f_pts) {
+        t->d_filter[0] = p + im.f_pts;
+        t->d_filter[1] = p + im.f_boxes;
+        t->d_filter[2] = p + im.f_medians;
+        t->d_filter[3] = p + im.f_frame;
+    }
     t->device_bytes = int64_t(im.total);
 }
 
@@ -802,7 +850,7 @@ size_t tk_tree_image_size(int64_t n, int dims, int dtype, int search_levels) {
 int tk_tree_search_levels(int64_t n, int dims, int dtype, int levels) {
     (void)dtype;
     // the deepest that query_levels asks for
-    const int deep = log2_round(double(std::max<int64_t>(n, 1)) / (dims > 3 ? 90.0 : kOneLaneLeaf));
+    const int deep = log2_round(double(std::max<int64_t>(n, 1)) / (dims > 3 ? 90.0 : one_lane_leaf(n)));
     return std::min(kMaxLevels, std::max(levels, deep));
 }
 
@@ -959,6 +1007,7 @@ tk_tree transient_tree(int64_t n, int64_t nq, int dims, int k, int dtype) {
     t.own_image = false;
     t.auto_depth = true;
     t.search_levels = kMaxLevels;
+    if (tree_image(n, dims, dtype, 1).f_pts) t.d_filter[0] = &t;  // it will have one: shapes the query (set_image places it)
     t.search_levels = query_levels(&t, auto_lanes(&t, nq, k), k);
     t.levels = t.search_levels;
     return t;

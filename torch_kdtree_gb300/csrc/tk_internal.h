@@ -68,10 +68,12 @@ namespace tk {
 struct HostPipe;
 void free_host_pipe(HostPipe* p);
 // Byte offsets of a GPU-built tree's device image, one allocation: points,
-// node boxes, split values, leaf offsets and (4-8 dims) original indices of
-// a tree whose leaves lie at depth `levels`.
+// node boxes, split values, leaf offsets, (4-8 dims) original indices and
+// (float64, 1-3 dims) the float filter of a tree whose leaves lie at depth `levels`.
 struct TreeImage {
     size_t pts = 0, boxes = 0, medians = 0, leaf_off = 0, perm = 0, total = 0;
+    // float64, 1-3 dims: the float filter (kd_filter.cuh)
+    size_t f_pts = 0, f_boxes = 0, f_medians = 0, f_frame = 0;
 };
 TreeImage tree_image(int64_t n, int dims, int dtype, int levels);
 // Scratch bytes of a GPU build.
@@ -124,6 +126,7 @@ struct tk_tree {
     int32_t* d_leaf_off = nullptr;  // int32[2^L + 1]
     void* d_boxes = nullptr;     // per node {lo.xyz, 0}, {hi.xyz, 0} (see tk_device.cuh); lo / hi rows when wide
     int32_t* d_perm = nullptr;   // trees of 4-8 dims: original index of each point (records hold coordinates only)
+    const void* d_filter[4] = {};  // float filter of float64 trees: points, boxes, split values, frame (kd_filter.cuh)
     bool one_image = false;      // the arrays above are parts of one allocation that starts at d_pts ...
     bool own_image = true;       // ... which the tree frees, unless the caller provided it
     int64_t device_bytes = 0;

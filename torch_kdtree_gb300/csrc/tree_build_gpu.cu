@@ -33,6 +33,7 @@
 #include <string>
 #include <vector>
 
+#include "kd_filter.cuh"
 #include "tk_device.cuh"
 #include "tk_internal.h"
 
@@ -701,6 +702,61 @@ __global__ void __launch_bounds__(kSubThreads) k_subtrees(const T* __restrict__ 
     for (int i = t; i < cnt; i += kSubThreads) write_point<T>(pts, dims, im, glo + i, ids[arr[fa * kSub + i]]);
 }
 
+// ---------------------------------------------------------- float filter --
+
+// Centre and scale of the cloud from its root box; a cloud with infinite
+// coordinates keeps its own.
+__device__ __forceinline__ Frame cloud_frame(const PointRec<double>* boxes) {
+    const PointRec<double> lo = boxes[0], hi = boxes[1];
+    const double l[3] = {lo.x, lo.y, lo.z}, h[3] = {hi.x, hi.y, hi.z};
+    Frame f;
+    double extent = 0.0;
+    for (int c = 0; c < 3; ++c) {
+        f.centre[c] = l[c] + 0.5 * (h[c] - l[c]);
+        if (!(fabs(f.centre[c]) <= 1.7e308)) f.centre[c] = 0.0;
+        extent = fmax(extent, h[c] - l[c]);
+    }
+    int e = 0;
+    if (extent > 0.0 && extent <= 1.7e308) e = -ilogb(extent);
+    f.scale = ldexp(1.0, max(-400, min(400, e)));
+    return f;
+}
+
+// Float images of points, boxes (rounded outwards) and split values.
+__global__ void __launch_bounds__(256) k_fill_filter(const PointRec<double>* __restrict__ pts, int64_t n,
+                                                     const PointRec<double>* __restrict__ boxes, int64_t nodes,
+                                                     const double* __restrict__ medians, int64_t splits, int dims,
+                                                     PointRec<float>* __restrict__ f_pts,
+                                                     PointRec<float>* __restrict__ f_boxes,
+                                                     float* __restrict__ f_medians, Frame* __restrict__ frame) {
+    __shared__ Frame f;
+    if (threadIdx.x == 0) f = cloud_frame(boxes);
+    __syncthreads();
+    if (blockIdx.x == 0 && threadIdx.x == 0) *frame = f;
+    const int64_t i = int64_t(blockIdx.x) * 256 + threadIdx.x;
+    if (i < n) {
+        const PointRec<double> p = pts[i];
+        f_pts[i] = PointRec<float>{__double2float_rn((p.x - f.centre[0]) * f.scale),
+                                   __double2float_rn((p.y - f.centre[1]) * f.scale),
+                                   __double2float_rn((p.z - f.centre[2]) * f.scale), 0.f};
+    }
+    if (i < nodes) {
+        const PointRec<double> lo = boxes[2 * i], hi = boxes[2 * i + 1];
+        f_boxes[2 * i] = PointRec<float>{__double2float_rd(frame_down(lo.x, f.centre[0], f.scale)),
+                                         __double2float_rd(frame_down(lo.y, f.centre[1], f.scale)),
+                                         __double2float_rd(frame_down(lo.z, f.centre[2], f.scale)),
+                                         __uint_as_float(rec_index(lo))};
+        f_boxes[2 * i + 1] = PointRec<float>{__double2float_ru(frame_up(hi.x, f.centre[0], f.scale)),
+                                             __double2float_ru(frame_up(hi.y, f.centre[1], f.scale)),
+                                             __double2float_ru(frame_up(hi.z, f.centre[2], f.scale)),
+                                             __uint_as_float(rec_index(hi))};
+    }
+    if (i < splits) {
+        const int ax = (31 - __clz(int(i) + 1)) % dims;
+        f_medians[i] = __double2float_rn((medians[i] - f.centre[ax]) * f.scale);
+    }
+}
+
 size_t subtree_smem(int dims) { return size_t(kSub) * (4 + 4 + 2 * dims + 1); }
 
 size_t align256(size_t v) { return (v + 255) / 256 * 256; }
@@ -771,6 +827,16 @@ TreeImage tree_image(int64_t n, int dims, int dtype, int levels) {
     o += align256(sizeof(int32_t) * (nleaves + 1));
     im.perm = o;
     if (wide) o += align256(sizeof(int32_t) * size_t(n));
+    if (!wide && dtype == TK_F64) {
+        im.f_pts = o;
+        o += align256(sizeof(PointRec<float>) * size_t(n));
+        im.f_boxes = o;
+        o += align256(sizeof(PointRec<float>) * 2 * (2 * nleaves - 1));
+        im.f_medians = o;
+        o += align256(sizeof(float) * nleaves);
+        im.f_frame = o;
+        o += align256(sizeof(Frame));
+    }
     im.total = o;
     return im;
 }
@@ -884,6 +950,20 @@ int enqueue_device_tree(const T* pts, int64_t n, int dims, void* stream, const t
                                                         reinterpret_cast<uint16_t*>(ws + w.key_b));
     }
     TK_TRY(cudaGetLastError());
+    if constexpr (sizeof(T) == 8) {
+        if (t->d_filter[0]) {
+            const int64_t nodes = (int64_t(2) << L) - 1, splits = (int64_t(1) << L) - 1;
+            const int64_t work = std::max(n, nodes);
+            k_fill_filter<<<unsigned((work + 255) / 256), 256, 0, s>>>(
+                static_cast<const PointRec<double>*>(t->d_pts), n, static_cast<const PointRec<double>*>(t->d_boxes), nodes,
+                static_cast<const double*>(t->d_medians), splits, dims,
+                static_cast<PointRec<float>*>(const_cast<void*>(t->d_filter[0])),
+                static_cast<PointRec<float>*>(const_cast<void*>(t->d_filter[1])),
+                static_cast<float*>(const_cast<void*>(t->d_filter[2])),
+                static_cast<Frame*>(const_cast<void*>(t->d_filter[3])));
+            TK_TRY(cudaGetLastError());
+        }
+    }
     return TK_OK;
 }
 
