@@ -410,7 +410,9 @@ __global__ void __launch_bounds__(kKdBlock) k_kd_query(const KdArgs<T> a) {
     const int gid = lane / G;
 
     for (int round = 0;;) {
-        const int base = next_queries(a.work, kGroupsPerWarp, a.nq, round);
+        int base;
+        if constexpr (G == 32) base = next_queries(a.work, 1);
+        else base = next_queries(a.work, kGroupsPerWarp, a.nq, round);
         if (base >= a.nq) break;
         const int t = base + gid;
         if (t < a.nq) {
@@ -418,6 +420,7 @@ __global__ void __launch_bounds__(kKdBlock) k_kd_query(const KdArgs<T> a) {
             kd_query_one<T, D, G, R>(a, s_med, buf, qi, gmask, gl, gbase);
         }
         __syncwarp();
+        if (G == 32 && !a.work) break;
     }
 }
 
