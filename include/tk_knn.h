@@ -243,8 +243,8 @@ int tk_batch_destroy(tk_batch* batch);
 size_t tk_batch_workspace_size(const tk_batch* batch);
 /* Number of output elements (sum of q_counts[c] * ks[c]). */
 int64_t tk_batch_output_size(const tk_batch* batch);
-/* All clouds in one persistent launch fed by a global work counter (plus
- * the binning kernels).  Device work only, no host synchronisation and no
+/* All clouds in persistent launches fed by work counters, one per power of
+ * two that the clouds' k round up to (plus the binning kernels).  Device work only, no host synchronisation and no
  * allocation: it can be captured in a CUDA graph.  threads_per_query: 0 =
  * auto, 1 (max k <= 16), or 8 / 32 (any k): trees of 1-3 dims run groups
  * of 8 lanes, trees of 4-8 dims groups of 32 (their kernels' shapes).

@@ -125,3 +125,39 @@ def test_random_batches(oracle):
             msg = f"case {case} cloud {c}: dims={dims} {np.dtype(dtype).name} n={len(r)} k={k} tpq={tpq}"
             np.testing.assert_array_equal(db.cpu().numpy(), bd, err_msg=msg)
             np.testing.assert_array_equal(ib.cpu().numpy(), bi, err_msg=msg)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float64])
+@pytest.mark.parametrize("dims", [1, 2, 3])
+@pytest.mark.parametrize("ks", [(1,), (16, 1, 2, 3, 4, 5, 9, 8, 1), (100, 8, 1, 9, 17, 33, 65, 128, 2)])
+def test_batch_launch_per_list_length(dtype, dims, ks):
+    """Every list length has a launch of its own: one alone, and all of them,
+    with clouds that have no queries, equal points, or queries without a
+    finite cost.  Captured as well, where the launches overlap too."""
+    from torch_kdtree_gb300.batched import BatchedKDTrees
+    gen = torch.Generator(device=cuda)
+    gen.manual_seed(5)
+    refs, qs = [], []
+    for c, k in enumerate(ks):
+        n = k + 37 * c + (3000 if c % 3 == 2 else 1)
+        m = (0, 1, 33, 1000)[c % 4] if len(ks) > 1 else 70
+        r = torch.randn(n, dims, device=cuda, dtype=dtype, generator=gen)
+        q = torch.randn(m, dims, device=cuda, dtype=dtype, generator=gen)
+        if c == 2:
+            r[:] = 1.0
+        if c == 3:
+            q[::7] = float("inf")
+            q[::11] = float("nan")
+        refs.append(r)
+        qs.append(q)
+    b = BatchedKDTrees(refs, list(ks), [q.shape[0] for q in qs])
+    d_b, i_b = b.query(qs)
+    replay = b.graph(torch.cat(qs))
+    b.out_dists.fill_(-1)
+    replay()
+    d_g, i_g = b.split(b.out_dists.clone()), b.split(b.out_idx.clone())
+    b.query_each(qs)
+    for c, (d, i) in enumerate(zip(b.split(b.out_dists), b.split(b.out_idx))):
+        for db, ib in ((d_b[c], i_b[c]), (d_g[c], i_g[c])):
+            np.testing.assert_array_equal(db.cpu().numpy(), d.cpu().numpy(), err_msg=str(c))
+            np.testing.assert_array_equal(ib.cpu().numpy(), i.cpu().numpy(), err_msg=str(c))

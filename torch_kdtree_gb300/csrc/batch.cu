@@ -8,12 +8,14 @@
 //
 //   1. k_batch_bin_count: each query finds its cloud (binary search over the
 //      query prefix), descends B_c levels of that cloud's tree and counts
-//      itself into the cloud's block of cells;
-//   2. exclusive_scan over all cells; 3. k_bin_scatter -> processing order;
-//   4. k_batch_query: warps pull chunks of the binned order from one global
-//      counter (the work queue); every group looks up its query's cloud and
-//      runs the same exact search as the single-cloud kernel with that
-//      cloud's tree and k.
+//      itself into a cell.  Cells are laid out by the clouds' k (rounded up
+//      to a power of two, largest first), then by the query's cost class
+//      (costliest first), then by cloud;
+//   2. exclusive_scan over all cells; 3. k_batch_scatter -> processing order;
+//   4. k_batch_query, once per list length: warps pull chunks of the launch's
+//      part of the order from a global counter (the work queue); every group
+//      looks up its query's cloud and runs the same exact search as the
+//      single-cloud kernel with that cloud's tree and k.
 // Trees of 4-8 dimensions take the same steps with the wide trees' records
 // and search (batch_wide.cuh); all clouds of a batch have one dims.
 #include <algorithm>
@@ -38,7 +40,8 @@ struct CloudDesc {
     int leaf_shift;  // image leaves below the searched depth (unused: boxes carry their ranges)
     int k;
     int bins;       // 2^B_c cells used for binning
-    int bin_base;   // first cell of this cloud in the global cell array
+    int bin_base;   // first cell of this cloud among those of the first cost class
+    int bin_stride; // cells from one cost class to the next
 };
 
 template <typename T>
@@ -52,11 +55,39 @@ struct BatchArgs {
     T* out_d;
     int32_t* out_i;
     int* work;
-    int use_boxes;
+    int first, last;            // the launch's part of the order
 };
 
 __device__ __forceinline__ int cloud_of(const long long* prefix, int n_clouds, long long qi) {
     return batch_cloud_of(prefix, n_clouds, qi);
+}
+
+// Cost class of a query, 0 = costliest: the squared distance to the farthest
+// corner of its cell (see cost_class), against that of a cell of the same size
+// in a uniform cloud, in steps of two octaves.  Few and relative, so that the
+// classes are part of the counting sort's cell and need no sort of their own:
+// the costliest searches do not end up in a launch's last chunks, and a warp's
+// queries cost much the same.  256 ragged clouds, 4.8M queries: 4.27 ms without
+// classes, 4.20 with 8, 4.24 with 16, 4.31 with 32; 64 clouds 1.00, 0.95, 0.95,
+// 0.97.
+constexpr int kCostClasses = 8;
+
+template <typename T, int D>
+__device__ __forceinline__ int batch_cost_class(const PointRec<T>* boxes, int node, const T (&p)[D]) {
+    float far2 = 0.f, diag2 = 0.f;
+    const PointRec<T> rlo = load_rec(boxes), rhi = load_rec(boxes + 1);
+    const PointRec<T> lo = load_rec(boxes + 2 * node), hi = load_rec(boxes + 2 * node + 1);
+    const T l[3] = {lo.x, lo.y, lo.z}, h[3] = {hi.x, hi.y, hi.z};
+    const T rl[3] = {rlo.x, rlo.y, rlo.z}, rh[3] = {rhi.x, rhi.y, rhi.z};
+#pragma unroll
+    for (int c = 0; c < D; ++c) {
+        const float f = float(fmax(fabs(p[c] - l[c]), fabs(p[c] - h[c]))), g = float(rh[c] - rl[c]);
+        far2 += f * f;
+        diag2 += g * g;
+    }
+    const float n = float(int(rec_index(rhi)) - int(rec_index(rlo)));
+    const float octaves = __log2f(far2) - __log2f(diag2) + 2.f / D * __log2f(n);
+    return kCostClasses - 1 - int(fminf(fmaxf(0.5f * octaves + 2.f, 0.f), kCostClasses - 1.f));
 }
 
 template <typename T, int D>
@@ -76,59 +107,56 @@ __global__ void k_batch_bin_count(const BatchArgs<T> a, int* counts, int* bin_of
         node = 2 * node + (pick<T, D>(p, ax) < m ? 1 : 2);
         ax = (ax + 1 == D) ? 0 : ax + 1;
     }
-    const int bin = cd.bin_base + node - ((1 << B) - 1);
+    const int cost = batch_cost_class<T, D>(cd.boxes, node, p);
+    const int bin = cd.bin_base + cost * cd.bin_stride + node - ((1 << B) - 1);
     bin_of[i] = bin;
     pos_of[i] = atomicAdd(counts + bin, 1);
 }
 
-template <typename T, int D, int G, int R>
-__device__ __forceinline__ void batch_search(const CloudDesc<T>& cd, const T (&q)[D], long long local,
-                                             const BatchArgs<T>& a, unsigned gmask, int gl, int gbase) {
-    const TreeView<T> tv{cd.pts, cd.medians, cd.leaf_off, cd.levels, 0, nullptr, cd.boxes};
-    const long long o = cd.out_off + local * cd.k;
-    kd_search<T, D, G, R>(tv, q, cd.k, a.out_d + o, a.out_i + o, gmask, gl, gbase);
-}
+constexpr int kBatchBlock = 128;  // threads per block of k_batch_query
 
-// G = 1: k <= 16 (registers per lane R in {1, 4, 16});
-// G = 8: k <= 128 (R in {2, 4, 8, 16}).  Capped at 4 blocks of 256 per SM (64
-// registers for float): left free the float kernels took 72-80 registers, 3
-// blocks per SM, and ran the 256 ragged clouds 9-14% slower (a few bytes of
-// spills cost less than a quarter of the resident warps).
-template <typename T, int D, int G>
-__global__ void __launch_bounds__(256, 4) k_batch_query(const BatchArgs<T> a) {
+// One launch serves the clouds whose lists take R keys a lane; `order` holds
+// these clouds' queries next to each other.  Bound by issue (the ALU pipe 72%
+// busy, 8 of 32 lanes active where searches differ).  One kernel for all list
+// lengths gave every search the registers and the instruction footprint of the
+// longest and mixed them in one warp; a launch after another, each with its own
+// tail, is slower still (256 ragged clouds, 4.8M queries 4.57 ms against 4.41;
+// 16 clouds 0.50 against 0.30), so a launch may start while the one before it
+// runs out (4.27; 0.27; with cost classes 4.20).  It reads only what was ready
+// before the first launch, and ends after the one before it, so whatever
+// follows on the stream waits for all.
+// 1024 threads an SM (64 registers for float): left free the kernels took up to
+// 80 and ran 13-20% slower.  Blocks of 64 or 256 threads: the same; of 32: 3%
+// slower.
+template <typename T, int D, int G, int R>
+__global__ void __launch_bounds__(kBatchBlock, sizeof(T) == 4 ? 1024 / kBatchBlock : 1) k_batch_query(const BatchArgs<T> a) {
     const int lane = threadIdx.x & 31;
     const int gl = lane & (G - 1);
     const int gbase = lane & ~(G - 1);
     const unsigned gmask = group_mask<G>(lane);
     constexpr int kGroupsPerWarp = 32 / G;
     const int gid = lane / G;
+    cudaTriggerProgrammaticLaunchCompletion();  // the next launch may take the place of blocks that end
     for (;;) {
         int base = 0;
-        if (lane == 0) base = atomicAdd(a.work, kGroupsPerWarp);
+        if (lane == 0) base = a.first + atomicAdd(a.work, kGroupsPerWarp);
         base = __shfl_sync(0xFFFFFFFFu, base, 0);
-        if (base >= a.total) break;
+        if (base >= a.last) break;
         const int t = base + gid;
-        if (t < a.total) {
-            const int qi = a.order ? __ldg(a.order + t) : t;
+        if (t < a.last) {
+            const int qi = __ldg(a.order + t);
             const int c = cloud_of(a.q_prefix, a.n_clouds, qi);
             const CloudDesc<T> cd = a.desc[c];
             T q[D];
 #pragma unroll
             for (int j = 0; j < D; ++j) q[j] = a.q[(long long)qi * D + j];
-            const long long local = qi - a.q_prefix[c];
-            if (G == 1) {
-                if (cd.k <= 1) batch_search<T, D, G, 1>(cd, q, local, a, gmask, gl, gbase);
-                else if (cd.k <= 4) batch_search<T, D, G, 4>(cd, q, local, a, gmask, gl, gbase);
-                else batch_search<T, D, G, 16>(cd, q, local, a, gmask, gl, gbase);
-            } else {
-                if (cd.k <= 2 * G) batch_search<T, D, G, 2>(cd, q, local, a, gmask, gl, gbase);
-                else if (cd.k <= 4 * G) batch_search<T, D, G, 4>(cd, q, local, a, gmask, gl, gbase);
-                else if (cd.k <= 8 * G) batch_search<T, D, G, 8>(cd, q, local, a, gmask, gl, gbase);
-                else batch_search<T, D, G, 16>(cd, q, local, a, gmask, gl, gbase);
-            }
+            const TreeView<T> tv{cd.pts, cd.medians, cd.leaf_off, cd.levels, 0, nullptr, cd.boxes};
+            const long long o = cd.out_off + (qi - a.q_prefix[c]) * cd.k;
+            kd_search<T, D, G, R>(tv, q, cd.k, a.out_d + o, a.out_i + o, gmask, gl, gbase);
         }
         __syncwarp();
     }
+    cudaGridDependencySynchronize();  // the launch before this one has ended
 }
 
 __global__ void k_batch_scatter(int total, const int* bin_of, const int* pos_of, const int* offsets, int* order) {
@@ -141,6 +169,8 @@ __global__ void k_batch_scatter(int total, const int* bin_of, const int* pos_of,
 
 using namespace tk;
 
+constexpr int kClasses = 8;  // k <= 1, 2, 4 .. 128
+
 struct tk_batch {
     int dtype = TK_F32, dims = 0, device = 0, n_clouds = 0;
     int max_k = 0;
@@ -149,6 +179,9 @@ struct tk_batch {
     void* d_desc = nullptr;
     long long* d_prefix = nullptr;
     std::vector<long long> q_prefix, out_off;
+    // queries of the clouds with 2^(c-1) < k <= 2^c; cells, and so the processing
+    // order, go from the largest c to the smallest
+    long long class_q[kClasses] = {};
 };
 
 namespace {
@@ -178,6 +211,12 @@ BatchWs batch_ws(const tk_batch* b) {
     return w;
 }
 
+int k_class(int k) {
+    int c = 0;
+    while ((1 << c) < k) ++c;
+    return c;
+}
+
 int batch_bin_levels(int L, long long nq) {
     int lg = 0;
     while ((1LL << (lg + 1)) <= nq) ++lg;
@@ -201,11 +240,21 @@ void fill_desc(WideCloudDesc<T>& d, const tk_tree* t) {
     d.boxes = static_cast<const T*>(t->d_boxes);
 }
 
+template <typename T>
+void place_cells(CloudDesc<T>& d, int base, int stride) {
+    d.bin_base += base;
+    d.bin_stride = stride;
+}
+template <typename T>
+void place_cells(WideCloudDesc<T>& d, int base, int) {
+    d.bin_base += base;
+}
+
 // Desc: CloudDesc<T> (trees of 1-3 dims) or WideCloudDesc<T> (4-8 dims).
 template <typename T, typename Desc>
 int upload_descs(tk_batch* b, const tk_tree* const* trees, const int64_t* q_counts, const int32_t* ks) {
     std::vector<Desc> h(b->n_clouds);
-    int bin_base = 0;
+    int cells[kClasses] = {};
     for (int c = 0; c < b->n_clouds; ++c) {
         const tk_tree* t = trees[c];
         Desc& d = h[c];
@@ -217,10 +266,22 @@ int upload_descs(tk_batch* b, const tk_tree* const* trees, const int64_t* q_coun
         d.k = ks[c];
         const int B = batch_bin_levels(d.levels, std::max<int64_t>(q_counts[c], 1));
         d.bins = 1 << B;
-        d.bin_base = bin_base;
-        bin_base += d.bins;
+        const int kc = k_class(ks[c]);
+        d.bin_base = cells[kc];  // within its class for now
+        cells[kc] += d.bins;
+        b->class_q[kc] += q_counts[c];
     }
-    b->total_bins = bin_base;
+    const int costs = b->dims <= 3 ? kCostClasses : 1;
+    b->total_bins = 0;
+    int base[kClasses];
+    for (int kc = kClasses - 1; kc >= 0; --kc) {
+        base[kc] = b->total_bins;
+        b->total_bins += costs * cells[kc];
+    }
+    for (int c = 0; c < b->n_clouds; ++c) {
+        const int kc = k_class(ks[c]);
+        place_cells(h[c], base[kc], cells[kc]);
+    }
     cudaError_t e = cudaMalloc(&b->d_desc, sizeof(Desc) * h.size());
     if (e == cudaSuccess) e = cudaMalloc(reinterpret_cast<void**>(&b->d_prefix), sizeof(long long) * b->q_prefix.size());
     if (e != cudaSuccess) return fail(TK_ENOMEM, std::string("batch allocation: ") + cudaGetErrorString(e));
@@ -231,8 +292,27 @@ int upload_descs(tk_batch* b, const tk_tree* const* trees, const int64_t* q_coun
     return TK_OK;
 }
 
+template <typename T, int D, int G, int R>
+cudaError_t launch_batch(const BatchArgs<T>& a, int sms, cudaStream_t s) {
+    auto* kfn = &k_batch_query<T, D, G, R>;
+    int per_sm = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kfn, kBatchBlock, 0) != cudaSuccess || per_sm <= 0) per_sm = 1;
+    const int per_block = kBatchBlock / G;
+    const int need = (a.last - a.first + per_block - 1) / per_block;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(std::max(1, std::min(need, per_sm * sms)));
+    cfg.blockDim = dim3(kBatchBlock);
+    cfg.stream = s;
+    cudaLaunchAttribute overlap;
+    overlap.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    overlap.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &overlap;
+    cfg.numAttrs = a.first > 0 ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, kfn, a);
+}
+
 template <typename T, int D>
-int run_batch(const tk_batch* b, const T* q, T* dists, int32_t* idx, int G, int boxes, char* ws, cudaStream_t s) {
+int run_batch(const tk_batch* b, const T* q, T* dists, int32_t* idx, int G, char* ws, cudaStream_t s) {
     const BatchWs w = batch_ws(b);
     BatchArgs<T> a;
     a.desc = static_cast<const CloudDesc<T>*>(b->d_desc);
@@ -242,33 +322,48 @@ int run_batch(const tk_batch* b, const T* q, T* dists, int32_t* idx, int G, int 
     a.total = int(b->total_q);
     a.out_d = dists;
     a.out_i = idx;
-    a.work = reinterpret_cast<int*>(ws + w.counter);
-    a.use_boxes = boxes;
+    int* work = reinterpret_cast<int*>(ws + w.counter);  // one per launch
     int* counts = reinterpret_cast<int*>(ws + w.counts);
     int* bin_of = reinterpret_cast<int*>(ws + w.bin_of);
     int* pos_of = reinterpret_cast<int*>(ws + w.pos_of);
     int* order = reinterpret_cast<int*>(ws + w.order);
     a.order = order;
-    cudaError_t e = cudaMemsetAsync(counts, 0, sizeof(int) * size_t(b->total_bins), s);
-    if (e == cudaSuccess) e = cudaMemsetAsync(a.work, 0, sizeof(int), s);
+    // the counters lie right before the cells
+    cudaError_t e = cudaMemsetAsync(work, 0, w.counts - w.counter + sizeof(int) * size_t(b->total_bins), s);
     if (e != cudaSuccess) return fail(TK_ECUDA, std::string("memset: ") + cudaGetErrorString(e));
     const int nb = (a.total + 255) / 256;
     k_batch_bin_count<T, D><<<nb, 256, 0, s>>>(a, counts, bin_of, pos_of);
     e = exclusive_scan(counts, b->total_bins, ws + w.scan, s);
     if (e != cudaSuccess) return fail(TK_ECUDA, std::string("batch scan: ") + cudaGetErrorString(e));
     k_batch_scatter<<<nb, 256, 0, s>>>(a.total, bin_of, pos_of, counts, order);
-    const void* kfn = G == 1 ? reinterpret_cast<const void*>(&k_batch_query<T, D, 1>)
-                             : reinterpret_cast<const void*>(&k_batch_query<T, D, 8>);
-    int per_sm = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kfn, 256, 0) != cudaSuccess || per_sm <= 0) per_sm = 1;
     int sms = 1;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, b->device);
-    const int need = (a.total + 256 / G - 1) / (256 / G);
-    const int grid = std::max(1, std::min(need, per_sm * sms));
-    if (G == 1) k_batch_query<T, D, 1><<<grid, 256, 0, s>>>(a);
-    else k_batch_query<T, D, 8><<<grid, 256, 0, s>>>(a);
-    e = cudaGetLastError();
-    if (e != cudaSuccess) return fail(TK_ECUDA, std::string("batch launch: ") + cudaGetErrorString(e));
+    a.last = 0;
+    for (int c = kClasses - 1; c >= 0;) {
+        const int lg = G == 1 ? c : std::max(0, c - 3);  // R = 2^lg keys a lane
+        a.first = a.last;
+        for (; c >= 0 && (G == 1 ? c : std::max(0, c - 3)) == lg; --c) a.last += int(b->class_q[c]);
+        if (a.last == a.first) continue;
+        a.work = work++;
+        if (G == 1) {
+            switch (lg) {
+                case 0: e = launch_batch<T, D, 1, 1>(a, sms, s); break;
+                case 1: e = launch_batch<T, D, 1, 2>(a, sms, s); break;
+                case 2: e = launch_batch<T, D, 1, 4>(a, sms, s); break;
+                case 3: e = launch_batch<T, D, 1, 8>(a, sms, s); break;
+                default: e = launch_batch<T, D, 1, 16>(a, sms, s); break;  // the caller saw to k <= 16
+            }
+        } else {
+            switch (lg) {
+                case 0: e = launch_batch<T, D, 8, 1>(a, sms, s); break;
+                case 1: e = launch_batch<T, D, 8, 2>(a, sms, s); break;
+                case 2: e = launch_batch<T, D, 8, 4>(a, sms, s); break;
+                case 3: e = launch_batch<T, D, 8, 8>(a, sms, s); break;
+                default: e = launch_batch<T, D, 8, 16>(a, sms, s); break;
+            }
+        }
+        if (e != cudaSuccess) return fail(TK_ECUDA, std::string("batch launch: ") + cudaGetErrorString(e));
+    }
     return TK_OK;
 }
 
@@ -406,15 +501,15 @@ int tk_batch_query(const tk_batch* b, const void* q, void* dists, int32_t* idx, 
     if (G == 32) G = 8;  // trees of 1-3 dims: 8-lane groups serve every k <= 128
     if (b->dtype == TK_F32) {
         switch (b->dims) {
-            case 1: return run_batch<float, 1>(b, static_cast<const float*>(q), static_cast<float*>(dists), idx, G, prune_boxes != 0, ws, s);
-            case 2: return run_batch<float, 2>(b, static_cast<const float*>(q), static_cast<float*>(dists), idx, G, prune_boxes != 0, ws, s);
-            default: return run_batch<float, 3>(b, static_cast<const float*>(q), static_cast<float*>(dists), idx, G, prune_boxes != 0, ws, s);
+            case 1: return run_batch<float, 1>(b, static_cast<const float*>(q), static_cast<float*>(dists), idx, G, ws, s);
+            case 2: return run_batch<float, 2>(b, static_cast<const float*>(q), static_cast<float*>(dists), idx, G, ws, s);
+            default: return run_batch<float, 3>(b, static_cast<const float*>(q), static_cast<float*>(dists), idx, G, ws, s);
         }
     }
     switch (b->dims) {
-        case 1: return run_batch<double, 1>(b, static_cast<const double*>(q), static_cast<double*>(dists), idx, G, prune_boxes != 0, ws, s);
-        case 2: return run_batch<double, 2>(b, static_cast<const double*>(q), static_cast<double*>(dists), idx, G, prune_boxes != 0, ws, s);
-        default: return run_batch<double, 3>(b, static_cast<const double*>(q), static_cast<double*>(dists), idx, G, prune_boxes != 0, ws, s);
+        case 1: return run_batch<double, 1>(b, static_cast<const double*>(q), static_cast<double*>(dists), idx, G, ws, s);
+        case 2: return run_batch<double, 2>(b, static_cast<const double*>(q), static_cast<double*>(dists), idx, G, ws, s);
+        default: return run_batch<double, 3>(b, static_cast<const double*>(q), static_cast<double*>(dists), idx, G, ws, s);
     }
 }
 
