@@ -390,3 +390,19 @@ def test_exact_mode_captured_in_a_graph():
         g.replay()
         torch.cuda.synchronize()
         assert torch.equal(dd, want[0]) and torch.equal(ii, want[1])
+
+
+@pytest.mark.parametrize("mode", ["tf32", "bf16_split"])
+@pytest.mark.parametrize("extra", [1, 300, 9000])
+@pytest.mark.parametrize("k", [1, 32])
+def test_tensor_core_rows_left_over(mode, extra, k, oracle):
+    """Row blocks left over after whole waves of blocks are searched in slices
+    of their own: a few of them, some, and more than half a wave."""
+    rng = np.random.default_rng(extra + k)
+    nq = 128 * torch.cuda.get_device_properties(0).multi_processor_count + extra
+    ref = rng.standard_normal((9000, 8)).astype(np.float32)
+    q = rng.standard_normal((nq, 8)).astype(np.float32)
+    bd, bi = oracle.brute(ref, q, k)
+    dd, ii = tk().nn_distance(torch.from_numpy(ref).to(cuda), torch.from_numpy(q).to(cuda), k, mode=mode)
+    np.testing.assert_array_equal(dd.cpu().numpy(), bd)
+    np.testing.assert_array_equal(ii.cpu().numpy(), bi)

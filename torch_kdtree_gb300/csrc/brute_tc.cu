@@ -44,7 +44,9 @@ struct TcWs {
     size_t a_pack, b_pack, a_lo, b_lo, rnorm, qnorm, fail_count, fail_list, brute, err, total;
     size_t cand_s, cand_i, tau;  // mma.sync search
     size_t hits, counts, thr;    // tcgen05 search
-    int KP, C, nsplit, pstride, rank, wanted;
+    int KP, C, nsplit, wanted;
+    int split_from;          // tcgen05 search: see first_slice
+    Tc5Slices head, tail;
     bool tc5;  // tcgen05 path
 };
 
@@ -83,38 +85,71 @@ TcWs tc_layout(int64_t n, int64_t nq, int d, int k, int mode, int sms) {
     if (w.tc5) {
         const int qblocks = int((nq + kT5Rows - 1) / kT5Rows);
         // Slices of the references per row block, and the sample that gives a
-        // slice's threshold: max(150, 5k) references of a row are to score
-        // below the thresholds of its slices together (the certificate wants
-        // about 2k with room), by the rank-th smallest minimum of every
-        // pstride-th tile, rank about 25 (the threshold scatters by 1 / sqrt(rank)) --
-        // so the more slices, the larger the sampled share.  One block per
-        // SM: the slice count with the least (1 + share) / SMs used, of at
-        // least 8 tiles a slice.
+        // slice's threshold: `wanted` references of a row are to score below
+        // the thresholds of its slices together (the certificate wants about
+        // 2k with room), by the `rank`-th smallest minimum of every pstride-th
+        // tile.  The threshold scatters by 1 / sqrt(rank), and every reference
+        // below it costs a list entry and an exact distance.  262,144 x 65,536,
+        // d=32, ms for (wanted, rank): TF32 k=16 (150, 25) 3.70, (100, 16)
+        // 3.38, (100, 12) 3.27, (80, 12) 3.46, where some rows miss their
+        // certificate; k=32 (5k, 25) 3.80, (4k, 20) 3.53, (4.5k, 12) 3.71;
+        // BF16 k=32 (5k, 25) 4.34, (4k, 20) 4.12, (5k, 12) 4.00.
         const int64_t tiles = (n + kT5Cols - 1) / kT5Cols;
         const int most = int(std::min<int64_t>(24, std::max<int64_t>(1, tiles / 8)));
         // small calls, where it costs little, want more: their many short
         // slices scatter more, and TF32's error is large against the spacing
         // of near neighbours in few dimensions
-        double wanted = std::max(150.0, 5.0 * k);
+        double wanted = std::max(100.0, (mode == TK_BRUTE_TF32 ? 4.0 : 5.0) * k);
+        const double rank = mode == TK_BRUTE_TF32 && wanted < 6.0 * k ? 20.0 : 12.0;
         if (qblocks <= (mode == TK_BRUTE_TF32 && d <= 8 ? sms : sms / 8)) wanted = std::max(wanted, 16.0 * k);
         w.wanted = int(wanted);
+        constexpr double kBlockTiles = 16.0;  // a block's start and its thresholds, in tiles
+        auto slices = [&](int ns, double below) {
+            const int64_t per = (tiles + ns - 1) / ns;
+            Tc5Slices sl;
+            sl.nsplit = ns;
+            sl.pstride = per >= 64 ? std::max(1, std::min(16, int(below / rank))) : 1;
+            // of at most 0.8 of the minima there are (see k_tc5_select)
+            const int64_t pre = (per + sl.pstride - 1) / sl.pstride;
+            const int minima = int(pre <= 8 ? 16 * pre : std::min<int64_t>(kT5Minima, 4 * std::min<int64_t>(pre, 32)));
+            sl.rank = std::max(8, std::min({64, minima * 4 / 5, int(below / sl.pstride + 0.5)}));
+            return sl;
+        };
+        // time of so many row blocks in ns slices each, in whole passes over the references
+        auto cost = [&](int blocks, const Tc5Slices& sl) {
+            return ((1.0 + 1.0 / sl.pstride) / sl.nsplit + kBlockTiles / double(tiles)) * std::ceil(double(blocks) * sl.nsplit / sms);
+        };
         double best = 1e30;
         for (int ns = 1; ns <= most; ++ns) {
-            const int64_t per = (tiles + ns - 1) / ns;
-            const double below = wanted / ns;
-            const int stride = per >= 64 ? std::max(1, std::min(8, int(below / 25.0))) : 1;
-            const double blocks = double(qblocks) * ns;
-            const double cost = (1.0 + 1.0 / stride) * std::ceil(blocks / sms) * sms / blocks;
-            if (cost < 0.98 * best) {
-                best = cost;
-                w.nsplit = ns;
-                w.pstride = stride;
-                // of at most 0.8 of the minima there are (see k_tc5_select)
-                const int64_t pre = (per + stride - 1) / stride;
-                const int minima = int(pre <= 8 ? 16 * pre : std::min<int64_t>(kT5Minima, 4 * std::min<int64_t>(pre, 32)));
-                w.rank = std::max(8, std::min({64, minima * 4 / 5, int(below / stride + 0.5)}));
+            const Tc5Slices sl = slices(ns, wanted / ns);
+            const double c = cost(qblocks, sl);
+            if (c < 0.98 * best) {
+                best = c;
+                w.head = w.tail = sl;
+                w.split_from = qblocks;
             }
         }
+        // Whole waves of row blocks, one block per SM, and slices for the blocks
+        // left over, which would hold the chip for a wave that is nearly empty:
+        // 512 row blocks on 152 SMs are 3 waves and half a wave of 56 x 2
+        // slices (262,144 x 65,536, d=32, TF32, k=1 4.05 -> 3.26 ms with the
+        // smaller sample above, of which the split 0.38; 20,000 queries 1.75 ->
+        // 1.14).  The certificate takes the lowest threshold of a row's slices,
+        // so they want more in all.
+        const int whole = qblocks / sms * sms;
+        for (int ns = 2; ns <= most && whole > 0 && whole < qblocks; ++ns) {
+            const double below = wanted / ns + std::sqrt(2.0 * std::log(double(ns)) * wanted / ns);
+            const Tc5Slices one = slices(1, wanted), sl = slices(ns, below);
+            const double c = cost(whole, one) + cost(qblocks - whole, sl);
+            if (c < 0.98 * best) {
+                best = c;
+                w.head = one;
+                w.tail = sl;
+                w.split_from = whole;
+                w.wanted = int(std::max(wanted, ns * below));
+            }
+        }
+        w.nsplit = w.head.nsplit;
         const size_t nq_pad = size_t(qblocks) * kT5Rows;
         const size_t n_pad = size_t((n + kT5Cols - 1) / kT5Cols) * kT5Cols;
         w.a_pack = o; o += align256(es * nq_pad * w.KP);
@@ -136,7 +171,8 @@ TcWs tc_layout(int64_t n, int64_t nq, int d, int k, int mode, int sms) {
     }
     w.err = o; o += 256;
     if (w.tc5) {
-        const size_t lists = (size_t(nq) + kT5Rows - 1) / kT5Rows * kT5Rows * w.nsplit * kT5Parts;
+        const int64_t rows = (nq + kT5Rows - 1) / kT5Rows * kT5Rows;
+        const size_t lists = size_t(first_slice(rows, w.split_from, w.head.nsplit, w.tail.nsplit)) * kT5Parts;
         w.hits = o; o += align256(8 * lists * kT5Cap);
         w.counts = o; o += align256(4 * lists);
         w.thr = o; o += align256(4 * lists);
@@ -232,9 +268,9 @@ int run_brute_tc(const float* ref, int64_t n, const float* q, int64_t nq, int d,
         t5.b_lo = blo;
         t5.nq = nq32;
         t5.tiles = tiles;
-        t5.nsplit = w.nsplit;
-        t5.pstride = w.pstride;
-        t5.rank = w.rank;
+        t5.split_from = w.split_from;
+        t5.head = w.head;
+        t5.tail = w.tail;
         t5.hits = reinterpret_cast<uint2*>(p + w.hits);
         t5.counts = reinterpret_cast<int*>(p + w.counts);
         t5.thr = reinterpret_cast<float*>(p + w.thr);
@@ -293,6 +329,8 @@ int run_brute_tc(const float* ref, int64_t n, const float* q, int64_t nq, int d,
     ra.k = k;
     ra.C = w.C;
     ra.nsplit = w.nsplit;
+    ra.split_from = w.split_from;
+    ra.tail_nsplit = w.tail.nsplit;
     ra.cand_s = a.cand_s;
     ra.cand_i = a.cand_i;
     ra.tau = a.tau;

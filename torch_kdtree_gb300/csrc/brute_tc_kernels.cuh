@@ -339,16 +339,30 @@ __global__ void __launch_bounds__(256) k_tc5_pack(const float* __restrict__ x, i
     }
 }
 
+// Slices of the references of a row block, and how their thresholds come about
+// (see k_tc5_select).
+struct Tc5Slices {
+    int nsplit;
+    int pstride;  // every pstride-th tile of a slice is sampled
+    int rank;     // the threshold is the rank-th smallest of the sample's minima
+};
+
+// The row blocks before `split_from` and those from there on may have
+// different slices; lists are kept by query, then slice, then part.
+__host__ __device__ inline long long first_slice(long long row, int split_from, int head, int tail) {
+    const long long b = (long long)split_from * kT5Rows;
+    return row < b ? row * head : b * head + (row - b) * tail;
+}
+
 struct Tc5Args {
     const unsigned char* a_hi;  // packed queries, blocks of 128 rows
     const unsigned char* a_lo;
     const unsigned char* b_hi;  // packed references, tiles of 256 rows
     const unsigned char* b_lo;
-    int nq, tiles, nsplit;
-    int pstride;                // every pstride-th tile of a slice is sampled
-    int rank;                   // the threshold is the rank-th smallest of the sample's minima
-    uint2* hits;                // [padded nq][nsplit][kT5Parts][CAP]: score bits, reference
-    int* counts;                // [padded nq][nsplit][kT5Parts]
+    int nq, tiles, split_from;  // row blocks with the head's slices
+    Tc5Slices head, tail;
+    uint2* hits;                // [slices of all rows, see first_slice][kT5Parts][CAP]: score bits, reference
+    int* counts;                // [slices of all rows][kT5Parts]
     float* thr;                 // same shape: every reference of the part scoring below it is in its list
     int* err;                   // kTcErrTimeout set when a bounded wait ran out
     uint32_t max_tries;         // polls of each mbarrier wait before giving up
@@ -440,13 +454,14 @@ __device__ __forceinline__ float min3(float a, float b, float c) {
 // in which threads only keep minima of groups of scores, 128 per row, rounded
 // up to 16 bits; the threshold is the rank-th smallest of a row's minima.  The
 // groups being spread over the cloud, about rank * pstride references of the
-// slice score below it; run_brute_tc picks both so that some 150 references
-// of a row do over all slices.  Nothing depends on that: a list that fills up
+// slice score below it; tc_layout picks both so that some 100 references (more
+// for large k) of a row do over all slices.  Nothing depends on that: a list that fills up
 // lowers its own threshold to its kT5Kept-th best, and whatever the threshold, the
 // references that no list holds score at or above it, which is all that the
 // certificate uses.
 //
-// 262,144 x 65,536, d=32, k=32, TF32: 3.5 ms, tensor pipe 45% busy, issue
+// 262,144 x 65,536, d=32, k=32, TF32: 2.9 ms; in whole waves of blocks 3.5 ms,
+// of which it was measured: tensor pipe 45% busy, issue
 // slots 51%: 4 epilogue warps per scheduler cannot cover the latency of their
 // own minima, votes and branches.  (Before: a short sample, then per-row
 // sorted lists kept up to date in the registers of 4-lane groups, a barrier
@@ -470,12 +485,19 @@ __global__ void __launch_bounds__(kT5Threads, 1) k_tc5_select(const Tc5Args a) {
     constexpr int NEPI = 32 * kT5EpiWarps;
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int per = (a.tiles + a.nsplit - 1) / a.nsplit;
-    const int tile0 = min(a.tiles, per * int(blockIdx.y));
+    // row blocks of the head come first, one after another for each of its slices
+    const bool in_tail = int(blockIdx.x) >= a.split_from * a.head.nsplit;
+    const Tc5Slices sl = in_tail ? a.tail : a.head;
+    const int in_part = int(blockIdx.x) - (in_tail ? a.split_from * a.head.nsplit : 0);
+    const int part_rows = in_tail ? (a.nq + kT5Rows - 1) / kT5Rows - a.split_from : a.split_from;
+    const int slice = in_part / part_rows;
+    const int rblock = in_part - slice * part_rows + (in_tail ? a.split_from : 0);
+    const int per = (a.tiles + sl.nsplit - 1) / sl.nsplit;
+    const int tile0 = min(a.tiles, per * slice);
     const int ntiles = min(a.tiles, tile0 + per) - tile0;
-    const int npre = (ntiles + a.pstride - 1) / a.pstride;  // sampled tiles
+    const int npre = (ntiles + sl.pstride - 1) / sl.pstride;  // sampled tiles
     const int nseq = npre + ntiles;  // tiles through the pipeline
-    auto tile_of = [&](int t) { return tile0 + (t < npre ? t * a.pstride : t - npre); };
+    auto tile_of = [&](int t) { return tile0 + (t < npre ? t * sl.pstride : t - npre); };
 
     if (tid == 0) {
         sm100::mbar_init(&full_a, 1);
@@ -510,8 +532,8 @@ __global__ void __launch_bounds__(kT5Threads, 1) k_tc5_select(const Tc5Args a) {
                 b_issued = t + 1;
             };
             sm100::mbar_arrive_expect_tx(&full_a, PL * A_BYTES);
-            sm100::bulk_g2s(sA, a.a_hi + (size_t)blockIdx.x * A_BYTES, A_BYTES, &full_a);
-            if (PL == 2) sm100::bulk_g2s(sA + A_BYTES, a.a_lo + (size_t)blockIdx.x * A_BYTES, A_BYTES, &full_a);
+            sm100::bulk_g2s(sA, a.a_hi + (size_t)rblock * A_BYTES, A_BYTES, &full_a);
+            if (PL == 2) sm100::bulk_g2s(sA + A_BYTES, a.a_lo + (size_t)rblock * A_BYTES, A_BYTES, &full_a);
             for (int t = 0; t < STAGES && t < nseq; ++t) load(t);
             for (int t = 0; t < nseq; ++t) {
                 const int st = t % STAGES, ac = t & 1;
@@ -648,7 +670,7 @@ __global__ void __launch_bounds__(kT5Threads, 1) k_tc5_select(const Tc5Args a) {
                 for (int i = 0; i < kT5Minima / 8; ++i) c += ((m[i] & 0xFFFFu) <= mid ? 1 : 0) + ((m[i] >> 16) <= mid ? 1 : 0);
                 c += __shfl_xor_sync(0xFFFFFFFFu, c, 1);
                 c += __shfl_xor_sync(0xFFFFFFFFu, c, 2);
-                if (c >= a.rank) hi = mid;
+                if (c >= sl.rank) hi = mid;
                 else lo = min(mid + 1u, 0xFFFFu);
             }
             // rounded up to the end of its 16-bit bucket, and low enough to
@@ -657,10 +679,12 @@ __global__ void __launch_bounds__(kT5Threads, 1) k_tc5_select(const Tc5Args a) {
             if (gl == 0) sThr[grow] = lo < 0xFF80u ? fminf(bits_score((lo << 16) | 0xFFFFu), kT5PadNorm) : kT5PadNorm;
         }
         bar_all();
-        const long long lidx = (((long long)blockIdx.x * kT5Rows + myrow) * a.nsplit + blockIdx.y) * kT5Parts + part;
+        const int row = rblock * kT5Rows + myrow;
+        const long long lidx =
+            (first_slice(row, a.split_from, a.head.nsplit, a.tail.nsplit) + slice) * kT5Parts + part;
         uint2* list = a.hits + lidx * CAP;
         // (rows past the last query take no hits: all their scores are equal)
-        float thr = blockIdx.x * kT5Rows + myrow < a.nq ? sThr[myrow] : -__int_as_float(0x7f800000);
+        float thr = row < a.nq ? sThr[myrow] : -__int_as_float(0x7f800000);
         int cnt = 0;
         // Hits of a half (32 columns from col0 on).  Branches are taken by the
         // whole warp (votes): few of its 512 scores of 16 columns are hits,
@@ -730,6 +754,7 @@ struct RerankArgs {
     const float* ref;     // [n, d] float32 originals
     const float* q;       // [nq, d]
     int n, nq, d, k, C, nsplit;
+    int split_from, tail_nsplit;  // tcgen05 search, see first_slice (nsplit: the head's)
     const float* cand_s;  // mma.sync search: [nq, nsplit, C]
     const int32_t* cand_i;
     const float* tau;     // [nq, nsplit]
@@ -862,14 +887,15 @@ static __global__ void __launch_bounds__(256) k_tc5_rerank(const RerankArgs a) {
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int qi = blockIdx.x * 8 + w;
     if (qi >= a.nq) return;
-    const int nl = a.nsplit * kT5Parts;
-    const int* counts = a.counts + (long long)qi * nl;
-    const uint2* hits = a.hits + (long long)qi * nl * CAP;
+    const int nl = (qi < (long long)a.split_from * kT5Rows ? a.nsplit : a.tail_nsplit) * kT5Parts;
+    const long long list0 = first_slice(qi, a.split_from, a.nsplit, a.tail_nsplit) * kT5Parts;
+    const int* counts = a.counts + list0;
+    const uint2* hits = a.hits + list0 * CAP;
     int total = 0;
     float tau = __int_as_float(0x7f800000);
     for (int l = lane; l < nl; l += 32) {
         total += counts[l];
-        tau = fminf(tau, a.thr[(long long)qi * nl + l]);
+        tau = fminf(tau, a.thr[list0 + l]);
     }
     total = __reduce_add_sync(0xFFFFFFFFu, total);
 #pragma unroll
@@ -952,7 +978,8 @@ int launch_tc5(const Tc5Args& a, int qblocks, cudaStream_t s) {
     const void* fn = reinterpret_cast<const void*>(&k_tc5_select<MODE, KP>);
     cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(Sh::SMEM));
     if (e != cudaSuccess) return fail(TK_ECUDA, std::string("tcgen05 select smem: ") + cudaGetErrorString(e));
-    k_tc5_select<MODE, KP><<<dim3(qblocks, a.nsplit), kT5Threads, Sh::SMEM, s>>>(a);
+    const int grid = a.split_from * a.head.nsplit + (qblocks - a.split_from) * a.tail.nsplit;
+    k_tc5_select<MODE, KP><<<grid, kT5Threads, Sh::SMEM, s>>>(a);
     return TK_OK;
 }
 
