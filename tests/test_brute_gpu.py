@@ -406,3 +406,21 @@ def test_tensor_core_rows_left_over(mode, extra, k, oracle):
     dd, ii = tk().nn_distance(torch.from_numpy(ref).to(cuda), torch.from_numpy(q).to(cuda), k, mode=mode)
     np.testing.assert_array_equal(dd.cpu().numpy(), bd)
     np.testing.assert_array_equal(ii.cpu().numpy(), bi)
+
+
+@pytest.mark.parametrize("n_listed", [1, 32, 33, 200])
+@pytest.mark.parametrize("k", [1, 20, 64])
+@pytest.mark.parametrize("d", [7, 8])
+def test_few_recomputed_queries(n_listed, k, d, oracle):
+    """The same with lists at the edges of the block-per-slice search, slices
+    that leave warps without a row, and rows read one float at a time."""
+    rng = np.random.default_rng(n_listed + k)
+    ref = np.concatenate([rng.standard_normal((1000, d)), np.tile(rng.standard_normal((1, d)) + 20, (300, 1))])
+    ref = ref[rng.permutation(len(ref))].astype(np.float32)
+    q = rng.standard_normal((1000, d)).astype(np.float32)
+    hard = rng.permutation(len(q))[:n_listed]
+    q[hard] = (20 + 0.1 * rng.standard_normal((n_listed, d))).astype(np.float32)
+    bd, bi = oracle.brute(ref, q, k)
+    dd, ii = tk().nn_distance(torch.from_numpy(ref).to(cuda), torch.from_numpy(q).to(cuda), k, mode="tf32")
+    np.testing.assert_array_equal(dd.cpu().numpy(), bd)
+    np.testing.assert_array_equal(ii.cpu().numpy(), bi)

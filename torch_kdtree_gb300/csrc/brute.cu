@@ -187,17 +187,21 @@ int check_common(const void* ref, int64_t n, const void* q, int64_t nq, int d, i
 // ------------------------------------------------- listed queries --
 //
 // The exact answers of the queries on a device-side list, whose length only
-// the device knows.  Usually it is empty or short: up to kFew queries, a warp
-// takes (query, slice) pairs, a lane per reference row read from global
-// memory (0.8 us per query of 262,144 references, d=32).  Longer lists go
-// through the tiled kernel above, its blocks looping over (query tile, slice)
-// pairs.  A last kernel merges a query's slices, a warp per query; whichever
-// kernel is not meant exits at once.  (The tiled kernel for any list, with a
-// lane merging a query's 128 slices, took 1.0 ms for a few dozen queries.)
+// the device knows.  Usually it is empty or short: up to kFew queries are
+// searched in (query, slice) pairs, a lane per reference row read from global
+// memory -- a chain of such reads, so up to kVeryFew queries a block's eight
+// warps share a pair (one query in 262,144 references, d=32: 0.2 ms -> 0.04),
+// above that a warp takes one (0.8 us per query).  Longer lists go through the
+// tiled kernel above, its blocks looping over (query tile, slice) pairs.  A
+// last kernel merges a query's slices, a block per query or for long lists a
+// warp; whichever kernel is not meant exits at once.  (The tiled kernel for any
+// list, with a lane merging a query's 128 slices, took 1.0 ms for a few dozen
+// queries.)
 namespace {
 
 constexpr int kFew = 256;
 constexpr int kFewSlices = 64;
+constexpr int kVeryFew = 32;
 constexpr int kMaxSlices = 128;
 constexpr int kSlots = 65536;  // (query, slice) pairs with a list in the shared buffer
 
@@ -231,18 +235,46 @@ __device__ __forceinline__ float row_dist(const float* __restrict__ q, const flo
     return acc;
 }
 
+// The lists of a block's eight warps, joined in the first warp's.  Every
+// thread of the block calls it.
+template <int R>
+__device__ __forceinline__ void join_lists(WarpList<float, R>& wl, Key<float> (*all)[32 * R], int k, int lane, int w) {
+    if (w > 0) {
+#pragma unroll
+        for (int i = 0; i < R; ++i) all[w][i * 32 + lane] = wl.list.slot[i];
+    }
+    __syncthreads();
+    if (w == 0) {
+        for (int o = 1; o < 8; ++o) {
+#pragma unroll
+            for (int i = 0; i < R; ++i)
+                wl.offer(i * 32 + lane >= 32 * R - k ? all[o][i * 32 + lane] : Key<float>::sentinel(), lane);
+        }
+        wl.flush(lane);
+    }
+    __syncthreads();
+}
+
 template <int R>
 __global__ void __launch_bounds__(256) k_few_search(const ListArgs a) {
     __shared__ Key<float> bufs[8][64];
+    __shared__ Key<float> all[8][32 * R];
     const int count = *a.qcount;
-    if (count > kFew) return;
+    if (count == 0 || count > kFew) return;
+    const int share = count <= kVeryFew ? 8 : 1;  // warps of a pair
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const bool vec = (a.d & 3) == 0 && ((reinterpret_cast<uintptr_t>(a.ref) | reinterpret_cast<uintptr_t>(a.q)) & 15) == 0;
     const int per = (a.n + kFewSlices - 1) / kFewSlices;
-    for (int item = blockIdx.x * 8 + w; item < count * kFewSlices; item += gridDim.x * 8) {
+    const int first = share == 8 ? int(blockIdx.x) : int(blockIdx.x) * 8 + w;
+    for (int item = first; item < count * kFewSlices; item += int(gridDim.x) * 8 / share) {
         const int slot = item / kFewSlices, slice = item % kFewSlices;
         const float* q = a.q + (long long)a.qlist[slot] * a.d;
-        const int r0 = int(min((long long)a.n, (long long)per * slice)), r1 = int(min((long long)a.n, (long long)r0 + per));
+        int r0 = int(min((long long)a.n, (long long)per * slice)), r1 = int(min((long long)a.n, (long long)r0 + per));
+        if (share == 8) {
+            const int sub = (r1 - r0 + 7) / 8;
+            r0 = min(r1, r0 + sub * w);
+            r1 = min(r1, r0 + sub);
+        }
         WarpList<float, R> wl;
         wl.init(a.k, bufs[w], lane);
         for (int r = r0; r < r1; r += 32) {
@@ -251,6 +283,10 @@ __global__ void __launch_bounds__(256) k_few_search(const ListArgs a) {
             wl.offer(mine, lane);
         }
         wl.flush(lane);
+        if (share == 8) {
+            join_lists<R>(wl, all, a.k, lane, w);
+            if (w > 0) continue;
+        }
         Key<float>* out = a.part + (long long)item * a.k;
 #pragma unroll
         for (int i = 0; i < R; ++i) {
@@ -263,9 +299,24 @@ __global__ void __launch_bounds__(256) k_few_search(const ListArgs a) {
 template <int R>
 __global__ void __launch_bounds__(256) k_list_merge(const ListArgs a) {
     __shared__ Key<float> bufs[8][64];
+    __shared__ Key<float> all[8][32 * R];
     const int count = *a.qcount;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const int slices = count <= kFew ? kFewSlices : list_slices(count, kSlots, a.max_slices);
+    if (count <= kFew) {  // a block per query
+        const int total = kFewSlices * a.k;
+        for (int slot = blockIdx.x; slot < count; slot += gridDim.x) {
+            WarpList<float, R> wl;
+            wl.init(a.k, bufs[w], lane);
+            const Key<float>* src = a.part + (long long)slot * total;
+            for (int e = threadIdx.x; e - lane < total; e += 256)
+                wl.offer(e < total ? src[e] : Key<float>::sentinel(), lane);
+            wl.flush(lane);
+            join_lists<R>(wl, all, a.k, lane, w);
+            if (w == 0) wl.list.store(a.k, lane, a.out_d, a.out_i, a.qlist[slot]);
+        }
+        return;
+    }
+    const int slices = list_slices(count, kSlots, a.max_slices);
     if (slices == 1) return;  // already in the outputs
     for (int slot = blockIdx.x * 8 + w; slot < count; slot += gridDim.x * 8) {
         WarpList<float, R> wl;
@@ -295,8 +346,8 @@ int brute_fallback(const float* ref, int64_t n, const float* q, int64_t nq, int 
     const int sms = sm_count_dev(), few = int(std::min<int64_t>(nq, kFew));
     const int max_slices = int(std::max<int64_t>(1, std::min<int64_t>(kMaxSlices, n / 2048)));
     ListArgs l{ref, q, int(n), d, k, qlist, qcount, static_cast<Key<float>*>(ws), max_slices, dists, idx};
-    const unsigned gs = unsigned(std::min(4 * sms, (few * kFewSlices + 7) / 8));
-    const unsigned gm = unsigned(std::min<int64_t>(4 * sms, (nq + 7) / 8));
+    const unsigned gs = unsigned(std::min(4 * sms, few * kFewSlices));
+    const unsigned gm = unsigned(std::min<int64_t>(4 * sms, std::max<int64_t>(few, (nq + 7) / 8)));
     if (k <= 32) k_few_search<1><<<gs, 256, 0, s>>>(l);
     else if (k <= 64) k_few_search<2><<<gs, 256, 0, s>>>(l);
     else k_few_search<4><<<gs, 256, 0, s>>>(l);
