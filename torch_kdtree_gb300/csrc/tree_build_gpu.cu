@@ -26,7 +26,7 @@
 // and level).  One sort per axis, seven launches per axis and level, boxes
 // bottom-up and seventeen allocations took (1M / 4M points, default levels,
 // build_kd_tree with the synchronisation) 2.7 / 4.7 ms and 0.93 ms for 10,000
-// points; this takes 0.58 / 1.75 ms and 0.24 ms.
+// points; this takes 0.49 / 1.73 ms and 0.20 ms.
 #include <algorithm>
 #include <cstring>
 #include <limits>
@@ -46,6 +46,29 @@ constexpr int kTile = 1024;        // positions per block of the partition passe
 constexpr int kSub = 4096;         // points of a subtree that one block finishes in shared memory
 constexpr int kSubThreads = 1024;
 constexpr int kSubItems = kSub / kSubThreads;
+
+// A build is a chain of some 30 short launches, each on the results of the one
+// before.  All but the first are set up while the one before still runs and
+// start when it has ended; every kernel waits for that (begin) before it
+// touches memory.  Buffers that the chain writes are not __restrict__ there: a
+// load of constant data may be moved above the wait.  (65,536 points 0.28 ->
+// 0.23 ms, 1M 0.55 -> 0.49; letting the next launch's blocks in early was no
+// faster, and slower for small clouds.)
+__device__ __forceinline__ void begin() { cudaGridDependencySynchronize(); }
+template <typename... P, typename... A>
+cudaError_t launch(bool after, void (*kernel)(P...), dim3 grid, unsigned block, size_t smem, cudaStream_t s, A... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = after ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, kernel, P(args)...);
+}
 
 template <typename T>
 struct KeyBits;
@@ -154,9 +177,10 @@ __device__ __forceinline__ int block_exclusive(int v, int* warp_sums, int* total
 
 template <typename T, bool FIRST>
 __global__ void __launch_bounds__(kSortThreads) k_radix_hist(const T* __restrict__ pts, int64_t n, int dims, int ax0,
-                                                             const typename KeyBits<T>::type* __restrict__ keys,
-                                                             int shift, int ntiles, int* __restrict__ hist,
+                                                             const typename KeyBits<T>::type* keys,
+                                                             int shift, int ntiles, int* hist,
                                                              int* __restrict__ odd) {
+    begin();
     __shared__ int h[256];
     const int t = threadIdx.x, a = blockIdx.y;
     if (t < 256) h[t] = 0;
@@ -183,7 +207,8 @@ __global__ void __launch_bounds__(kSortThreads) k_radix_hist(const T* __restrict
 
 // Exclusive scan of every row (blockIdx.y * gridDim.x + blockIdx.x) of `len`
 // counts in place; the row's total goes to totals.
-__global__ void __launch_bounds__(kScanThreads) k_row_scan(int* __restrict__ rows, int len, int* __restrict__ totals) {
+__global__ void __launch_bounds__(kScanThreads) k_row_scan(int* rows, int len, int* totals) {
+    begin();
     __shared__ int warp_sums[32];
     const int64_t row = int64_t(blockIdx.y) * gridDim.x + blockIdx.x;
     int* d = rows + row * len;
@@ -210,9 +235,10 @@ __global__ void __launch_bounds__(kScanThreads) k_row_scan(int* __restrict__ row
 
 template <typename T, bool FIRST, bool LAST>
 __global__ void __launch_bounds__(kSortThreads, 2) k_radix_scatter(
-    const T* __restrict__ pts, int64_t n, int dims, int ax0, const typename KeyBits<T>::type* __restrict__ kin,
-    const Arrays vin, int shift, int ntiles, const int* __restrict__ hist, const int* __restrict__ totals,
-    typename KeyBits<T>::type* __restrict__ kout, const Arrays vout) {
+    const T* __restrict__ pts, int64_t n, int dims, int ax0, const typename KeyBits<T>::type* kin,
+    const Arrays vin, int shift, int ntiles, const int* hist, const int* totals,
+    typename KeyBits<T>::type* kout, const Arrays vout) {
+    begin();
     using K = typename KeyBits<T>::type;
     constexpr int ITEMS = KeyBits<T>::kItems, TILE = radix_tile<T>(), WARPS = kSortThreads / 32;
     __shared__ K skey[TILE];
@@ -500,8 +526,9 @@ __device__ __forceinline__ void write_point(const T* __restrict__ pts, int dims,
 template <typename T>
 __global__ void __launch_bounds__(256) k_level_count(const T* __restrict__ pts, int n, int dims, int s, const Arrays P,
                                                      const Image<T> im, const Arrays in, int naxes,
-                                                     uint32_t* __restrict__ bits, int words, int ntiles,
-                                                     int* __restrict__ counts) {
+                                                     uint32_t* bits, int words, int ntiles,
+                                                     int* counts) {
+    begin();
     __shared__ int warp_cnt[8];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, b = blockIdx.y;
     if (b == naxes) {
@@ -547,10 +574,16 @@ __global__ void __launch_bounds__(256) k_level_count(const T* __restrict__ pts, 
 }
 
 // Stable partition of every node's range by side (lefts first); counts holds
-// the exclusive scan of the tiles' left counts.
+// the tiles' left counts or, `scanned`, their exclusive scan.  Up to
+// kCountedTiles tiles a block adds up the counts before its own (a few
+// kilobytes from L2, while its own bits arrive), which saves the scan's launch
+// (1M points 0.57 -> 0.55 ms).
+constexpr int kCountedTiles = 2048;
+
 __global__ void __launch_bounds__(256) k_level_partition(int n, int s, const Arrays in, const Arrays out,
-                                                         const uint32_t* __restrict__ bits, int words, int ntiles,
-                                                         const int* __restrict__ counts) {
+                                                         const uint32_t* bits, int words, int ntiles, bool scanned,
+                                                         const int* counts) {
+    begin();
     __shared__ int warp_cnt[8];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, b = blockIdx.y;
     const uint32_t* pb = in[b];
@@ -561,8 +594,20 @@ __global__ void __launch_bounds__(256) k_level_partition(int n, int s, const Arr
     int c = __popc(mine);
     c = __reduce_add_sync(0xFFFFFFFFu, c);
     if (lane == 0) warp_cnt[w] = c;
-    __syncthreads();
-    int run = counts[int64_t(b) * ntiles + blockIdx.x];
+    int run = 0;
+    if (!scanned) {
+        __shared__ int before[8];
+        int sum = 0;
+        for (int i = threadIdx.x; i < int(blockIdx.x); i += 256) sum += counts[int64_t(b) * ntiles + i];
+        sum = __reduce_add_sync(0xFFFFFFFFu, sum);
+        if (lane == 0) before[w] = sum;
+        __syncthreads();
+#pragma unroll
+        for (int i = 0; i < 8; ++i) run += before[i];
+    } else {
+        __syncthreads();
+        run = counts[int64_t(b) * ntiles + blockIdx.x];
+    }
     for (int i = 0; i < w; ++i) run += warp_cnt[i];
     const unsigned below = (1u << lane) - 1u;
 #pragma unroll
@@ -582,7 +627,8 @@ __global__ void __launch_bounds__(256) k_level_partition(int n, int s, const Arr
 
 template <typename T>
 __global__ void __launch_bounds__(256) k_write_points(const T* __restrict__ pts, int n, int dims,
-                                                      const uint32_t* __restrict__ order, const Image<T> im) {
+                                                      const uint32_t* order, const Image<T> im) {
+    begin();
     const int64_t p = int64_t(blockIdx.x) * 256 + threadIdx.x;
     if (p < n) write_point<T>(pts, dims, im, p, order[p]);
 }
@@ -597,6 +643,7 @@ template <typename T>
 __global__ void __launch_bounds__(kSubThreads) k_subtrees(const T* __restrict__ pts, int n, int dims, int t0,
                                                           const Arrays P, const Image<T> im,
                                                           uint16_t* __restrict__ place) {
+    begin();
     extern __shared__ __align__(16) unsigned char smem[];
     uint32_t* ids = reinterpret_cast<uint32_t*>(smem);                    // [kSub]
     uint32_t* start = ids + kSub;                                         // [kSub] scan at each node's start
@@ -723,12 +770,13 @@ __device__ __forceinline__ Frame cloud_frame(const PointRec<double>* boxes) {
 }
 
 // Float images of points, boxes (rounded outwards) and split values.
-__global__ void __launch_bounds__(256) k_fill_filter(const PointRec<double>* __restrict__ pts, int64_t n,
-                                                     const PointRec<double>* __restrict__ boxes, int64_t nodes,
-                                                     const double* __restrict__ medians, int64_t splits, int dims,
+__global__ void __launch_bounds__(256) k_fill_filter(const PointRec<double>* pts, int64_t n,
+                                                     const PointRec<double>* boxes, int64_t nodes,
+                                                     const double* medians, int64_t splits, int dims,
                                                      PointRec<float>* __restrict__ f_pts,
                                                      PointRec<float>* __restrict__ f_boxes,
                                                      float* __restrict__ f_medians, Frame* __restrict__ frame) {
+    begin();
     __shared__ Frame f;
     if (threadIdx.x == 0) f = cloud_frame(boxes);
     __syncthreads();
@@ -895,12 +943,12 @@ int enqueue_device_tree(const T* pts, int64_t n, int dims, void* stream, const t
                 const Arrays& vin = pass & 1 ? spare : dst;
                 const Arrays& vout = pass & 1 ? dst : spare;  // an even number of passes ends in dst
                 const int shift = 8 * pass;
-                if (pass == 0) k_radix_hist<T, true><<<grid, kSortThreads, 0, s>>>(pts, n, dims, a0, kin, shift, rtiles, hist, odd);
-                else k_radix_hist<T, false><<<grid, kSortThreads, 0, s>>>(pts, n, dims, a0, kin, shift, rtiles, hist, odd);
-                k_row_scan<<<dim3(256, na), kScanThreads, 0, s>>>(hist, rtiles, totals);
-                if (pass == 0) k_radix_scatter<T, true, false><<<grid, kSortThreads, 0, s>>>(pts, n, dims, a0, kin, vin, shift, rtiles, hist, totals, kout, vout);
-                else if (pass + 1 < passes) k_radix_scatter<T, false, false><<<grid, kSortThreads, 0, s>>>(pts, n, dims, a0, kin, vin, shift, rtiles, hist, totals, kout, vout);
-                else k_radix_scatter<T, false, true><<<grid, kSortThreads, 0, s>>>(pts, n, dims, a0, kin, vin, shift, rtiles, hist, totals, kout, vout);
+                if (pass == 0) TK_TRY(launch(a0 > 0, k_radix_hist<T, true>, grid, kSortThreads, 0, s, pts, n, dims, a0, kin, shift, rtiles, hist, odd));
+                else TK_TRY(launch(true, k_radix_hist<T, false>, grid, kSortThreads, 0, s, pts, n, dims, a0, kin, shift, rtiles, hist, odd));
+                TK_TRY(launch(true, k_row_scan, dim3(256, na), kScanThreads, 0, s, hist, rtiles, totals));
+                if (pass == 0) TK_TRY(launch(true, k_radix_scatter<T, true, false>, grid, kSortThreads, 0, s, pts, n, dims, a0, kin, vin, shift, rtiles, hist, totals, kout, vout));
+                else if (pass + 1 < passes) TK_TRY(launch(true, k_radix_scatter<T, false, false>, grid, kSortThreads, 0, s, pts, n, dims, a0, kin, vin, shift, rtiles, hist, totals, kout, vout));
+                else TK_TRY(launch(true, k_radix_scatter<T, false, true>, grid, kSortThreads, 0, s, pts, n, dims, a0, kin, vin, shift, rtiles, hist, totals, kout, vout));
                 TK_TRY(cudaGetLastError());
             }
         }
@@ -924,10 +972,11 @@ int enqueue_device_tree(const T* pts, int64_t n, int dims, void* stream, const t
                 const Arrays out = spare;
                 for (int i = 0; i < m; ++i) in.set(i, P.slot(axes[g + i]));
                 // the nodes' entries need every axis's order as it was before this level: with the first group
-                k_level_count<T><<<dim3(ntiles, m + (g == 0)), 256, 0, s>>>(pts, n32, dims, lev, P, im, in, m, bits, words, ntiles, counts);
+                TK_TRY(launch(true, k_level_count<T>, dim3(ntiles, m + (g == 0)), 256, 0, s, pts, n32, dims, lev, P, im, in, m, bits, words, ntiles, counts));
                 if (m > 0) {
-                    k_row_scan<<<dim3(1, m), kScanThreads, 0, s>>>(counts, ntiles, totals);
-                    k_level_partition<<<dim3(ntiles, m), 256, 0, s>>>(n32, lev, in, out, bits, words, ntiles, counts);
+                    const bool scan = ntiles > kCountedTiles;
+                    if (scan) TK_TRY(launch(true, k_row_scan, dim3(1, m), kScanThreads, 0, s, counts, ntiles, totals));
+                    TK_TRY(launch(true, k_level_partition, dim3(ntiles, m), 256, 0, s, n32, lev, in, out, bits, words, ntiles, scan, counts));
                 }
                 for (int i = 0; i < m; ++i) {
                     P.set(axes[g + i], out.slot(i));
@@ -941,26 +990,26 @@ int enqueue_device_tree(const T* pts, int64_t n, int dims, void* stream, const t
 
     // 3. the rest, a block per node
     if (n > kSub && ((n - 1) >> t0) + 1 > kSub) {  // leaves larger than a block's capacity
-        k_level_count<T><<<dim3(ntiles, 1), 256, 0, s>>>(pts, n32, dims, L, P, im, P, 0, nullptr, 0, ntiles, nullptr);
-        k_write_points<T><<<unsigned((n + 255) / 256), 256, 0, s>>>(pts, n32, dims, P[(L - 1) % dims], im);
+        TK_TRY(launch(true, k_level_count<T>, dim3(ntiles, 1), 256, 0, s, pts, n32, dims, L, P, im, P, 0, nullptr, 0, ntiles, nullptr));
+        TK_TRY(launch(true, k_write_points<T>, dim3(unsigned((n + 255) / 256)), 256, 0, s, pts, n32, dims, P[(L - 1) % dims], im));
     } else {
         const size_t smem = subtree_smem(dims);
         TK_TRY(cudaFuncSetAttribute(k_subtrees<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
-        k_subtrees<T><<<1u << t0, kSubThreads, smem, s>>>(pts, n32, dims, t0, P, im,
-                                                        reinterpret_cast<uint16_t*>(ws + w.key_b));
+        TK_TRY(launch(true, k_subtrees<T>, dim3(1u << t0), kSubThreads, smem, s, pts, n32, dims, t0, P, im,
+                      reinterpret_cast<uint16_t*>(ws + w.key_b)));
     }
     TK_TRY(cudaGetLastError());
     if constexpr (sizeof(T) == 8) {
         if (t->d_filter[0]) {
             const int64_t nodes = (int64_t(2) << L) - 1, splits = (int64_t(1) << L) - 1;
             const int64_t work = std::max(n, nodes);
-            k_fill_filter<<<unsigned((work + 255) / 256), 256, 0, s>>>(
+            TK_TRY(launch(true, k_fill_filter, dim3(unsigned((work + 255) / 256)), 256, 0, s,
                 static_cast<const PointRec<double>*>(t->d_pts), n, static_cast<const PointRec<double>*>(t->d_boxes), nodes,
                 static_cast<const double*>(t->d_medians), splits, dims,
                 static_cast<PointRec<float>*>(const_cast<void*>(t->d_filter[0])),
                 static_cast<PointRec<float>*>(const_cast<void*>(t->d_filter[1])),
                 static_cast<float*>(const_cast<void*>(t->d_filter[2])),
-                static_cast<Frame*>(const_cast<void*>(t->d_filter[3])));
+                static_cast<Frame*>(const_cast<void*>(t->d_filter[3]))));
             TK_TRY(cudaGetLastError());
         }
     }
