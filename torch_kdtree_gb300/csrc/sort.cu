@@ -12,6 +12,7 @@
 //      equals its rank in input order among equal digits (stability).
 #include <algorithm>
 
+#include "launch.cuh"
 #include "sort.cuh"
 
 namespace tk {
@@ -58,6 +59,7 @@ __device__ __forceinline__ int block_exclusive_sum(int v, int* warp_sums, int* t
 
 // Tile-local exclusive scan; writes the tile total to sums[blockIdx.x].
 __global__ void k_scan_tiles(int* data, int64_t n, int* sums) {
+    begin();
     __shared__ int warp_sums[32];
     const int64_t base = int64_t(blockIdx.x) * kScanTile + int64_t(threadIdx.x) * kScanItems;
     int v[kScanItems];
@@ -79,6 +81,7 @@ __global__ void k_scan_tiles(int* data, int64_t n, int* sums) {
 
 // One block: exclusive scan of sums[0..m) in place, any m (chunked).
 __global__ void k_scan_single(int* sums, int m) {
+    begin();
     __shared__ int warp_sums[32];
     const int per = (m + blockDim.x - 1) / blockDim.x;
     const int beg = min(m, int(threadIdx.x) * per), end = min(m, beg + per);
@@ -92,14 +95,33 @@ __global__ void k_scan_single(int* sums, int m) {
     }
 }
 
-__global__ void k_scan_add(int* data, int64_t n, const int* sums) {
-    const int64_t base = int64_t(blockIdx.x) * kScanTile;
-    const int add = sums[blockIdx.x];
-    for (int i = threadIdx.x; i < kScanTile; i += blockDim.x)
-        if (base + i < n) data[base + i] += add;
+// Adds what lies before each tile.  Up to kOwnSums tiles, `sums` holds the
+// tiles' totals and a block adds up those before its own; beyond, their
+// exclusive scan.
+constexpr int kOwnSums = 2048;
+
+__global__ void __launch_bounds__(kScanThreads) k_scan_add(int* data, int64_t n, const int* sums, bool scanned) {
+    begin();
+    __shared__ int warp_sums[32];
+    const int64_t base = int64_t(blockIdx.x) * kScanTile + threadIdx.x;
+    int v[kScanItems];
+#pragma unroll
+    for (int i = 0; i < kScanItems; ++i) v[i] = base + i * kScanThreads < n ? data[base + i * kScanThreads] : 0;
+    int add = 0;
+    if (scanned) {
+        add = sums[blockIdx.x];
+    } else {
+        int s = 0;
+        for (int i = threadIdx.x; i < int(blockIdx.x); i += kScanThreads) s += sums[i];
+        block_exclusive_sum(s, warp_sums, &add);
+    }
+#pragma unroll
+    for (int i = 0; i < kScanItems; ++i)
+        if (base + i * kScanThreads < n) data[base + i * kScanThreads] = v[i] + add;
 }
 
 __global__ void k_digit_hist(const uint32_t* keys, int64_t n, int shift, int ntiles, int* hist) {
+    begin();
     __shared__ int h[256];
     h[threadIdx.x] = 0;
     __syncthreads();
@@ -115,6 +137,7 @@ __global__ void k_digit_hist(const uint32_t* keys, int64_t n, int shift, int nti
 
 __global__ void k_digit_scatter(const uint32_t* keys, const uint32_t* vals, int64_t n, int shift, int ntiles,
                                 const int* offs, uint32_t* keys_out, uint32_t* vals_out) {
+    begin();
     __shared__ int warp_cnt[kWarps][256];
     __shared__ int run_cnt[256];
     const int t = threadIdx.x, lane = t & 31, wid = t >> 5;
@@ -169,10 +192,12 @@ cudaError_t exclusive_scan(int* data, int64_t n, void* ws, cudaStream_t s) {
     if (n <= 0) return cudaSuccess;
     const int64_t tiles = (n + kScanTile - 1) / kScanTile;
     int* sums = static_cast<int*>(ws);
-    k_scan_tiles<<<unsigned(tiles), kScanThreads, 0, s>>>(data, n, sums);
-    k_scan_single<<<1, kScanThreads, 0, s>>>(sums, int(tiles));
-    k_scan_add<<<unsigned(tiles), 256, 0, s>>>(data, n, sums);
-    return cudaGetLastError();
+    cudaError_t e = launch(true, k_scan_tiles, dim3(unsigned(tiles)), kScanThreads, 0, s, data, n, sums);
+    if (e != cudaSuccess || tiles == 1) return e;
+    const bool scan = tiles > kOwnSums;
+    if (scan) e = launch(true, k_scan_single, dim3(1), kScanThreads, 0, s, sums, int(tiles));
+    if (e != cudaSuccess) return e;
+    return launch(true, k_scan_add, dim3(unsigned(tiles)), kScanThreads, 0, s, data, n, sums, scan);
 }
 
 size_t sort_pass8_workspace_bytes(int64_t n) {
@@ -189,12 +214,12 @@ cudaError_t sort_pass8(const uint32_t* keys_in, const uint32_t* vals_in, uint32_
     const int64_t hist_n = 256 * ntiles;
     int* hist = static_cast<int*>(ws);
     void* scan_ws = static_cast<char*>(ws) + align256(sizeof(int) * size_t(hist_n));
-    k_digit_hist<<<unsigned(ntiles), kSortThreads, 0, s>>>(keys_in, n, 0, int(ntiles), hist);
-    cudaError_t e = exclusive_scan(hist, hist_n, scan_ws, s);
+    cudaError_t e = launch(true, k_digit_hist, dim3(unsigned(ntiles)), kSortThreads, 0, s, keys_in, n, 0, int(ntiles), hist);
     if (e != cudaSuccess) return e;
-    k_digit_scatter<<<unsigned(ntiles), kSortThreads, 0, s>>>(keys_in, vals_in, n, 0, int(ntiles), hist, keys_out,
-                                                             vals_out);
-    return cudaGetLastError();
+    e = exclusive_scan(hist, hist_n, scan_ws, s);
+    if (e != cudaSuccess) return e;
+    return launch(true, k_digit_scatter, dim3(unsigned(ntiles)), kSortThreads, 0, s, keys_in, vals_in, n, 0, int(ntiles),
+                  hist, keys_out, vals_out);
 }
 
 }  // namespace tk

@@ -34,6 +34,7 @@
 #include <vector>
 
 #include "kd_filter.cuh"
+#include "launch.cuh"
 #include "tk_device.cuh"
 #include "tk_internal.h"
 
@@ -48,27 +49,8 @@ constexpr int kSubThreads = 1024;
 constexpr int kSubItems = kSub / kSubThreads;
 
 // A build is a chain of some 30 short launches, each on the results of the one
-// before.  All but the first are set up while the one before still runs and
-// start when it has ended; every kernel waits for that (begin) before it
-// touches memory.  Buffers that the chain writes are not __restrict__ there: a
-// load of constant data may be moved above the wait.  (65,536 points 0.28 ->
-// 0.23 ms, 1M 0.55 -> 0.49; letting the next launch's blocks in early was no
-// faster, and slower for small clouds.)
-__device__ __forceinline__ void begin() { cudaGridDependencySynchronize(); }
-template <typename... P, typename... A>
-cudaError_t launch(bool after, void (*kernel)(P...), dim3 grid, unsigned block, size_t smem, cudaStream_t s, A... args) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = grid;
-    cfg.blockDim = dim3(block);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = s;
-    cudaLaunchAttribute attr;
-    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr.val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = &attr;
-    cfg.numAttrs = after ? 1 : 0;
-    return cudaLaunchKernelEx(&cfg, kernel, P(args)...);
-}
+// before: all but the first are set up ahead of time (launch.cuh; 65,536 points
+// 0.28 -> 0.23 ms, 1M 0.55 -> 0.49).
 
 template <typename T>
 struct KeyBits;
@@ -233,6 +215,12 @@ __global__ void __launch_bounds__(kScanThreads) k_row_scan(int* rows, int len, i
     if (threadIdx.x == 0) totals[row] = carry;
 }
 
+// Up to kOwnScanTiles tiles there is no scan (totals null): a scatter block
+// adds up its digits' rows of the histogram itself, which saves a launch per
+// pass (30,000 points built in 0.208 -> 0.195 ms; with 64 tiles the rows cost
+// more than the launch, 260,000 points 0.26 -> 0.30).
+constexpr int kOwnScanTiles = 32;
+
 template <typename T, bool FIRST, bool LAST>
 __global__ void __launch_bounds__(kSortThreads, 2) k_radix_scatter(
     const T* __restrict__ pts, int64_t n, int dims, int ax0, const typename KeyBits<T>::type* kin,
@@ -264,6 +252,22 @@ __global__ void __launch_bounds__(kSortThreads, 2) k_radix_scatter(
             val[i] = FIRST ? uint32_t(e) : vin[a][e];
         }
     }
+    // of digit t: items in tiles before this one, and in all
+    int tiles_before = 0, row_total = 0;
+    if (t < 256) {
+        const int* row = hist + (int64_t(a) * 256 + t) * ntiles;
+        if (totals) {
+            tiles_before = row[blockIdx.x];
+            row_total = totals[a * 256 + t];
+        } else {
+#pragma unroll 4
+            for (int i = 0; i < ntiles; ++i) {
+                const int c = row[i];
+                tiles_before += i < int(blockIdx.x) ? c : 0;
+                row_total += c;
+            }
+        }
+    }
     const unsigned below = (1u << lane) - 1u;
 #pragma unroll
     for (int i = 0; i < ITEMS; ++i) {
@@ -286,9 +290,9 @@ __global__ void __launch_bounds__(kSortThreads, 2) k_radix_scatter(
             run += c;
         }
     const int lstart = block_exclusive(run, warp_sums);
-    const int gstart = block_exclusive(t < 256 ? totals[a * 256 + t] : 0, warp_sums);
+    const int gstart = block_exclusive(row_total, warp_sums);
     if (t < 256) {
-        gbase[t] = gstart + hist[(int64_t(a) * 256 + t) * ntiles + blockIdx.x] - lstart;
+        gbase[t] = gstart + tiles_before - lstart;
         for (int i = 0; i < WARPS; ++i) cnt[i][t] = uint16_t(cnt[i][t] + lstart);
     }
     __syncthreads();
@@ -929,8 +933,8 @@ int enqueue_device_tree(const T* pts, int64_t n, int dims, void* stream, const t
         K* key_a = reinterpret_cast<K*>(ws + w.key_a);
         K* key_b = reinterpret_cast<K*>(ws + w.key_b);
         int* hist = reinterpret_cast<int*>(ws + w.hist);
-        int* totals = reinterpret_cast<int*>(ws + w.totals);
         const int rtiles = int((n + radix_tile<T>() - 1) / radix_tile<T>());
+        int* totals = rtiles > kOwnScanTiles ? reinterpret_cast<int*>(ws + w.totals) : nullptr;
         const int passes = int(sizeof(K));
         for (int a0 = 0; a0 < dims; a0 += A) {
             const int na = std::min(A, dims - a0);
@@ -945,7 +949,7 @@ int enqueue_device_tree(const T* pts, int64_t n, int dims, void* stream, const t
                 const int shift = 8 * pass;
                 if (pass == 0) TK_TRY(launch(a0 > 0, k_radix_hist<T, true>, grid, kSortThreads, 0, s, pts, n, dims, a0, kin, shift, rtiles, hist, odd));
                 else TK_TRY(launch(true, k_radix_hist<T, false>, grid, kSortThreads, 0, s, pts, n, dims, a0, kin, shift, rtiles, hist, odd));
-                TK_TRY(launch(true, k_row_scan, dim3(256, na), kScanThreads, 0, s, hist, rtiles, totals));
+                if (totals) TK_TRY(launch(true, k_row_scan, dim3(256, na), kScanThreads, 0, s, hist, rtiles, totals));
                 if (pass == 0) TK_TRY(launch(true, k_radix_scatter<T, true, false>, grid, kSortThreads, 0, s, pts, n, dims, a0, kin, vin, shift, rtiles, hist, totals, kout, vout));
                 else if (pass + 1 < passes) TK_TRY(launch(true, k_radix_scatter<T, false, false>, grid, kSortThreads, 0, s, pts, n, dims, a0, kin, vin, shift, rtiles, hist, totals, kout, vout));
                 else TK_TRY(launch(true, k_radix_scatter<T, false, true>, grid, kSortThreads, 0, s, pts, n, dims, a0, kin, vin, shift, rtiles, hist, totals, kout, vout));
