@@ -145,3 +145,20 @@ def test_no_queries_gives_zero_reference_gradient():
     g = torch.empty(0, 4, device=cuda)
     gq, gr = knn_backward(q, ref, idx, g, True, True)
     assert gq.shape == (0, 3) and torch.equal(gr, torch.zeros_like(ref))
+
+
+@pytest.mark.parametrize("n", [1, 4095, 4096, 2048 * 4096 - 1, 2048 * 4096])
+def test_segment_scan_limits(n):
+    """Segment starts of n references: one scan tile, several, and more than
+    the blocks add up themselves."""
+    from torch_kdtree_gb300.nn_distance import nn_distance
+    ref = torch.arange(n, device="cuda", dtype=torch.float32)[:, None].requires_grad_()
+    at = torch.unique(torch.tensor([0, n // 3, n // 2, n - 2, n - 1], device="cuda").clamp(min=0))
+    at = at.repeat_interleave(3)
+    q = ref.detach()[at] + 0.25
+    d, i = nn_distance(ref, q, 1)
+    assert torch.equal(i[:, 0].long(), at)
+    (g,) = torch.autograd.grad(d.sum(), ref)
+    # (the quarter is rounded away where the coordinates are large)
+    want = torch.zeros_like(g).index_add_(0, at, 2 * (ref.detach()[at] - q))
+    assert torch.equal(g, want)

@@ -256,3 +256,14 @@ def test_device_build_refuses_nan_at_every_size(dtype, n):
     good = torch.randn(n, 3, device=cuda)
     d, _ = tk.build_kd_tree(good).query(good[:100])
     assert float(d.max()) == 0.0
+
+
+@pytest.mark.parametrize("dtype,n", [(np.float32, 131_072), (np.float32, 131_073), (np.float64, 65_536),
+                                     (np.float64, 65_537), (np.float32, 2_097_152), (np.float32, 2_097_153)])
+def test_device_build_around_scan_limits(dtype, n):
+    """Clouds whose radix or level tiles just fit, or no longer fit, the sums
+    that the blocks take themselves."""
+    rng = np.random.default_rng(n)
+    pts = rng.standard_normal((n, 2)).astype(dtype)
+    pts[: n // 4] = np.round(pts[: n // 4], 1)
+    assert_same_layout(pts, 7)
