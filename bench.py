@@ -460,11 +460,11 @@ def run_ours(args, rank, world):
                 "transfer": "tk_tree_query_host: queries in one H2D copy; results written by the query kernel "
                             "straight into the pinned host buffers",
                 "ms_per_step": t_e2e / args.steps},
-        # per chosen step (one graph replay): k_bin_count, the three kernels of the
-        # cell-count scan (k_scan_tiles, k_scan_single, k_scan_add), k_bin_scatter,
-        # the cost-class pass (k_digit_hist, three scan kernels, k_digit_scatter)
-        # and the KD query kernel
-        "gpu_launches": 11 * args.steps,
+        # per chosen step (one graph replay): k_bin_count, the two kernels of the
+        # cell-count scan (k_scan_tiles, k_scan_add), k_bin_scatter, the cost-class
+        # pass (k_digit_hist, the two scan kernels, k_digit_scatter) and the KD query
+        # kernel
+        "gpu_launches": 9 * args.steps,
         "clocks": clocks,
         "other_workloads": rows,
     }
