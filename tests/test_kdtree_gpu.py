@@ -478,3 +478,21 @@ def test_float64_filter(d, data, oracle):
                 dd, ii = tree.query(torch.from_numpy(q).to(cuda), nr_nns_searches=k)
                 np.testing.assert_array_equal(dd.cpu().numpy(), bd, err_msg=f"{k} {levels}")
                 np.testing.assert_array_equal(ii.cpu().numpy(), bi, err_msg=f"{k} {levels}")
+
+
+@pytest.mark.parametrize("scale", [1e-300, 1e-160, 1e-20, 1.0, 1e20, 1e150])
+@pytest.mark.parametrize("dims", [1, 2, 3])
+def test_float64_filter_at_any_scale(scale, dims, oracle):
+    """The filter's reach over the exponents: distances that vanish, are
+    subnormal, or come near the largest double, and k-th distances of zero."""
+    from torch_kdtree_gb300 import build_kd_tree
+    rng = np.random.default_rng(dims)
+    ref = rng.standard_normal((3000, dims)) * scale
+    ref[:300] = ref[300]
+    q = np.concatenate([rng.standard_normal((200, dims)) * scale, ref[300:301], ref[:20], 1e3 * scale * np.ones((3, dims))])
+    tree = build_kd_tree(torch.from_numpy(ref).to("cuda"))
+    for k in (1, 8, 33):
+        d, i = tree.query(torch.from_numpy(q).to("cuda"), nr_nns_searches=k)
+        bd, bi = oracle.brute(ref, q, k)
+        np.testing.assert_array_equal(d.cpu().numpy(), bd)
+        np.testing.assert_array_equal(i.cpu().numpy(), bi)

@@ -14,8 +14,11 @@
 // descent takes is free, since siblings are tested by their boxes.
 //
 // 65,536 queries in 200,000 points, k=8: 0.77 ms without the filter (1.06 ms on
-// four lanes per query), 0.32 ms with it; the image grows from 32 to 48 bytes
-// per point.
+// four lanes per query), 0.27 ms with it; the image grows from 32 to 48 bytes
+// per point.  The double pipe was still 75% busy at 0.32 ms, a good part of it
+// with the query's place in the frame, now an axis per lane, and the reach,
+// now in integers.  What is left is the survivors' distances; keeping those of
+// several leaves for one batch costs more in reach (4 or more: 2-10% slower).
 #pragma once
 
 #include <cuda_runtime.h>
@@ -53,6 +56,18 @@ struct FilterArgs {
 __device__ __forceinline__ double frame_down(double v, double c, double s) { return __dmul_rd(__dsub_rd(v, c), s); }
 __device__ __forceinline__ double frame_up(double v, double c, double s) { return __dmul_ru(__dsub_ru(v, c), s); }
 
+// A float no less than d 2^e, d a distance given by its bits (never negative,
+// never NaN): at most an ulp more than the next float, at least 2^-126.  In
+// integers: a search asks for it at every leaf.
+__device__ __forceinline__ float scaled_up(unsigned long long d, int e) {
+    const int field = int(d >> 52);
+    if (field == 0x7FF) return __int_as_float(0x7f800000);
+    const int f = max(field, 1) - 1023 + e + 127;
+    if (f <= 0) return __int_as_float(0x00800000);
+    if (f >= 255) return __int_as_float(0x7f800000);
+    return __int_as_float((f << 23) + int((d >> 29) & 0x7FFFFFull) + 1);
+}
+
 template <int D, int R>
 __device__ __forceinline__ void kd_search_filtered(const FilterArgs& a, const double (&q)[D], double* out_d,
                                                    int32_t* out_i, Key<double>* buf, uint32_t* todo, int lane) {
@@ -61,17 +76,25 @@ __device__ __forceinline__ void kd_search_filtered(const FilterArgs& a, const do
     const int L = a.levels;
     const double scale = a.f.frame->scale;
     bool nan_q = false;  // all distances are NaN and enter no list: the home leaf is enough
-    float lo[D], hi[D];  // the query's place in the frame
+    float lo[D], hi[D];  // the query's place in the frame, an axis per lane
+    {
+        const int c = lane < D ? lane : 0;
+        double qc = q[0];
+        if (D > 1) qc = c == 1 ? q[D > 1 ? 1 : 0] : qc;
+        if (D > 2) qc = c == 2 ? q[D > 2 ? 2 : 0] : qc;
+        const double centre = a.f.frame->centre[c];
+        const float down = __double2float_rd(frame_down(qc, centre, scale));
+        const float up = __double2float_ru(frame_up(qc, centre, scale));
 #pragma unroll
-    for (int c = 0; c < D; ++c) {
-        nan_q |= q[c] != q[c];
-        lo[c] = __double2float_rd(frame_down(q[c], a.f.frame->centre[c], scale));
-        hi[c] = __double2float_ru(frame_up(q[c], a.f.frame->centre[c], scale));
+        for (int i = 0; i < D; ++i) {
+            nan_q |= (__double_as_longlong(q[i]) & 0x7FFFFFFFFFFFFFFFll) > 0x7FF0000000000000ll;
+            lo[i] = __shfl_sync(0xFFFFFFFFu, down, i);
+            hi[i] = __shfl_sync(0xFFFFFFFFu, up, i);
+        }
     }
+    const int scale_exp = 2 * (int((__double_as_longlong(scale) >> 52) & 0x7FF) - 1023);
     float reach = __int_as_float(0x7f800000);  // the k-th distance in the frame, rounded up
-    auto set_reach = [&]() {
-        reach = __fmul_ru(__double2float_ru(__dmul_ru(__dmul_ru(wl.worst.dist(), scale), scale)), 1.0f + 0x1p-21f);
-    };
+    auto set_reach = [&]() { reach = __fmul_ru(scaled_up(wl.worst.d, scale_exp), 1.0f + 0x1p-21f); };
     // sum of squares of lower bounds on the per-axis distances
     auto sum_sq = [&](const float (&g)[D]) {
         float s = 0.f;
