@@ -138,8 +138,11 @@ int log2_round(double v) { return v <= 1.0 ? 0 : int(std::lround(std::log2(v)));
 // queries 0.97 / 2.1; 200,000 points, 131,072 queries, k=4 0.19 / 0.24), lower
 // for k = 1, higher for k = 16, and lower in fewer dimensions, where a search
 // is shorter (131,072 queries in 200,000 points, k=4: d=2 0.10 / 0.16, d=1
-// 0.05 / 0.13).  Leaves of more than 192 points (a depth the caller asked for)
-// always take a warp.  Trees of 4-8 dimensions (1M refs x 262k queries N(0,1),
+// 0.05 / 0.13).  Small clouds fall slower than the large ones' slope (1,000
+// points, d = 3: 20,000 queries, k=4 0.054 / 0.040, k=1 0.043 / 0.036, 40,000
+// 0.056 / 0.061 and 0.043 / 0.049; k=16 40,000 0.115 / 0.077, 131,072 0.195 /
+// 0.203; 5,000 points, d = 2, k=16 40,000 0.083 / 0.068).  Leaves of more than
+// 192 points (a depth the caller asked for) always take a warp.  Trees of 4-8 dimensions (1M refs x 262k queries N(0,1),
 // depth 12-13): one lane only for k = 1 up to 6 dimensions from half a wave of
 // queries on (d=4: 0.40 vs 0.70 ms), a warp otherwise (d=8, k=16: 21.4 vs 38.3).
 int auto_lanes(const tk_tree* t, int64_t nq, int k) {
@@ -160,9 +163,12 @@ int auto_lanes(const tk_tree* t, int64_t nq, int k) {
     }
     const double avg_leaf = double(t->n) / double(int64_t(1) << t->search_levels);
     if (!t->auto_depth && avg_leaf > 192) return 32;
-    const double crossing = sms * 120.0 * std::max(1.0, std::log2(double(t->n)) - 10.3);
+    const double lg = std::log2(double(t->n));
+    double crossing = sms * 120.0 * std::max({1.0, lg - 10.3, t->dims > 1 ? 0.3 * lg - 1.05 : 0.0});
     const double by_k = k == 1 ? 0.6 : (k > 8 ? 1.4 : 0.9), by_dims = t->dims == 1 ? 0.4 : (t->dims == 2 ? 0.65 : 1.0);
-    return double(nq) >= crossing * by_k * by_dims ? 1 : 32;
+    crossing *= by_k;
+    if (k > 8 && t->dims > 1) crossing = std::max(crossing, sms * 660.0);
+    return double(nq) >= crossing * by_dims ? 1 : 32;
 }
 
 int pow2_ceil(int v) {
