@@ -424,3 +424,23 @@ def test_few_recomputed_queries(n_listed, k, d, oracle):
     dd, ii = tk().nn_distance(torch.from_numpy(ref).to(cuda), torch.from_numpy(q).to(cuda), k, mode="tf32")
     np.testing.assert_array_equal(dd.cpu().numpy(), bd)
     np.testing.assert_array_equal(ii.cpu().numpy(), bi)
+
+
+@pytest.mark.parametrize("d,mode", [(23, "tf32"), (24, "tf32"), (32, "tf32"), (39, "tf32"), (24, "bf16_split"), (47, "bf16_split")])
+@pytest.mark.parametrize("data", ["normal", "repeated", "clusters"])
+def test_tensor_core_staged_rerank(d, mode, data, oracle):
+    """The re-rank that recomputes the best scores first, at the edges of its
+    dimensions: lists of distinct scores, of ties, and of far more than wanted."""
+    rng = np.random.default_rng(d)
+    n, nq = 20_000, 2_000
+    ref = rng.standard_normal((n, d)).astype(np.float32)
+    if data == "repeated":
+        ref = ref[rng.integers(0, n // 20, n)]
+    elif data == "clusters":
+        ref = (ref[rng.integers(0, 40, n)] + 0.05 * rng.standard_normal((n, d))).astype(np.float32)
+    q = (ref[rng.integers(0, n, nq)] + 0.2 * rng.standard_normal((nq, d))).astype(np.float32)
+    for k in (1, 10, 32):
+        bd, bi = oracle.brute(ref, q, k)
+        dd, ii = tk().nn_distance(torch.from_numpy(ref).to(cuda), torch.from_numpy(q).to(cuda), k, mode=mode)
+        np.testing.assert_array_equal(dd.cpu().numpy(), bd)
+        np.testing.assert_array_equal(ii.cpu().numpy(), bi)
