@@ -444,3 +444,22 @@ def test_tensor_core_staged_rerank(d, mode, data, oracle):
         dd, ii = tk().nn_distance(torch.from_numpy(ref).to(cuda), torch.from_numpy(q).to(cuda), k, mode=mode)
         np.testing.assert_array_equal(dd.cpu().numpy(), bd)
         np.testing.assert_array_equal(ii.cpu().numpy(), bi)
+
+
+@pytest.mark.parametrize("mode", ["exact", "tf32", "bf16_split"])
+@pytest.mark.parametrize("d", [8, 32])
+@pytest.mark.parametrize("share", [0.01, 0.1, 0.5])
+@pytest.mark.parametrize("value", [np.inf, -np.inf])
+def test_many_infinite_references(mode, d, share, value, oracle):
+    """References with an infinite coordinate, and nothing else unusual in the
+    cloud: many of them, so that whole samples of scores come from such rows."""
+    rng = np.random.default_rng(d)
+    ref = rng.standard_normal((20_000, d)).astype(np.float32)
+    ref[rng.permutation(len(ref))[:int(share * len(ref))], 1] = value
+    q = rng.standard_normal((1_000, d)).astype(np.float32)
+    for k in (1, 8, 32):
+        bd, bi = oracle.brute(ref, q, k)
+        assert np.isfinite(bd).all()
+        dd, ii = tk().nn_distance(torch.from_numpy(ref).to(cuda), torch.from_numpy(q).to(cuda), k, mode=mode)
+        np.testing.assert_array_equal(dd.cpu().numpy(), bd)
+        np.testing.assert_array_equal(ii.cpu().numpy(), bi)

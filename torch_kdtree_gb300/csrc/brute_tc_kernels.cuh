@@ -30,8 +30,8 @@ inline size_t align256(size_t v) { return (v + 255) / 256 * 256; }
 // non-finite coordinates) enter no list, and overflowing ones break the error
 // bound, so a query is certified only when |q|^2 < 2^125 and every reference
 // has |r|^2 < 2^125 (the pack kernel flags any other reference in `err`,
-// which certifies nothing; the tcgen05 path takes references with infinite or
-// NaN coordinates for padding).  Then every partial sum of a score is below
+// which certifies nothing; the tcgen05 path packs references with infinite or
+// NaN coordinates as padding).  Then every partial sum of a score is below
 // |r|^2 + 2|q||r| <= 2 (|q|^2 + |r|^2) < 2^127: finite.  Uncertified queries
 // are answered by the exact kernel.
 constexpr float kTcNormLimit = 0x1p125f;
@@ -297,30 +297,32 @@ __global__ void __launch_bounds__(256) k_tc5_pack(const float* __restrict__ x, i
     const long long r = is_query ? p : (long long)packed_ref(uint32_t(tile), uint32_t(c), uint32_t(tiles));
     const bool real = r < rows;
     const float* row = x + r * d;
+    // A reference with an infinite or NaN coordinate is at distance inf or NaN:
+    // it is in no certified answer (those have k finite distances), and all of
+    // its row becomes padding's.  Packed as it is, its products are infinite,
+    // scores of -inf take the sample's threshold down to -inf, and tau with it.
+    float nrm = 0.f, odd = 0.f;  // odd: NaN if a coordinate is not finite
+    if (!is_query) {
+        for (int j = 0; real && j < d; ++j) {
+            nrm = fmaf(row[j], row[j], nrm);
+            odd += row[j] - row[j];
+        }
+    }
+    const bool used = real && odd == 0.f;
     float v[E];
 #pragma unroll
     for (int e = 0; e < E; ++e) {
         const int k = cb * E + e;
         v[e] = 0.f;
         if (k < d) {
-            v[e] = real ? row[k] : 0.f;
+            v[e] = used ? row[k] : 0.f;
             if (is_query) v[e] = -2.f * v[e];
         } else if (k == d) {
             if (is_query) {
                 v[e] = real ? 1.f : 0.f;
             } else {
-                float nrm = 0.f, odd = 0.f;  // odd: NaN if a coordinate is not finite
-                for (int j = 0; real && j < d; ++j) {
-                    nrm = fmaf(row[j], row[j], nrm);
-                    odd += row[j] - row[j];
-                }
-                // An infinite or NaN coordinate puts the reference at distance
-                // inf or NaN: it is in no certified answer (those have k
-                // finite distances) and counts as padding.  For the rest see
-                // kTcNormLimit.
-                const bool finite = odd == 0.f;
-                if (finite && !(nrm < kTcNormLimit)) atomicOr(err, kTcErrRange);
-                v[e] = real && finite ? nrm : kT5PadNorm;
+                if (used && !(nrm < kTcNormLimit)) atomicOr(err, kTcErrRange);  // see kTcNormLimit
+                v[e] = used ? nrm : kT5PadNorm;
             }
         }
     }
@@ -831,7 +833,7 @@ __device__ __forceinline__ float squared_norm(const float* qrow, int d, int lane
 __device__ __forceinline__ bool certified(const RerankArgs& a, float qq, float tau, float D) {
     if (a.err && *a.err) return false;
     if (!(qq < kTcNormLimit)) return false;  // see kTcNormLimit (also NaN / inf coordinates)
-    if (isinf(tau)) return true;
+    if (tau == __int_as_float(0x7f800000)) return true;  // every other reference was recomputed
     const float u = 1.0f / 16777216.0f;           // 2^-24
     const float m = float(a.d + 4) * u;           // rounding of the exact FP32 distance
     const float Dp = D * (1.0f + 2.0f * m);       // at least the real |q-r|^2 of any r with dist(r) <= D
