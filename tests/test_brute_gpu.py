@@ -463,3 +463,30 @@ def test_many_infinite_references(mode, d, share, value, oracle):
         dd, ii = tk().nn_distance(torch.from_numpy(ref).to(cuda), torch.from_numpy(q).to(cuda), k, mode=mode)
         np.testing.assert_array_equal(dd.cpu().numpy(), bd)
         np.testing.assert_array_equal(ii.cpu().numpy(), bi)
+
+
+def test_default_mode_workspace_covers_every_pass():
+    """Calls of more queries than one pass over the tensor cores: the size that
+    is asked for covers the full passes and the rest, whatever its length."""
+    from torch_kdtree_gb300 import _lib
+    from torch_kdtree_gb300._lib import LIB
+    full = 262_144
+    for n, d, k in ((20_000, 32, 8), (20_000, 8, 8), (262_144, 32, 32), (5_000, 16, 1)):
+        def size(nq, mode):
+            return LIB.tk_nn_distance_workspace_size(n, nq, d, k, _lib.TK_F32, mode)
+        one = size(full, _lib.TK_BRUTE_BF16_SPLIT)
+        for rest in range(1, full, 128):
+            need = size(rest, _lib.TK_BRUTE_BF16_SPLIT)
+            assert size(full + rest, _lib.TK_BRUTE_ROUTED) >= max(one, need), (n, d, k, rest)
+
+
+@pytest.mark.parametrize("nq", [262_144 + 255_000, 262_144 + 1, 2 * 262_144])
+def test_default_mode_in_several_passes(nq, oracle):
+    rng = np.random.default_rng(nq)
+    ref = rng.standard_normal((20_000, 8)).astype(np.float32)
+    q = rng.standard_normal((nq, 8)).astype(np.float32)
+    dd, ii = tk().nn_distance(torch.from_numpy(ref).to(cuda), torch.from_numpy(q).to(cuda), 8)
+    rows = np.concatenate([np.arange(100), np.arange(262_044, 262_244) % nq, np.arange(nq - 300, nq)])
+    bd, bi = oracle.brute(ref, q[rows], 8)
+    np.testing.assert_array_equal(dd.cpu().numpy()[rows], bd)
+    np.testing.assert_array_equal(ii.cpu().numpy()[rows], bi)
