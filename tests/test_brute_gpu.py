@@ -490,3 +490,25 @@ def test_default_mode_in_several_passes(nq, oracle):
     bd, bi = oracle.brute(ref, q[rows], 8)
     np.testing.assert_array_equal(dd.cpu().numpy()[rows], bd)
     np.testing.assert_array_equal(ii.cpu().numpy()[rows], bi)
+
+
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+@pytest.mark.parametrize("nq", [30_000, 400_000])
+@pytest.mark.parametrize("k", [1, 4, 8, 16, 20])
+def test_nan_queries_through_a_tree(dtype, nq, k):
+    """A query with a NaN coordinate has no neighbour, whichever search the
+    default mode takes: distance inf, index -1 (the CUDA cores' answer)."""
+    from torch_kdtree_gb300.nn_distance import nn_distance_raw
+    g = torch.Generator(device=cuda).manual_seed(k)
+    for d in (1, 2, 3):
+        ref = torch.randn(20_000, d, generator=g, device=cuda, dtype=torch.float64).to(getattr(torch, np.dtype(dtype).name))
+        q = torch.randn(nq, d, generator=g, device=cuda, dtype=torch.float64).to(ref.dtype)
+        rows = torch.tensor([0, 5, nq // 2, nq - 1], device=cuda)
+        q[rows, d - 1] = float("nan")
+        dd, ii = tk().nn_distance(ref, q, k)
+        assert torch.isinf(dd[rows]).all() and (ii[rows] == -1).all()
+        few = torch.cat([rows, torch.arange(1000, 1100, device=cuda)])
+        want_d = torch.empty(len(few), k, dtype=ref.dtype, device=cuda)
+        want_i = torch.empty(len(few), k, dtype=torch.int32, device=cuda)
+        nn_distance_raw(ref, q[few].contiguous(), k, want_d, want_i, "exact")
+        assert torch.equal(dd[few], want_d) and torch.equal(ii[few], want_i)

@@ -57,6 +57,7 @@ struct KdArgs {
     T* out_d;                // [nq, k]
     int32_t* out_i;          // [nq, k]
     int* work;               // global work counter, zero at launch; null: the grid covers all queries once
+    bool nan_empty = false;  // a NaN query's row stays empty, as the exhaustive search leaves it (see kd_search)
 };
 
 template <typename T, int D>
@@ -157,9 +158,13 @@ __device__ __forceinline__ void bitonic_sort(Key<T> (&v)[R]) {
 // -- then by its bounding box, whose per-axis gaps also become the axis
 // bounds its own descent starts from.  All lanes of a group hold the same
 // trail: no local memory, for any group size.
+//
+// With `fill`, one lane takes its first k points from the home leaf without a
+// comparison; a query with a NaN coordinate keeps them, at distance NaN.
+// Without it they are offered like the others, and NaN enters no list.
 template <typename T, int D, int G, int R>
 __device__ __forceinline__ void kd_search(const TreeView<T>& tv, const T (&q)[D], int k, T* out_d,
-                                          int32_t* out_i, unsigned gmask, int gl, int gbase) {
+                                          int32_t* out_i, unsigned gmask, int gl, int gbase, bool fill = true) {
     TopK<T, G, R> list;
     list.init(k, gl);
     Key<T> worst = Key<T>::sentinel();
@@ -189,7 +194,7 @@ __device__ __forceinline__ void kd_search(const TreeView<T>& tv, const T (&q)[D]
         ax = (ax + 1 == D) ? 0 : ax + 1;
     }
     uint32_t pending = (1u << L) - 1u;  // every far sibling on the home path (L <= 24)
-    bool home = true;
+    bool home = fill;
 
     for (;;) {
         // `node` is a leaf; its box records carry its point range (one round trip for both)
@@ -377,7 +382,12 @@ __device__ __forceinline__ void kd_query_one(const KdArgs<T>& a, const T* s_med,
     T* out_d = a.out_d + (long long)qi * a.k;
     int32_t* out_i = a.out_i + (long long)qi * a.k;
     if constexpr (G == 32) kd_search_warp<T, D, R>(tv, q, a.k, out_d, out_i, buf, gl);
-    else kd_search<T, D, G, R>(tv, q, a.k, out_d, out_i, gmask, gl, gbase);
+    else {
+        bool nan_q = false;
+#pragma unroll
+        for (int c = 0; c < D; ++c) nan_q |= q[c] != q[c];
+        kd_search<T, D, G, R>(tv, q, a.k, out_d, out_i, gmask, gl, gbase, !(a.nan_empty && nan_q));
+    }
 }
 
 constexpr int kKdBlock = 256;  // threads per block of the KD query kernels

@@ -346,6 +346,7 @@ int run_query(const tk_tree* t, const T* q, int nq, int k, T* dists, int32_t* id
     a.out_d = dists;
     a.out_i = idx;
     a.work = counter;
+    a.nan_empty = t->nan_empty;
     KdLaunch l{G, R, block, grid, smem};
     if (o.kernel_start_event) cudaEventRecord(static_cast<cudaEvent_t>(o.kernel_start_event), s);
     int rc;
@@ -1012,6 +1013,7 @@ tk_tree transient_tree(int64_t n, int64_t nq, int dims, int k, int dtype) {
     t.one_image = true;
     t.own_image = false;
     t.auto_depth = true;
+    t.nan_empty = true;
     t.search_levels = kMaxLevels;
     if (tree_image(n, dims, dtype, 1).f_pts) t.d_filter[0] = &t;  // it will have one: shapes the query (set_image places it)
     t.search_levels = query_levels(&t, auto_lanes(&t, nq, k), k);

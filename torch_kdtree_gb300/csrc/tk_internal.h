@@ -112,6 +112,7 @@ struct tk_tree {
     // The library chose search_levels: a query may stop at any shallower depth
     // (every node of the image knows its point range), see query_levels.
     bool auto_depth = false;
+    bool nan_empty = false;  // built for one exhaustive search's call: a NaN query's row stays empty
     int device = 0;
     int64_t n = 0;
     // host layout (one of the two is filled when the tree was built on the
