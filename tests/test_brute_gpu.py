@@ -512,3 +512,19 @@ def test_nan_queries_through_a_tree(dtype, nq, k):
         want_i = torch.empty(len(few), k, dtype=torch.int32, device=cuda)
         nn_distance_raw(ref, q[few].contiguous(), k, want_d, want_i, "exact")
         assert torch.equal(dd[few], want_d) and torch.equal(ii[few], want_i)
+
+
+@pytest.mark.parametrize("mode", ["exact", "tf32", "bf16_split"])
+@pytest.mark.parametrize("d", [4, 8, 32])
+def test_tiny_coordinates(mode, d, oracle):
+    """Clouds so small that products of coordinates are subnormal or zero,
+    where the relative error bounds of the tensor-core products do not hold."""
+    rng = np.random.default_rng(d)
+    ref = rng.standard_normal((5_000, d))
+    q = rng.standard_normal((500, d))
+    for e in np.arange(-23.0, -16.0, 0.25):
+        r, p = (ref * 10.0 ** e).astype(np.float32), (q * 10.0 ** e).astype(np.float32)
+        bd, bi = oracle.brute(r, p, 8)
+        dd, ii = tk().nn_distance(torch.from_numpy(r).to(cuda), torch.from_numpy(p).to(cuda), 8, mode=mode)
+        np.testing.assert_array_equal(dd.cpu().numpy(), bd, err_msg=f"1e{e}")
+        np.testing.assert_array_equal(ii.cpu().numpy(), bi, err_msg=f"1e{e}")

@@ -841,7 +841,10 @@ __device__ __forceinline__ bool certified(const RerankArgs& a, float qq, float t
     const float rho = qn + sqrtf(Dp);             // |r| of any such r
     const float eps = 2.0f * a.eps_dot + m;       // score error, relative
     const float big = qn * rho + rho * rho + fmaxf(Dp, qq);
-    const float E = 2.0f * eps * big + 4.0f * float(a.d + 16) * u * (big + fabsf(tau));  // first term: x2 safety
+    // first term: x2 safety; the last: operands, products and sums below 2^-126
+    // may be taken for zero, each of the at most 3 (d + 1) <= 195 products and
+    // sums at a loss of that much (relative bounds say nothing down there)
+    const float E = 2.0f * eps * big + 4.0f * float(a.d + 16) * u * (big + fabsf(tau)) + 0x1p-112f;
     return (qq + tau) - E > Dp;                   // false for NaN
 }
 
