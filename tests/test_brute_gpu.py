@@ -528,3 +528,22 @@ def test_tiny_coordinates(mode, d, oracle):
         dd, ii = tk().nn_distance(torch.from_numpy(r).to(cuda), torch.from_numpy(p).to(cuda), 8, mode=mode)
         np.testing.assert_array_equal(dd.cpu().numpy(), bd, err_msg=f"1e{e}")
         np.testing.assert_array_equal(ii.cpu().numpy(), bi, err_msg=f"1e{e}")
+
+
+@pytest.mark.parametrize("n_listed", [257, 1_000, 1_025, 3_000])
+@pytest.mark.parametrize("n", [600, 9_000])
+@pytest.mark.parametrize("k,d", [(1, 8), (20, 8), (64, 20)])
+def test_many_recomputed_queries(n_listed, n, k, d, oracle):
+    """Lists of some tiles of queries up to all of them, searched by a block
+    per tile and slice, with one slice of the references and with several."""
+    rng = np.random.default_rng(n_listed + k)
+    ref = np.concatenate([rng.standard_normal((n, d)), np.tile(rng.standard_normal((1, d)) + 20, (400, 1))])
+    ref = ref[rng.permutation(len(ref))].astype(np.float32)
+    q = rng.standard_normal((3_000, d)).astype(np.float32)
+    hard = rng.permutation(len(q))[:n_listed]
+    q[hard] = (20 + 0.1 * rng.standard_normal((n_listed, d))).astype(np.float32)
+    bd, bi = oracle.brute(ref, q, k)
+    for mode in ("tf32", "bf16_split"):
+        dd, ii = tk().nn_distance(torch.from_numpy(ref).to(cuda), torch.from_numpy(q).to(cuda), k, mode=mode)
+        np.testing.assert_array_equal(dd.cpu().numpy(), bd)
+        np.testing.assert_array_equal(ii.cpu().numpy(), bi)

@@ -76,23 +76,7 @@ size_t brute_ws_bytes(const BrutePlan& p, int64_t nq, int k) {
 }
 
 template <typename T>
-int run_brute(const T* ref, int64_t n, const T* q, int64_t nq, int d, int k, T* dists, int32_t* idx, void* ws,
-              size_t ws_bytes, cudaStream_t s, const int* gate = nullptr) {
-    const BrutePlan p = plan_brute(n, nq, d, k, sizeof(T) == 4);
-    if (ws_bytes < brute_ws_bytes<T>(p, nq, k) || (p.nsplit > 1 && !ws))
-        return fail(TK_EWORKSPACE, "workspace too small");
-    BruteArgs<T> a;
-    a.ref = ref;
-    a.q = q;
-    a.n = int(n);
-    a.nq = int(nq);
-    a.d = d;
-    a.k = k;
-    a.nsplit = p.nsplit;
-    a.out_d = dists;
-    a.out_i = idx;
-    a.part = static_cast<Key<T>*>(ws);
-    a.gate = gate;
+int launch_brute(const BruteArgs<T>& a, const BrutePlan& p, cudaStream_t s) {
     switch (p.DP) {
         case 1: return launch_dp<T, 1>(a, p, s);
         case 2: return launch_dp<T, 2>(a, p, s);
@@ -113,6 +97,27 @@ int run_brute(const T* ref, int64_t n, const T* q, int64_t nq, int d, int k, T* 
         return launch_brute_f64_wide(a, p, s);  // brute_f64.cu: d = 5 .. 128
     }
     return fail(TK_EUNSUPPORTED, "no brute-force kernel for this dimension");
+}
+
+template <typename T>
+int run_brute(const T* ref, int64_t n, const T* q, int64_t nq, int d, int k, T* dists, int32_t* idx, void* ws,
+              size_t ws_bytes, cudaStream_t s, const int* gate = nullptr) {
+    const BrutePlan p = plan_brute(n, nq, d, k, sizeof(T) == 4);
+    if (ws_bytes < brute_ws_bytes<T>(p, nq, k) || (p.nsplit > 1 && !ws))
+        return fail(TK_EWORKSPACE, "workspace too small");
+    BruteArgs<T> a;
+    a.ref = ref;
+    a.q = q;
+    a.n = int(n);
+    a.nq = int(nq);
+    a.d = d;
+    a.k = k;
+    a.nsplit = p.nsplit;
+    a.out_d = dists;
+    a.out_i = idx;
+    a.part = static_cast<Key<T>*>(ws);
+    a.gate = gate;
+    return launch_brute<T>(a, p, s);
 }
 
 // Route of a call that only wants the exact answer (TK_BRUTE_ROUTED).
@@ -202,7 +207,7 @@ int check_common(const void* ref, int64_t n, const void* q, int64_t nq, int d, i
 // memory -- a chain of such reads, so up to kVeryFew queries a block's eight
 // warps share a pair (one query in 262,144 references, d=32: 0.2 ms -> 0.04),
 // above that a warp takes one (0.8 us per query).  Longer lists go through the
-// tiled kernel above, its blocks looping over (query tile, slice) pairs.  A
+// tiled kernel above, a block per (query tile, slice) pair.  A
 // last kernel merges a query's slices, a block per query or for long lists a
 // warp; whichever kernel is not meant exits at once.  (The tiled kernel for any
 // list, with a lane merging a query's 128 slices, took 1.0 ms for a few dozen
@@ -213,7 +218,15 @@ constexpr int kFew = 256;
 constexpr int kFewSlices = 64;
 constexpr int kVeryFew = 32;
 constexpr int kMaxSlices = 128;
-constexpr int kSlots = 65536;  // (query, slice) pairs with a list in the shared buffer
+
+// The tiled kernel's plan for a list: enough blocks for the tiles of all
+// queries, and for 8 an SM.
+BrutePlan plan_list(int64_t n, int64_t nq, int d, int k) {
+    BrutePlan p = plan_brute(n, nq, d, k, true);
+    p.nsplit = int(std::max<int64_t>(1, std::min<int64_t>(kMaxSlices, n / 2048)));
+    p.list_blocks = std::max(p.qtiles, 8 * sm_count_dev());
+    return p;
+}
 
 struct ListArgs {
     const float* ref;
@@ -222,7 +235,7 @@ struct ListArgs {
     const int* qlist;
     const int* qcount;
     Key<float>* part;  // [listed query][slice][k]
-    int max_slices;    // of the tiled kernel
+    int max_slices, tile_blocks, per_tile;  // of the tiled kernel
     float* out_d;
     int32_t* out_i;
 };
@@ -326,7 +339,7 @@ __global__ void __launch_bounds__(256) k_list_merge(const ListArgs a) {
         }
         return;
     }
-    const int slices = list_slices(count, kSlots, a.max_slices);
+    const int slices = list_slices(count, a.tile_blocks, a.per_tile, a.max_slices);
     if (slices == 1) return;  // already in the outputs
     for (int slot = blockIdx.x * 8 + w; slot < count; slot += gridDim.x * 8) {
         WarpList<float, R> wl;
@@ -341,21 +354,24 @@ __global__ void __launch_bounds__(256) k_list_merge(const ListArgs a) {
 
 }  // namespace
 
-// Both kernels share one buffer of per-slice lists: 16.8 MB for k = 32,
-// whatever the list's length.
+// Both kernels share one buffer of per-slice lists, some 80 MB for k = 32
+// however many queries there are: a list per query of each of the tiled
+// kernel's blocks, or of the slices of a short list.
 size_t brute_fallback_workspace_bytes(int64_t n, int64_t nq, int d, int k) {
-    (void)n;
-    (void)d;
-    const int64_t slots = std::min<int64_t>(kSlots, std::max<int64_t>(nq, 1) * kMaxSlices);
-    return align256(sizeof(Key<float>) * size_t(slots) * k);
+    nq = std::max<int64_t>(nq, 1);
+    const BrutePlan p = plan_list(n, nq, d, k);
+    const int64_t tiled = std::min(nq * p.nsplit, int64_t(p.list_blocks) * (256 / p.G));
+    const int64_t few = std::min<int64_t>(nq, kFew) * kFewSlices;
+    return align256(sizeof(Key<float>) * size_t(std::max(tiled, few)) * k);
 }
 
 int brute_fallback(const float* ref, int64_t n, const float* q, int64_t nq, int d, int k, float* dists,
                    int32_t* idx, const int* qlist, const int* qcount, void* ws, size_t ws_bytes, cudaStream_t s) {
     if (ws_bytes < brute_fallback_workspace_bytes(n, nq, d, k)) return fail(TK_EWORKSPACE, "fallback workspace");
     const int sms = sm_count_dev(), few = int(std::min<int64_t>(nq, kFew));
-    const int max_slices = int(std::max<int64_t>(1, std::min<int64_t>(kMaxSlices, n / 2048)));
-    ListArgs l{ref, q, int(n), d, k, qlist, qcount, static_cast<Key<float>*>(ws), max_slices, dists, idx};
+    const BrutePlan p = plan_list(n, nq, d, k);
+    ListArgs l{ref, q, int(n), d, k, qlist, qcount, static_cast<Key<float>*>(ws), p.nsplit, p.list_blocks, 256 / p.G,
+               dists, idx};
     const unsigned gs = unsigned(std::min(4 * sms, few * kFewSlices));
     const unsigned gm = unsigned(std::min<int64_t>(4 * sms, std::max<int64_t>(few, (nq + 7) / 8)));
     if (k <= 32) k_few_search<1><<<gs, 256, 0, s>>>(l);
@@ -363,11 +379,7 @@ int brute_fallback(const float* ref, int64_t n, const float* q, int64_t nq, int 
     else k_few_search<4><<<gs, 256, 0, s>>>(l);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return fail(TK_ECUDA, std::string("listed queries: ") + cudaGetErrorString(e));
-    int rc = TK_OK;
     if (nq > kFew) {
-        BrutePlan p = plan_brute(n, nq, d, k, true);
-        p.nsplit = max_slices;
-        p.list_blocks = int(std::min<int64_t>(int64_t(p.qtiles) * max_slices, 8 * sms));
         BruteArgs<float> a;
         a.ref = ref;
         a.q = q;
@@ -382,18 +394,7 @@ int brute_fallback(const float* ref, int64_t n, const float* q, int64_t nq, int 
         a.qlist = qlist;
         a.qcount = qcount;
         a.qmore = kFew;
-        a.slots = kSlots;
-        switch (p.DP) {
-            case 1: rc = launch_dp<float, 1>(a, p, s); break;
-            case 2: rc = launch_dp<float, 2>(a, p, s); break;
-            case 3: rc = launch_dp<float, 3>(a, p, s); break;
-            case 4: rc = launch_dp<float, 4>(a, p, s); break;
-            case 8: rc = launch_dp<float, 8>(a, p, s); break;
-            case 16: rc = launch_dp<float, 16>(a, p, s); break;
-            case 32: rc = launch_dp<float, 32>(a, p, s); break;
-            case 64: rc = launch_dp<float, 64>(a, p, s); break;
-            default: rc = launch_dp<float, 128>(a, p, s); break;
-        }
+        const int rc = launch_brute<float>(a, p, s);
         if (rc != TK_OK) return rc;
     }
     if (k <= 32) k_list_merge<1><<<gm, 256, 0, s>>>(l);
