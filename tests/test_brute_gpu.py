@@ -547,3 +547,30 @@ def test_many_recomputed_queries(n_listed, n, k, d, oracle):
         dd, ii = tk().nn_distance(torch.from_numpy(ref).to(cuda), torch.from_numpy(q).to(cuda), k, mode=mode)
         np.testing.assert_array_equal(dd.cpu().numpy(), bd)
         np.testing.assert_array_equal(ii.cpu().numpy(), bi)
+
+
+@pytest.mark.parametrize("mode", ["exact", "tf32", "bf16_split"])
+@pytest.mark.parametrize("d", [4, 8, 32, 39])
+@pytest.mark.parametrize("mean", [30.0, -3000.0, "one coordinate"])
+def test_clouds_far_from_the_origin(mode, d, mean, oracle):
+    """The candidate search takes points relative to the cloud's middle; its
+    answers stay exact, and hardly a query needs the exhaustive search."""
+    from test_bounded_wait_gpu import run
+    rng = np.random.default_rng(d)
+    ref = rng.standard_normal((20_000, d))
+    q = rng.standard_normal((1_000, d))
+    if mean == "one coordinate":
+        ref[:, d - 1] += 500
+        q[:, d - 1] += 500
+    else:
+        ref, q = ref + mean, q + mean
+    ref, q = ref.astype(np.float32), q.astype(np.float32)
+    rt, qt = torch.from_numpy(ref).to(cuda), torch.from_numpy(q).to(cuda)
+    for k in (1, 8):
+        bd, bi = oracle.brute(ref, q, k)
+        dd, ii = tk().nn_distance(rt, qt, k, mode=mode)
+        np.testing.assert_array_equal(dd.cpu().numpy(), bd)
+        np.testing.assert_array_equal(ii.cpu().numpy(), bi)
+    if mode == "bf16_split" and mean != -3000.0:
+        recomputed = run(rt, qt, 8, mode)[4]
+        assert recomputed < len(q) // 10, recomputed

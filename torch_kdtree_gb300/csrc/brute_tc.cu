@@ -4,6 +4,7 @@
 //
 //   score(q, r) = |r|^2 - 2 q.r   (ranks like |q - r|^2 for a fixed query)
 //
+// 0. k_tc5_centre: the point that q and r are taken relative to (tcgen05 path).
 // 1. k_tc_pack: operands for the tensor cores (TF32 rounded to nearest, or a
 //    BF16 hi/lo split x = hi + lo) and |x|^2 in FP32.
 // 2. k_tc5_select (brute_tc_kernels.cuh): tcgen05 products of 128 queries and
@@ -41,7 +42,7 @@ using namespace tcx;
 namespace {
 
 struct TcWs {
-    size_t a_pack, b_pack, a_lo, b_lo, rnorm, qnorm, fail_count, fail_list, brute, err, total;
+    size_t a_pack, b_pack, a_lo, b_lo, rnorm, qnorm, centre, fail_count, fail_list, brute, err, total;
     size_t cand_s, cand_i, tau;  // mma.sync search
     size_t hits, counts, thr;    // tcgen05 search
     int KP, C, nsplit, wanted;
@@ -171,6 +172,7 @@ TcWs tc_layout(int64_t n, int64_t nq, int d, int k, int mode, int sms) {
     }
     w.err = o; o += 256;
     if (w.tc5) {
+        w.centre = o; o += 256;
         const int64_t rows = (nq + kT5Rows - 1) / kT5Rows * kT5Rows;
         const size_t lists = size_t(first_slice(rows, w.split_from, w.head.nsplit, w.tail.nsplit)) * kT5Parts;
         w.hits = o; o += align256(8 * lists * kT5Cap);
@@ -221,9 +223,8 @@ int run_brute_tc(const float* ref, int64_t n, const float* q, int64_t nq, int d,
     if (!ws || ws_bytes < w.total) return fail(TK_EWORKSPACE, "workspace too small");
     char* p = static_cast<char*>(ws);
     const int n32 = int(n), nq32 = int(nq);
-    cudaError_t e0 = cudaMemsetAsync(p + w.err, 0, sizeof(int), s);
     int* err = reinterpret_cast<int*>(p + w.err);  // no certificates when set (see kTcNormLimit)
-    if (e0 != cudaSuccess) return fail(TK_ECUDA, std::string("memset: ") + cudaGetErrorString(e0));
+    int* fail_count = reinterpret_cast<int*>(p + w.fail_count);
     if (!w.tc5) {
         // The mma.sync candidate search keeps 128 rows' lists and a score tile
         // in shared memory; for k > 32 with d > 32 (C = 128, KP = 64) that is
@@ -235,15 +236,24 @@ int run_brute_tc(const float* ref, int64_t n, const float* q, int64_t nq, int d,
         if (cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess) optin = 0;
         if (select_smem_bytes(mode, w.KP, w.C) > size_t(optin)) {
             int* list = reinterpret_cast<int*>(p + w.fail_list);
-            int* count = reinterpret_cast<int*>(p + w.fail_count);
-            k_all_queries<<<(nq32 + 255) / 256, 256, 0, s>>>(nq32, list, count);
+            cudaError_t e0 = cudaMemsetAsync(err, 0, sizeof(int), s);
+            if (e0 != cudaSuccess) return fail(TK_ECUDA, std::string("memset: ") + cudaGetErrorString(e0));
+            k_all_queries<<<(nq32 + 255) / 256, 256, 0, s>>>(nq32, list, fail_count);
             const cudaError_t e1 = cudaGetLastError();
             if (e1 != cudaSuccess) return fail(TK_ECUDA, std::string("fallback list: ") + cudaGetErrorString(e1));
-            return brute_fallback(ref, n, q, nq, d, k, dists, idx, list, count, p + w.brute,
+            return brute_fallback(ref, n, q, nq, d, k, dists, idx, list, fail_count, p + w.brute,
                                   brute_fallback_workspace_bytes(n, nq, d, k), s);
         }
     }
     int crc = TK_OK;
+    const float* centre = w.tc5 ? reinterpret_cast<const float*>(p + w.centre) : nullptr;
+    if (w.tc5) {
+        k_tc5_centre<<<1, 1024, 0, s>>>(ref, n32, d, reinterpret_cast<float*>(p + w.centre), err, fail_count);
+    } else {
+        cudaError_t e0 = cudaMemsetAsync(err, 0, sizeof(int), s);
+        if (e0 == cudaSuccess) e0 = cudaMemsetAsync(fail_count, 0, sizeof(int), s);
+        if (e0 != cudaSuccess) return fail(TK_ECUDA, std::string("memset: ") + cudaGetErrorString(e0));
+    }
     if (w.tc5) {
         // 1-2. pack into the core-matrix layout and run the tcgen05 candidate kernel
         const int qblocks = (nq32 + kT5Rows - 1) / kT5Rows, tiles = int((n + kT5Cols - 1) / kT5Cols);
@@ -254,13 +264,13 @@ int run_brute_tc(const float* ref, int64_t n, const float* q, int64_t nq, int d,
         const int chunks = w.KP * (mode == TK_BRUTE_TF32 ? 4 : 2) / 16;  // 16-byte pieces of a packed row
         auto grid = [&](int64_t rows) { return unsigned((rows * chunks + 255) / 256); };
         const unsigned ga = grid(int64_t(qblocks) * kT5Rows), gb = grid(int64_t(tiles) * kT5Cols);
-        if (mode == TK_BRUTE_TF32) {
-            k_tc5_pack<TK_BRUTE_TF32><<<ga, 256, 0, s>>>(q, nq32, qblocks, d, w.KP, 1, ahi, alo, err);
-            k_tc5_pack<TK_BRUTE_TF32><<<gb, 256, 0, s>>>(ref, n32, tiles, d, w.KP, 0, bhi, blo, err);
-        } else {
-            k_tc5_pack<TK_BRUTE_BF16_SPLIT><<<ga, 256, 0, s>>>(q, nq32, qblocks, d, w.KP, 1, ahi, alo, err);
-            k_tc5_pack<TK_BRUTE_BF16_SPLIT><<<gb, 256, 0, s>>>(ref, n32, tiles, d, w.KP, 0, bhi, blo, err);
-        }
+        const Tc5Pack pq{q, nq32, qblocks, ahi, alo}, pr{ref, n32, tiles, bhi, blo};
+        // set up while the kernel before it runs
+        const cudaError_t e0 =
+            mode == TK_BRUTE_TF32
+                ? launch(true, k_tc5_pack<TK_BRUTE_TF32>, dim3(ga + gb), 256, 0, s, pq, pr, int(ga), d, w.KP, centre, err)
+                : launch(true, k_tc5_pack<TK_BRUTE_BF16_SPLIT>, dim3(ga + gb), 256, 0, s, pq, pr, int(ga), d, w.KP, centre, err);
+        if (e0 != cudaSuccess) return fail(TK_ECUDA, std::string("packing: ") + cudaGetErrorString(e0));
         Tc5Args t5{};
         t5.a_hi = ahi;
         t5.a_lo = alo;
@@ -318,8 +328,6 @@ int run_brute_tc(const float* ref, int64_t n, const float* q, int64_t nq, int d,
         if (crc != TK_OK) return crc;
     }
     // 3. exact re-rank + certificate
-    cudaError_t e = cudaMemsetAsync(p + w.fail_count, 0, sizeof(int), s);
-    if (e != cudaSuccess) return fail(TK_ECUDA, std::string("memset: ") + cudaGetErrorString(e));
     RerankArgs ra{};
     ra.ref = ref;
     ra.q = q;
@@ -343,15 +351,16 @@ int run_brute_tc(const float* ref, int64_t n, const float* q, int64_t nq, int d,
                                              : (3.1 / 65536.0 + 3.0 * (d + 2) * 2.0 * u));
     ra.out_d = dists;
     ra.out_i = idx;
-    ra.fail_count = reinterpret_cast<int*>(p + w.fail_count);
+    ra.centre = centre;
+    ra.fail_count = fail_count;
     ra.fail_list = reinterpret_cast<int*>(p + w.fail_list);
-    ra.err = reinterpret_cast<const int*>(p + w.err);
+    ra.err = err;
     const int rb = (nq32 + 7) / 8;
     if (w.tc5) {
         k_tc5_rerank<<<rb, 256, 0, s>>>(ra);
     } else if (k <= 32) k_tc_rerank<1><<<rb, 256, 0, s>>>(ra);
     else k_tc_rerank<2><<<rb, 256, 0, s>>>(ra);
-    e = cudaGetLastError();
+    const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return fail(TK_ECUDA, std::string("tc launch: ") + cudaGetErrorString(e));
     // 4. exact recomputation of the uncertified queries
     return brute_fallback(ref, n, q, nq, d, k, dists, idx, ra.fail_list, ra.fail_count, p + w.brute,

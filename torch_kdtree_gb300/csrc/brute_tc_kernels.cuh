@@ -12,6 +12,7 @@
 
 #include "brute.cuh"
 #include "kd_warp.cuh"
+#include "launch.cuh"
 #include "tc_sm100.cuh"
 #include "tk_internal.h"
 
@@ -260,6 +261,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_tc_select(const TcArgs a) {
 // memory, often neighbours in space, fall into different tiles (see the sample
 // below) and different column groups (see the lists).  Padding rows carry a
 // huge |r|^2.
+constexpr int kT5MaxDims = 47;
 constexpr int kT5Rows = 128;   // M (queries per block)
 constexpr int kT5Cols = 256;   // N (references per tile)
 constexpr int kT5EpiWarps = 16; // 4 per 32-lane quarter of the accumulator when reading tensor memory
@@ -279,17 +281,59 @@ __device__ __forceinline__ uint32_t packed_ref(uint32_t tile, uint32_t col, uint
     return ((col - 67u * tile) & uint32_t(kT5Cols - 1)) * tiles + tile;
 }
 
-// A thread per 16 bytes of a packed row.  is_query selects [-2q, 1]
-// (tiles of kT5Rows rows) or [r, |r|^2] (tiles of kT5Cols rows).
+// The point that queries and references are taken relative to: a score's error
+// grows with their squared norms, so a cloud far from the origin (its mean 30
+// times its spread) would get no certificate.  Per coordinate the median of 32
+// references, where it exceeds half their interquartile range, else 0 (a cloud
+// around the origin keeps its operands).  A warp per coordinate, a lane per
+// reference, one block; it also zeroes the words of the report.
+static __global__ void __launch_bounds__(1024) k_tc5_centre(const float* __restrict__ ref, int n, int d,
+                                                            float* __restrict__ centre, int* __restrict__ err,
+                                                            int* __restrict__ fail_count) {
+    const int lane = threadIdx.x & 31;
+    if (threadIdx.x == 0) *err = *fail_count = 0;
+    for (int c = threadIdx.x >> 5; c < d; c += 32) {
+        float v = ref[(long long)lane * n / 32 * d + c];
+        if (!(fabsf(v) < 0x1p60f)) v = 0.f;  // infinite and NaN coordinates, too
+        int rank = 0;
+#pragma unroll
+        for (int j = 0; j < 32; ++j) {
+            const float o = __shfl_sync(0xFFFFFFFFu, v, j);
+            rank += o < v || (o == v && j < lane) ? 1 : 0;
+        }
+        auto ranked = [&](int r) { return __shfl_sync(0xFFFFFFFFu, v, __ffs(__ballot_sync(0xFFFFFFFFu, rank == r)) - 1); };
+        const float lower = ranked(8), median = ranked(16), upper = ranked(24);
+        if (lane == 0) centre[c] = fabsf(median) >= 0.5f * (upper - lower) ? median : 0.f;
+    }
+}
+
+// One side's points and where they go.
+struct Tc5Pack {
+    const float* x;
+    int rows, tiles;
+    unsigned char *hi, *lo;
+};
+
+// A thread per 16 bytes of a packed row, [-2q, 1] (tiles of kT5Rows rows) in
+// the first q_blocks blocks, [r, |r|^2] (tiles of kT5Cols rows) in the others,
+// q and r relative to `centre`.
 template <int MODE>
-__global__ void __launch_bounds__(256) k_tc5_pack(const float* __restrict__ x, int rows, int tiles, int d, int KP,
-                                                  int is_query, unsigned char* __restrict__ hi,
-                                                  unsigned char* __restrict__ lo, int* __restrict__ err) {
+__global__ void __launch_bounds__(256) k_tc5_pack(const Tc5Pack queries, const Tc5Pack refs, int q_blocks, int d,
+                                                  int KP, const float* centre, int* err) {
+    begin();
+    const bool is_query = int(blockIdx.x) < q_blocks;
+    const Tc5Pack& side = is_query ? queries : refs;
+    const float* __restrict__ x = side.x;
+    const int rows = side.rows, tiles = side.tiles;
+    unsigned char *hi = side.hi, *lo = side.lo;
+    __shared__ float mid[kT5MaxDims];
+    if (threadIdx.x < d) mid[threadIdx.x] = centre[threadIdx.x];
+    __syncthreads();
     constexpr int ESZ = MODE == TK_BRUTE_TF32 ? 4 : 2;
     constexpr int E = 16 / ESZ;  // elements of 16 bytes
     const int KB = KP * ESZ, chunks = KB / 16;
     const int tile_rows = is_query ? kT5Rows : kT5Cols;
-    const long long i = (long long)blockIdx.x * 256 + threadIdx.x;
+    const long long i = (long long)(int(blockIdx.x) - (is_query ? 0 : q_blocks)) * 256 + threadIdx.x;
     const long long p = i / chunks;
     const int cb = int(i - p * chunks);
     if (p >= (long long)tiles * tile_rows) return;
@@ -304,7 +348,8 @@ __global__ void __launch_bounds__(256) k_tc5_pack(const float* __restrict__ x, i
     float nrm = 0.f, odd = 0.f;  // odd: NaN if a coordinate is not finite
     if (!is_query) {
         for (int j = 0; real && j < d; ++j) {
-            nrm = fmaf(row[j], row[j], nrm);
+            const float v = __fsub_rn(row[j], mid[j]);
+            nrm = fmaf(v, v, nrm);
             odd += row[j] - row[j];
         }
     }
@@ -315,7 +360,7 @@ __global__ void __launch_bounds__(256) k_tc5_pack(const float* __restrict__ x, i
         const int k = cb * E + e;
         v[e] = 0.f;
         if (k < d) {
-            v[e] = used ? row[k] : 0.f;
+            v[e] = used ? __fsub_rn(row[k], mid[k]) : 0.f;
             if (is_query) v[e] = -2.f * v[e];
         } else if (k == d) {
             if (is_query) {
@@ -760,6 +805,7 @@ struct RerankArgs {
     const float* cand_s;  // mma.sync search: [nq, nsplit, C]
     const int32_t* cand_i;
     const float* tau;     // [nq, nsplit]
+    const float* centre;  // tcgen05 search: what the scores are relative to (else null)
     int keep;             // tcgen05 search: references per query worth recomputing
     const uint2* hits;    // see Tc5Args
     const int* counts;
@@ -815,10 +861,13 @@ __device__ __forceinline__ float rerank_dist(const float* __restrict__ qrow, con
     return acc;
 }
 
-// |q|^2 on every lane of the warp, a lane per coordinate.
-__device__ __forceinline__ float squared_norm(const float* qrow, int d, int lane) {
+// |q|^2, relative to `centre` if there is one, on every lane of the warp.
+__device__ __forceinline__ float squared_norm(const float* qrow, const float* centre, int d, int lane) {
     float qq = 0.f;
-    for (int c = lane; c < d; c += 32) qq = fmaf(qrow[c], qrow[c], qq);
+    for (int c = lane; c < d; c += 32) {
+        const float v = centre ? __fsub_rn(qrow[c], centre[c]) : qrow[c];
+        qq = fmaf(v, v, qq);
+    }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) qq += __shfl_xor_sync(0xFFFFFFFFu, qq, o);
     return qq;
@@ -827,8 +876,9 @@ __device__ __forceinline__ float squared_norm(const float* qrow, int d, int lane
 // Certificate of a query (|q|^2 = qq) whose k-th exact distance among the
 // recomputed references is D; every other reference scores at or above tau.
 // In single precision: E already doubles the bound on the score's error, and
-// its last term covers the rounding of this arithmetic, below 2 (d + 16) u of
-// the largest operand.  (In double it kept the slow pipe busy for a third of
+// its second term covers the rounding of this arithmetic, below 2 (d + 16) u of
+// the largest operand, and that of taking q and r relative to the centre (u of
+// each coordinate, which moves |q - r|^2 by at most 4.1 u (|q|^2 + |r|^2)).  (In double it kept the slow pipe busy for a third of
 // the re-rank.)  Overflow or NaN anywhere refuses the certificate.
 __device__ __forceinline__ bool certified(const RerankArgs& a, float qq, float tau, float D) {
     if (a.err && *a.err) return false;
@@ -844,7 +894,7 @@ __device__ __forceinline__ bool certified(const RerankArgs& a, float qq, float t
     // first term: x2 safety; the last: operands, products and sums below 2^-126
     // may be taken for zero, each of the at most 3 (d + 1) <= 195 products and
     // sums at a loss of that much (relative bounds say nothing down there)
-    const float E = 2.0f * eps * big + 4.0f * float(a.d + 16) * u * (big + fabsf(tau)) + 0x1p-112f;
+    const float E = 2.0f * eps * big + 4.0f * float(a.d + 18) * u * (big + fabsf(tau)) + 0x1p-112f;
     return (qq + tau) - E > Dp;                   // false for NaN
 }
 
@@ -870,7 +920,7 @@ __global__ void __launch_bounds__(256) k_tc_rerank(const RerankArgs a) {
         worst = offer<float, 32, R>(list, mine, worst, 0xFFFFFFFFu, lane, 0);
     }
     list.store(a.k, lane, a.out_d, a.out_i, qi);
-    const float qq = squared_norm(qrow, a.d, lane);
+    const float qq = squared_norm(qrow, a.centre, a.d, lane);
     if (lane == 0) {
         float tau = __int_as_float(0x7f800000);
         for (int s = 0; s < a.nsplit; ++s) tau = fminf(tau, a.tau[(long long)qi * a.nsplit + s]);
@@ -979,7 +1029,7 @@ static __global__ void __launch_bounds__(256) k_tc5_rerank(const RerankArgs a) {
         __syncwarp();
         wl.flush(lane);
     };
-    const float qq = squared_norm(qrow, a.d, lane);
+    const float qq = squared_norm(qrow, a.centre, a.d, lane);
     if (a.d >= kStagedDims && nl <= 8 && total > a.k + 48 && total <= 32 * HELD) {
         uint2 hit[HELD];  // hit h of all lists on lane h % 32
         const int mine = lane < nl ? counts[lane] : 0;
