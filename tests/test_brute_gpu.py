@@ -574,3 +574,38 @@ def test_clouds_far_from_the_origin(mode, d, mean, oracle):
     if mode == "bf16_split" and mean != -3000.0:
         recomputed = run(rt, qt, 8, mode)[4]
         assert recomputed < len(q) // 10, recomputed
+
+
+@pytest.mark.parametrize("mode", ["exact", "tf32", "bf16_split"])
+@pytest.mark.parametrize("d", [4, 8, 32])
+@pytest.mark.parametrize("clusters,apart", [(2, 300.0), (64, 100.0), (64, 10.0), (1000, 100.0)])
+def test_distant_clusters(mode, d, clusters, apart, oracle):
+    """Clusters whose distances to one another dwarf those within: the lists go
+    on by the scores' error where they hold what is there, and rows without a
+    chance take no hits; also next to rows of a cloud around the middle."""
+    rng = np.random.default_rng(clusters + d)
+    n, nq = 20_000, 1_500
+    at = (rng.standard_normal((clusters, d)) * apart).astype(np.float32)
+    at[0] = 0
+    pick = rng.integers(0, clusters, nq)
+    pick[: nq // 3] = 0  # whole blocks of rows around the middle
+    ref = (at[rng.integers(0, clusters, n)] + rng.standard_normal((n, d))).astype(np.float32)
+    q = (at[pick] + rng.standard_normal((nq, d))).astype(np.float32)
+    rt, qt = torch.from_numpy(ref).to(cuda), torch.from_numpy(q).to(cuda)
+    for k in (1, 8, 32):
+        bd, bi = oracle.brute(ref, q, k)
+        dd, ii = tk().nn_distance(rt, qt, k, mode=mode)
+        np.testing.assert_array_equal(dd.cpu().numpy(), bd)
+        np.testing.assert_array_equal(ii.cpu().numpy(), bi)
+
+
+def test_clusters_that_the_lists_hold_are_certified():
+    """312 references a cluster, 100 spreads apart: more of them lie within the
+    scores' error than the sample's threshold lets through, and fit the lists."""
+    from test_bounded_wait_gpu import run
+    rng = np.random.default_rng(0)
+    at = (rng.standard_normal((64, 8)) * 100).astype(np.float32)
+    ref = (at[rng.integers(0, 64, 20_000)] + rng.standard_normal((20_000, 8))).astype(np.float32)
+    q = (at[rng.integers(0, 64, 2_000)] + rng.standard_normal((2_000, 8))).astype(np.float32)
+    recomputed = run(torch.from_numpy(ref).to(cuda), torch.from_numpy(q).to(cuda), 8, "bf16_split")[4]
+    assert recomputed < len(q) // 4, recomputed

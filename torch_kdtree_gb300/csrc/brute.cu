@@ -223,7 +223,7 @@ constexpr int kMaxSlices = 128;
 // queries, and for 8 an SM.
 BrutePlan plan_list(int64_t n, int64_t nq, int d, int k) {
     BrutePlan p = plan_brute(n, nq, d, k, true);
-    p.nsplit = int(std::max<int64_t>(1, std::min<int64_t>(kMaxSlices, n / 2048)));
+    p.nsplit = int(std::max<int64_t>(1, std::min<int64_t>(kMaxSlices, n / 256)));
     p.list_blocks = std::max(p.qtiles, 8 * sm_count_dev());
     return p;
 }

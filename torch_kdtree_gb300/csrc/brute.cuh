@@ -68,16 +68,29 @@ __device__ __forceinline__ T sqdist_padded(const T (&q)[DP], const T* r) {
     return acc;
 }
 
+// A block's share: query tile, slice, and how many there are of queries and
+// slices.  Of a list only the device knows; kept in shared memory (`at`) and
+// read again after the search, whose registers it took to a fourth more time.
+struct BrutePlace {
+    int live, nsplit, qtile, slice;
+};
+template <typename T, bool LIST>
+__device__ __forceinline__ BrutePlace brute_place(const BruteArgs<T>& a, const volatile int* at) {
+    if constexpr (LIST) return BrutePlace{at[0], at[1], at[2], at[3]};
+    else return BrutePlace{a.nq, a.nsplit, int(blockIdx.x), int(blockIdx.y)};
+}
+
 // One query tile against one slice (LIST: of the listed queries).
 template <typename T, int DP, int G, int R, bool LIST>
-__device__ __forceinline__ void brute_block(const BruteArgs<T>& a, T* tile, int live, int nsplit, int qtile, int slice) {
+__device__ __forceinline__ void brute_block(const BruteArgs<T>& a, T* tile, const volatile int* at) {
     constexpr int TR = BruteTile<T, DP>::kRefs;
     const int lane = threadIdx.x & 31;
     const int gl = lane & (G - 1);
     const int gbase = lane & ~(G - 1);
     const unsigned gmask = group_mask<G>(lane);
-    const int slot = qtile * (blockDim.x / G) + threadIdx.x / G;
-    const bool active = slot < live;
+    const BrutePlace b = brute_place<T, LIST>(a, at);
+    const int slot = b.qtile * (blockDim.x / G) + threadIdx.x / G;
+    const bool active = slot < b.live;
     const int qi = active ? (LIST ? a.qlist[slot] : slot) : 0;
 
     T q[DP];
@@ -88,9 +101,9 @@ __device__ __forceinline__ void brute_block(const BruteArgs<T>& a, T* tile, int 
     list.init(a.k, gl);
     Key<T> worst = Key<T>::sentinel();
 
-    const long long per = ((long long)a.n + nsplit - 1) / nsplit;
-    const int r0 = int(min((long long)a.n, per * slice));
-    const int r1 = int(min((long long)a.n, per * (slice + 1)));
+    const long long per = ((long long)a.n + b.nsplit - 1) / b.nsplit;
+    const int r0 = int(min((long long)a.n, per * b.slice));
+    const int r1 = int(min((long long)a.n, per * (b.slice + 1)));
     for (int t0 = r0; t0 < r1; t0 += TR) {
         const int len = min(TR, r1 - t0);
         __syncthreads();
@@ -178,11 +191,13 @@ __device__ __forceinline__ void brute_block(const BruteArgs<T>& a, T* tile, int 
             }
         }
     }
-    if (!active) return;
-    if (nsplit == 1) {
-        list.store(a.k, gl, a.out_d, a.out_i, LIST ? a.qlist[slot] : slot);
+    const BrutePlace e = brute_place<T, LIST>(a, at);
+    const int row = e.qtile * (blockDim.x / G) + threadIdx.x / G;
+    if (row >= e.live) return;
+    if (e.nsplit == 1) {
+        list.store(a.k, gl, a.out_d, a.out_i, LIST ? a.qlist[row] : row);
     } else {
-        Key<T>* dst = a.part + ((long long)slot * nsplit + slice) * a.k;
+        Key<T>* dst = a.part + ((long long)row * e.nsplit + e.slice) * a.k;
 #pragma unroll
         for (int r = 0; r < R; ++r) {
             const int s = r * G + gl;
@@ -196,7 +211,7 @@ template <typename T, int DP, int G, int R>
 __global__ void __launch_bounds__(256) k_brute(const BruteArgs<T> a) {
     __shared__ __align__(16) T tile[BruteTile<T, DP>::kRefs * DP];
     if (a.gate && *a.gate == 0) return;
-    brute_block<T, DP, G, R, false>(a, tile, a.nq, a.nsplit, blockIdx.x, blockIdx.y);
+    brute_block<T, DP, G, R, false>(a, tile, nullptr);
 }
 
 // The queries of a list: a block per (query tile, slice) pair, the rest exit.
@@ -204,12 +219,20 @@ __global__ void __launch_bounds__(256) k_brute(const BruteArgs<T> a) {
 template <typename T, int DP, int G, int R>
 __global__ void __launch_bounds__(256) k_brute_list(const BruteArgs<T> a) {
     __shared__ __align__(16) T tile[BruteTile<T, DP>::kRefs * DP];
+    __shared__ int at[4];
     const int live = *a.qcount;
     if (live <= a.qmore) return;
     const int per_tile = blockDim.x / G, qtiles = (live + per_tile - 1) / per_tile;
     const int nsplit = list_slices(live, gridDim.x, per_tile, a.nsplit);
-    if (int(blockIdx.x) < qtiles * nsplit)
-        brute_block<T, DP, G, R, true>(a, tile, live, nsplit, blockIdx.x % qtiles, blockIdx.x / qtiles);
+    if (int(blockIdx.x) >= qtiles * nsplit) return;
+    if (threadIdx.x == 0) {
+        at[0] = live;
+        at[1] = nsplit;
+        at[2] = int(blockIdx.x) % qtiles;
+        at[3] = int(blockIdx.x) / qtiles;
+    }
+    __syncthreads();
+    brute_block<T, DP, G, R, true>(a, tile, at);
 }
 
 // Combine the per-slice lists of every query (group of G lanes per query).

@@ -157,7 +157,8 @@ TcWs tc_layout(int64_t n, int64_t nq, int d, int k, int mode, int sms) {
         w.b_pack = o; o += align256(es * n_pad * w.KP);
         w.a_lo = o; o += mode == TK_BRUTE_TF32 ? 0 : align256(es * nq_pad * w.KP);
         w.b_lo = o; o += mode == TK_BRUTE_TF32 ? 0 : align256(es * n_pad * w.KP);
-        w.rnorm = w.qnorm = o;
+        w.rnorm = o;
+        w.qnorm = o; o += align256(4 * size_t(nq));
     } else {
         const int qblocks = int((nq + kRows - 1) / kRows);
         int ns = std::max(1, (2 * sms + qblocks - 1) / std::max(1, qblocks));
@@ -246,7 +247,11 @@ int run_brute_tc(const float* ref, int64_t n, const float* q, int64_t nq, int d,
         }
     }
     int crc = TK_OK;
-    const float* centre = w.tc5 ? reinterpret_cast<const float*>(p + w.centre) : nullptr;
+    const float* centre = reinterpret_cast<const float*>(p + w.centre);
+    float* qnorm = reinterpret_cast<float*>(p + w.qnorm);
+    const double u = 1.0 / 16777216.0;
+    const float eps_dot = float(mode == TK_BRUTE_TF32 ? (1.0 / 1024.0 + 1.0 / 4194304.0 + (d + 2) * 2.0 * u)
+                                                      : (3.1 / 65536.0 + 3.0 * (d + 2) * 2.0 * u));
     if (w.tc5) {
         k_tc5_centre<<<1, 1024, 0, s>>>(ref, n32, d, reinterpret_cast<float*>(p + w.centre), err, fail_count);
     } else {
@@ -268,8 +273,8 @@ int run_brute_tc(const float* ref, int64_t n, const float* q, int64_t nq, int d,
         // set up while the kernel before it runs
         const cudaError_t e0 =
             mode == TK_BRUTE_TF32
-                ? launch(true, k_tc5_pack<TK_BRUTE_TF32>, dim3(ga + gb), 256, 0, s, pq, pr, int(ga), d, w.KP, centre, err)
-                : launch(true, k_tc5_pack<TK_BRUTE_BF16_SPLIT>, dim3(ga + gb), 256, 0, s, pq, pr, int(ga), d, w.KP, centre, err);
+                ? launch(true, k_tc5_pack<TK_BRUTE_TF32>, dim3(ga + gb), 256, 0, s, pq, pr, int(ga), d, w.KP, centre, qnorm, err)
+                : launch(true, k_tc5_pack<TK_BRUTE_BF16_SPLIT>, dim3(ga + gb), 256, 0, s, pq, pr, int(ga), d, w.KP, centre, qnorm, err);
         if (e0 != cudaSuccess) return fail(TK_ECUDA, std::string("packing: ") + cudaGetErrorString(e0));
         Tc5Args t5{};
         t5.a_hi = ahi;
@@ -284,7 +289,10 @@ int run_brute_tc(const float* ref, int64_t n, const float* q, int64_t nq, int d,
         t5.hits = reinterpret_cast<uint2*>(p + w.hits);
         t5.counts = reinterpret_cast<int*>(p + w.counts);
         t5.thr = reinterpret_cast<float*>(p + w.thr);
-        t5.err = reinterpret_cast<int*>(p + w.err);
+        t5.qnorm = qnorm;
+        t5.eps_dot = eps_dot;
+        t5.d = d;
+        t5.err = err;
         const uint32_t polls = g_wait_polls.load();
         t5.max_tries = polls ? polls : kT5MaxTries;
         crc = mode == TK_BRUTE_TF32 ? tc5_dispatch_tf32(t5, w.KP, qblocks, s)
@@ -292,7 +300,7 @@ int run_brute_tc(const float* ref, int64_t n, const float* q, int64_t nq, int d,
         if (crc != TK_OK) return crc;
     } else if (mode == TK_BRUTE_TF32) {
         k_tc_pack<TK_BRUTE_TF32><<<(nq32 + 255) / 256, 256, 0, s>>>(q, nq32, d, w.KP, reinterpret_cast<uint32_t*>(p + w.a_pack),
-                                                                  nullptr, nullptr, reinterpret_cast<float*>(p + w.qnorm),
+                                                                  nullptr, nullptr, qnorm,
                                                                   nullptr);
         k_tc_pack<TK_BRUTE_TF32><<<(n32 + 255) / 256, 256, 0, s>>>(ref, n32, d, w.KP, reinterpret_cast<uint32_t*>(p + w.b_pack),
                                                                  nullptr, nullptr, reinterpret_cast<float*>(p + w.rnorm),
@@ -300,7 +308,7 @@ int run_brute_tc(const float* ref, int64_t n, const float* q, int64_t nq, int d,
     } else {
         k_tc_pack<TK_BRUTE_BF16_SPLIT><<<(nq32 + 255) / 256, 256, 0, s>>>(
             q, nq32, d, w.KP, nullptr, reinterpret_cast<__nv_bfloat16*>(p + w.a_pack),
-            reinterpret_cast<__nv_bfloat16*>(p + w.a_lo), reinterpret_cast<float*>(p + w.qnorm), nullptr);
+            reinterpret_cast<__nv_bfloat16*>(p + w.a_lo), qnorm, nullptr);
         k_tc_pack<TK_BRUTE_BF16_SPLIT><<<(n32 + 255) / 256, 256, 0, s>>>(
             ref, n32, d, w.KP, nullptr, reinterpret_cast<__nv_bfloat16*>(p + w.b_pack),
             reinterpret_cast<__nv_bfloat16*>(p + w.b_lo), reinterpret_cast<float*>(p + w.rnorm), err);
@@ -346,12 +354,10 @@ int run_brute_tc(const float* ref, int64_t n, const float* q, int64_t nq, int d,
     ra.hits = reinterpret_cast<const uint2*>(p + w.hits);
     ra.counts = reinterpret_cast<const int*>(p + w.counts);
     ra.thr = reinterpret_cast<const float*>(p + w.thr);
-    const double u = 1.0 / 16777216.0;
-    ra.eps_dot = float(mode == TK_BRUTE_TF32 ? (1.0 / 1024.0 + 1.0 / 4194304.0 + (d + 2) * 2.0 * u)
-                                             : (3.1 / 65536.0 + 3.0 * (d + 2) * 2.0 * u));
+    ra.eps_dot = eps_dot;
     ra.out_d = dists;
     ra.out_i = idx;
-    ra.centre = centre;
+    ra.qnorm = qnorm;
     ra.fail_count = fail_count;
     ra.fail_list = reinterpret_cast<int*>(p + w.fail_list);
     ra.err = err;

@@ -316,10 +316,10 @@ struct Tc5Pack {
 
 // A thread per 16 bytes of a packed row, [-2q, 1] (tiles of kT5Rows rows) in
 // the first q_blocks blocks, [r, |r|^2] (tiles of kT5Cols rows) in the others,
-// q and r relative to `centre`.
+// q and r relative to `centre`; |q|^2 goes to qnorm.
 template <int MODE>
 __global__ void __launch_bounds__(256) k_tc5_pack(const Tc5Pack queries, const Tc5Pack refs, int q_blocks, int d,
-                                                  int KP, const float* centre, int* err) {
+                                                  int KP, const float* centre, float* qnorm, int* err) {
     begin();
     const bool is_query = int(blockIdx.x) < q_blocks;
     const Tc5Pack& side = is_query ? queries : refs;
@@ -346,14 +346,13 @@ __global__ void __launch_bounds__(256) k_tc5_pack(const Tc5Pack queries, const T
     // its row becomes padding's.  Packed as it is, its products are infinite,
     // scores of -inf take the sample's threshold down to -inf, and tau with it.
     float nrm = 0.f, odd = 0.f;  // odd: NaN if a coordinate is not finite
-    if (!is_query) {
-        for (int j = 0; real && j < d; ++j) {
-            const float v = __fsub_rn(row[j], mid[j]);
-            nrm = fmaf(v, v, nrm);
-            odd += row[j] - row[j];
-        }
+    const bool norm = !is_query || d / E == cb;  // a query's only where it is written
+    for (int j = 0; real && norm && j < d; ++j) {
+        const float v = __fsub_rn(row[j], mid[j]);
+        nrm = fmaf(v, v, nrm);
+        odd += row[j] - row[j];
     }
-    const bool used = real && odd == 0.f;
+    const bool used = real && (is_query || odd == 0.f);
     float v[E];
 #pragma unroll
     for (int e = 0; e < E; ++e) {
@@ -365,6 +364,7 @@ __global__ void __launch_bounds__(256) k_tc5_pack(const Tc5Pack queries, const T
         } else if (k == d) {
             if (is_query) {
                 v[e] = real ? 1.f : 0.f;
+                if (real) qnorm[r] = nrm;
             } else {
                 if (used && !(nrm < kTcNormLimit)) atomicOr(err, kTcErrRange);  // see kTcNormLimit
                 v[e] = used ? nrm : kT5PadNorm;
@@ -411,9 +411,44 @@ struct Tc5Args {
     uint2* hits;                // [slices of all rows, see first_slice][kT5Parts][CAP]: score bits, reference
     int* counts;                // [slices of all rows][kT5Parts]
     float* thr;                 // same shape: every reference of the part scoring below it is in its list
+    const float* qnorm;         // |q|^2
+    float eps_dot;              // see RerankArgs
+    int d;
     int* err;                   // kTcErrTimeout set when a bounded wait ran out
     uint32_t max_tries;         // polls of each mbarrier wait before giving up
 };
+
+// Whether a query's certificate holds: |q|^2 = qq, the k-th exact distance among
+// the recomputed references is D, every other reference scores at or above
+// tau.  In single precision: E already doubles the bound on the score's error,
+// and its second term covers the rounding of this arithmetic, below 2 (d + 16) u of
+// the largest operand, and that of taking q and r relative to the centre (u of
+// each coordinate, which moves |q - r|^2 by at most 4.1 u (|q|^2 + |r|^2)).  (In
+// double it kept the slow pipe busy for a third of the re-rank.)  Overflow or
+// NaN anywhere, and tau = -inf, refuse it; what fails for some D and tau fails
+// for every larger D and smaller tau.
+struct ScoreBound {
+    float Dp;  // at least the real |q-r|^2 of any r with dist(r) <= D
+    float E;   // bound on the error of any such r's score, and of the comparison
+};
+__device__ __forceinline__ ScoreBound score_bound(float eps_dot, int d, float qq, float tau, float D) {
+    const float u = 1.0f / 16777216.0f;           // 2^-24
+    const float m = float(d + 4) * u;             // rounding of the exact FP32 distance
+    const float Dp = D * (1.0f + 2.0f * m);
+    const float qn = sqrtf(qq);
+    const float rho = qn + sqrtf(Dp);             // |r|
+    const float eps = 2.0f * eps_dot + m;         // score error, relative
+    const float big = qn * rho + rho * rho + fmaxf(Dp, qq);
+    // first term: x2 safety; the last: operands, products and sums below 2^-126
+    // may be taken for zero, each of the at most 3 (d + 1) <= 195 products and
+    // sums at a loss of that much (relative bounds say nothing down there)
+    const float E = 2.0f * eps * big + 4.0f * float(d + 18) * u * (big + fabsf(tau)) + 0x1p-112f;
+    return ScoreBound{Dp, E};
+}
+__device__ __forceinline__ bool certifies(float eps_dot, int d, float qq, float tau, float D) {
+    const ScoreBound b = score_bound(eps_dot, d, qq, tau, D);
+    return (qq + tau) - b.E > b.Dp;               // false for NaN
+}
 
 // Order-preserving uint32 image of a score (negative scores included).
 __device__ __forceinline__ uint32_t score_bits(float sc) {
@@ -483,6 +518,25 @@ static __device__ __noinline__ uint2 prune_hits(uint2* list, int n, int lane) {
     return make_uint2(uint32_t(kept), __float_as_uint(bits_score(lo)));
 }
 
+// 16 bits of a squared distance (the negative ones, errors of scores, are 0),
+// ordered like it, and the largest distance with given bits.
+constexpr uint32_t kT5CodeInf = 0xFF00u;
+__device__ __forceinline__ uint16_t dist_code(float x) { return uint16_t(__float_as_uint(fmaxf(x, 0.f)) >> 15); }
+__device__ __forceinline__ float code_end(uint32_t code) { return __uint_as_float((code << 15) | 0x7FFFu); }
+
+// Threshold of a row at distance `far` (see k_tc5_select), t where more
+// references lie below that than the lists hold; by 4 lanes per row, each with
+// a quarter of its minima, which stand for `groups` groups.
+static __device__ __noinline__ float blurred_threshold(const uint16_t* mins, float t, float far, int groups, int pstride) {
+    const uint32_t end = min(uint32_t(dist_code(far)), kT5CodeInf - 1u);
+    int c = 0;
+    for (int i = 0; i < kT5Minima / 4; ++i) c += mins[i] <= end ? 1 : 0;
+    c += __shfl_xor_sync(0xFFFFFFFFu, c, 1);
+    c += __shfl_xor_sync(0xFFFFFFFFu, c, 2);
+    const float most = float(groups) * (1.f - __expf(-float(kT5Parts * 96) / float(groups * pstride)));
+    return float(c) <= most ? code_end(end) : t;
+}
+
 __device__ __forceinline__ float min3(float a, float b, float c) {
     float r;
     asm("min.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
@@ -505,7 +559,9 @@ __device__ __forceinline__ float min3(float a, float b, float c) {
 // for large k) of a row do over all slices.  Nothing depends on that: a list that fills up
 // lowers its own threshold to its kT5Kept-th best, and whatever the threshold, the
 // references that no list holds score at or above it, which is all that the
-// certificate uses.
+// certificate uses.  Rows whose threshold is too low for a certificate whatever
+// the distances (clusters far apart: scores differ by less than their error)
+// take no hits, and a block of such rows only waits for its products.
 //
 // 262,144 x 65,536, d=32, k=32, TF32: 2.9 ms; in whole waves of blocks 3.5 ms,
 // of which it was measured: tensor pipe 45% busy, issue
@@ -529,6 +585,7 @@ __global__ void __launch_bounds__(kT5Threads, 1) k_tc5_select(const Tc5Args a) {
     float* sThr = reinterpret_cast<float*>(sMin + kT5Rows * kT5MinStride);     // [kT5Rows]
     __shared__ __align__(8) uint64_t full_a, full_b[STAGES], mma_done[2], epi_done[2];
     __shared__ uint32_t tmem_base_sh;
+    __shared__ volatile int some_row;  // whether a row of the block is searched
     constexpr int NEPI = 32 * kT5EpiWarps;
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -547,6 +604,7 @@ __global__ void __launch_bounds__(kT5Threads, 1) k_tc5_select(const Tc5Args a) {
     auto tile_of = [&](int t) { return tile0 + (t < npre ? t * sl.pstride : t - npre); };
 
     if (tid == 0) {
+        some_row = 0;
         sm100::mbar_init(&full_a, 1);
         for (int i = 0; i < STAGES; ++i) sm100::mbar_init(&full_b[i], 1);
         sm100::mbar_init(&mma_done[0], 1);
@@ -647,14 +705,20 @@ __global__ void __launch_bounds__(kT5Threads, 1) k_tc5_select(const Tc5Args a) {
         const int myrow = 32 * quarter + lane;
         const uint32_t trow = tmem + (uint32_t(32 * quarter) << 16) + uint32_t(part * 64);
         auto bar_all = [&]() { asm volatile("bar.sync 1, %0;" ::"r"(NEPI) : "memory"); };
+        // |q|^2 of this thread's row, and of the row whose threshold it helps to find
+        const int grow = 32 * quarter + 8 * part + (lane >> 2), gl = lane & 3;
+        const float qq = rblock * kT5Rows + myrow < a.nq ? __ldg(a.qnorm + rblock * kT5Rows + myrow) : 0.f;
         bool alive = true;
         float va[32], vb[32];  // the thread's first and last 32 scores of a tile
-        // Waits for pipeline step t's products and loads both halves; the
-        // second is still on its way.  False when the wait ran out.
-        auto begin = [&](int t) {
+        // Waits for pipeline step t's products; false when the wait ran out.
+        auto products = [&](int t) {
             int ok = 1;
             if (lane == 0) ok = sm100::mbar_wait(&mma_done[t & 1], (t >> 1) & 1, a.max_tries);
-            if (!__shfl_sync(0xFFFFFFFFu, ok, 0)) return false;
+            return __shfl_sync(0xFFFFFFFFu, ok, 0) != 0;
+        };
+        // The same, and loads both halves; the second is still on its way.
+        auto begin = [&](int t) {
+            if (!products(t)) return false;
             sm100::tc_fence_after();
             const uint32_t at = trow + uint32_t((t & 1) * kT5Cols);
             sm100::tmem_ld32(at, va);
@@ -688,14 +752,14 @@ __global__ void __launch_bounds__(kT5Threads, 1) k_tc5_select(const Tc5Args a) {
             const float m2 = min16(vb, 0, g), m3 = min16(vb, 1, g);
             uint16_t* out = sMin + myrow * kT5MinStride;
             if (npre <= 8) {
-                out[(t * 4 + 0) * 4 + part] = uint16_t(score_bits(m0) >> 16);
-                out[(t * 4 + 1) * 4 + part] = uint16_t(score_bits(m1) >> 16);
-                out[(t * 4 + 2) * 4 + part] = uint16_t(score_bits(m2) >> 16);
-                out[(t * 4 + 3) * 4 + part] = uint16_t(score_bits(m3) >> 16);
+                out[(t * 4 + 0) * 4 + part] = dist_code(qq + m0);
+                out[(t * 4 + 1) * 4 + part] = dist_code(qq + m1);
+                out[(t * 4 + 2) * 4 + part] = dist_code(qq + m2);
+                out[(t * 4 + 3) * 4 + part] = dist_code(qq + m3);
             } else {
                 run = fminf(min3(run, m0, m1), fminf(m2, m3));
                 if ((t + 1) % tpg == 0 || t + 1 == npre) {
-                    out[(t / tpg) * 4 + part] = uint16_t(score_bits(run) >> 16);
+                    out[(t / tpg) * 4 + part] = dist_code(qq + run);
                     run = __int_as_float(0x7f800000);
                 }
             }
@@ -703,7 +767,6 @@ __global__ void __launch_bounds__(kT5Threads, 1) k_tc5_select(const Tc5Args a) {
         bar_all();
         {
             // the rank-th smallest of a row's minima, by 4 lanes: bisection on their 16-bit images
-            const int grow = 32 * quarter + 8 * part + (lane >> 2), gl = lane & 3;
             const uint16_t* mins = sMin + grow * kT5MinStride + gl * (kT5Minima / 4);
             uint32_t m[kT5Minima / 8];
 #pragma unroll
@@ -720,18 +783,35 @@ __global__ void __launch_bounds__(kT5Threads, 1) k_tc5_select(const Tc5Args a) {
                 if (c >= sl.rank) hi = mid;
                 else lo = min(mid + 1u, 0xFFFFu);
             }
-            // rounded up to the end of its 16-bit bucket, and low enough to
-            // keep the padding rows out (NaN minima give a NaN threshold: no
-            // hits, and no certificate for such rows)
-            if (gl == 0) sThr[grow] = lo < 0xFF80u ? fminf(bits_score((lo << 16) | 0xFFFFu), kT5PadNorm) : kT5PadNorm;
+            // t: rounded up to the end of its 16-bit bucket
+            float t = lo < kT5CodeInf ? code_end(lo) : kT5PadNorm;
+            // Where the scores' error is not small against t (clusters far
+            // apart), the certificate may want lists that go on by that error;
+            // groups without a reference that near tell whether they can hold
+            // what is there.  Where it exceeds t there is none, see below.
+            const int grow_q = rblock * kT5Rows + grow;
+            const float gqq = grow_q < a.nq ? __ldg(a.qnorm + grow_q) : 0.f;
+            const float E = score_bound(a.eps_dot, a.d, gqq, t - gqq, t).E;
+            const bool blurred = E > 0.0625f * t;
+            if (__any_sync(0xFFFFFFFFu, blurred)) {
+                const int groups = npre <= 8 ? 16 * npre : 4 * ((npre + tpg - 1) / tpg);
+                const float far = blurred_threshold(mins, t, t + 1.01f * E, groups, sl.pstride);
+                if (blurred) t = far;
+            }
+            // Low enough to keep the padding rows out.  (NaN scores have code 0
+            // and are no hits; such a row's |q|^2 is no certificate's.  Rows past
+            // the last query take no hits: all their scores are equal.)
+            const float low = fminf(t - gqq, kT5PadNorm);
+            const bool search = grow_q < a.nq && certifies(a.eps_dot, a.d, gqq, low, 0.f);
+            if (gl == 0) sThr[grow] = search ? low : -__int_as_float(0x7f800000);
+            if (__any_sync(0xFFFFFFFFu, search) && lane == 0) some_row = 1;
         }
         bar_all();
         const int row = rblock * kT5Rows + myrow;
         const long long lidx =
             (first_slice(row, a.split_from, a.head.nsplit, a.tail.nsplit) + slice) * kT5Parts + part;
         uint2* list = a.hits + lidx * CAP;
-        // (rows past the last query take no hits: all their scores are equal)
-        float thr = row < a.nq ? sThr[myrow] : -__int_as_float(0x7f800000);
+        float thr = sThr[myrow];
         int cnt = 0;
         // Hits of a half (32 columns from col0 on).  Branches are taken by the
         // whole warp (votes): few of its 512 scores of 16 columns are hits,
@@ -766,7 +846,16 @@ __global__ void __launch_bounds__(kT5Threads, 1) k_tc5_select(const Tc5Args a) {
                 }
             }
         };
-        for (int t = npre; alive && t < nseq; ++t) {
+        // A block without a row to search lets the products pass.  (The issuer
+        // looking whether it could stop took every block 13% more time.)
+        int next = npre;
+        if (some_row == 0) {
+            for (; alive && next < nseq; ++next) {
+                alive = products(next);
+                if (alive && lane == 0) sm100::mbar_arrive(&epi_done[next & 1]);
+            }
+        }
+        for (int t = next; alive && t < nseq; ++t) {
             alive = begin(t);
             if (!alive) break;
             const uint32_t tile = uint32_t(tile_of(t)), col0 = uint32_t(64 * part);
@@ -805,7 +894,7 @@ struct RerankArgs {
     const float* cand_s;  // mma.sync search: [nq, nsplit, C]
     const int32_t* cand_i;
     const float* tau;     // [nq, nsplit]
-    const float* centre;  // tcgen05 search: what the scores are relative to (else null)
+    const float* qnorm;   // |q|^2
     int keep;             // tcgen05 search: references per query worth recomputing
     const uint2* hits;    // see Tc5Args
     const int* counts;
@@ -861,41 +950,13 @@ __device__ __forceinline__ float rerank_dist(const float* __restrict__ qrow, con
     return acc;
 }
 
-// |q|^2, relative to `centre` if there is one, on every lane of the warp.
-__device__ __forceinline__ float squared_norm(const float* qrow, const float* centre, int d, int lane) {
-    float qq = 0.f;
-    for (int c = lane; c < d; c += 32) {
-        const float v = centre ? __fsub_rn(qrow[c], centre[c]) : qrow[c];
-        qq = fmaf(v, v, qq);
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) qq += __shfl_xor_sync(0xFFFFFFFFu, qq, o);
-    return qq;
-}
-
 // Certificate of a query (|q|^2 = qq) whose k-th exact distance among the
 // recomputed references is D; every other reference scores at or above tau.
-// In single precision: E already doubles the bound on the score's error, and
-// its second term covers the rounding of this arithmetic, below 2 (d + 16) u of
-// the largest operand, and that of taking q and r relative to the centre (u of
-// each coordinate, which moves |q - r|^2 by at most 4.1 u (|q|^2 + |r|^2)).  (In double it kept the slow pipe busy for a third of
-// the re-rank.)  Overflow or NaN anywhere refuses the certificate.
 __device__ __forceinline__ bool certified(const RerankArgs& a, float qq, float tau, float D) {
     if (a.err && *a.err) return false;
     if (!(qq < kTcNormLimit)) return false;  // see kTcNormLimit (also NaN / inf coordinates)
     if (tau == __int_as_float(0x7f800000)) return true;  // every other reference was recomputed
-    const float u = 1.0f / 16777216.0f;           // 2^-24
-    const float m = float(a.d + 4) * u;           // rounding of the exact FP32 distance
-    const float Dp = D * (1.0f + 2.0f * m);       // at least the real |q-r|^2 of any r with dist(r) <= D
-    const float qn = sqrtf(qq);
-    const float rho = qn + sqrtf(Dp);             // |r| of any such r
-    const float eps = 2.0f * a.eps_dot + m;       // score error, relative
-    const float big = qn * rho + rho * rho + fmaxf(Dp, qq);
-    // first term: x2 safety; the last: operands, products and sums below 2^-126
-    // may be taken for zero, each of the at most 3 (d + 1) <= 195 products and
-    // sums at a loss of that much (relative bounds say nothing down there)
-    const float E = 2.0f * eps * big + 4.0f * float(a.d + 18) * u * (big + fabsf(tau)) + 0x1p-112f;
-    return (qq + tau) - E > Dp;                   // false for NaN
+    return certifies(a.eps_dot, a.d, qq, tau, D);
 }
 
 // One warp per query: exact distances of the candidates, top-k, certificate.
@@ -920,7 +981,7 @@ __global__ void __launch_bounds__(256) k_tc_rerank(const RerankArgs a) {
         worst = offer<float, 32, R>(list, mine, worst, 0xFFFFFFFFu, lane, 0);
     }
     list.store(a.k, lane, a.out_d, a.out_i, qi);
-    const float qq = squared_norm(qrow, a.centre, a.d, lane);
+    const float qq = a.qnorm[qi];
     if (lane == 0) {
         float tau = __int_as_float(0x7f800000);
         for (int s = 0; s < a.nsplit; ++s) tau = fminf(tau, a.tau[(long long)qi * a.nsplit + s]);
@@ -945,7 +1006,7 @@ __global__ void __launch_bounds__(256) k_tc_rerank(const RerankArgs a) {
 // 0.52 -> 0.47; d=13 the same, d=8 1 to 7% slower.
 constexpr int kStagedDims = 24;
 
-static __global__ void __launch_bounds__(256) k_tc5_rerank(const RerankArgs a) {
+static __global__ void __launch_bounds__(256, 4) k_tc5_rerank(const RerankArgs a) {
     constexpr int CAP = kT5Cap, HELD = 8;
     __shared__ Key<float> bufs[8][64];
     __shared__ uint32_t todo[8][64];
@@ -991,8 +1052,11 @@ static __global__ void __launch_bounds__(256) k_tc5_rerank(const RerankArgs a) {
             else lo = mid + 1u;
             if (below >= a.keep && below <= a.keep + 32) break;  // near enough
         }
-        cut = hi;
-        tau = fminf(tau, bits_score(cut));
+        // (unless only the rest can give the certificate, see k_tc5_select)
+        if (certifies(a.eps_dot, a.d, a.qnorm[qi], bits_score(hi), 0.f)) {
+            cut = hi;
+            tau = fminf(tau, bits_score(cut));
+        }
     }
     WarpList<float, 1> wl;
     wl.init(a.k, bufs[w], lane);
@@ -1029,7 +1093,7 @@ static __global__ void __launch_bounds__(256) k_tc5_rerank(const RerankArgs a) {
         __syncwarp();
         wl.flush(lane);
     };
-    const float qq = squared_norm(qrow, a.centre, a.d, lane);
+    const float qq = a.qnorm[qi];
     if (a.d >= kStagedDims && nl <= 8 && total > a.k + 48 && total <= 32 * HELD) {
         uint2 hit[HELD];  // hit h of all lists on lane h % 32
         const int mine = lane < nl ? counts[lane] : 0;
