@@ -609,3 +609,28 @@ def test_clusters_that_the_lists_hold_are_certified():
     q = (at[rng.integers(0, 64, 2_000)] + rng.standard_normal((2_000, 8))).astype(np.float32)
     recomputed = run(torch.from_numpy(ref).to(cuda), torch.from_numpy(q).to(cuda), 8, "bf16_split")[4]
     assert recomputed < len(q) // 4, recomputed
+
+
+@pytest.mark.parametrize("mode", ["tf32", "bf16_split"])
+def test_tensor_core_modes_in_several_passes(mode, oracle):
+    """The modes that name the tensor cores take a million queries a pass: ten
+    million ask for no more workspace than that; the report counts all passes."""
+    from torch_kdtree_gb300 import _lib
+    from torch_kdtree_gb300._lib import LIB
+    from torch_kdtree_gb300.nn_distance import _BRUTE_MODES
+    from test_bounded_wait_gpu import run
+    for d, k in ((8, 1), (32, 32)):
+        assert LIB.tk_nn_distance_workspace_size(1_000_000, 10_000_000, d, k, _lib.TK_F32, _BRUTE_MODES[mode]) < 6 << 30
+    rng = np.random.default_rng(1)
+    nq = (1 << 20) + 1_000
+    ref = np.concatenate([rng.standard_normal((2_000, 4)), np.tile(rng.standard_normal((1, 4)) + 20, (700, 1))])
+    ref = ref.astype(np.float32)
+    q = rng.standard_normal((nq, 4)).astype(np.float32)
+    hard = np.concatenate([np.arange(300, 340), np.arange(nq - 50, nq - 20)])  # no certificate: all equally far
+    q[hard] = (20 + 0.1 * rng.standard_normal((len(hard), 4))).astype(np.float32)
+    dd, ii, rc, flags, recomputed = run(torch.from_numpy(ref).to(cuda), torch.from_numpy(q).to(cuda), 2, mode)
+    assert rc == 0 and flags == 0 and recomputed >= len(hard)
+    rows = np.concatenate([np.arange(250, 450), np.arange((1 << 20) - 100, nq)])
+    bd, bi = oracle.brute(ref, q[rows], 2)
+    np.testing.assert_array_equal(dd.cpu().numpy()[rows], bd)
+    np.testing.assert_array_equal(ii.cpu().numpy()[rows], bi)

@@ -128,17 +128,6 @@ enum class Route { kCudaCores, kTensorCores, kTree };
 constexpr int64_t kRoutePass = 262144;
 constexpr size_t kRouteBytes = size_t(4) << 30;
 
-// Workspace of those passes: a last, shorter pass may need more than a full
-// one (rows left over after whole waves of blocks are searched in slices, each
-// with lists of its own).
-size_t route_tc_bytes(int64_t n, int64_t nq, int d, int k) {
-    const int64_t rest = nq % kRoutePass;
-    size_t b = 0;
-    if (nq >= kRoutePass) b = brute_tc_workspace_bytes(n, kRoutePass, d, k, TK_BRUTE_BF16_SPLIT);
-    if (rest > 0) b = std::max(b, brute_tc_workspace_bytes(n, rest, d, k, TK_BRUTE_BF16_SPLIT));
-    return b;
-}
-
 // Up to three dimensions a tree that is built for the call pays from the
 // pairs on at which the comparisons cost more than its build (ms, exhaustive /
 // tree: 65,536 x 65,536, d=3, k=1 1.87 / 0.29; 20,000 x 20,000 k=1 0.22 / 0.21,
@@ -161,7 +150,7 @@ Route route_of(int64_t n, int64_t nq, int d, int k, int dtype) {
     if (dtype != TK_F32 || d > 47 || k > 32 || n < 512 || pairs < 6e4) return Route::kCudaCores;
     if (narrow && (k < 4 || (k < 8 && pairs > 5e7))) return Route::kCudaCores;
     if (k < 4 && pairs < (d <= 8 ? 5e8 : 1e6)) return Route::kCudaCores;
-    if (route_tc_bytes(n, nq, d, k) > kRouteBytes) return Route::kCudaCores;
+    if (brute_tc_workspace_bytes(n, nq, d, k, TK_BRUTE_BF16_SPLIT, kRoutePass) > kRouteBytes) return Route::kCudaCores;
     return Route::kTensorCores;
 }
 
@@ -413,10 +402,10 @@ extern "C" {
 
 size_t tk_nn_distance_workspace_size(int64_t n, int64_t nq, int dims, int k, int dtype, int mode) {
     if (n < 1 || nq < 0 || k < 1 || dims < 1) return 0;
-    if (mode == TK_BRUTE_TF32 || mode == TK_BRUTE_BF16_SPLIT) return brute_tc_workspace_bytes(n, nq, dims, k, mode);
+    if (mode == TK_BRUTE_TF32 || mode == TK_BRUTE_BF16_SPLIT) return brute_tc_workspace_bytes(n, nq, dims, k, mode, kTcPass);
     nq = std::max<int64_t>(nq, 1);
     const Route route = mode == TK_BRUTE_ROUTED ? route_of(n, nq, dims, k, dtype) : Route::kCudaCores;
-    if (route == Route::kTensorCores) return route_tc_bytes(n, nq, dims, k);
+    if (route == Route::kTensorCores) return brute_tc_workspace_bytes(n, nq, dims, k, TK_BRUTE_BF16_SPLIT, kRoutePass);
     return exact_ws_bytes(n, nq, dims, k, dtype) +
            (route == Route::kTree ? transient_tree_workspace_bytes(n, nq, dims, k, dtype) : 0);
 }
@@ -438,13 +427,10 @@ int tk_nn_distance(const void* ref, int64_t n, const void* q, int64_t nq, int di
         return run_tree_route<double>(static_cast<const double*>(ref), n, static_cast<const double*>(q), nq, dims, k,
                                       dtype, static_cast<double*>(dists), idx, ws, workspace_bytes, s);
     }
-    if (route == Route::kTensorCores) {
-        for (int64_t q0 = 0; q0 < nq && rc == TK_OK; q0 += kRoutePass)
-            rc = run_brute_tc(static_cast<const float*>(ref), n, static_cast<const float*>(q) + q0 * dims,
-                              std::min(kRoutePass, nq - q0), dims, k, TK_BRUTE_BF16_SPLIT,
-                              static_cast<float*>(dists) + q0 * k, idx + q0 * k, workspace, workspace_bytes, s);
-        return rc;
-    }
+    if (route == Route::kTensorCores)
+        return run_brute_tc(static_cast<const float*>(ref), n, static_cast<const float*>(q), nq, dims, k,
+                            TK_BRUTE_BF16_SPLIT, static_cast<float*>(dists), idx, workspace, workspace_bytes,
+                            kRoutePass, s);
     if (mode == TK_BRUTE_EXACT || mode == TK_BRUTE_ROUTED) {
         if (dtype == TK_F32)
             return run_brute<float>(static_cast<const float*>(ref), n, static_cast<const float*>(q), nq, dims, k,
@@ -455,7 +441,7 @@ int tk_nn_distance(const void* ref, int64_t n, const void* q, int64_t nq, int di
     if (mode == TK_BRUTE_TF32 || mode == TK_BRUTE_BF16_SPLIT) {
         if (dtype != TK_F32) return fail(TK_EINVAL, "tensor-core modes take float32 inputs");
         return run_brute_tc(static_cast<const float*>(ref), n, static_cast<const float*>(q), nq, dims, k, mode,
-                            static_cast<float*>(dists), idx, workspace, workspace_bytes, s);
+                            static_cast<float*>(dists), idx, workspace, workspace_bytes, kTcPass, s);
     }
     return fail(TK_EINVAL, "unknown brute-force mode");
 }

@@ -33,6 +33,7 @@
 #include <atomic>
 #include <cmath>
 #include <string>
+#include <vector>
 
 #include "brute_tc.cuh"
 #include "brute_tc_kernels.cuh"
@@ -42,7 +43,7 @@ using namespace tcx;
 namespace {
 
 struct TcWs {
-    size_t a_pack, b_pack, a_lo, b_lo, rnorm, qnorm, centre, fail_count, fail_list, brute, err, total;
+    size_t a_pack, b_pack, a_lo, b_lo, rnorm, qnorm, centre, fail_list, brute, total;
     size_t cand_s, cand_i, tau;  // mma.sync search
     size_t hits, counts, thr;    // tcgen05 search
     int KP, C, nsplit, wanted;
@@ -171,7 +172,6 @@ TcWs tc_layout(int64_t n, int64_t nq, int d, int k, int mode, int sms) {
         w.rnorm = o; o += align256(4 * size_t(n));
         w.qnorm = o; o += align256(4 * size_t(nq));
     }
-    w.err = o; o += 256;
     if (w.tc5) {
         w.centre = o; o += 256;
         const int64_t rows = (nq + kT5Rows - 1) / kT5Rows * kT5Rows;
@@ -184,7 +184,6 @@ TcWs tc_layout(int64_t n, int64_t nq, int d, int k, int mode, int sms) {
         w.cand_i = o; o += align256(4 * size_t(nq) * w.nsplit * w.C);
         w.tau = o; o += align256(4 * size_t(nq) * w.nsplit);
     }
-    w.fail_count = o; o += 256;
     w.fail_list = o; o += align256(4 * size_t(nq));
     w.brute = o; o += brute_fallback_workspace_bytes(n, nq, d, k);
     w.total = o;
@@ -212,20 +211,38 @@ int sm_count_now() {
 
 }  // namespace
 
-size_t brute_tc_workspace_bytes(int64_t n, int64_t nq, int d, int k, int mode) {
-    return tc_layout(n, std::max<int64_t>(nq, 1), d, k, mode, sm_count_now()).total;
+// The workspace starts with two words a pass (see kTcErrTimeout; queries
+// recomputed), which tk_nn_distance_report reads; every pass uses the rest.
+namespace {
+
+int64_t pass_length(int d, int k, int mode, int64_t pass) {
+    return tc5_eligible(d, k, mode) ? pass : int64_t(1) << 31;  // the mma.sync search's lists are short
+}
+int64_t pass_count(int64_t nq, int64_t len) { return (std::max<int64_t>(nq, 1) + len - 1) / len; }
+size_t words_bytes(int64_t passes) { return align256(2 * sizeof(int) * size_t(passes)); }
+
+}  // namespace
+
+// A last, shorter pass may need more than a full one: rows left over after
+// whole waves of blocks are searched in slices, each with lists of its own.
+size_t brute_tc_workspace_bytes(int64_t n, int64_t nq, int d, int k, int mode, int64_t pass) {
+    nq = std::max<int64_t>(nq, 1);
+    const int64_t len = pass_length(d, k, mode, pass), rest = nq % len;
+    const int sms = sm_count_now();
+    size_t most = 0;
+    if (nq >= len) most = tc_layout(n, len, d, k, mode, sms).total;
+    if (rest > 0) most = std::max(most, tc_layout(n, rest, d, k, mode, sms).total);
+    return words_bytes(pass_count(nq, len)) + most;
 }
 
-int run_brute_tc(const float* ref, int64_t n, const float* q, int64_t nq, int d, int k, int mode, float* dists,
-                 int32_t* idx, void* ws, size_t ws_bytes, cudaStream_t s) {
-    if (k > 64) return fail(TK_EUNSUPPORTED, "tensor-core modes support k <= 64 (use TK_BRUTE_EXACT)");
-    if (d > 64) return fail(TK_EUNSUPPORTED, "tensor-core modes support d <= 64 (use TK_BRUTE_EXACT)");
+namespace {
+
+int run_pass(const float* ref, int64_t n, const float* q, int64_t nq, int d, int k, int mode, float* dists,
+             int32_t* idx, int* words, char* p, cudaStream_t s) {
     const TcWs w = tc_layout(n, nq, d, k, mode, sm_count_now());
-    if (!ws || ws_bytes < w.total) return fail(TK_EWORKSPACE, "workspace too small");
-    char* p = static_cast<char*>(ws);
     const int n32 = int(n), nq32 = int(nq);
-    int* err = reinterpret_cast<int*>(p + w.err);  // no certificates when set (see kTcNormLimit)
-    int* fail_count = reinterpret_cast<int*>(p + w.fail_count);
+    int* err = words;  // no certificates when set (see kTcNormLimit)
+    int* fail_count = words + 1;
     if (!w.tc5) {
         // The mma.sync candidate search keeps 128 rows' lists and a score tile
         // in shared memory; for k > 32 with d > 32 (C = 128, KP = 64) that is
@@ -255,8 +272,7 @@ int run_brute_tc(const float* ref, int64_t n, const float* q, int64_t nq, int d,
     if (w.tc5) {
         k_tc5_centre<<<1, 1024, 0, s>>>(ref, n32, d, reinterpret_cast<float*>(p + w.centre), err, fail_count);
     } else {
-        cudaError_t e0 = cudaMemsetAsync(err, 0, sizeof(int), s);
-        if (e0 == cudaSuccess) e0 = cudaMemsetAsync(fail_count, 0, sizeof(int), s);
+        const cudaError_t e0 = cudaMemsetAsync(words, 0, 2 * sizeof(int), s);
         if (e0 != cudaSuccess) return fail(TK_ECUDA, std::string("memset: ") + cudaGetErrorString(e0));
     }
     if (w.tc5) {
@@ -373,6 +389,23 @@ int run_brute_tc(const float* ref, int64_t n, const float* q, int64_t nq, int d,
                           brute_fallback_workspace_bytes(n, nq, d, k), s);
 }
 
+}  // namespace
+
+int run_brute_tc(const float* ref, int64_t n, const float* q, int64_t nq, int d, int k, int mode, float* dists,
+                 int32_t* idx, void* ws, size_t ws_bytes, int64_t pass, cudaStream_t s) {
+    if (k > 64) return fail(TK_EUNSUPPORTED, "tensor-core modes support k <= 64 (use TK_BRUTE_EXACT)");
+    if (d > 64) return fail(TK_EUNSUPPORTED, "tensor-core modes support d <= 64 (use TK_BRUTE_EXACT)");
+    if (!ws || ws_bytes < brute_tc_workspace_bytes(n, nq, d, k, mode, pass))
+        return fail(TK_EWORKSPACE, "workspace too small");
+    const int64_t len = pass_length(d, k, mode, pass), passes = pass_count(nq, len);
+    char* rest = static_cast<char*>(ws) + words_bytes(passes);
+    int rc = TK_OK;
+    for (int64_t i = 0; i < passes && rc == TK_OK; ++i)
+        rc = run_pass(ref, n, q + i * len * d, std::min(len, nq - i * len), d, k, mode, dists + i * len * k,
+                      idx + i * len * k, static_cast<int*>(ws) + 2 * i, rest, s);
+    return rc;
+}
+
 }  // namespace tk
 
 extern "C" uint32_t tk_set_device_wait_limit(uint32_t polls) { return tk::g_wait_polls.exchange(polls); }
@@ -388,11 +421,13 @@ extern "C" int tk_nn_distance_report(const void* workspace, int64_t n, int64_t n
     if (mode != TK_BRUTE_TF32 && mode != TK_BRUTE_BF16_SPLIT) return TK_OK;  // the exact kernel has no certificate
     if (dtype != TK_F32) return fail(TK_EINVAL, "tensor-core modes take float32 inputs");
     if (!workspace || n < 1 || nq < 1 || k < 1 || dims < 1) return fail(TK_EINVAL, "bad shape or null workspace");
-    const TcWs w = tc_layout(n, nq, dims, k, mode, sm_count_now());
-    const char* p = static_cast<const char*>(workspace);
-    cudaError_t e = cudaMemcpy(flags, p + w.err, sizeof(int), cudaMemcpyDeviceToHost);
-    if (e == cudaSuccess) e = cudaMemcpy(recomputed, p + w.fail_count, sizeof(int), cudaMemcpyDeviceToHost);
+    std::vector<int> words(2 * size_t(pass_count(nq, pass_length(dims, k, mode, kTcPass))));
+    const cudaError_t e = cudaMemcpy(words.data(), workspace, sizeof(int) * words.size(), cudaMemcpyDeviceToHost);
     if (e != cudaSuccess) return fail(TK_ECUDA, std::string("report: ") + cudaGetErrorString(e));
+    for (size_t i = 0; i < words.size(); i += 2) {
+        *flags |= words[i];
+        *recomputed += words[i + 1];
+    }
     if (*flags & kTcErrTimeout)
         return fail(TK_ETIMEOUT, "a bounded device wait ran out; the exact kernel recomputed every query");
     return TK_OK;
