@@ -496,3 +496,25 @@ def test_float64_filter_at_any_scale(scale, dims, oracle):
         bd, bi = oracle.brute(ref, q, k)
         np.testing.assert_array_equal(d.cpu().numpy(), bd)
         np.testing.assert_array_equal(i.cpu().numpy(), bi)
+
+
+@pytest.mark.parametrize("d", [1, 2, 3])
+@pytest.mark.parametrize("leaf", [8, 16, 64, 128])
+def test_lanes_at_a_depth_of_the_caller(d, leaf):
+    """The number of lanes that the library takes at a depth the caller named
+    moves with the leaves' size; the answers are those of either number."""
+    from torch_kdtree_gb300 import build_kd_tree
+    from torch_kdtree_gb300._lib import QueryOpts
+    n = 20_000
+    g = torch.Generator(device=cuda).manual_seed(leaf)
+    ref = torch.randn(n, d, generator=g, device=cuda)
+    tree = build_kd_tree(ref, levels=int(np.round(np.log2(n / leaf))))
+    for nq in (20_000, 50_000, 90_000, 150_000):
+        q = torch.randn(nq, d, generator=g, device=cuda)
+        for k in (1, 8, 16):
+            tree.query_opts = None
+            want = tree.query(q, k)
+            for lanes in (1, 32):
+                tree.query_opts = QueryOpts.make(threads_per_query=lanes)
+                got = tree.query(q, k)
+                assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1])

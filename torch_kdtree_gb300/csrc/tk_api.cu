@@ -141,10 +141,16 @@ int log2_round(double v) { return v <= 1.0 ? 0 : int(std::lround(std::log2(v)));
 // 0.05 / 0.13).  Small clouds fall slower than the large ones' slope (1,000
 // points, d = 3: 20,000 queries, k=4 0.054 / 0.040, k=1 0.043 / 0.036, 40,000
 // 0.056 / 0.061 and 0.043 / 0.049; k=16 40,000 0.115 / 0.077, 131,072 0.195 /
-// 0.203; 5,000 points, d = 2, k=16 40,000 0.083 / 0.068).  Leaves of more than
-// 192 points (a depth the caller asked for) always take a warp.  Trees of 4-8 dimensions (1M refs x 262k queries N(0,1),
-// depth 12-13): one lane only for k = 1 up to 6 dimensions from half a wave of
-// queries on (d=4: 0.40 vs 0.70 ms), a warp otherwise (d=8, k=16: 21.4 vs 38.3).
+// 0.203; 5,000 points, d = 2, k=16 40,000 0.083 / 0.068).  At a depth the
+// caller asked for both search the same leaves, and the crossing moves with
+// them: small ones leave most of a warp's lanes without a point, large ones are
+// a long scan for one lane (a warp's time over one lane's, d = 3, k=16: 100,000
+// points in leaves of 12, 130,000 queries 1.44, of 49 0.7; 10,000 in leaves of
+// 10, 80,000 queries 1.4; 1M in leaves of 15, k=8, 80,000 0.95, 110,000 1.13);
+// more than 192 points always take a warp.  Trees of 4-8 dimensions (1M refs x
+// 262k queries N(0,1), depth 12-13): one lane only for k = 1 up to 6 dimensions
+// from half a wave of queries on (d=4: 0.40 vs 0.70 ms), a warp otherwise (d=8,
+// k=16: 21.4 vs 38.3).
 int auto_lanes(const tk_tree* t, int64_t nq, int k) {
     if (k > 16) return 32;
     const double sms = sm_count(t->device);
@@ -168,6 +174,11 @@ int auto_lanes(const tk_tree* t, int64_t nq, int k) {
     const double by_k = k == 1 ? 0.6 : (k > 8 ? 1.4 : 0.9), by_dims = t->dims == 1 ? 0.4 : (t->dims == 2 ? 0.65 : 1.0);
     crossing *= by_k;
     if (k > 8 && t->dims > 1) crossing = std::max(crossing, sms * 660.0);
+    if (!t->auto_depth) {
+        if (k == 1) crossing = sms * (165.0 + 28.0 * std::max(0.0, lg - 10.0)) * std::pow(std::max(1.0, avg_leaf / 16), 0.45);
+        else crossing *= std::pow(avg_leaf / 32, 0.75);
+        if (t->dims == 1) crossing = std::min(crossing, sms * 1000.0);  // by_dims makes it 400
+    }
     return double(nq) >= crossing * by_dims ? 1 : 32;
 }
 
