@@ -518,3 +518,22 @@ def test_lanes_at_a_depth_of_the_caller(d, leaf):
                 tree.query_opts = QueryOpts.make(threads_per_query=lanes)
                 got = tree.query(q, k)
                 assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1])
+
+
+@pytest.mark.parametrize("d", [4, 6, 8])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float64])
+def test_wide_trees_on_one_lane(d, dtype):
+    """One lane per query in 4-8 dimensions, in calls of less than a block an
+    SM, of a few more, and of several; the answers are a warp's."""
+    from torch_kdtree_gb300 import build_kd_tree
+    from torch_kdtree_gb300._lib import QueryOpts
+    g = torch.Generator(device=cuda).manual_seed(d)
+    tree = build_kd_tree(torch.randn(20_000, d, generator=g, device=cuda, dtype=dtype))
+    for nq in (5_000, 40_000, 80_000):
+        q = torch.randn(nq, d, generator=g, device=cuda, dtype=dtype)
+        for k in (1, 4, 16):
+            tree.query_opts = QueryOpts.make(threads_per_query=32)
+            want = tree.query(q, k)
+            tree.query_opts = QueryOpts.make(threads_per_query=1)
+            got = tree.query(q, k)
+            assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1])

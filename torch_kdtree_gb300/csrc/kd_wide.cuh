@@ -248,7 +248,7 @@ __device__ __forceinline__ void kd_search_wide_warp(const KdWideArgs<T>& a, cons
 // and 8 dims than the 62 registers it takes freely; the next rows loaded
 // while the last are offered: 4%.
 template <typename T, int W, int G, int R>
-__global__ void __launch_bounds__(256, G == 32 && sizeof(T) == 4 ? (R < 4 ? 5 : 4) : 1) k_kd_wide(const KdWideArgs<T> a) {
+__global__ void __launch_bounds__(256, G == 1 ? 0 : (sizeof(T) == 4 ? (R < 4 ? 5 : 4) : 1)) k_kd_wide(const KdWideArgs<T> a) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     T* s_med = reinterpret_cast<T*>(smem_raw);
     Key<T>* buf = nullptr;

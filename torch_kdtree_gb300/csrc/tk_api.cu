@@ -276,14 +276,15 @@ int prepare_order(const tk_tree* t, int L, int G, int nq, int k, const tk_query_
 // wants small leaves; a warp scans 32 points at a time and, with a longer
 // list, has more to gain from scanning on than from another descent.  Best
 // depths measured (k; points per leaf at 10,000 / 100,000 / 1M / 4M points):
-// one lane 10 / 24 / 30 / 16 (5,000 points: 10); a warp k=1 39 / 49 / 61 / 64, k=8 156 / 98 / 61 /
+// one lane 10 / 24 / 30 / 16 (5,000 points: 10; 100,000 points of 5 and 6 dims
+// 12); a warp k=1 39 / 49 / 61 / 64, k=8 156 / 98 / 61 /
 // 128, k=16 156 / 98 / 122 / 128, k=100 156 / 195 / 244 / 128; 4-8 dims 61 to
 // 122.  float64 without the float filter pays more for a point than for a
 // descent.
 int query_levels(const tk_tree* t, int lanes, int k) {
     if (!t->auto_depth) return t->search_levels;
     double leaf = one_lane_leaf(t->n);
-    if (t->dims > 3) leaf = lanes == 1 ? leaf : 90;
+    if (t->dims > 3) leaf = lanes == 1 ? (t->dims > 4 ? std::min(leaf, 12.0) : leaf) : 90;
     else if (lanes == 32) leaf = t->dtype == TK_F64 && !t->d_filter[0] ? 50 : (k <= 2 ? 50 : (k <= 48 ? 110 : 180));
     else if (lanes > 1) leaf = 40;
     return std::max(1, std::min(t->search_levels, log2_round(double(t->n) / leaf)));
@@ -420,7 +421,10 @@ int run_query_wide(const tk_tree* t, const T* q, int nq, int k, T* dists, int32_
     const int need = (nq + groups_per_block - 1) / groups_per_block;
     const int grid = std::max(1, std::min(need, per_sm * sm_count(t->device)));
 
-    int* counter = grid < need || binned(t, L, G, nq, k, o) ? reinterpret_cast<int*>(ws + ws_layout(t->search_levels, nq).counter) : nullptr;
+    // One lane a query, more than a block an SM: uneven loads, which the counter
+    // levels (300,000 points of 6 dims, k=1, 80,000 queries 1.44 -> 1.31 ms).
+    const bool level = G == 1 && need > sm_count(t->device);
+    int* counter = grid < need || level || binned(t, L, G, nq, k, o) ? reinterpret_cast<int*>(ws + ws_layout(t->search_levels, nq).counter) : nullptr;
     const int32_t* order = nullptr;
     const int rc0 = prepare_order(t, L, G, nq, k, o, ws, s, &counter, &order, true, [&](int B, int* counts, int* bin_of, int* pos_of) {
         bin_count_wide_launch<T>(q, nq, t->dims, static_cast<const T*>(t->d_medians), B, L,
