@@ -537,3 +537,20 @@ def test_wide_trees_on_one_lane(d, dtype):
             tree.query_opts = QueryOpts.make(threads_per_query=1)
             got = tree.query(q, k)
             assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1])
+
+
+@pytest.mark.parametrize("d,sizes", [(1, (1_000, 300_000)), (2, (1_000, 262_143, 262_144)), (3, (1_000, 65_535, 65_536)),
+                                     (6, (1_000, 9_999, 10_000))])
+def test_long_searches_binned_or_not(d, sizes):
+    """Long lists of many queries on both sides of the cloud sizes from which
+    their queries are ordered by cell; the answers do not depend on it."""
+    from torch_kdtree_gb300 import build_kd_tree
+    from torch_kdtree_gb300._lib import QueryOpts
+    g = torch.Generator(device=cuda).manual_seed(d)
+    q = torch.randn(50_000, d, generator=g, device=cuda)
+    for n in sizes:
+        tree = build_kd_tree(torch.randn(n, d, generator=g, device=cuda))
+        got = tree.query(q, 50)
+        tree.query_opts = QueryOpts.make(threads_per_query=32, bin_queries=0)
+        want = tree.query(q, 50)
+        assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1])

@@ -211,11 +211,17 @@ int blocks_per_sm(const void* kfn, int block, size_t smem) {
 // where a search is long (4-8 dims, or long lists), from ten queries per
 // resident warp on: 65,536 queries of 1M points, ms in input order / binned:
 // 6 dims k=16 1.93 / 1.78, 8 dims 8.0 / 7.0, 3 dims k=100 0.66 / 0.60; but 3
-// dims k=16 0.24 / 0.25, and 10,000 queries lose wherever they are.
+// dims k=16 0.24 / 0.25, and 10,000 queries lose wherever they are.  So does
+// every call on a small cloud, whose searches are alike (80,000 queries, k=50,
+// unbinned over binned: 3 dims 1,000 points 0.84, 30,000 0.96, 100,000 1.00,
+// 300,000 1.12; 2 dims 100,000 0.93, 300,000 1.03; 6 dims, k=16, 1,000 0.89,
+// 10,000 1.00, 100,000 1.02).
 bool binned(const tk_tree* t, int L, int G, int64_t nq, int k, const tk_query_opts& o) {
     if (o.bin_queries >= 0) return o.bin_queries == 1;
     const int64_t sms = sm_count(t->device);
-    const bool long_search = G == 32 && (t->dims > 3 ? k > 4 : k > 48) && nq >= sms * 320;
+    const bool long_search = G == 32 && nq >= sms * 320 &&
+                             (t->dims > 3 ? k > 4 && t->n >= 10000
+                                          : k > 48 && t->n >= (t->dims == 3 ? int64_t(1) << 16 : int64_t(1) << 18));
     return L >= 2 && (nq >= sms * 1024 || long_search);
 }
 
