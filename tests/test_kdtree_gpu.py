@@ -554,3 +554,27 @@ def test_long_searches_binned_or_not(d, sizes):
         tree.query_opts = QueryOpts.make(threads_per_query=32, bin_queries=0)
         want = tree.query(q, 50)
         assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1])
+
+
+@pytest.mark.parametrize("d", [1, 2, 3, 4, 6, 8])
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+@pytest.mark.parametrize("n", [1, 33, 5_000])
+def test_nearest_on_a_warp(d, dtype, n, oracle):
+    """k = 1 on a warp keeps no list: ties go to the lower index, infinite and
+    NaN queries as with any other shape, in leaves of any size."""
+    from torch_kdtree_gb300 import build_kd_tree
+    from torch_kdtree_gb300._lib import QueryOpts
+    rng = np.random.default_rng(d)
+    ref = np.round(rng.standard_normal((n, d)) * 4).astype(dtype)
+    q = np.round(rng.standard_normal((700, d)) * 4).astype(dtype)
+    q[3, 0], q[4, 0] = np.inf, -np.inf
+    bd, bi = oracle.brute(ref, q, 1)
+    q[5, d - 1] = np.nan
+    for levels in sorted({1, max(1, int(np.log2(n)) - 2)}):
+        tree = build_kd_tree(torch.from_numpy(ref).to(cuda), levels=levels)
+        tree.query_opts = QueryOpts.make(threads_per_query=32)
+        dd, ii = (x.cpu().numpy() for x in tree.query(torch.from_numpy(q).to(cuda), 1))
+        rows_ = np.arange(700) != 5
+        np.testing.assert_array_equal(dd[rows_], bd[rows_])
+        np.testing.assert_array_equal(ii[rows_], bi[rows_])
+        assert np.isinf(dd[5]) and ii[5] == -1

@@ -5,7 +5,8 @@
 
 namespace tk {
 
-#define TK_FILTER_LIST(X) X(1, 1) X(1, 2) X(1, 4) X(2, 1) X(2, 2) X(2, 4) X(3, 1) X(3, 2) X(3, 4)
+#define TK_FILTER_LIST(X) \
+    X(1, 0) X(1, 1) X(1, 2) X(1, 4) X(2, 0) X(2, 1) X(2, 2) X(2, 4) X(3, 0) X(3, 1) X(3, 2) X(3, 4)
 
 const void* kd_filtered_kernel(int D, int R) {
 #define TK_FPTR(d, r) \

@@ -114,4 +114,35 @@ struct WarpList {
     }
 };
 
+// k = 1 (kernels of R = 0): the nearest of a batch's candidates is the new
+// worst key at once.  Buffered until the end of a leaf they kept the reach wide
+// and cost a sort of 32 where one exchange does (1M queries in 1,000 points, 500
+// a leaf, 1.27 -> 0.94 ms; 262,144 in 4M, 512 a leaf 0.58 -> 0.49).
+template <typename T>
+struct WarpList<T, 0> {
+    struct Nearest {
+        Key<T> key;
+        __device__ __forceinline__ void store(int, int lane, T* out_d, int32_t* out_i, long long row) const {
+            if (lane == 0) {
+                out_d[row] = key.dist();
+                out_i[row] = int32_t(key.index());
+            }
+        }
+    } list;
+    Key<T> worst;
+
+    __device__ __forceinline__ void init(int, Key<T>*, int) { worst = list.key = Key<T>::sentinel(); }
+    __device__ __forceinline__ void offer(const Key<T>& mine, int lane) {
+        Key<T> x = mine.lt(worst) ? mine : worst;
+        if (!__any_sync(0xFFFFFFFFu, mine.lt(worst))) return;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            const Key<T> y = x.shfl(0xFFFFFFFFu, lane ^ o, 32);
+            x = y.lt(x) ? y : x;
+        }
+        worst = list.key = x;
+    }
+    __device__ __forceinline__ void flush(int) {}
+};
+
 }  // namespace tk

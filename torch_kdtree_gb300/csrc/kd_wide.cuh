@@ -320,7 +320,7 @@ __global__ void k_bin_count_wide(const T* __restrict__ q, int nq, int dims, cons
 }
 
 // Launchers (kd_wide_f32.cu, kd_wide_f64.cu): G in {1, 32}; R in {1, 2, 4, 8,
-// 16} for G = 1, {1, 2, 4} for G = 32.
+// 16} for G = 1, {0, 1, 2, 4} for G = 32.
 template <typename T>
 const void* kd_wide_kernel(int W, int G, int R);
 template <typename T>

@@ -320,6 +320,7 @@ int run_query(const tk_tree* t, const T* q, int nq, int k, T* dists, int32_t* id
             R = pow2_ceil((k + G - 1) / G);
         }
         if (!gr_available(t->dtype, D, G, R)) return fail(TK_EUNSUPPORTED, "no kernel shape for this k");
+        if (G == 32 && k == 1) R = 0;  // WarpList<T, 0>
     }
 
     const int L = packet ? t->search_levels : query_levels(t, G, k);
@@ -410,7 +411,7 @@ int run_query_wide(const tk_tree* t, const T* q, int nq, int k, T* dists, int32_
     if (G != 1 && G != 2 && G != 4 && G != 8 && G != 16 && G != 32)
         return fail(TK_EINVAL, "threads_per_query must be 1, 2, 4, 8, 16 or 32");
     if (G != 1 || k > 16) G = 32;  // kernels of wide trees: 1 (k <= 16) or 32 lanes per query
-    const int R = pow2_ceil((k + G - 1) / G);
+    const int R = G == 32 && k == 1 ? 0 : pow2_ceil((k + G - 1) / G);  // 0: WarpList<T, 0>
     const int W = record_width(t->dims);
     const int L = query_levels(t, G, k);
     int S = o.smem_levels >= 0 ? o.smem_levels : 10;
