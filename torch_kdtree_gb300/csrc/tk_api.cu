@@ -343,7 +343,13 @@ int run_query(const tk_tree* t, const T* q, int nq, int k, T* dists, int32_t* id
     if (o.blocks_per_sm > 0) per_sm = std::min(per_sm, int(o.blocks_per_sm));
     const int groups_per_block = block / G;
     const int need = (nq + groups_per_block - 1) / groups_per_block;
-    const int grid = std::max(1, std::min(need, per_sm * sm_count(t->device)));
+    const int sms = sm_count(t->device);
+    int grid = std::max(1, std::min(need, per_sm * sms));
+    // A few blocks left over after as many on every SM would have the last word
+    // with long lists on one lane; the counter (grid < need) deals out what they
+    // would do (2 dims, 10,000 points, k=16, 80,000 queries, 313 blocks -> 304:
+    // 0.119 -> 0.108 ms).
+    if (grid == need && G == 1 && k > 8 && grid > sms && grid % sms <= sms / 8) grid -= grid % sms;
 
     // a grid that holds all queries at once needs no counter
     int* counter = grid < need || binned(t, L, G, nq, k, o) ? reinterpret_cast<int*>(ws + ws_layout(t->search_levels, nq).counter) : nullptr;
