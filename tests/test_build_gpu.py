@@ -267,3 +267,21 @@ def test_device_build_around_scan_limits(dtype, n):
     pts = rng.standard_normal((n, 2)).astype(dtype)
     pts[: n // 4] = np.round(pts[: n // 4], 1)
     assert_same_layout(pts, 7)
+
+
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+@pytest.mark.parametrize("d", [1, 2, 3, 5])
+@pytest.mark.parametrize("n", [1_000, 4_097, 300_000])
+def test_layout_of_a_deeper_image(dtype, d, n):
+    """The layout that a default-depth tree reports, put in order from its
+    deeper image: the host builder's, with ties, zeros of both signs and
+    infinite coordinates."""
+    from torch_kdtree_gb300 import build_kd_tree
+    rng = np.random.default_rng(d)
+    pts = np.round(rng.standard_normal((n, d)) * 50).astype(dtype)
+    pts[rng.integers(0, n, n // 10)] *= -0.0
+    pts[rng.integers(0, n, 5), 0] = np.inf
+    td = build_kd_tree(torch.from_numpy(pts).cuda())
+    th = build_kd_tree(torch.from_numpy(pts), device=torch.device("cuda"))
+    assert torch.equal(td.shuffled_ind, th.shuffled_ind)
+    assert torch.equal(td.structured_points, th.structured_points)
