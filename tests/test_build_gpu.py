@@ -285,3 +285,29 @@ def test_layout_of_a_deeper_image(dtype, d, n):
     th = build_kd_tree(torch.from_numpy(pts), device=torch.device("cuda"))
     assert torch.equal(td.shuffled_ind, th.shuffled_ind)
     assert torch.equal(td.structured_points, th.structured_points)
+
+
+def test_tree_in_a_graph_is_kept_from_its_stream():
+    """A query captured on the stream that built the tree may be replayed on
+    any other: the tree's memory waits for all of them when it goes."""
+    from torch_kdtree_gb300 import build_kd_tree
+    from torch_kdtree_gb300.batched import BatchedKDTrees
+    s = torch.cuda.Stream()
+    ref, q = torch.randn(5_000, 3, device="cuda"), torch.randn(200, 3, device="cuda")
+    torch.cuda.synchronize()
+    with torch.cuda.stream(s):
+        tree = build_kd_tree(ref)
+        batch = BatchedKDTrees([ref], [4], [len(q)])
+        want = tree.query(q, 4)
+        batch.query_flat(q)
+        s.synchronize()
+        assert not tree._tree.other_streams and not batch.trees[0]._tree.other_streams
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g, stream=s):
+        got = tree.query(q, 4)
+        batch.query_flat(q)
+    assert tree._tree.other_streams and batch.trees[0]._tree.other_streams
+    g.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1])
+    assert torch.equal(batch.out_dists.view(-1, 4), want[0])
