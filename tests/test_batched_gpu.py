@@ -161,3 +161,20 @@ def test_batch_launch_per_list_length(dtype, dims, ks):
         for db, ib in ((d_b[c], i_b[c]), (d_g[c], i_g[c])):
             np.testing.assert_array_equal(db.cpu().numpy(), d.cpu().numpy(), err_msg=str(c))
             np.testing.assert_array_equal(ib.cpu().numpy(), i.cpu().numpy(), err_msg=str(c))
+
+
+@pytest.mark.parametrize("d", [1, 2, 3, 5])
+def test_host_built_clouds_in_a_batch(d):
+    """Clouds whose trees were built on the host, alone and next to others:
+    the same answers as every tree on its own."""
+    from torch_kdtree_gb300.batched import BatchedKDTrees
+    g = torch.Generator(device="cuda").manual_seed(d)
+    refs = [torch.randn(n, d, generator=g, device="cuda") for n in (40, 3_000, 20_000)]
+    qs = [torch.randn(n, d, generator=g, device="cuda") * 1.5 for n in (10, 700, 5_000)]
+    for clouds in ([r.cpu() for r in refs], [refs[0].cpu(), refs[1], refs[2].cpu()]):
+        batch = BatchedKDTrees(clouds, [3, 16, 1], [len(q) for q in qs], device=torch.device("cuda"))
+        assert batch.trees[0].built_on == "host"
+        dists, inds = batch.query(qs)
+        for tree, q, k, dd, ii in zip(batch.trees, qs, [3, 16, 1], dists, inds):
+            want = tree.query(q, k)
+            assert torch.equal(dd, want[0]) and torch.equal(ii, want[1])

@@ -34,10 +34,10 @@ struct CloudDesc {
     const PointRec<T>* pts;
     const T* medians;
     const int32_t* leaf_off;
-    const PointRec<T>* boxes;  // null: prune with split planes only
+    const PointRec<T>* boxes;
     long long out_off;  // element offset of the cloud's [nq_c, k_c] block in the outputs
     int levels;
-    int leaf_shift;  // image leaves below the searched depth (unused: boxes carry their ranges)
+    int n;          // points
     int k;
     int bins;       // 2^B_c cells used for binning
     int bin_base;   // first cell of this cloud among those of the first cost class
@@ -73,7 +73,7 @@ __device__ __forceinline__ int cloud_of(const long long* prefix, int n_clouds, l
 constexpr int kCostClasses = 8;
 
 template <typename T, int D>
-__device__ __forceinline__ int batch_cost_class(const PointRec<T>* boxes, int node, const T (&p)[D]) {
+__device__ __forceinline__ int batch_cost_class(const PointRec<T>* boxes, int points, int node, const T (&p)[D]) {
     float far2 = 0.f, diag2 = 0.f;
     const PointRec<T> rlo = load_rec(boxes), rhi = load_rec(boxes + 1);
     const PointRec<T> lo = load_rec(boxes + 2 * node), hi = load_rec(boxes + 2 * node + 1);
@@ -85,8 +85,7 @@ __device__ __forceinline__ int batch_cost_class(const PointRec<T>* boxes, int no
         far2 += f * f;
         diag2 += g * g;
     }
-    const float n = float(int(rec_index(rhi)) - int(rec_index(rlo)));
-    const float octaves = __log2f(far2) - __log2f(diag2) + 2.f / D * __log2f(n);
+    const float octaves = __log2f(far2) - __log2f(diag2) + 2.f / D * __log2f(float(points));
     return kCostClasses - 1 - int(fminf(fmaxf(0.5f * octaves + 2.f, 0.f), kCostClasses - 1.f));
 }
 
@@ -107,7 +106,7 @@ __global__ void k_batch_bin_count(const BatchArgs<T> a, int* counts, int* bin_of
         node = 2 * node + (pick<T, D>(p, ax) < m ? 1 : 2);
         ax = (ax + 1 == D) ? 0 : ax + 1;
     }
-    const int cost = batch_cost_class<T, D>(cd.boxes, node, p);
+    const int cost = batch_cost_class<T, D>(cd.boxes, cd.n, node, p);
     const int bin = cd.bin_base + cost * cd.bin_stride + node - ((1 << B) - 1);
     bin_of[i] = bin;
     pos_of[i] = atomicAdd(counts + bin, 1);
@@ -223,12 +222,14 @@ int batch_bin_levels(int L, long long nq) {
     return std::max(1, std::min({L, kMaxBinLevels, lg - 4}));
 }
 
+// of trees whose search stops at d.levels
 template <typename T>
 void fill_desc(CloudDesc<T>& d, const tk_tree* t) {
     d.pts = static_cast<const PointRec<T>*>(t->d_pts);
     d.medians = static_cast<const T*>(t->d_medians);
     d.leaf_off = t->d_leaf_off;
     d.boxes = static_cast<const PointRec<T>*>(t->d_boxes);
+    d.n = int(t->n);
 }
 
 template <typename T>
@@ -238,6 +239,7 @@ void fill_desc(WideCloudDesc<T>& d, const tk_tree* t) {
     d.medians = static_cast<const T*>(t->d_medians);
     d.leaf_off = t->d_leaf_off;
     d.boxes = static_cast<const T*>(t->d_boxes);
+    d.leaf_shift = t->search_levels - d.levels;
 }
 
 template <typename T>
@@ -258,11 +260,10 @@ int upload_descs(tk_batch* b, const tk_tree* const* trees, const int64_t* q_coun
     for (int c = 0; c < b->n_clouds; ++c) {
         const tk_tree* t = trees[c];
         Desc& d = h[c];
-        fill_desc<T>(d, t);
         d.out_off = b->out_off[c];
         // the batch runs one lane per query up to k = 16, else 8 lanes (32 with 4-8 dims)
         d.levels = query_levels(t, b->max_k <= 16 ? 1 : (t->dims > 3 ? 32 : 8), ks[c]);
-        d.leaf_shift = t->search_levels - d.levels;
+        fill_desc<T>(d, t);
         d.k = ks[c];
         const int B = batch_bin_levels(d.levels, std::max<int64_t>(q_counts[c], 1));
         d.bins = 1 << B;
