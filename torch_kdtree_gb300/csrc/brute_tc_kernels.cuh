@@ -269,7 +269,10 @@ constexpr int kT5Parts = kT5EpiWarps / 4;           // column groups of 64: list
 constexpr int kT5Minima = 128;                      // sample minima per row
 constexpr int kT5MinStride = kT5Minima + 2;         // their row stride (16-bit words): lanes of a read on other banks
 constexpr int kT5Threads = 32 * (kT5EpiWarps + 1);
-constexpr float kT5PadNorm = 1e30f;
+// |r|^2 of a padding row, and the highest threshold: a power of two, exact in
+// TF32 and in BF16, so that a padding row scores just that, never below it
+// (rounded down it would let r >= n into the lists).
+constexpr float kT5PadNorm = 0x1p99f;
 constexpr uint32_t kT5MaxTries = 1u << 22;  // bounded mbarrier polls (default; Tc5Args::max_tries)
 
 __device__ __forceinline__ uint32_t core_offset(int row, int kb, int KB) {

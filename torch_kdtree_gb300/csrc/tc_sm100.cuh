@@ -90,11 +90,6 @@ __device__ __forceinline__ void tc_fence_after() {
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 }
 
-// Generic-proxy writes to shared memory -> visible to the async proxy.
-__device__ __forceinline__ void fence_proxy_async_smem() {
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-}
-
 // Shared-memory matrix descriptor, no swizzle: start address, leading-dimension
 // byte offset (between core matrices adjacent along K), stride-dimension byte
 // offset (between 8-row groups), fixed 0b001 at bits 46-48.
