@@ -527,17 +527,32 @@ constexpr uint32_t kT5CodeInf = 0xFF00u;
 __device__ __forceinline__ uint16_t dist_code(float x) { return uint16_t(__float_as_uint(fmaxf(x, 0.f)) >> 15); }
 __device__ __forceinline__ float code_end(uint32_t code) { return __uint_as_float((code << 15) | 0x7FFFu); }
 
-// Threshold of a row at distance `far` (see k_tc5_select), t where more
-// references lie below that than the lists hold; by 4 lanes per row, each with
-// a quarter of its minima, which stand for `groups` groups.
-static __device__ __noinline__ float blurred_threshold(const uint16_t* mins, float t, float far, int groups, int pstride) {
-    const uint32_t end = min(uint32_t(dist_code(far)), kT5CodeInf - 1u);
-    int c = 0;
-    for (int i = 0; i < kT5Minima / 4; ++i) c += mins[i] <= end ? 1 : 0;
-    c += __shfl_xor_sync(0xFFFFFFFFu, c, 1);
-    c += __shfl_xor_sync(0xFFFFFFFFu, c, 2);
-    const float most = float(groups) * (1.f - __expf(-float(kT5Parts * 96) / float(groups * pstride)));
-    return float(c) <= most ? code_end(end) : t;
+// Threshold (a score) of a row whose minima's rank-th smallest has code `lo`,
+// -inf where no certificate can come of it; see k_tc5_select.  By 4 lanes per
+// row, each with a quarter of its minima, which stand for `groups` groups.
+static __device__ __noinline__ float row_threshold(const uint16_t* mins, uint32_t lo, float qq, bool real, float eps_dot,
+                                                   int d, int groups, int pstride) {
+    float t = lo < kT5CodeInf ? code_end(lo) : kT5PadNorm;  // rounded up to the end of its 16-bit bucket
+    // Where the scores' error is not small against t (clusters far apart), the
+    // certificate may want lists that go on by that error; groups without a
+    // reference that near tell whether they can hold what is there.  Where it
+    // exceeds t there is none, see below.
+    const float E = score_bound(eps_dot, d, qq, t - qq, t).E;
+    const bool blurred = E > 0.0625f * t;
+    if (__any_sync(0xFFFFFFFFu, blurred)) {
+        const uint32_t end = min(uint32_t(dist_code(t + 1.01f * E)), kT5CodeInf - 1u);
+        int c = 0;
+        for (int i = 0; i < kT5Minima / 4; ++i) c += mins[i] <= end ? 1 : 0;
+        c += __shfl_xor_sync(0xFFFFFFFFu, c, 1);
+        c += __shfl_xor_sync(0xFFFFFFFFu, c, 2);
+        const float most = float(groups) * (1.f - __expf(-float(kT5Parts * 96) / float(groups * pstride)));
+        if (blurred && float(c) <= most) t = code_end(end);
+    }
+    // Low enough to keep the padding rows out.  (NaN scores have code 0 and are
+    // no hits; such a row's |q|^2 is no certificate's.  Rows past the last query
+    // take no hits: all their scores are equal.)
+    const float low = fminf(t - qq, kT5PadNorm);
+    return real && certifies(eps_dot, d, qq, low, 0.f) ? low : -__int_as_float(0x7f800000);
 }
 
 __device__ __forceinline__ float min3(float a, float b, float c) {
@@ -566,7 +581,7 @@ __device__ __forceinline__ float min3(float a, float b, float c) {
 // the distances (clusters far apart: scores differ by less than their error)
 // take no hits, and a block of such rows only waits for its products.
 //
-// 262,144 x 65,536, d=32, k=32, TF32: 2.9 ms; in whole waves of blocks 3.5 ms,
+// 262,144 x 65,536, d=32, k=32, TF32: 3.1 ms; in whole waves of blocks 3.5 ms,
 // of which it was measured: tensor pipe 45% busy, issue
 // slots 51%: 4 epilogue warps per scheduler cannot cover the latency of their
 // own minima, votes and branches.  (Before: a short sample, then per-row
@@ -786,28 +801,12 @@ __global__ void __launch_bounds__(kT5Threads, 1) k_tc5_select(const Tc5Args a) {
                 if (c >= sl.rank) hi = mid;
                 else lo = min(mid + 1u, 0xFFFFu);
             }
-            // t: rounded up to the end of its 16-bit bucket
-            float t = lo < kT5CodeInf ? code_end(lo) : kT5PadNorm;
-            // Where the scores' error is not small against t (clusters far
-            // apart), the certificate may want lists that go on by that error;
-            // groups without a reference that near tell whether they can hold
-            // what is there.  Where it exceeds t there is none, see below.
             const int grow_q = rblock * kT5Rows + grow;
-            const float gqq = grow_q < a.nq ? __ldg(a.qnorm + grow_q) : 0.f;
-            const float E = score_bound(a.eps_dot, a.d, gqq, t - gqq, t).E;
-            const bool blurred = E > 0.0625f * t;
-            if (__any_sync(0xFFFFFFFFu, blurred)) {
-                const int groups = npre <= 8 ? 16 * npre : 4 * ((npre + tpg - 1) / tpg);
-                const float far = blurred_threshold(mins, t, t + 1.01f * E, groups, sl.pstride);
-                if (blurred) t = far;
-            }
-            // Low enough to keep the padding rows out.  (NaN scores have code 0
-            // and are no hits; such a row's |q|^2 is no certificate's.  Rows past
-            // the last query take no hits: all their scores are equal.)
-            const float low = fminf(t - gqq, kT5PadNorm);
-            const bool search = grow_q < a.nq && certifies(a.eps_dot, a.d, gqq, low, 0.f);
-            if (gl == 0) sThr[grow] = search ? low : -__int_as_float(0x7f800000);
-            if (__any_sync(0xFFFFFFFFu, search) && lane == 0) some_row = 1;
+            const bool real = grow_q < a.nq;
+            const float low = row_threshold(mins, lo, real ? __ldg(a.qnorm + grow_q) : 0.f, real, a.eps_dot, a.d,
+                                            npre <= 8 ? 16 * npre : 4 * ((npre + tpg - 1) / tpg), sl.pstride);
+            if (gl == 0) sThr[grow] = low;
+            if (__any_sync(0xFFFFFFFFu, low > -__int_as_float(0x7f800000)) && lane == 0) some_row = 1;
         }
         bar_all();
         const int row = rblock * kT5Rows + myrow;
