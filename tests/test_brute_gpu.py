@@ -634,3 +634,16 @@ def test_tensor_core_modes_in_several_passes(mode, oracle):
     bd, bi = oracle.brute(ref, q[rows], 2)
     np.testing.assert_array_equal(dd.cpu().numpy()[rows], bd)
     np.testing.assert_array_equal(ii.cpu().numpy()[rows], bi)
+
+
+@pytest.mark.parametrize("d", [4, 8, 16, 32])
+@pytest.mark.parametrize("n", [1, 3, 4, 5, 8, 255, 256, 257, 511, 1023])
+def test_nearest_at_the_edges_of_a_tile(d, n, oracle):
+    """k = 1 takes eight references at a time: tiles that end anywhere in them."""
+    rng = np.random.default_rng(n)
+    ref = np.round(rng.standard_normal((n, d)) * 2).astype(np.float32)
+    q = np.round(rng.standard_normal((300, d)) * 2).astype(np.float32)
+    dd, ii = tk().nn_distance(torch.from_numpy(ref).to(cuda), torch.from_numpy(q).to(cuda), 1)
+    bd, bi = oracle.brute(ref, q, 1)
+    np.testing.assert_array_equal(dd.cpu().numpy(), bd)
+    np.testing.assert_array_equal(ii.cpu().numpy(), bi)

@@ -119,8 +119,12 @@ __device__ __forceinline__ void brute_block(const BruteArgs<T>& a, T* tile, cons
             // accumulation order as sqdist (dimension by dimension).
             constexpr int U = 4;
             static_assert(TR % U == 0, "tile rows must be a multiple of the step");
+            // two steps at once where the list is one key (k = 1, 20,000 x 2,000,
+            // d = 8 0.155 -> 0.125 ms; with more keys 2% slower to 20%)
+            constexpr int kSteps = R == 1 ? 2 : 1;
             if (active) {
                 const float4* rows = reinterpret_cast<const float4*>(tile);
+#pragma unroll kSteps
                 for (int j0 = 0; j0 < len; j0 += U) {
                     T acc[U];
 #pragma unroll
