@@ -294,13 +294,19 @@ int prepare_order(const tk_tree* t, int L, int G, int nq, int k, const tk_query_
 // 12); a warp k=1 39 / 49 / 61 / 64, k=8 156 / 98 / 61 /
 // 128, k=16 156 / 98 / 122 / 128, k=100 156 / 195 / 244 / 128; 4-8 dims 61 to
 // 122.  float64 without the float filter pays more for a point than for a
-// descent.
+// descent.  Of the shapes between, which only callers ask for, two lanes want
+// one lane's leaves, four a little more, eight and sixteen 20 to 40 points
+// (10,000 points, d = 3, 1M queries, k=1 / 8, 10 and 20 points over 40: 2 lanes
+// 0.61, 0.72 / 0.65, 0.76; 4 0.77, 0.81 / 0.85, 0.84; 8 0.92, 0.91 / 1.07, 0.96;
+// 16 0.92, 0.94 / 1.09, 0.99).
 int query_levels(const tk_tree* t, int lanes, int k) {
     if (!t->auto_depth) return t->search_levels;
     double leaf = one_lane_leaf(t->n);
     if (t->dims > 3) leaf = lanes == 1 ? (t->dims > 4 ? std::min(leaf, 12.0) : leaf) : 90;
     else if (lanes == 32) leaf = t->dtype == TK_F64 && !t->d_filter[0] ? 50 : (k <= 2 ? 50 : (k <= 48 ? 110 : 180));
-    else if (lanes > 1) leaf = 40;
+    else if (lanes >= 8) leaf = k == 1 || (lanes == 8 && k <= 16) ? 25 : 40;
+    else if (lanes == 4 && t->dims == 3 && k > 1) leaf *= 1.5;
+    else if (lanes > 1) leaf = std::min(leaf, 12.0);
     return std::max(1, std::min(t->search_levels, log2_round(double(t->n) / leaf)));
 }
 
