@@ -260,10 +260,12 @@ typedef enum tk_brute_mode {
     TK_BRUTE_TF32 = 1,       /* q.r on tensor cores in TF32, over-fetch, exact FP32 re-rank */
     TK_BRUTE_BF16_SPLIT = 2, /* q.r as BF16 hi/lo split products with FP32 accumulation, then exact re-rank */
     TK_BRUTE_ROUTED = 3      /* whichever search is fastest for the sizes, any dtype, dims and k of TK_BRUTE_EXACT:
-                                CUDA cores, BF16 hi/lo, or (1-3 dims) a KD-tree that lives for the call */
+                                CUDA cores, BF16 hi/lo (float32), or (1-3 dims) a KD-tree that lives for the call */
 } tk_brute_mode;
 
-/* Bytes of device scratch tk_nn_distance needs. */
+/* Bytes of device scratch tk_nn_distance needs.  The tensor-core searches
+ * keep 4.6 KB of lists per query, in passes of at most 2^20 queries (262,144
+ * with TK_BRUTE_ROUTED): some 5 (1.3) GB however many queries there are. */
 size_t tk_nn_distance_workspace_size(int64_t n, int64_t nq, int dims, int k, int dtype, int mode);
 
 /* Exhaustive exact k nearest neighbours (the nn_distance op).

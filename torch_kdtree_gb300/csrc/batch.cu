@@ -67,7 +67,7 @@ __device__ __forceinline__ int cloud_of(const long long* prefix, int n_clouds, l
 // in a uniform cloud, in steps of two octaves.  Few and relative, so that the
 // classes are part of the counting sort's cell and need no sort of their own:
 // the costliest searches do not end up in a launch's last chunks, and a warp's
-// queries cost much the same.  256 ragged clouds, 4.8M queries: 4.27 ms without
+// queries cost much the same.  256 ragged clouds, 5.8M queries: 4.27 ms without
 // classes, 4.20 with 8, 4.24 with 16, 4.31 with 32; 64 clouds 1.00, 0.95, 0.95,
 // 0.97.
 constexpr int kCostClasses = 8;
@@ -119,7 +119,7 @@ constexpr int kBatchBlock = 128;  // threads per block of k_batch_query
 // busy, 8 of 32 lanes active where searches differ).  One kernel for all list
 // lengths gave every search the registers and the instruction footprint of the
 // longest and mixed them in one warp; a launch after another, each with its own
-// tail, is slower still (256 ragged clouds, 4.8M queries 4.57 ms against 4.41;
+// tail, is slower still (256 ragged clouds, 5.8M queries 4.57 ms against 4.41;
 // 16 clouds 0.50 against 0.30), so a launch may start while the one before it
 // runs out (4.27; 0.27; with cost classes 4.20).  It reads only what was ready
 // before the first launch, and ends after the one before it, so whatever

@@ -117,7 +117,7 @@ struct WarpList {
 // k = 1 (kernels of R = 0): the nearest of a batch's candidates is the new
 // worst key at once.  Buffered until the end of a leaf they kept the reach wide
 // and cost a sort of 32 where one exchange does (1M queries in 1,000 points, 500
-// a leaf, 1.27 -> 0.94 ms; 262,144 in 4M, 512 a leaf 0.58 -> 0.49).
+// a leaf, 1.27 -> 0.82 ms; 262,144 in 4M, 512 a leaf 0.58 -> 0.41).
 template <typename T>
 struct WarpList<T, 0> {
     struct Nearest {

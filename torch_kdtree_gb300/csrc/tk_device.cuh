@@ -341,8 +341,8 @@ __device__ __forceinline__ int next_queries(int* work, int count, int nq, int& r
 
 // The same for a loop that ends by itself where there is no counter: no count
 // of the rounds is held across the search.  Which form a kernel takes is
-// measured: a warp per query of k_kd_query spilled with the count (262,144
-// queries in 4M points, k = 100: 8.07 ms against 7.57); the other shapes run 3
+// measured: a warp per query of k_kd_query spilled with the count (1M queries
+// in 1M points, k = 100: 8.07 ms against 7.57); the other shapes run 3
 // to 14% faster with it (one lane, k = 16, 262,144 queries in 200,000 points,
 // 2 dims 0.31 ms against 0.36; 65,536 in 1M points, 8 dims 6.9 against 7.9).
 __device__ __forceinline__ int next_queries(int* work, int count) {

@@ -476,11 +476,17 @@ def nn_distance(points_ref: torch.Tensor, points_query: torch.Tensor, nr_nns_sea
     """Exhaustive exact KNN: ``(dists, inds)`` of every query among all
     reference points, squared distances ``[Q, k]`` and int32 indices.
 
-    ``mode``: "exact" (float32 or float64; the fastest search for the sizes:
-    CUDA cores, tensor cores with an exact re-rank, or in 1-3 dimensions a
-    KD-tree that lives for the call), "tf32" or "bf16_split" (tensor-core
-    candidate search with an exact float32 re-rank; same answer), or "auto" (the fastest of these for the shapes, timed once
-    by :func:`torch_kdtree_gb300.autotune.autotune_brute` and cached).
+    ``mode``: "exact" ("fp32" and "fp64" are other names of it; float32 or
+    float64; the fastest search for the sizes: CUDA cores, in 1-3 dimensions a
+    KD-tree that lives for the call, or for float32 tensor cores), "tf32" or
+    "bf16_split" (tensor cores), or "auto" (the fastest of these for the shapes,
+    timed once by :func:`torch_kdtree_gb300.autotune.autotune_brute` and cached).
+    The tensor cores only choose candidates, in products of BF16 pairs or TF32
+    with a bound on their error; distances and order come from the points' own
+    precision, and queries without a certificate are searched exhaustively in
+    it, so every mode gives the same answer.  Tensor-core searches take 4.6 KB
+    of scratch per query, up to 1.3 GB in mode "exact" (queries go in passes
+    of 262,144) and 5 GB in the modes that name them (passes of 2^20).
     Differentiable in both point sets.  The reference shipped this search as
     an unbound CUDA launcher (src/nndistance_g.cu:191-220) for d = 3 only;
     here any 1 <= d <= 128, float32 or float64."""
