@@ -9,7 +9,6 @@
 #include <mutex>
 #include <new>
 #include <string>
-#include <system_error>
 #include <thread>
 #include <tuple>
 #include <vector>
@@ -669,7 +668,7 @@ void in_threads(size_t count, size_t piece, F work) {
     pool.reserve(want);
     try {
         while (pool.size() + 1 < want) pool.emplace_back(run);
-    } catch (const std::system_error&) {
+    } catch (...) {  // no more threads than there are
     }
     run();
     for (std::thread& t : pool) t.join();
