@@ -72,7 +72,7 @@ class BatchedKDTrees:
         if not q_flat.is_contiguous() or q_flat.device != self.device:
             raise AssertionError("queries must be contiguous on the batch's device")
         stream = _stream_ptr(self.device)
-        if stream != self._stream or torch._C._cuda_isCurrentStreamCapturing():
+        if stream != self._stream or (stream and torch._C._cuda_isCurrentStreamCapturing()):
             for t in self.trees:
                 t._tree.used_on(stream)
             self._stream = stream

@@ -101,8 +101,9 @@ class _Tree:
         return self._scratch_free
 
     def used_on(self, stream: int) -> None:
-        # a captured query runs wherever its graph is replayed
-        if stream != self.stream or torch._C._cuda_isCurrentStreamCapturing():
+        # a captured query runs wherever its graph is replayed (the default
+        # stream, 0, cannot be captured: not asked, 0.2 us a call)
+        if stream != self.stream or (stream and torch._C._cuda_isCurrentStreamCapturing()):
             self.other_streams = True
 
     def info(self) -> TreeInfo:
@@ -126,7 +127,7 @@ def knn_query_raw(tree: _Tree, q: torch.Tensor, k: int, dists: torch.Tensor, idx
     """Enqueue one tk_tree_query on the current stream (inputs already on the device)."""
     nq = q.shape[0]
     stream = _stream_ptr(q.device)
-    if not tree.other_streams:
+    if (stream or stream != tree.stream) and not tree.other_streams:
         tree.used_on(stream)
     if nq <= tree.scratch_free and (opts is None or (opts.bin_queries <= 0 and opts.blocks_per_sm <= 0)):
         ws_ptr, ws_bytes = None, 0
